@@ -46,7 +46,7 @@ def _stale(target, deps):
 
 def build(verbose=False, force=False, extra_flags=()):
     os.makedirs(OUT, exist_ok=True)
-    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
     jobs = []
     objs = []
     for src in sources():

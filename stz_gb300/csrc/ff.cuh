@@ -6,37 +6,9 @@
 // error (a*b - p exactly = fmaf(a, b, -p)).
 #pragma once
 
+#include "ffnum.cuh"
+
 namespace stzg {
-
-struct ff {
-    float hi, lo;
-};
-
-__device__ __forceinline__ ff ff_fast2sum(float a, float b) {
-    const float s = a + b;
-    return ff{s, b - (s - a)};
-}
-__device__ __forceinline__ ff ff_add(ff a, ff b) {
-    const float s = a.hi + b.hi, bb = s - a.hi;
-    float e = (a.hi - (s - bb)) + (b.hi - bb);
-    e += a.lo + b.lo;
-    return ff_fast2sum(s, e);
-}
-__device__ __forceinline__ ff ff_neg(ff a) { return ff{-a.hi, -a.lo}; }
-__device__ __forceinline__ ff ff_sub(ff a, ff b) { return ff_add(a, ff_neg(b)); }
-__device__ __forceinline__ ff ff_mul(ff a, ff b) {
-    const float p = a.hi * b.hi;
-    float e = fmaf(a.hi, b.hi, -p);
-    e = fmaf(a.hi, b.lo, e);
-    e = fmaf(a.lo, b.hi, e);
-    return ff_fast2sum(p, e);
-}
-__device__ __forceinline__ ff ff_add_f(ff a, float b) {
-    const float s = a.hi + b, bb = s - a.hi;
-    float e = (a.hi - (s - bb)) + (b - bb);
-    e += a.lo;
-    return ff_fast2sum(s, e);
-}
 
 // double -> hi + lo on the integer pipe: hi keeps the sign, the exponent and
 // the leading 24 significant bits, lo the remaining 29 bits rounded to a

@@ -1,6 +1,7 @@
 // Multigrid kernels and hierarchy set-up (see mg.cuh for the design).
 #include "mg.cuh"
 #include "mg_device.cuh"
+#include "mg_window.cuh"
 #include "ff.cuh"
 #include "transfer1d.cuh"
 
@@ -300,7 +301,30 @@ template <typename T> int hierarchy<T>::allocate(int m, int n, V *top_z, V *top_
         L.b = p[1];
         L.r = p[2];
     }
+    if (sizeof(T) == 8) {
+        const size_t bytes = sizeof(float4) * (size_t)m * n;
+        void *p = nullptr;
+        cudaError_t e = cudaMalloc(&p, bytes);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(top correction)");
+        owned_.push_back(p);
+        bytes_ += bytes;
+        top_pairs = (float4 *)p;
+    }
     return STZG_OK;
+}
+
+// A stencil as float pairs: per block the high parts, then the low ones.
+static void split_stencil(const stencil9<double> &s, float4 *out) {
+    for (int e = 0; e < 10; e++) {
+        const double v[4] = {s.e[e].a, s.e[e].b, s.e[e].c, s.e[e].d};
+        float h[4], l[4];
+        for (int q = 0; q < 4; q++) {
+            h[q] = (float)v[q];
+            l[q] = (float)(v[q] - (double)h[q]);
+        }
+        out[2 * e] = make_float4(h[0], h[1], h[2], h[3]);
+        out[2 * e + 1] = make_float4(l[0], l[1], l[2], l[3]);
+    }
 }
 
 template <typename T> cudaError_t prepare_tail_kernel();
@@ -325,6 +349,21 @@ template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> 
         D.ncls = (int)L.cls.size();
         STZG_CUDA(cudaMemcpy((void *)D.st, tab.data(), sizeof(stencil9<T>) * tab.size(), cudaMemcpyHostToDevice));
         STZG_CUDA(cudaMemcpy((void *)D.cls, L.cls.data(), sizeof(int) * L.cls.size(), cudaMemcpyHostToDevice));
+        {
+            std::vector<float4> pairs(20 * L.table.size());
+            for (size_t k = 0; k < L.table.size(); k++) split_stencil(L.table[k], pairs.data() + 20 * k);
+            if (L.table.size() > pair_cap_[l]) {
+                void *p;
+                cudaError_t e = cudaMalloc(&p, sizeof(float4) * pairs.size());
+                if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(stencil pairs)");
+                owned_.push_back(p);
+                bytes_ += sizeof(float4) * pairs.size();
+                st_pairs[l] = (const float4 *)p;
+                pair_cap_[l] = L.table.size();
+            }
+            STZG_CUDA(cudaMemcpy((void *)st_pairs[l], pairs.data(), sizeof(float4) * pairs.size(),
+                                 cudaMemcpyHostToDevice));
+        }
     }
     STZG_CUDA(prepare_tail_kernel<T>());
     bottom_inv = nullptr;
@@ -345,6 +384,7 @@ template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> 
             bottom_inv = inv_dev_;
             bottom_unknowns = 2 * ops.back().m * ops.back().n;
         }
+        STZG_CHECK(build_dense(*this, inv, owned_, dense_cap_));
     }
     return STZG_OK;
 }
@@ -373,7 +413,13 @@ template <typename T> int hierarchy<T>::grow(int l, size_t st_need, size_t cls_n
 }
 
 template <typename T> void hierarchy<T>::release() {
-    for (int l = 0; l < 17; l++) st_cap_[l] = cls_cap_[l] = 0;
+    for (int l = 0; l < 17; l++) {
+        st_cap_[l] = cls_cap_[l] = pair_cap_[l] = dense_cap_[l] = 0;
+        st_pairs[l] = nullptr;
+        dense_buf[l] = nullptr;
+    }
+    top_pairs = nullptr;
+    dense = nullptr;
     inv_cap_ = 0;
     inv_dev_ = nullptr;
     bottom_inv = nullptr;
@@ -1842,6 +1888,8 @@ struct tail_levels {
     const double *inv;
     int inv_n;
     int inv_off;  // byte offset of a shared-memory copy of inv (pair tail), -1: none
+    const float4 *dense = nullptr;  // pair tail: the levels from d on as one matrix (hierarchy::dense)
+    int d = 0;
 };
 
 template <typename T>
@@ -2104,7 +2152,8 @@ __device__ void tail_pairs_body(const tail_levels &tl, const hierarchy_view<floa
             offs[l][4] = l < tl.ml ? (unsigned)((const unsigned char *)S[l].cls - tail_raw) : 0u;
         }
     __syncthreads();
-    for (int l = tl.t; l < tl.ml; l++) {
+    const int bottom = tl.dense ? tl.d : tl.ml;
+    for (int l = tl.t; l < bottom; l++) {
         const pair_level V = pair_view(tail_raw, offs, l), Cv = pair_view(tail_raw, offs, l + 1);
         const int P = S[l].m >> 1, n = S[l].n, cn = S[l + 1].n, ln = lane < P ? lane : P - 1;
         const int lsrc = ln == 0 ? P - 1 : ln - 1, rsrc = ln + 1 == P ? 0 : ln + 1;
@@ -2129,14 +2178,26 @@ __device__ void tail_pairs_body(const tail_levels &tl, const hierarchy_view<floa
         }
         __syncthreads();
     }
-    if (tl.inv_off >= 0) {
+    if (tl.dense) {
+        const pair_level B = pair_view(tail_raw, offs, tl.d);
+        const int nd = S[tl.d].m * S[tl.d].n;
+        for (int r = w; r < 2 * nd; r += nw) {
+            const ff v = mgw::warp_pair_sum(
+                mgw::dense_share<32, float>(tl.dense + (size_t)r * nd, B.b2, nd, lane));
+            if (lane == 0) {
+                if (r & 1) B.z2[r >> 1].y = v.hi + v.lo;
+                else B.z2[r >> 1].x = v.hi + v.lo;
+            }
+        }
+        __syncthreads();
+    } else if (tl.inv_off >= 0) {
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
         tail_bottom(tl, reinterpret_cast<const double *>(tail_raw + tl.inv_off), S[tl.ml], tsh, tid, nth);
     } else {
         tail_bottom(tl, tl.inv, S[tl.ml], tsh, tid, nth);
     }
-    for (int l = tl.ml - 1; l >= tl.t; l--) {
+    for (int l = bottom - 1; l >= tl.t; l--) {
         const pair_level V = pair_view(tail_raw, offs, l), Cv = pair_view(tail_raw, offs, l + 1);
         const int P = S[l].m >> 1, n = S[l].n, ln = lane < P ? lane : P - 1;
         const int lsrc = ln == 0 ? P - 1 : ln - 1, rsrc = ln + 1 == P ? 0 : ln + 1;
@@ -2516,6 +2577,9 @@ static int persist_start(const hierarchy<float> &h, int t) {
     if (!h.persist || !h.bar || !h.bar_err) return 0;
     const int ml = h.nl - 1;
     if (t > ml || t < 2 || !pair_tail(h, t)) return 0;
+    // the same results as the default schedule, whose levels from dense_from
+    // on are one matrix: the tail has to reach that level
+    if (h.dense && h.dense_from <= t) return 0;
     int p = t;
     while (p > 1 && march_level(h, h.lv[p - 1]) && h.lv[p - 1].m <= kPersistWidth) p--;
     return p < t ? p : 0;
@@ -2557,6 +2621,11 @@ static void coarse_persist(hierarchy<float> &h, int p, int t, cudaStream_t st) {
     cp.t = t;
     cp.tl = tail_levels{t, h.nl - 1, h.bottom_inv, h.bottom_unknowns, -1};
     size_t smem = pair_tail_smem(h, t, &cp.tl.inv_off);
+    if (h.dense) {
+        cp.tl.dense = h.dense;
+        cp.tl.d = h.dense_from;
+        cp.tl.inv_off = -1;
+    }
     if (smem < kPersistStage) smem = kPersistStage;
     cp.bar = h.bar;
     cp.err = h.bar_err;
@@ -2640,7 +2709,23 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
         top_sweep(h, st);
         return;
     }
-    const int t = tail_start(h);
+    int t = tail_start(h);
+    int small = -1;  // first level of the small-level kernel (-1: none)
+    if constexpr (sizeof(T) == 8) {
+        if (pair_cycle_supported(h)) {
+            if (zero_start) cudaMemsetAsync(T0.z, 0, sizeof(V) * (size_t)T0.m * T0.n, st);
+            pair_residual(h, nullptr, reduction_blocks(), st);
+            pair_cycle(h, st);
+            return;
+        }
+    } else {
+        if (h.fuse && h.tail_limit < 0 && !persist_start(h, t)) small = small_first(h);
+        if (small == 0) {
+            small_levels(h, zero_start, st);
+            return;
+        }
+        if (small > 0) t = small;
+    }
     if (zero_start && !fused) cudaMemsetAsync(T0.z, 0, sizeof(V) * (size_t)T0.m * T0.n, st);
     if (fused) {
         launch_top_down(h, st, zero_start);
@@ -2653,7 +2738,7 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
         note_launch();
     }
     int p = 0;  // first level of the persistent coarse kernel (0: none)
-    if constexpr (sizeof(T) == 4) p = persist_start(h, t);
+    if constexpr (sizeof(T) == 4) p = small > 0 ? 0 : persist_start(h, t);
     // levels [1, down_end) go down outside the tail (and the persistent kernel)
     const int down_end = p ? p : (t <= ml ? t : ml);
     for (int i = 1; i < down_end; i++) {
@@ -2678,6 +2763,9 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
     if (p) {
         if constexpr (sizeof(T) == 4) coarse_persist(h, p, t, st);
         up_from = p;
+    } else if (small > 0) {
+        if constexpr (sizeof(T) == 4) small_levels(h, true, st);
+        up_from = t;
     } else if (t <= ml) {
         hierarchy_view<T> hv;
         for (int l = 0; l < h.nl; l++) hv.lv[l] = h.lv[l];
@@ -2735,6 +2823,14 @@ template <typename T>
 void top_residual_sqnorm(hierarchy<T> &h, double *partials, int npart, double *out, double *out_b,
                          cudaStream_t st) {
     level_view<T> &L = h.lv[0];
+    if constexpr (sizeof(T) == 8) {
+        if (pair_cycle_supported(h)) {
+            pair_residual(h, partials, npart, st);
+            k_final_sum<<<1, 256, 0, st>>>(partials, npart, out, out_b);
+            note_launch();
+            return;
+        }
+    }
     k_top_sqnorm<T><<<npart, kRedThreads, 0, st>>>(h.op, L.z, L.b, L.m, L.n, partials); note_launch();
     k_final_sum<<<1, 256, 0, st>>>(partials, npart, out, out_b); note_launch();
 }

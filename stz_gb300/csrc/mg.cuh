@@ -95,6 +95,8 @@ template <typename T> class hierarchy {
     // and whether wide single-precision levels use the fused tile kernels
     long tail_limit = -1;
     int fuse = 1;
+    // most blocks of the small-level kernel's cluster (mg_small.cu)
+    int small_blocks = 16;
     // single precision: the coarse levels at most 512 wide and the tail in
     // one cooperative persistent kernel (set by the owner once
     // coarse_persist_supported() holds; bar: two zeroed device words for its
@@ -104,13 +106,22 @@ template <typename T> class hierarchy {
     int persist = 0;
     unsigned *bar = nullptr;
     int *bar_err = nullptr;
+    // the coarse stencils as float pairs (20 float4 each: per block the high
+    // parts, then the low ones; FP32 hierarchies: from dense_from on), the
+    // V-cycle from level dense_from on as one matrix of float pairs (null: none),
+    // and for FP64 hierarchies the top level's correction
+    const float4 *st_pairs[17] = {nullptr};
+    const float4 *dense = nullptr;
+    int dense_from = 0;
+    float2 *dense_buf[17] = {nullptr};
+    float4 *top_pairs = nullptr;
     void release();
     ~hierarchy() { release(); }
     size_t device_bytes() const { return bytes_; }
   private:
     std::vector<void *> owned_;
     size_t bytes_ = 0;
-    size_t st_cap_[17] = {0}, cls_cap_[17] = {0}, inv_cap_ = 0;
+    size_t st_cap_[17] = {0}, cls_cap_[17] = {0}, pair_cap_[17] = {0}, dense_cap_[17] = {0}, inv_cap_ = 0;
     int grow(int l, size_t st_need, size_t cls_need);
     double *inv_dev_ = nullptr;
 };
@@ -121,6 +132,22 @@ template <typename T> class hierarchy {
 template <typename T>
 void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64, bool zero_start = false);
 template <typename T> void top_sweep(hierarchy<T> &h, cudaStream_t st);
+// FP64 V-cycles in correction form (mg_small.cu): pair_residual leaves
+// r = b - A z of the top level as float pairs in its r array (and, with
+// partials, the per-block sums of r^2 and b^2 for k_final_sum); pair_cycle
+// adds one V-cycle on A d = r to z.  Where supported, vcycle<double> is the
+// two of them.
+bool pair_cycle_supported(const hierarchy<double> &h);
+void pair_residual(const hierarchy<double> &h, double *partials, int npart, cudaStream_t st);
+void pair_cycle(const hierarchy<double> &h, cudaStream_t st);
+// Lays out the matrix of the levels from dense_from on (inverse: of the
+// coarsest level); own and caps: the hierarchy's allocations and their sizes.
+template <typename T>
+int build_dense(hierarchy<T> &h, const std::vector<double> &inverse, std::vector<void *> &own, size_t *caps);
+// FP32: the levels from small_first (-1: none) on in one launch, from and to
+// that level's global b and z.
+int small_first(const hierarchy<float> &h);
+void small_levels(const hierarchy<float> &h, bool zero_start, cudaStream_t st);
 // One launch of the streaming top-level kernel down (0) or up (1) of the FP32
 // V-cycle, for timing; false where the top level does not use them.
 bool top_level_kernel(hierarchy<float> &h, int which, cudaStream_t st);

@@ -1,0 +1,1058 @@
+// Phases of a V-cycle on a window of a level that sits in shared memory,
+// templated on the number type: float, or ff (a float pair, ~48 significant
+// bits).  A window holds the nodes of a range of rows, either whole periodic
+// rows (WRAP) or a range of columns with a halo, each row stored parity-major
+// (even columns, then odd ones) so that the points of one colour, and their
+// neighbours, are consecutive.  Every phase is a loop over points by thread
+// index without synchronisation; the caller separates phases by barriers.
+//
+// The smoother is the one of mg.cu: two colours on the matrix-free top level
+// (colour c updates x where (i + j) & 1 == c and y elsewhere), on coarse
+// levels the even rows (even columns, odd columns, the last column of an odd
+// line) and then the odd rows; float results are the bits of the streaming
+// kernels' operations in their order.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "transfer1d.cuh"
+
+#ifdef __CUDACC__
+#define MGW_FN __device__ __forceinline__
+#define MGW_BOTH __host__ __device__ inline
+#else
+#define MGW_FN inline
+#define MGW_BOTH inline
+#endif
+
+#include "ffnum.cuh"
+
+namespace stzg {
+namespace mgw {
+
+// ---- numbers -----------------------------------------------------------------
+
+template <typename S> struct num;
+template <> struct num<float> {
+    typedef float2 node;            // x, y
+    static constexpr int quads = 1; // float4 words of a 2x2 block
+};
+template <> struct num<ff> {
+    typedef float4 node;            // x.hi, y.hi, x.lo, y.lo
+    static constexpr int quads = 2; // the high parts, then the low parts
+};
+
+template <typename S> struct val2 {
+    S x, y;
+};
+
+MGW_FN val2<float> get(const float2 &p) { return val2<float>{p.x, p.y}; }
+MGW_FN val2<ff> get(const float4 &p) { return val2<ff>{ff{p.x, p.z}, ff{p.y, p.w}}; }
+MGW_FN float2 put(const val2<float> &v) { return make_float2(v.x, v.y); }
+MGW_FN float4 put(const val2<ff> &v) { return make_float4(v.x.hi, v.y.hi, v.x.lo, v.y.lo); }
+MGW_FN float get_x(const float2 *p) { return p->x; }
+MGW_FN float get_y(const float2 *p) { return p->y; }
+MGW_FN ff get_x(const float4 *p) { return ff{p->x, p->z}; }
+MGW_FN ff get_y(const float4 *p) { return ff{p->y, p->w}; }
+MGW_FN void put_x(float2 *p, float v) { p->x = v; }
+MGW_FN void put_y(float2 *p, float v) { p->y = v; }
+MGW_FN void put_x(float4 *p, ff v) { p->x = v.hi; p->z = v.lo; }
+MGW_FN void put_y(float4 *p, ff v) { p->y = v.hi; p->w = v.lo; }
+
+MGW_FN float add(float a, float b) { return a + b; }
+MGW_FN ff add(ff a, ff b) { return ff_add(a, b); }
+MGW_FN float sub(float a, float b) { return a - b; }
+MGW_FN ff sub(ff a, ff b) { return ff_sub(a, b); }
+MGW_FN float mul(float a, float b) { return a * b; }
+MGW_FN ff mul(ff a, ff b) { return ff_mul(a, b); }
+// by a power of two
+MGW_FN float scale(float a, float w) { return a * w; }
+MGW_FN ff scale(ff a, float w) { return ff{a.hi * w, a.lo * w}; }
+
+// A running sum of products.  ff: the high parts by TwoSum, every rounding
+// error and low part gathered in lo (relative 2^-48 of the terms' magnitude),
+// renormalised once at the end.
+struct facc {
+    float v = 0.f;
+    MGW_FN void mad(float a, float b) { v = fmaf(a, b, v); }
+    MGW_FN float done() const { return v; }
+};
+struct ffacc {
+    float hi = 0.f, lo = 0.f;
+    MGW_FN void mad(ff a, ff b) {
+        const float p = ff_prod(a.hi, b.hi);
+        float e = fmaf(a.hi, b.hi, -p);
+        e = fmaf(a.hi, b.lo, e);
+        e = fmaf(a.lo, b.hi, e);
+        const float s = hi + p, bb = s - hi;
+        lo += ((hi - (s - bb)) + (p - bb)) + e;
+        hi = s;
+    }
+    MGW_FN ff done() const { return ff_fast2sum(hi, lo); }
+};
+template <typename S> struct acc_of;
+template <> struct acc_of<float> { typedef facc type; };
+template <> struct acc_of<ff> { typedef ffacc type; };
+
+// a + b - c - d of the corner terms, and a + b, as operands of a product (not
+// renormalised for ff: the product folds the low part in).
+MGW_FN float sum2(float a, float b) { return a + b; }
+MGW_FN ff sum2(ff a, ff b) {
+    const float s = a.hi + b.hi, bb = s - a.hi;
+    return ff{s, ((a.hi - (s - bb)) + (b.hi - bb)) + (a.lo + b.lo)};
+}
+MGW_FN float cross4(float a, float b, float c, float d) { return a + b - c - d; }
+MGW_FN ff cross4(ff a, ff b, ff c, ff d) { return sum2(sum2(a, ff_neg(c)), sum2(b, ff_neg(d))); }
+
+// Constants of the top-level operator (top_op in mg.cuh) in the number type.
+template <typename S> struct top_consts {
+    S Kmx, Kmy, mx, my, qK, cxx, cyy, icxx, icyy, bcxx, bcyy, ibcxx, ibcyy;
+};
+
+MGW_FN float three(float k1, float s1, float k2, float s2, float k3, float s3) { return k1 * s1 + k2 * s2 + k3 * s3; }
+MGW_FN ff three(ff k1, ff s1, ff k2, ff s2, ff k3, ff s3) {
+    ffacc a;
+    a.mad(k1, s1);
+    a.mad(k2, s2);
+    a.mad(k3, s3);
+    return a.done();
+}
+
+// ---- windows -----------------------------------------------------------------
+
+template <typename S, bool WRAP> struct window {
+    typedef typename num<S>::node node;
+    node *z, *b, *r;
+    int W, He;          // columns; even ones
+    int jb, rb;         // rows of local row 0 of z and b; of r
+    int m, n;           // the level
+    int x0;             // global column of window column 0 (even; 0 when WRAP)
+    const float4 *st;   // stencils: 10 blocks each
+    const int *cls;     // class per row (homog) or per point
+    int homog;
+    MGW_FN int col(int w) const { return (w & 1) * He + (w >> 1); }
+    MGW_FN int at(int j, int w) const { return (j - jb) * W + col(w); }
+    MGW_FN int rat(int j, int w) const { return (j - rb) * W + col(w); }
+    MGW_FN int left(int w) const { return WRAP && w == 0 ? W - 1 : w - 1; }
+    MGW_FN int right(int w) const { return WRAP && w == W - 1 ? 0 : w + 1; }
+    MGW_FN int gcol(int w) const {
+        if (WRAP) return w;
+        const int g = x0 + w;
+        return g < 0 ? g + m : (g >= m ? g % m : g);
+    }
+    MGW_FN const float4 *sten(int j, int w) const {
+        const int c = homog ? cls[j] : cls[(size_t)j * m + gcol(w)];
+        return st + (size_t)c * (10 * num<S>::quads);
+    }
+};
+
+// idx -> (idx / per, idx % per) for idx < 2^20: the half keeps the float
+// quotient away from whole numbers.
+struct divider {
+    float inv;
+    int per;
+    MGW_FN explicit divider(int p) : inv(1.f / (float)(p > 0 ? p : 1)), per(p) {}
+    MGW_FN int quot(int k) const { return (int)(((float)k + 0.5f) * inv); }
+};
+
+// acc += A z of block e.
+MGW_FN void madd(facc &ax, facc &ay, const float4 *s, int e, const val2<float> &z) {
+    const float4 A = s[e];
+    ax.mad(A.x, z.x);
+    ax.mad(A.y, z.y);
+    ay.mad(A.z, z.x);
+    ay.mad(A.w, z.y);
+}
+MGW_FN void madd(ffacc &ax, ffacc &ay, const float4 *s, int e, const val2<ff> &z) {
+    const float4 H = s[2 * e], L = s[2 * e + 1];
+    ax.mad(ff{H.x, L.x}, z.x);
+    ax.mad(ff{H.y, L.y}, z.y);
+    ay.mad(ff{H.z, L.z}, z.x);
+    ay.mad(ff{H.w, L.w}, z.y);
+}
+// A v of block e (the inverse of the centre block)
+MGW_FN val2<float> apply(const float4 *s, int e, const val2<float> &v) {
+    const float4 A = s[e];
+    return val2<float>{A.x * v.x + A.y * v.y, A.z * v.x + A.w * v.y};
+}
+MGW_FN val2<ff> apply(const float4 *s, int e, const val2<ff> &v) {
+    ffacc ax, ay;
+    madd(ax, ay, s, e, v);
+    return val2<ff>{ax.done(), ay.done()};
+}
+
+// Off-diagonal products of a coarse level (tgmg_level::mul_a,
+// tgmg.in.cc:536-547).  rows: whether the rows below and above take part;
+// mid: whether the neighbours in the row do (a sweep that starts from zero
+// skips what is still zero: adding exact zeros changes nothing).
+template <typename S, bool WRAP>
+MGW_FN void offdiag(const window<S, WRAP> &V, const float4 *s, int j, int w, bool rows, bool mid,
+                    typename acc_of<S>::type &ax, typename acc_of<S>::type &ay) {
+    const int wl = V.left(w), wr = V.right(w);
+    if (rows && j > 0) {
+        madd(ax, ay, s, 0, get(V.z[V.at(j - 1, wl)]));
+        madd(ax, ay, s, 1, get(V.z[V.at(j - 1, w)]));
+        madd(ax, ay, s, 2, get(V.z[V.at(j - 1, wr)]));
+    }
+    if (mid) {
+        madd(ax, ay, s, 3, get(V.z[V.at(j, wl)]));
+        madd(ax, ay, s, 5, get(V.z[V.at(j, wr)]));
+    }
+    if (rows && j < V.n - 1) {
+        madd(ax, ay, s, 6, get(V.z[V.at(j + 1, wl)]));
+        madd(ax, ay, s, 7, get(V.z[V.at(j + 1, w)]));
+        madd(ax, ay, s, 8, get(V.z[V.at(j + 1, wr)]));
+    }
+}
+
+MGW_FN int imax(int a, int b) { return a > b ? a : b; }
+MGW_FN int imin(int a, int b) { return a < b ? a : b; }
+
+// Colours of a sweep: rows of parity cy, columns of parity cx (cx == 2: the
+// last column of an odd line), rows jlo..jhi and window columns wlo..whi (all
+// when WRAP).
+template <typename S, bool WRAP>
+MGW_FN void lev_color(const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int cx, int cy, bool from_zero,
+                      int tid, int nth) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    const int j0 = jlo + ((jlo ^ cy) & 1);
+    if (j0 > jhi) return;
+    int w0, nw;
+    if (cx == 2) {
+        w0 = V.W - 1;
+        nw = 1;
+    } else if (WRAP) {
+        w0 = cx;
+        nw = V.W >> 1;  // even columns without the last one of an odd line
+    } else {
+        w0 = wlo + ((wlo ^ cx) & 1);
+        nw = whi >= w0 ? ((whi - w0) >> 1) + 1 : 0;
+    }
+    const int total = (((jhi - j0) >> 1) + 1) * nw;
+    const divider dv(nw);
+    for (int k = tid; k < total; k += nth) {
+        const int q = dv.quot(k), j = j0 + 2 * q, w = w0 + 2 * (k - q * nw);
+        const float4 *s = V.sten(j, w);
+        typename acc_of<S>::type ax, ay;
+        offdiag(V, s, j, w, !(from_zero && cy == 0), !(from_zero && cx == 0), ax, ay);
+        const int c = V.at(j, w);
+        const val2<S> bb = get(V.b[c]);
+        V.z[c] = put(apply(s, 9, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())}));
+    }
+}
+
+// z = 0 on the last column of an odd line (the third colour, read before its
+// first update in a sweep from zero).
+template <typename S, bool WRAP>
+MGW_FN void lev_clear_last(const window<S, WRAP> &V, int jlo, int jhi, int tid, int nth) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    for (int j = jlo + tid; j <= jhi; j += nth) {
+        val2<S> o{};
+        V.z[V.at(j, V.W - 1)] = put(o);
+    }
+}
+
+// r = b - A z after a sweep.  On an even line the odd columns of odd rows took
+// the last colour: their residual is zero up to rounding and set to zero.
+template <typename S, bool WRAP>
+MGW_FN void lev_residual(const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int tid, int nth) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    if (jlo > jhi) return;
+    if (WRAP) {
+        wlo = 0;
+        whi = V.W - 1;
+    }
+    const int nw = whi - wlo + 1, total = (jhi - jlo + 1) * nw;
+    const bool odd_line = V.m & 1;
+    const divider dv(nw);
+    for (int k = tid; k < total; k += nth) {
+        const int q = dv.quot(k), j = jlo + q, w = wlo + (k - q * nw);
+        val2<S> o{};
+        if (odd_line || !(j & w & 1)) {
+            const float4 *s = V.sten(j, w);
+            typename acc_of<S>::type ax, ay;
+            offdiag(V, s, j, w, true, true, ax, ay);
+            const int c = V.at(j, w);
+            madd(ax, ay, s, 4, get(V.z[c]));
+            const val2<S> bb = get(V.b[c]);
+            o = val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())};
+        }
+        V.r[V.rat(j, w)] = put(o);
+    }
+}
+
+// Off-diagonal sums of the top level (qs_multi::mul_a, qs_multi.hh:41-50).
+template <typename S, bool WRAP>
+MGW_FN S top_off_x(const top_consts<S> &o, const window<S, WRAP> &V, int j, int w) {
+    const int wl = V.left(w), wr = V.right(w);
+    return three(o.Kmx, sum2(get_x(V.z + V.at(j, wl)), get_x(V.z + V.at(j, wr))), o.my,
+                 sum2(get_x(V.z + V.at(j - 1, w)), get_x(V.z + V.at(j + 1, w))), o.qK,
+                 cross4(get_y(V.z + V.at(j - 1, wl)), get_y(V.z + V.at(j + 1, wr)), get_y(V.z + V.at(j - 1, wr)),
+                        get_y(V.z + V.at(j + 1, wl))));
+}
+template <typename S, bool WRAP>
+MGW_FN S top_off_y(const top_consts<S> &o, const window<S, WRAP> &V, int j, int w) {
+    const int wl = V.left(w), wr = V.right(w);
+    return three(o.mx, sum2(get_y(V.z + V.at(j, wl)), get_y(V.z + V.at(j, wr))), o.Kmy,
+                 sum2(get_y(V.z + V.at(j - 1, w)), get_y(V.z + V.at(j + 1, w))), o.qK,
+                 cross4(get_x(V.z + V.at(j - 1, wl)), get_x(V.z + V.at(j + 1, wr)), get_x(V.z + V.at(j - 1, wr)),
+                        get_x(V.z + V.at(j + 1, wl))));
+}
+
+// One colour of the top level: a thread takes a pair of columns, the x
+// equation at one and the y equation at the other, so that lanes do not
+// diverge on the component.  from_zero: z is zero, so only b counts.
+template <typename S, bool WRAP>
+MGW_FN void top_color(const top_consts<S> &o, const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int color,
+                      bool from_zero, int tid, int nth) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    if (jlo > jhi) return;
+    if (WRAP) {
+        wlo = 0;
+        whi = V.W - 1;
+    }
+    const int p0 = wlo >> 1, np = (whi >> 1) - p0 + 1, total = (jhi - jlo + 1) * np;
+    const divider dv(np);
+    for (int k = tid; k < total; k += nth) {
+        const int q = dv.quot(k), j = jlo + q, wa = 2 * (p0 + (k - q * np));
+        const bool even_is_x = (j & 1) == color;
+        const int wx = even_is_x ? wa : wa + 1, wy = even_is_x ? wa + 1 : wa;
+        const bool wall = j == 0 || j == V.n - 1;
+        if (wx >= wlo && wx <= whi) {
+            const int c = V.at(j, wx);
+            const S bb = get_x(V.b + c);
+            if (wall) put_x(V.z + c, mul(o.ibcxx, bb));
+            else if (from_zero) put_x(V.z + c, mul(o.icxx, bb));
+            else put_x(V.z + c, mul(o.icxx, sub(bb, top_off_x(o, V, j, wx))));
+        }
+        if (wy >= wlo && wy <= whi) {
+            const int c = V.at(j, wy);
+            const S bb = get_y(V.b + c);
+            if (wall) put_y(V.z + c, mul(o.ibcyy, bb));
+            else if (from_zero) put_y(V.z + c, mul(o.icyy, bb));
+            else put_y(V.z + c, mul(o.icyy, sub(bb, top_off_y(o, V, j, wy))));
+        }
+    }
+}
+
+// Residual of the colour-0 equations after a sweep (the colour-1 ones, whose
+// unknowns were updated last, and the wall rows are zero up to rounding).
+template <typename S, bool WRAP>
+MGW_FN void top_residual(const top_consts<S> &o, const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int tid,
+                         int nth) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    if (jlo > jhi) return;
+    if (WRAP) {
+        wlo = 0;
+        whi = V.W - 1;
+    }
+    const int p0 = wlo >> 1, np = (whi >> 1) - p0 + 1, total = (jhi - jlo + 1) * np;
+    const divider dv(np);
+    for (int k = tid; k < total; k += nth) {
+        const int q = dv.quot(k), j = jlo + q, wa = 2 * (p0 + (k - q * np));
+        const int wx = (j & 1) ? wa + 1 : wa, wy = (j & 1) ? wa : wa + 1;
+        const bool wall = j == 0 || j == V.n - 1;
+        if (wx >= wlo && wx <= whi) {
+            const int c = V.at(j, wx);
+            val2<S> r{};
+            if (!wall) r.x = sub(sub(get_x(V.b + c), top_off_x(o, V, j, wx)), mul(o.cxx, get_x(V.z + c)));
+            V.r[V.rat(j, wx)] = put(r);
+        }
+        if (wy >= wlo && wy <= whi) {
+            const int c = V.at(j, wy);
+            val2<S> r{};
+            if (!wall) r.y = sub(sub(get_y(V.b + c), top_off_y(o, V, j, wy)), mul(o.cyy, get_y(V.z + c)));
+            V.r[V.rat(j, wy)] = put(r);
+        }
+    }
+}
+
+// halves_of(2J + q - 1, n, 0, J), q = 0, 1, 2 on a bounded line of n points.
+MGW_FN int row_halves(int q, int J, int n) {
+    const int fy = 2 * J + q - 1;
+    if (fy < 0 || fy >= n) return 0;
+    if (q == 1) return 2;
+    if ((n & 1) || fy != n - 1) return 1;
+    return q == 0 ? 2 : 0;
+}
+
+// Full weighting of r at the coarse points of rows Jlo..Jhi, columns
+// Ilo..Ihi (global): out(J, I, value).
+template <typename S, bool WRAP, typename Out>
+MGW_FN void restrict_rows(const window<S, WRAP> &V, int Jlo, int Jhi, int Ilo, int Ihi, int cm, Out out, int tid,
+                          int nth) {
+    const int nI = Ihi - Ilo + 1, total = (Jhi - Jlo + 1) * nI;
+    if (Jhi < Jlo || nI <= 0) return;
+    const bool odd_line = V.m & 1;
+    const divider dv(nI);
+    for (int k = tid; k < total; k += nth) {
+        const int qk = dv.quot(k), J = Jlo + qk, I = Ilo + (k - qk * nI), w = 2 * I - V.x0;
+        // an odd periodic line: its last (even) point injects, so the two
+        // coarse points at the seam have no neighbour across it
+        const bool hl = !(odd_line && I == 0), hr = !(odd_line && I == cm - 1);
+        val2<S> a{};
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const int hy = row_halves(q, J, V.n);
+            if (!hy) continue;
+            const int fy = 2 * J + q - 1;
+            const float w1 = (float)hy * 0.25f, w2 = (float)(2 * hy) * 0.25f;
+            if (hl) {
+                const val2<S> v = get(V.r[V.rat(fy, V.left(w))]);
+                a.x = add(a.x, scale(v.x, w1));
+                a.y = add(a.y, scale(v.y, w1));
+            }
+            const val2<S> c = get(V.r[V.rat(fy, w)]);
+            a.x = add(a.x, scale(c.x, w2));
+            a.y = add(a.y, scale(c.y, w2));
+            if (hr) {
+                const val2<S> v = get(V.r[V.rat(fy, V.right(w))]);
+                a.x = add(a.x, scale(v.x, w1));
+                a.y = add(a.y, scale(v.y, w1));
+            }
+        }
+        out(J, I, put(a));
+    }
+}
+
+// z += P zc on rows jlo..jhi, window columns wlo..whi: zc(J, I) is the child's
+// value at row J and the coarse column I of window column 2 (I - x0/2) (WRAP:
+// 0 <= I < cm; else unwrapped).
+template <typename S, bool WRAP, typename Child>
+MGW_FN void prolong_rows(const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int cm, Child zc, int tid,
+                         int nth) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    if (jlo > jhi) return;
+    if (WRAP) {
+        wlo = 0;
+        whi = V.W - 1;
+    }
+    const int nw = whi - wlo + 1, total = (jhi - jlo + 1) * nw;
+    const divider dv(nw);
+    for (int k = tid; k < total; k += nth) {
+        const int qk = dv.quot(k), j = jlo + qk, w = wlo + (k - qk * nw);
+        int cy[2], hy[2];
+        const int ny = p1d_halves(j, V.n, 0, cy, hy);
+        const int I = (V.x0 + w) >> 1;  // floor: x0 is even
+        val2<S> a{};
+        if (w & 1) {
+            const int I1 = WRAP && I + 1 == cm ? 0 : I + 1;
+            for (int q = 0; q < ny; q++) {
+                const float wy = (float)hy[q] * 0.25f;
+                const val2<S> v0 = get(zc(cy[q], I)), v1 = get(zc(cy[q], I1));
+                a.x = add(a.x, scale(add(v0.x, v1.x), wy));
+                a.y = add(a.y, scale(add(v0.y, v1.y), wy));
+            }
+        } else {
+            for (int q = 0; q < ny; q++) {
+                const float wy = (float)hy[q] * 0.25f;
+                const val2<S> v0 = get(zc(cy[q], I));
+                a.x = add(a.x, scale(v0.x, 2.f * wy));
+                a.y = add(a.y, scale(v0.y, 2.f * wy));
+            }
+        }
+        const int c = V.at(j, w);
+        const val2<S> f = get(V.z[c]);
+        V.z[c] = put(val2<S>{add(f.x, a.x), add(f.y, a.y)});
+    }
+}
+
+// ---- even levels in 2 x 2 blocks --------------------------------------------------
+//
+// The same phases for a band of an even line with one stencil class per row
+// and its tables in shared memory: a thread keeps one block of 2 x 2 nodes
+// (rows 2q, 2q + 1 of the band, columns 2k, 2k + 1) through every phase, so
+// that indices are formed once per level; small levels are bound by the
+// latency of a phase, of which index arithmetic was the larger part.
+
+// A thread's blocks: q, k of the first one, and the step to the next.
+struct block_walk {
+    int q, k, dq, dk, P;
+    MGW_FN block_walk(int tid, int nth, int p) : P(p) {
+        const divider dv(p);
+        q = dv.quot(tid);
+        k = tid - q * p;
+        dq = dv.quot(nth);
+        dk = nth - dq * p;
+    }
+    MGW_FN void next() {
+        k += dk;
+        q += dq;
+        if (k >= P) {
+            k -= P;
+            q++;
+        }
+    }
+};
+
+// The nodes around a point: its column and its neighbours' columns as offsets
+// in a parity-major row.
+struct columns3 {
+    int l, c, r;
+    MGW_FN columns3(int k, int P, int cx)
+        : l(cx ? k : P + (k ? k - 1 : P - 1)), c(cx ? P + k : k), r(cx ? (k + 1 == P ? 0 : k + 1) : P + k) {}
+};
+
+template <typename S>
+MGW_FN void offdiag3(const float4 *s, const typename num<S>::node *row, int W, const columns3 &c, bool dn, bool mid,
+                     bool up, typename acc_of<S>::type &ax, typename acc_of<S>::type &ay) {
+    if (dn) {
+        madd(ax, ay, s, 0, get(row[c.l - W]));
+        madd(ax, ay, s, 1, get(row[c.c - W]));
+        madd(ax, ay, s, 2, get(row[c.r - W]));
+    }
+    if (mid) {
+        madd(ax, ay, s, 3, get(row[c.l]));
+        madd(ax, ay, s, 5, get(row[c.r]));
+    }
+    if (up) {
+        madd(ax, ay, s, 6, get(row[c.l + W]));
+        madd(ax, ay, s, 7, get(row[c.c + W]));
+        madd(ax, ay, s, 8, get(row[c.r + W]));
+    }
+}
+
+// Colour (cx, cy) on the rows jlo..jhi of the band (qn block rows).
+template <typename S>
+MGW_FN void block_color(const window<S, true> &V, block_walk w, int qn, int jlo, int jhi, int cx, int cy,
+                        bool from_zero) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    for (; w.q < qn; w.next()) {
+        const int lr = 2 * w.q + cy, j = V.jb + lr;
+        if (j < jlo || j > jhi) continue;
+        const float4 *s = V.st + V.cls[j] * (10 * num<S>::quads);
+        const columns3 c(w.k, w.P, cx);
+        typename num<S>::node *row = V.z + lr * V.W;
+        const bool rows = !(from_zero && cy == 0);
+        const val2<S> bb = get(V.b[lr * V.W + c.c]);
+        typename acc_of<S>::type ax, ay;
+        offdiag3<S>(s, row, V.W, c, rows && j > 0, !(from_zero && cx == 0), rows && j < V.n - 1, ax, ay);
+        row[c.c] = put(apply(s, 9, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())}));
+    }
+}
+
+// Residual of the rows jlo..jhi (the odd columns of odd rows: zero).
+template <typename S> MGW_FN void block_residual(const window<S, true> &V, block_walk w, int qn, int jlo, int jhi) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    for (; w.q < qn; w.next()) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int cx = e & 1, cy = e >> 1, lr = 2 * w.q + cy, j = V.jb + lr;
+            if (j < jlo || j > jhi) continue;
+            const columns3 c(w.k, w.P, cx);
+            val2<S> o{};
+            if (e < 3) {
+                const float4 *s = V.st + V.cls[j] * (10 * num<S>::quads);
+                const typename num<S>::node *row = V.z + lr * V.W;
+                const val2<S> bb = get(V.b[lr * V.W + c.c]);
+                typename acc_of<S>::type ax, ay;
+                offdiag3<S>(s, row, V.W, c, j > 0, true, j < V.n - 1, ax, ay);
+                madd(ax, ay, s, 4, get(row[c.c]));
+                o = val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())};
+            }
+            V.r[(j - V.rb) * V.W + c.c] = put(o);
+        }
+    }
+}
+
+// Restriction to the coarse rows Jlo..Jhi: coarse point (J, k) under block
+// (J - jb/2, k).
+template <typename S, typename Out>
+MGW_FN void block_restrict(const window<S, true> &V, block_walk w, int qn, int Jlo, int Jhi, Out out) {
+    for (; w.q < qn; w.next()) {
+        const int J = (V.jb >> 1) + w.q;
+        if (J < Jlo || J > Jhi) continue;
+        const columns3 c(w.k, w.P, 0);
+        val2<S> a{};
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const int hy = row_halves(q, J, V.n);
+            if (!hy) continue;
+            const typename num<S>::node *row = V.r + (2 * J + q - 1 - V.rb) * V.W;
+            const float w1 = (float)hy * 0.25f, w2 = (float)(2 * hy) * 0.25f;
+            const val2<S> l = get(row[c.l]), m = get(row[c.c]), r = get(row[c.r]);
+            a.x = add(a.x, scale(l.x, w1));
+            a.y = add(a.y, scale(l.y, w1));
+            a.x = add(a.x, scale(m.x, w2));
+            a.y = add(a.y, scale(m.y, w2));
+            a.x = add(a.x, scale(r.x, w1));
+            a.y = add(a.y, scale(r.y, w1));
+        }
+        out(J, w.k, put(a));
+    }
+}
+
+// Prolongation on the rows jlo..jhi: crow(J) is the child's row J (natural or
+// parity-major, col(I) its column).
+template <typename S, typename Row, typename Col>
+MGW_FN void block_prolong(const window<S, true> &V, block_walk w, int qn, int jlo, int jhi, Row crow, Col col) {
+    typedef typename num<S>::node node;
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    for (; w.q < qn; w.next()) {
+        const int je = V.jb + 2 * w.q, J = je >> 1;
+        if (je > jhi || je + 1 < jlo) continue;
+        const int c0 = col(w.k), c1 = col(w.k + 1 == w.P ? 0 : w.k + 1);
+        const bool even = je >= jlo, odd = je + 1 <= jhi;
+        // an even line injects its last point into the last coarse one
+        const bool inject = !(V.n & 1) && je + 1 == V.n - 1;
+        val2<S> a0{}, a1{}, b0{}, b1{};
+        if (even || !inject) {
+            const node *r = crow(J);
+            a0 = get(r[c0]);
+            a1 = get(r[c1]);
+        }
+        if (odd) {
+            const node *r = crow(J + 1);
+            b0 = get(r[c0]);
+            b1 = get(r[c1]);
+        }
+        node *z = V.z + 2 * w.q * V.W;
+        if (even) {
+            const val2<S> f = get(z[w.k]), g = get(z[w.P + w.k]);
+            z[w.k] = put(val2<S>{add(f.x, a0.x), add(f.y, a0.y)});
+            z[w.P + w.k] =
+                put(val2<S>{add(g.x, scale(add(a0.x, a1.x), 0.5f)), add(g.y, scale(add(a0.y, a1.y), 0.5f))});
+        }
+        if (odd) {
+            node *y = z + V.W;
+            const val2<S> f = get(y[w.k]), g = get(y[w.P + w.k]);
+            val2<S> u, v;
+            if (inject) {
+                u = b0;
+                v = val2<S>{scale(add(b0.x, b1.x), 0.5f), scale(add(b0.y, b1.y), 0.5f)};
+            } else {
+                u = val2<S>{add(scale(a0.x, 0.5f), scale(b0.x, 0.5f)), add(scale(a0.y, 0.5f), scale(b0.y, 0.5f))};
+                v = val2<S>{add(scale(add(a0.x, a1.x), 0.25f), scale(add(b0.x, b1.x), 0.25f)),
+                            add(scale(add(a0.y, a1.y), 0.25f), scale(add(b0.y, b1.y), 0.25f))};
+            }
+            y[w.k] = put(val2<S>{add(f.x, u.x), add(f.y, u.y)});
+            y[w.P + w.k] = put(val2<S>{add(g.x, v.x), add(g.y, v.y)});
+        }
+    }
+}
+
+// Off-diagonal sums of the top level around a point (comp 0: the x equation).
+template <typename S>
+MGW_FN S top_off3(const top_consts<S> &o, const typename num<S>::node *row, int W, const columns3 &c, int comp) {
+    if (comp == 0)
+        return three(o.Kmx, sum2(get_x(row + c.l), get_x(row + c.r)), o.my,
+                     sum2(get_x(row + c.c - W), get_x(row + c.c + W)), o.qK,
+                     cross4(get_y(row + c.l - W), get_y(row + c.r + W), get_y(row + c.r - W), get_y(row + c.l + W)));
+    return three(o.mx, sum2(get_y(row + c.l), get_y(row + c.r)), o.Kmy,
+                 sum2(get_y(row + c.c - W), get_y(row + c.c + W)), o.qK,
+                 cross4(get_x(row + c.l - W), get_x(row + c.r + W), get_x(row + c.r - W), get_x(row + c.l + W)));
+}
+
+// One colour of the top level on the rows jlo..jhi: of the block's four nodes
+// the x equation at the two with (i + j) & 1 == color, the y one at the others.
+template <typename S>
+MGW_FN void block_top_color(const top_consts<S> &o, const window<S, true> &V, block_walk w, int qn, int jlo, int jhi,
+                            int color, bool from_zero) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    for (; w.q < qn; w.next()) {
+#pragma unroll
+        for (int cy = 0; cy < 2; cy++) {
+            const int lr = 2 * w.q + cy, j = V.jb + lr;
+            if (j < jlo || j > jhi) continue;
+            const bool wall = j == 0 || j == V.n - 1;
+            const int cxx = (cy ^ color) & 1;  // the column whose x equation is due
+            typename num<S>::node *row = V.z + lr * V.W;
+            const typename num<S>::node *b = V.b + lr * V.W;
+            const columns3 cx(w.k, w.P, cxx), cyc(w.k, w.P, cxx ^ 1);
+            const S bx = get_x(b + cx.c), by = get_y(b + cyc.c);
+            if (wall) {
+                put_x(row + cx.c, mul(o.ibcxx, bx));
+                put_y(row + cyc.c, mul(o.ibcyy, by));
+            } else if (from_zero) {
+                put_x(row + cx.c, mul(o.icxx, bx));
+                put_y(row + cyc.c, mul(o.icyy, by));
+            } else {
+                const S ex = top_off3(o, row, V.W, cx, 0), ey = top_off3(o, row, V.W, cyc, 1);
+                put_x(row + cx.c, mul(o.icxx, sub(bx, ex)));
+                put_y(row + cyc.c, mul(o.icyy, sub(by, ey)));
+            }
+        }
+    }
+}
+
+template <typename S>
+MGW_FN void block_top_residual(const top_consts<S> &o, const window<S, true> &V, block_walk w, int qn, int jlo,
+                               int jhi) {
+    jlo = imax(jlo, 0);
+    jhi = imin(jhi, V.n - 1);
+    for (; w.q < qn; w.next()) {
+#pragma unroll
+        for (int cy = 0; cy < 2; cy++) {
+            const int lr = 2 * w.q + cy, j = V.jb + lr;
+            if (j < jlo || j > jhi) continue;
+            const bool wall = j == 0 || j == V.n - 1;
+            const typename num<S>::node *row = V.z + lr * V.W, *b = V.b + lr * V.W;
+            const columns3 cx(w.k, w.P, cy), cyc(w.k, w.P, cy ^ 1);
+            val2<S> rx{}, ry{};
+            if (!wall) {
+                rx.x = sub(sub(get_x(b + cx.c), top_off3(o, row, V.W, cx, 0)), mul(o.cxx, get_x(row + cx.c)));
+                ry.y = sub(sub(get_y(b + cyc.c), top_off3(o, row, V.W, cyc, 1)), mul(o.cyy, get_y(row + cyc.c)));
+            }
+            typename num<S>::node *r = V.r + (j - V.rb) * V.W;
+            r[cx.c] = put(rx);
+            r[cyc.c] = put(ry);
+        }
+    }
+}
+
+// ---- distributed small levels ---------------------------------------------------
+//
+// The levels t .. d-1 of a V-cycle in the shared memory of a cluster of blocks
+// (or one block), each cut into row bands, one per block, so that block c owns
+// the coarse rows that restrict from its own fine rows; a band carries the
+// halo rows that make its sweep, residual and restriction exact without an
+// exchange inside a level, so a level costs one cluster barrier on the way
+// down (the child's right-hand side, with its halo) and one on the way up (the
+// child's solution).  From level d on the rest of the V-cycle (it starts from
+// zero, so it is one linear map of d's right-hand side, coarsest solve
+// included) is a matrix of float pairs laid out with the operators, its rows
+// shared out over the blocks: ten levels' worth of dependent phases become
+// one product.
+
+constexpr int kMaxLevels = 17;
+constexpr int kTopBelow = 4, kTopAbove = 4;  // halo rows of the top level: below y0, from y1 up
+constexpr int kLevBelow = 2, kLevAbove = 4;  // of a coarse level (three are read; block rows are pairs)
+
+template <typename S> struct small_level {
+    typedef typename num<S>::node node;
+    int m, n, homog, nst, ncls;
+    const int *cls;     // global
+    const float4 *st;   // global
+    unsigned zo, bo;    // shared offsets of the band's z and b (level d: all of them)
+    unsigned ho;        // the three rows of the solution beyond the band (levels above t)
+    unsigned so, co;    // stencils and row classes (kNone: read from global memory)
+    node *zg;           // global z, b (level t)
+    const node *bg;
+};
+
+constexpr unsigned kNone = 0xffffffffu;
+
+template <typename S> struct small_plan {
+    int t, d, blocks;
+    int top;                 // level t is the matrix-free top level
+    int zero_start;          // its z starts from zero
+    unsigned ro;             // residual rows of the level in hand
+    unsigned bytes;
+    const float4 *dense;     // row-major, per column node (x.hi, x.lo, y.hi, y.lo)
+    double2 *sum;            // not null: the top level's result is added to this iterate
+    top_consts<S> op;
+    small_level<S> lv[kMaxLevels];
+};
+
+// First row of block c on level l: level d's cut scaled up, the line's end
+// for c == blocks.
+template <typename S> MGW_BOTH int band_row(const small_plan<S> &P, int l, int c) {
+    if (c >= P.blocks) return P.lv[l].n;
+    return (int)((long)c * P.lv[P.d].n / P.blocks) << (P.d - l);
+}
+template <typename S> MGW_BOTH int band_below(const small_plan<S> &P, int l) {
+    return P.top && l == P.t ? kTopBelow : kLevBelow;
+}
+template <typename S> MGW_BOTH int band_above(const small_plan<S> &P, int l) {
+    return P.top && l == P.t ? kTopAbove : kLevAbove;
+}
+
+// FAST: every level t .. d-1 is an even line with one class per row and its
+// tables in shared memory (known at compile time).
+template <bool FAST, typename S>
+MGW_FN window<S, true> band_window(const small_plan<S> &P, int l, int c, unsigned char *base) {
+    typedef typename num<S>::node node;
+    const small_level<S> &L = P.lv[l];
+    window<S, true> V;
+    V.z = reinterpret_cast<node *>(base + L.zo);
+    V.b = reinterpret_cast<node *>(base + L.bo);
+    V.r = reinterpret_cast<node *>(base + P.ro);
+    V.W = V.m = L.m;
+    V.He = (L.m + 1) >> 1;
+    V.n = L.n;
+    const int y0 = band_row(P, l, c);
+    V.jb = y0 - band_below(P, l);
+    V.rb = y0 - 1;
+    V.x0 = 0;
+    V.homog = L.homog;
+    if (FAST) {
+        V.st = reinterpret_cast<const float4 *>(base + L.so);
+        V.cls = reinterpret_cast<const int *>(base + L.co);
+    } else {
+        V.st = L.so != kNone ? reinterpret_cast<const float4 *>(base + L.so) : L.st;
+        V.cls = L.co != kNone ? reinterpret_cast<const int *>(base + L.co) : L.cls;
+    }
+    return V;
+}
+
+MGW_FN ff as_pair(float a) { return ff{a, 0.f}; }
+MGW_FN ff as_pair(ff a) { return a; }
+MGW_FN float from_pair(ff a, float) { return a.hi + a.lo; }
+MGW_FN ff from_pair(ff a, ff) { return a; }
+
+#ifdef __CUDACC__
+// The sum of a pair over a warp, on every lane.
+MGW_FN ff warp_pair_sum(ff a) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ff b;
+        b.hi = __shfl_xor_sync(0xffffffffu, a.hi, o);
+        b.lo = __shfl_xor_sync(0xffffffffu, a.lo, o);
+        a = ff_add(a, b);
+    }
+    return a;
+}
+#endif
+
+// This lane's share of one row of the dense levels' product.
+template <int LANES, typename S>
+MGW_FN ff dense_share(const float4 *row, const typename num<S>::node *b, int nd, int lane) {
+    ffacc a;
+    for (int k = lane; k < nd; k += LANES) {
+#ifdef __CUDACC__
+        const float4 M = __ldg(row + k);
+#else
+        const float4 M = row[k];
+#endif
+        const val2<S> v = get(b[k]);
+        a.mad(ff{M.x, M.y}, as_pair(v.x));
+        a.mad(ff{M.z, M.w}, as_pair(v.y));
+    }
+    return a.done();
+}
+
+// The V-cycle on the levels of the plan.  E: the block's environment -
+// rank(), local() and base(rank) (a block's shared memory, this or another
+// one's), par(f) (f(thread, threads) on every thread, then a block barrier),
+// csync() (a barrier of all blocks), kLanes and lane_sum(v) (threads of a
+// product row and the sum over them), ld(p) (a global load), store(P, k, v)
+// (the result of level t at its node k), wait_input() (before the first read
+// of what an earlier kernel wrote).
+template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const small_plan<S> &P, E &env) {
+    typedef typename num<S>::node node;
+    const int me = env.rank(), nb = P.blocks;
+    unsigned char *base = env.local();
+    const small_level<S> &D = P.lv[P.d];
+    node *bd = reinterpret_cast<node *>(base + D.bo), *zd = reinterpret_cast<node *>(base + D.zo);
+    // the tables; level t's own and halo rows of b (and z)
+    env.par([&](int tid, int nth) {
+        for (int l = P.t; l < P.d; l++) {
+            const small_level<S> &L = P.lv[l];
+            if (L.so != kNone) {
+                float4 *d = reinterpret_cast<float4 *>(base + L.so);
+                for (int k = tid; k < L.nst * 10 * num<S>::quads; k += nth) d[k] = L.st[k];
+            }
+            if (L.co != kNone) {
+                int *d = reinterpret_cast<int *>(base + L.co);
+                for (int k = tid; k < L.ncls; k += nth) d[k] = L.cls[k];
+            }
+        }
+        env.wait_input();
+        const small_level<S> &L = P.lv[P.t];
+        const window<S, true> V = band_window<FAST>(P, P.t, me, base);
+        const int y1 = band_row(P, P.t, me + 1);
+        const int lo = imax(0, V.jb), hi = imin(L.n, y1 + band_above(P, P.t));
+        const int total = (hi - lo) * L.m;
+        const divider dv(L.m);
+        for (int k = tid; k < total; k += nth) {
+            const int q = dv.quot(k), j = lo + q, w = k - q * L.m;
+            V.b[V.at(j, w)] = env.ld(L.bg + (size_t)j * L.m + w);
+            if (P.top && !P.zero_start) V.z[V.at(j, w)] = env.ld(L.zg + (size_t)j * L.m + w);
+        }
+    });
+    if (nb > 1) env.csync();  // every block runs: its shared memory may be written
+    // down
+    for (int l = P.t; l < P.d; l++) {
+        const window<S, true> V = band_window<FAST>(P, l, me, base);
+        const int y0 = band_row(P, l, me), y1 = band_row(P, l, me + 1), cm = P.lv[l + 1].m;
+        const int qn = (y1 - V.jb + band_above(P, l) + 1) >> 1;
+        const bool top = P.top && l == P.t;
+        if (FAST) {
+            const block_walk w(env.thread(), env.threads(), V.W >> 1);
+            if (top) {
+                env.par([&](int tid, int nth) {
+                    block_top_color(P.op, V, env.walk(w, tid, nth), qn, y0 - 3, y1 + 2, 0, P.zero_start != 0);
+                });
+                env.par([&](int tid, int nth) {
+                    block_top_color(P.op, V, env.walk(w, tid, nth), qn, y0 - 2, y1 + 1, 1, false);
+                });
+                env.par([&](int tid, int nth) {
+                    block_top_residual(P.op, V, env.walk(w, tid, nth), qn, y0 - 1, y1 - 1);
+                });
+            } else {
+#pragma unroll 1
+                for (int c = 0; c < 4; c++)
+                    env.par([&](int tid, int nth) {
+                        block_color(V, env.walk(w, tid, nth), qn, y0 - 2 + (c >> 1), y1 + 2 - (c >> 1), c & 1, c >> 1,
+                                    true);
+                    });
+                env.par([&](int tid, int nth) { block_residual(V, env.walk(w, tid, nth), qn, y0 - 1, y1 - 1); });
+            }
+        } else if (top) {
+            env.par([&](int tid, int nth) {
+                top_color(P.op, V, y0 - 3, y1 + 2, 0, 0, 0, P.zero_start != 0, tid, nth);
+            });
+            env.par([&](int tid, int nth) { top_color(P.op, V, y0 - 2, y1 + 1, 0, 0, 1, false, tid, nth); });
+            env.par([&](int tid, int nth) { top_residual(P.op, V, y0 - 1, y1 - 1, 0, 0, tid, nth); });
+        } else {
+            const int ncx = (V.m & 1) ? 3 : 2;
+#pragma unroll 1
+            for (int cy = 0; cy < 2; cy++)
+#pragma unroll 1
+                for (int cx = 0; cx < ncx; cx++)
+                    env.par([&](int tid, int nth) {
+                        if (ncx == 3 && cy == 0 && cx == 0) lev_clear_last(V, y0 - 2, y1 + 2, tid, nth);
+                        lev_color(V, y0 - 2 + cy, y1 + 2 - cy, 0, 0, cx, cy, true, tid, nth);
+                    });
+            env.par([&](int tid, int nth) { lev_residual(V, y0 - 1, y1 - 1, 0, 0, tid, nth); });
+        }
+        // restriction: the child's own rows, and to every block whose band
+        // (with its halo) holds the row; level d goes to all of them
+        const int J0 = band_row(P, l + 1, me), J1 = band_row(P, l + 1, me + 1);
+        env.par([&](int tid, int nth) {
+            if (l + 1 < P.d) {
+                const window<S, true> CV = band_window<FAST>(P, l + 1, me, base);
+                const int He = CV.He;
+                node *to[4];  // b of the neighbours at distance -2, -1, 1, 2, shifted to absolute rows
+                int lo[4], hi[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int c = me + (q < 2 ? q - 2 : q - 1);
+                    lo[q] = 1;
+                    hi[q] = 0;
+                    to[q] = nullptr;
+                    if (c < 0 || c >= nb) continue;
+                    lo[q] = band_row(P, l + 1, c) - kLevBelow;
+                    hi[q] = band_row(P, l + 1, c + 1) + kLevAbove - 2;  // the last row a sweep reads
+                    if (lo[q] >= J1 || hi[q] < J0) hi[q] = lo[q] - 1;
+                    else to[q] = reinterpret_cast<node *>(env.base(c) + P.lv[l + 1].bo);
+                }
+                auto out = [&](int J, int I, node v) {
+                    const int c = (I & 1) * He + (I >> 1);
+                    CV.b[(J - CV.jb) * cm + c] = v;
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (J >= lo[q] && J <= hi[q]) to[q][(J - lo[q]) * cm + c] = v;
+                };
+                if (FAST) block_restrict(V, block_walk(tid, nth, V.W >> 1), qn, J0, J1 - 1, out);
+                else restrict_rows(V, J0, J1 - 1, 0, cm - 1, cm, out, tid, nth);
+            } else {
+                auto out = [&](int J, int I, node v) {
+                    for (int c = 0; c < nb; c++)
+                        reinterpret_cast<node *>((c == me ? base : env.base(c)) + D.bo)[J * cm + I] = v;
+                };
+                if (FAST) block_restrict(V, block_walk(tid, nth, V.W >> 1), qn, J0, J1 - 1, out);
+                else restrict_rows(V, J0, J1 - 1, 0, cm - 1, cm, out, tid, nth);
+            }
+        });
+        if (nb > 1) env.csync();
+    }
+    // level d: z = M b, a group of threads per row, the result to every block
+    env.par([&](int tid, int nth) {
+        const int nd = D.m * D.n, r0 = 2 * (int)((long)nd * me / nb), r1 = 2 * (int)((long)nd * (me + 1) / nb);
+        const int lane = tid % E::kLanes;
+        for (int r = r0 + tid / E::kLanes; r < r1; r += nth / E::kLanes) {
+            const float4 *row = P.dense + (size_t)r * nd;
+            const S v = from_pair(env.lane_sum(dense_share<E::kLanes, S>(row, bd, nd, lane)), S());
+            for (int c = lane; c < nb; c += E::kLanes) {
+                node *z = reinterpret_cast<node *>((c == me ? base : env.base(c)) + D.zo) + (r >> 1);
+                if (r & 1) put_y(z, v);
+                else put_x(z, v);
+            }
+        }
+    });
+    if (nb > 1) env.csync();
+    // up
+    for (int l = P.d - 1; l >= P.t; l--) {
+        const window<S, true> V = band_window<FAST>(P, l, me, base);
+        const int y0 = band_row(P, l, me), y1 = band_row(P, l, me + 1), cm = P.lv[l + 1].m;
+        const int qn = (y1 - V.jb + band_above(P, l) + 1) >> 1;
+        const bool top = P.top && l == P.t, last = l + 1 == P.d;
+        const window<S, true> CV = band_window<FAST>(P, l + 1, me, base);
+        const int J0 = band_row(P, l + 1, me), J1 = band_row(P, l + 1, me + 1), cHe = CV.He;
+        const node *halo = last ? nullptr : reinterpret_cast<const node *>(base + P.lv[l + 1].ho);
+        auto crow = [&](int J) -> const node * {
+            if (last) return zd + J * cm;
+            if (J < J0) return halo;
+            if (J >= J1) return halo + (1 + J - J1) * cm;
+            return CV.z + (J - CV.jb) * cm;
+        };
+        auto ccol = [&](int I) { return last ? I : (I & 1) * cHe + (I >> 1); };
+        if (FAST) {
+            const block_walk w(env.thread(), env.threads(), V.W >> 1);
+            env.par([&](int tid, int nth) {
+                block_prolong(V, env.walk(w, tid, nth), qn, y0 - (top ? 2 : 1), y1 + 1, crow, ccol);
+            });
+            if (top) {
+                env.par([&](int tid, int nth) {
+                    block_top_color(P.op, V, env.walk(w, tid, nth), qn, y0 - 1, y1, 0, false);
+                });
+                env.par([&](int tid, int nth) {
+                    block_top_color(P.op, V, env.walk(w, tid, nth), qn, y0, y1 - 1, 1, false);
+                });
+            } else {
+#pragma unroll 1
+                for (int c = 0; c < 4; c++)
+                    env.par([&](int tid, int nth) {
+                        block_color(V, env.walk(w, tid, nth), qn, y0, y1 - (c >> 1), c & 1, c >> 1, false);
+                    });
+            }
+        } else {
+            env.par([&](int tid, int nth) {
+                prolong_rows(V, y0 - (top ? 2 : 1), y1 + 1, 0, 0, cm,
+                             [&](int J, int I) -> node { return crow(J)[ccol(I)]; }, tid, nth);
+            });
+            if (top) {
+                env.par([&](int tid, int nth) { top_color(P.op, V, y0 - 1, y1, 0, 0, 0, false, tid, nth); });
+                env.par([&](int tid, int nth) { top_color(P.op, V, y0, y1 - 1, 0, 0, 1, false, tid, nth); });
+            } else {
+                const int ncx = (V.m & 1) ? 3 : 2;
+#pragma unroll 1
+                for (int cy = 0; cy < 2; cy++)
+#pragma unroll 1
+                    for (int cx = 0; cx < ncx; cx++)
+                        env.par([&](int tid, int nth) {
+                            lev_color(V, y0, y1 - cy, 0, 0, cx, cy, false, tid, nth);
+                        });
+            }
+        }
+        if (l == P.t) {
+            env.par([&](int tid, int nth) {
+                const int total = (y1 - y0) * V.m;
+                const divider dv(V.m);
+                for (int k = tid; k < total; k += nth) {
+                    const int q = dv.quot(k), w = k - q * V.m;
+                    env.store(P, (size_t)(y0 + q) * V.m + w, V.z[V.at(y0 + q, w)]);
+                }
+            });
+        } else if (nb > 1) {
+            // rows next to the band's edges, for the neighbours' prolongation
+            env.par([&](int tid, int nth) {
+                const int m = V.m;
+                node *lo = me > 0 ? reinterpret_cast<node *>(env.base(me - 1) + P.lv[l].ho) : nullptr;
+                node *hi = me + 1 < nb ? reinterpret_cast<node *>(env.base(me + 1) + P.lv[l].ho) : nullptr;
+                for (int k = tid; k < m; k += nth) {
+                    if (lo) {
+                        lo[m + k] = V.z[(y0 - V.jb) * m + k];
+                        lo[2 * m + k] = V.z[(y0 + 1 - V.jb) * m + k];
+                    }
+                    if (hi) hi[k] = V.z[(y1 - 1 - V.jb) * m + k];
+                }
+            });
+            env.csync();
+        }
+    }
+}
+
+}  // namespace mgw
+}  // namespace stzg
