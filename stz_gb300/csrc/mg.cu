@@ -2182,8 +2182,9 @@ __device__ void tail_pairs_body(const tail_levels &tl, const hierarchy_view<floa
         const pair_level B = pair_view(tail_raw, offs, tl.d);
         const int nd = S[tl.d].m * S[tl.d].n;
         for (int r = w; r < 2 * nd; r += nw) {
-            const ff v = mgw::warp_pair_sum(
-                mgw::dense_share<32, float>(tl.dense + (size_t)r * nd, B.b2, nd, lane));
+            ff share[1];
+            mgw::dense_share<32, 1, float>(tl.dense + (size_t)r * nd, 0, 1, B.b2, nd, lane, share);
+            const ff v = mgw::warp_pair_sum(share[0]);
             if (lane == 0) {
                 if (r & 1) B.z2[r >> 1].y = v.hi + v.lo;
                 else B.z2[r >> 1].x = v.hi + v.lo;

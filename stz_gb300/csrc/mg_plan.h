@@ -8,7 +8,7 @@ namespace stzg {
 namespace mgw {
 
 // Fills the offsets of P for levels t..d (their sizes, classes and stencil
-// counts already in P.lv) over `blocks` blocks with at most max_bytes of
+// counts already in P.lv) over `blocks` blocks (a power of two) with at most max_bytes of
 // shared memory each; false where it does not fit.  Every block needs a row
 // of level d, so that the bands above have the two rows their neighbours'
 // halos read.
@@ -17,6 +17,8 @@ template <typename S> bool layout_small(small_plan<S> &P, int t, int d, int bloc
     P.t = t;
     P.d = d;
     P.blocks = blocks;
+    P.shift = 0;
+    while ((1 << P.shift) < blocks) P.shift++;
     if (t >= d || (blocks > 1 && P.lv[d].n < blocks)) return false;
     unsigned off = 0;
     auto place = [&](unsigned long bytes) {
@@ -26,6 +28,7 @@ template <typename S> bool layout_small(small_plan<S> &P, int t, int d, int bloc
     };
     const unsigned long nd = (unsigned long)P.lv[d].m * P.lv[d].n;
     if (nd * sizeof(node) * 2 > max_bytes) return false;
+    P.lv[d].ps = (int)nd;
     P.lv[d].zo = place(nd * sizeof(node));
     P.lv[d].bo = place(nd * sizeof(node));
     P.lv[d].ho = P.lv[d].so = P.lv[d].co = kNone;
@@ -40,14 +43,16 @@ template <typename S> bool layout_small(small_plan<S> &P, int t, int d, int bloc
         const int rows = (own + band_below(P, l) + band_above(P, l) + 1) & ~1;
         const unsigned long nodes = (unsigned long)L.m * rows;
         if (nodes * sizeof(node) * 2 > max_bytes) return false;
+        L.ps = (int)nodes;
         L.zo = place(nodes * sizeof(node));
         L.bo = place(nodes * sizeof(node));
         L.ho = l > t ? place(3ul * L.m * sizeof(node)) : kNone;
-        const unsigned long rb = (unsigned long)L.m * (own + 1) * sizeof(node);
+        const unsigned long rb = (unsigned long)L.m * (own + 1);
         if (rb > rmax) rmax = rb;
         if (off > max_bytes) return false;
     }
-    P.ro = place(rmax);
+    P.rs = (int)rmax;
+    P.ro = place(rmax * sizeof(node));
     if (off > max_bytes) return false;
     // tables: small ones in shared memory (one class per row, a few stencils)
     for (int l = t; l < d; l++) {
@@ -86,6 +91,38 @@ template <typename F> int dense_level(int ml, F nodes) {
     int d = ml;
     while (d > 1 && nodes(d - 1) <= kDenseNodes) d--;
     return d;
+}
+
+// Tile of a wide level: coarse columns and rows, threads, shared memory of one
+// launch.  top: 0 a coarse level, 1 the top level down, 2 up; bands: whole
+// rows.  A row of blocks is a warp's; 16, 8 or 4 of them per tile, the most
+// that still gives three blocks per SM (the halo of a tile of 14, 6 or 2
+// coarse rows costs 1.14, 1.33 or 2 times the rows).
+struct tile_shape {
+    int tw, th, threads;
+    unsigned long bytes;
+};
+inline tile_shape shape_tile(int m, int cm, int cn, int table, int top, bool bands, unsigned long max_bytes) {
+    const int extra = top == 1 ? 3 : 2;
+    tile_shape T;
+    T.threads = 256;
+    auto bytes = [&] {
+        const unsigned long W = bands ? m : 64, cw = bands ? cm : 33;
+        return W * 2 * (T.th + extra) * 32 + table + cw * (T.th + 3) * 16;
+    };
+    if (bands) {
+        T.tw = cm;
+        for (T.th = 4; T.th > 2 && (bytes() > max_bytes || (cn + T.th - 1) / T.th < 152); T.th >>= 1) {}
+    } else {
+        T.tw = top == 1 ? 29 : (top == 2 ? 30 : 28);
+        for (int rows = 16; rows >= 4; rows >>= 1) {
+            T.th = rows - extra;
+            T.threads = rows >= 8 ? 256 : 128;
+            if ((long)((cm + T.tw - 1) / T.tw) * ((cn + T.th - 1) / T.th) >= 3 * 152) break;
+        }
+    }
+    T.bytes = bytes();
+    return T;
 }
 
 }  // namespace mgw

@@ -278,9 +278,10 @@ template <typename S> void launch_small(const small_plan<S> &P, cudaStream_t st)
 
 constexpr size_t kTileMax = 200 * 1024;
 
-// Geometry of a wide level's tiles; false where not even the smallest fits.
-bool plan_tile(const hierarchy<double> &h, int l, tile_level &L, bool &wrap, size_t &down, size_t &up) {
+// A wide level's arrays and tiles on the way down (up = false) or up.
+tile_level plan_tile(const hierarchy<double> &h, int l, bool up, bool &bands, size_t &bytes) {
     const level_view<double> &A = h.lv[l], &C = h.lv[l + 1];
+    tile_level L;
     std::memset(&L, 0, sizeof(L));
     L.m = A.m;
     L.n = A.n;
@@ -296,35 +297,21 @@ bool plan_tile(const hierarchy<double> &h, int l, tile_level &L, bool &wrap, siz
     L.zup = reinterpret_cast<float4 *>(A.z);
     L.bc = reinterpret_cast<float4 *>(C.b);
     L.zc = reinterpret_cast<const float4 *>(C.z);
-    wrap = l && ((A.m & 1) || !A.homog);
-    const size_t tab = L.staged ? (size_t)A.nst * 320 : 0;
-    auto bytes = [&](bool u) {
-        const size_t W = wrap ? L.m : 2 * L.tw + 8, rows = 2 * L.th + 5;
-        const size_t cw = wrap ? L.cm : L.tw + 5;
-        return 32 * W * rows + tab + (u ? 16 * cw * (L.th + 3) : 0);
-    };
-    if (wrap) {
-        L.tw = L.cm;
-        for (L.th = 4; L.th > 1 && (bytes(true) > kTileMax || (L.th > 2 && ceil_div(L.cn, L.th) < 152)); L.th >>= 1) {}
-    } else {
-        // the largest tile that still gives two blocks per SM
-        const int shapes[4][2] = {{32, 8}, {16, 8}, {16, 4}, {8, 4}};
-        for (int k = 0; k < 4; k++) {
-            L.tw = shapes[k][0];
-            L.th = shapes[k][1];
-            if ((long)ceil_div(L.cm, L.tw) * ceil_div(L.cn, L.th) >= 2 * 152) break;
-        }
-    }
-    down = bytes(false);
-    up = bytes(true);
-    return up <= kTileMax;
+    if (!l) L.sum = h.lv[0].z;
+    bands = l && ((A.m & 1) || !A.homog);
+    const tile_shape T = shape_tile(L.m, L.cm, L.cn, L.staged ? A.nst * 320 : 0, l ? 0 : (up ? 2 : 1), bands, kTileMax);
+    L.tw = T.tw;
+    L.th = T.th;
+    L.threads = T.threads;
+    bytes = T.bytes;
+    return L;
 }
 
 template <typename... K, typename... A>
-void launch_tile(void (*kern)(K...), const tile_level &L, bool wrap, size_t smem, cudaStream_t st, A... args) {
+void launch_tile(void (*kern)(K...), const tile_level &L, bool bands, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(wrap ? 1 : ceil_div(L.cm, L.tw), ceil_div(L.cn, L.th));
-    cfg.blockDim = dim3(kTileThreads);
+    cfg.gridDim = dim3(bands ? 1 : ceil_div(L.cm, L.tw), ceil_div(L.cn, L.th));
+    cfg.blockDim = dim3(L.threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -405,10 +392,10 @@ bool pair_cycle_supported(const hierarchy<double> &h) {
     small_plan<ff> P;
     if (!choose_small(h, true, P)) return false;
     for (int l = 0; l < P.t; l++) {
-        tile_level L;
-        bool wrap;
-        size_t d, u;
-        if (!plan_tile(h, l, L, wrap, d, u)) return false;
+        bool bands;
+        size_t bytes;
+        plan_tile(h, l, true, bands, bytes);
+        if (bytes > kTileMax) return false;
     }
     return true;
 }
@@ -426,13 +413,12 @@ void pair_cycle(const hierarchy<double> &h, cudaStream_t st) {
     if (!choose_small(h, true, P)) return;
     const top_consts<ff> op = consts_of(h.op);
     for (int l = 0; l < P.t; l++) {
-        tile_level L;
-        bool wrap;
-        size_t d, u;
-        plan_tile(h, l, L, wrap, d, u);
-        if (l == 0) launch_tile(k_pair_top_down, L, false, d, st, op, L);
-        else if (wrap) launch_tile(k_pair_lev_down<true>, L, true, d, st, L);
-        else launch_tile(k_pair_lev_down<false>, L, false, d, st, L);
+        bool bands;
+        size_t bytes;
+        const tile_level L = plan_tile(h, l, false, bands, bytes);
+        if (l == 0) launch_tile(k_pair_top_down, L, false, bytes, st, op, L);
+        else if (bands) launch_tile(k_pair_lev_down<true>, L, true, bytes, st, L);
+        else launch_tile(k_pair_lev_down<false>, L, false, bytes, st, L);
     }
     if (P.t == 0) {
         P.lv[0].bg = reinterpret_cast<const float4 *>(h.lv[0].r);
@@ -440,15 +426,12 @@ void pair_cycle(const hierarchy<double> &h, cudaStream_t st) {
     }
     launch_small(P, st);
     for (int l = P.t - 1; l >= 0; l--) {
-        tile_level L;
-        bool wrap;
-        size_t d, u;
-        plan_tile(h, l, L, wrap, d, u);
-        if (l == 0) {
-            L.sum = h.lv[0].z;
-            launch_tile(k_pair_top_up, L, false, u, st, op, L);
-        } else if (wrap) launch_tile(k_pair_lev_up<true>, L, true, u, st, L);
-        else launch_tile(k_pair_lev_up<false>, L, false, u, st, L);
+        bool bands;
+        size_t bytes;
+        const tile_level L = plan_tile(h, l, true, bands, bytes);
+        if (l == 0) launch_tile(k_pair_top_up, L, false, bytes, st, op, L);
+        else if (bands) launch_tile(k_pair_lev_up<true>, L, true, bytes, st, L);
+        else launch_tile(k_pair_lev_up<false>, L, false, bytes, st, L);
     }
 }
 

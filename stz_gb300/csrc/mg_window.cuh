@@ -50,14 +50,23 @@ MGW_FN val2<float> get(const float2 &p) { return val2<float>{p.x, p.y}; }
 MGW_FN val2<ff> get(const float4 &p) { return val2<ff>{ff{p.x, p.z}, ff{p.y, p.w}}; }
 MGW_FN float2 put(const val2<float> &v) { return make_float2(v.x, v.y); }
 MGW_FN float4 put(const val2<ff> &v) { return make_float4(v.x.hi, v.y.hi, v.x.lo, v.y.lo); }
-MGW_FN float get_x(const float2 *p) { return p->x; }
-MGW_FN float get_y(const float2 *p) { return p->y; }
-MGW_FN ff get_x(const float4 *p) { return ff{p->x, p->z}; }
-MGW_FN ff get_y(const float4 *p) { return ff{p->y, p->w}; }
-MGW_FN void put_x(float2 *p, float v) { p->x = v; }
-MGW_FN void put_y(float2 *p, float v) { p->y = v; }
-MGW_FN void put_x(float4 *p, ff v) { p->x = v.hi; p->z = v.lo; }
-MGW_FN void put_y(float4 *p, ff v) { p->y = v.hi; p->w = v.lo; }
+
+// Nodes in shared memory: the x components, then the y ones, so that a sweep
+// over one component (the top level's) reads consecutive words.
+template <typename S> struct plane {
+    S *p;    // x; y at p + ps
+    int ps;
+    MGW_FN plane operator+(int k) const { return plane{p + k, ps}; }
+    MGW_FN S x(int k) const { return p[k]; }
+    MGW_FN S y(int k) const { return p[k + ps]; }
+    MGW_FN void set_x(int k, S v) const { p[k] = v; }
+    MGW_FN void set_y(int k, S v) const { p[k + ps] = v; }
+    MGW_FN val2<S> get(int k) const { return val2<S>{p[k], p[k + ps]}; }
+    MGW_FN void set(int k, const val2<S> &v) const {
+        p[k] = v.x;
+        p[k + ps] = v.y;
+    }
+};
 
 MGW_FN float add(float a, float b) { return a + b; }
 MGW_FN ff add(ff a, ff b) { return ff_add(a, b); }
@@ -121,8 +130,7 @@ MGW_FN ff three(ff k1, ff s1, ff k2, ff s2, ff k3, ff s3) {
 // ---- windows -----------------------------------------------------------------
 
 template <typename S, bool WRAP> struct window {
-    typedef typename num<S>::node node;
-    node *z, *b, *r;
+    plane<S> z, b, r;
     int W, He;          // columns; even ones
     int jb, rb;         // rows of local row 0 of z and b; of r
     int m, n;           // the level
@@ -190,18 +198,18 @@ MGW_FN void offdiag(const window<S, WRAP> &V, const float4 *s, int j, int w, boo
                     typename acc_of<S>::type &ax, typename acc_of<S>::type &ay) {
     const int wl = V.left(w), wr = V.right(w);
     if (rows && j > 0) {
-        madd(ax, ay, s, 0, get(V.z[V.at(j - 1, wl)]));
-        madd(ax, ay, s, 1, get(V.z[V.at(j - 1, w)]));
-        madd(ax, ay, s, 2, get(V.z[V.at(j - 1, wr)]));
+        madd(ax, ay, s, 0, V.z.get(V.at(j - 1, wl)));
+        madd(ax, ay, s, 1, V.z.get(V.at(j - 1, w)));
+        madd(ax, ay, s, 2, V.z.get(V.at(j - 1, wr)));
     }
     if (mid) {
-        madd(ax, ay, s, 3, get(V.z[V.at(j, wl)]));
-        madd(ax, ay, s, 5, get(V.z[V.at(j, wr)]));
+        madd(ax, ay, s, 3, V.z.get(V.at(j, wl)));
+        madd(ax, ay, s, 5, V.z.get(V.at(j, wr)));
     }
     if (rows && j < V.n - 1) {
-        madd(ax, ay, s, 6, get(V.z[V.at(j + 1, wl)]));
-        madd(ax, ay, s, 7, get(V.z[V.at(j + 1, w)]));
-        madd(ax, ay, s, 8, get(V.z[V.at(j + 1, wr)]));
+        madd(ax, ay, s, 6, V.z.get(V.at(j + 1, wl)));
+        madd(ax, ay, s, 7, V.z.get(V.at(j + 1, w)));
+        madd(ax, ay, s, 8, V.z.get(V.at(j + 1, wr)));
     }
 }
 
@@ -237,8 +245,8 @@ MGW_FN void lev_color(const window<S, WRAP> &V, int jlo, int jhi, int wlo, int w
         typename acc_of<S>::type ax, ay;
         offdiag(V, s, j, w, !(from_zero && cy == 0), !(from_zero && cx == 0), ax, ay);
         const int c = V.at(j, w);
-        const val2<S> bb = get(V.b[c]);
-        V.z[c] = put(apply(s, 9, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())}));
+        const val2<S> bb = V.b.get(c);
+        V.z.set(c, apply(s, 9, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())}));
     }
 }
 
@@ -250,7 +258,7 @@ MGW_FN void lev_clear_last(const window<S, WRAP> &V, int jlo, int jhi, int tid, 
     jhi = imin(jhi, V.n - 1);
     for (int j = jlo + tid; j <= jhi; j += nth) {
         val2<S> o{};
-        V.z[V.at(j, V.W - 1)] = put(o);
+        V.z.set(V.at(j, V.W - 1), o);
     }
 }
 
@@ -276,11 +284,11 @@ MGW_FN void lev_residual(const window<S, WRAP> &V, int jlo, int jhi, int wlo, in
             typename acc_of<S>::type ax, ay;
             offdiag(V, s, j, w, true, true, ax, ay);
             const int c = V.at(j, w);
-            madd(ax, ay, s, 4, get(V.z[c]));
-            const val2<S> bb = get(V.b[c]);
+            madd(ax, ay, s, 4, V.z.get(c));
+            const val2<S> bb = V.b.get(c);
             o = val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())};
         }
-        V.r[V.rat(j, w)] = put(o);
+        V.r.set(V.rat(j, w), o);
     }
 }
 
@@ -288,18 +296,18 @@ MGW_FN void lev_residual(const window<S, WRAP> &V, int jlo, int jhi, int wlo, in
 template <typename S, bool WRAP>
 MGW_FN S top_off_x(const top_consts<S> &o, const window<S, WRAP> &V, int j, int w) {
     const int wl = V.left(w), wr = V.right(w);
-    return three(o.Kmx, sum2(get_x(V.z + V.at(j, wl)), get_x(V.z + V.at(j, wr))), o.my,
-                 sum2(get_x(V.z + V.at(j - 1, w)), get_x(V.z + V.at(j + 1, w))), o.qK,
-                 cross4(get_y(V.z + V.at(j - 1, wl)), get_y(V.z + V.at(j + 1, wr)), get_y(V.z + V.at(j - 1, wr)),
-                        get_y(V.z + V.at(j + 1, wl))));
+    return three(o.Kmx, sum2(V.z.x(V.at(j, wl)), V.z.x(V.at(j, wr))), o.my,
+                 sum2(V.z.x(V.at(j - 1, w)), V.z.x(V.at(j + 1, w))), o.qK,
+                 cross4(V.z.y(V.at(j - 1, wl)), V.z.y(V.at(j + 1, wr)), V.z.y(V.at(j - 1, wr)),
+                        V.z.y(V.at(j + 1, wl))));
 }
 template <typename S, bool WRAP>
 MGW_FN S top_off_y(const top_consts<S> &o, const window<S, WRAP> &V, int j, int w) {
     const int wl = V.left(w), wr = V.right(w);
-    return three(o.mx, sum2(get_y(V.z + V.at(j, wl)), get_y(V.z + V.at(j, wr))), o.Kmy,
-                 sum2(get_y(V.z + V.at(j - 1, w)), get_y(V.z + V.at(j + 1, w))), o.qK,
-                 cross4(get_x(V.z + V.at(j - 1, wl)), get_x(V.z + V.at(j + 1, wr)), get_x(V.z + V.at(j - 1, wr)),
-                        get_x(V.z + V.at(j + 1, wl))));
+    return three(o.mx, sum2(V.z.y(V.at(j, wl)), V.z.y(V.at(j, wr))), o.Kmy,
+                 sum2(V.z.y(V.at(j - 1, w)), V.z.y(V.at(j + 1, w))), o.qK,
+                 cross4(V.z.x(V.at(j - 1, wl)), V.z.x(V.at(j + 1, wr)), V.z.x(V.at(j - 1, wr)),
+                        V.z.x(V.at(j + 1, wl))));
 }
 
 // One colour of the top level: a thread takes a pair of columns, the x
@@ -324,17 +332,17 @@ MGW_FN void top_color(const top_consts<S> &o, const window<S, WRAP> &V, int jlo,
         const bool wall = j == 0 || j == V.n - 1;
         if (wx >= wlo && wx <= whi) {
             const int c = V.at(j, wx);
-            const S bb = get_x(V.b + c);
-            if (wall) put_x(V.z + c, mul(o.ibcxx, bb));
-            else if (from_zero) put_x(V.z + c, mul(o.icxx, bb));
-            else put_x(V.z + c, mul(o.icxx, sub(bb, top_off_x(o, V, j, wx))));
+            const S bb = V.b.x(c);
+            if (wall) V.z.set_x(c, mul(o.ibcxx, bb));
+            else if (from_zero) V.z.set_x(c, mul(o.icxx, bb));
+            else V.z.set_x(c, mul(o.icxx, sub(bb, top_off_x(o, V, j, wx))));
         }
         if (wy >= wlo && wy <= whi) {
             const int c = V.at(j, wy);
-            const S bb = get_y(V.b + c);
-            if (wall) put_y(V.z + c, mul(o.ibcyy, bb));
-            else if (from_zero) put_y(V.z + c, mul(o.icyy, bb));
-            else put_y(V.z + c, mul(o.icyy, sub(bb, top_off_y(o, V, j, wy))));
+            const S bb = V.b.y(c);
+            if (wall) V.z.set_y(c, mul(o.ibcyy, bb));
+            else if (from_zero) V.z.set_y(c, mul(o.icyy, bb));
+            else V.z.set_y(c, mul(o.icyy, sub(bb, top_off_y(o, V, j, wy))));
         }
     }
 }
@@ -360,14 +368,14 @@ MGW_FN void top_residual(const top_consts<S> &o, const window<S, WRAP> &V, int j
         if (wx >= wlo && wx <= whi) {
             const int c = V.at(j, wx);
             val2<S> r{};
-            if (!wall) r.x = sub(sub(get_x(V.b + c), top_off_x(o, V, j, wx)), mul(o.cxx, get_x(V.z + c)));
-            V.r[V.rat(j, wx)] = put(r);
+            if (!wall) r.x = sub(sub(V.b.x(c), top_off_x(o, V, j, wx)), mul(o.cxx, V.z.x(c)));
+            V.r.set(V.rat(j, wx), r);
         }
         if (wy >= wlo && wy <= whi) {
             const int c = V.at(j, wy);
             val2<S> r{};
-            if (!wall) r.y = sub(sub(get_y(V.b + c), top_off_y(o, V, j, wy)), mul(o.cyy, get_y(V.z + c)));
-            V.r[V.rat(j, wy)] = put(r);
+            if (!wall) r.y = sub(sub(V.b.y(c), top_off_y(o, V, j, wy)), mul(o.cyy, V.z.y(c)));
+            V.r.set(V.rat(j, wy), r);
         }
     }
 }
@@ -403,20 +411,20 @@ MGW_FN void restrict_rows(const window<S, WRAP> &V, int Jlo, int Jhi, int Ilo, i
             const int fy = 2 * J + q - 1;
             const float w1 = (float)hy * 0.25f, w2 = (float)(2 * hy) * 0.25f;
             if (hl) {
-                const val2<S> v = get(V.r[V.rat(fy, V.left(w))]);
+                const val2<S> v = V.r.get(V.rat(fy, V.left(w)));
                 a.x = add(a.x, scale(v.x, w1));
                 a.y = add(a.y, scale(v.y, w1));
             }
-            const val2<S> c = get(V.r[V.rat(fy, w)]);
+            const val2<S> c = V.r.get(V.rat(fy, w));
             a.x = add(a.x, scale(c.x, w2));
             a.y = add(a.y, scale(c.y, w2));
             if (hr) {
-                const val2<S> v = get(V.r[V.rat(fy, V.right(w))]);
+                const val2<S> v = V.r.get(V.rat(fy, V.right(w)));
                 a.x = add(a.x, scale(v.x, w1));
                 a.y = add(a.y, scale(v.y, w1));
             }
         }
-        out(J, I, put(a));
+        out(J, I, a);
     }
 }
 
@@ -445,21 +453,21 @@ MGW_FN void prolong_rows(const window<S, WRAP> &V, int jlo, int jhi, int wlo, in
             const int I1 = WRAP && I + 1 == cm ? 0 : I + 1;
             for (int q = 0; q < ny; q++) {
                 const float wy = (float)hy[q] * 0.25f;
-                const val2<S> v0 = get(zc(cy[q], I)), v1 = get(zc(cy[q], I1));
+                const val2<S> v0 = zc(cy[q], I), v1 = zc(cy[q], I1);
                 a.x = add(a.x, scale(add(v0.x, v1.x), wy));
                 a.y = add(a.y, scale(add(v0.y, v1.y), wy));
             }
         } else {
             for (int q = 0; q < ny; q++) {
                 const float wy = (float)hy[q] * 0.25f;
-                const val2<S> v0 = get(zc(cy[q], I));
+                const val2<S> v0 = zc(cy[q], I);
                 a.x = add(a.x, scale(v0.x, 2.f * wy));
                 a.y = add(a.y, scale(v0.y, 2.f * wy));
             }
         }
         const int c = V.at(j, w);
-        const val2<S> f = get(V.z[c]);
-        V.z[c] = put(val2<S>{add(f.x, a.x), add(f.y, a.y)});
+        const val2<S> f = V.z.get(c);
+        V.z.set(c, val2<S>{add(f.x, a.x), add(f.y, a.y)});
     }
 }
 
@@ -500,21 +508,21 @@ struct columns3 {
 };
 
 template <typename S>
-MGW_FN void offdiag3(const float4 *s, const typename num<S>::node *row, int W, const columns3 &c, bool dn, bool mid,
+MGW_FN void offdiag3(const float4 *s, const plane<S> &row, int W, const columns3 &c, bool dn, bool mid,
                      bool up, typename acc_of<S>::type &ax, typename acc_of<S>::type &ay) {
     if (dn) {
-        madd(ax, ay, s, 0, get(row[c.l - W]));
-        madd(ax, ay, s, 1, get(row[c.c - W]));
-        madd(ax, ay, s, 2, get(row[c.r - W]));
+        madd(ax, ay, s, 0, row.get(c.l - W));
+        madd(ax, ay, s, 1, row.get(c.c - W));
+        madd(ax, ay, s, 2, row.get(c.r - W));
     }
     if (mid) {
-        madd(ax, ay, s, 3, get(row[c.l]));
-        madd(ax, ay, s, 5, get(row[c.r]));
+        madd(ax, ay, s, 3, row.get(c.l));
+        madd(ax, ay, s, 5, row.get(c.r));
     }
     if (up) {
-        madd(ax, ay, s, 6, get(row[c.l + W]));
-        madd(ax, ay, s, 7, get(row[c.c + W]));
-        madd(ax, ay, s, 8, get(row[c.r + W]));
+        madd(ax, ay, s, 6, row.get(c.l + W));
+        madd(ax, ay, s, 7, row.get(c.c + W));
+        madd(ax, ay, s, 8, row.get(c.r + W));
     }
 }
 
@@ -529,37 +537,37 @@ MGW_FN void block_color(const window<S, true> &V, block_walk w, int qn, int jlo,
         if (j < jlo || j > jhi) continue;
         const float4 *s = V.st + V.cls[j] * (10 * num<S>::quads);
         const columns3 c(w.k, w.P, cx);
-        typename num<S>::node *row = V.z + lr * V.W;
+        const plane<S> row = V.z + lr * V.W;
         const bool rows = !(from_zero && cy == 0);
-        const val2<S> bb = get(V.b[lr * V.W + c.c]);
+        const val2<S> bb = V.b.get(lr * V.W + c.c);
         typename acc_of<S>::type ax, ay;
         offdiag3<S>(s, row, V.W, c, rows && j > 0, !(from_zero && cx == 0), rows && j < V.n - 1, ax, ay);
-        row[c.c] = put(apply(s, 9, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())}));
+        row.set(c.c, apply(s, 9, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())}));
     }
 }
 
-// Residual of the rows jlo..jhi (the odd columns of odd rows: zero).
-template <typename S> MGW_FN void block_residual(const window<S, true> &V, block_walk w, int qn, int jlo, int jhi) {
+// Residual of the rows jlo..jhi (the odd columns of odd rows: zero): the three
+// points of a block on different threads.
+template <typename S>
+MGW_FN void block_residual(const window<S, true> &V, int P, int qn, int jlo, int jhi, int tid, int nth) {
     jlo = imax(jlo, 0);
     jhi = imin(jhi, V.n - 1);
-    for (; w.q < qn; w.next()) {
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int cx = e & 1, cy = e >> 1, lr = 2 * w.q + cy, j = V.jb + lr;
-            if (j < jlo || j > jhi) continue;
-            const columns3 c(w.k, w.P, cx);
-            val2<S> o{};
-            if (e < 3) {
-                const float4 *s = V.st + V.cls[j] * (10 * num<S>::quads);
-                const typename num<S>::node *row = V.z + lr * V.W;
-                const val2<S> bb = get(V.b[lr * V.W + c.c]);
-                typename acc_of<S>::type ax, ay;
-                offdiag3<S>(s, row, V.W, c, j > 0, true, j < V.n - 1, ax, ay);
-                madd(ax, ay, s, 4, get(row[c.c]));
-                o = val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())};
-            }
-            V.r[(j - V.rb) * V.W + c.c] = put(o);
-        }
+    const int blocks = P * qn;
+    const divider dv(P);
+    for (int t = tid; t < 3 * blocks; t += nth) {
+        const int e = t >= 2 * blocks ? 2 : (t >= blocks ? 1 : 0), i = t - e * blocks, q = dv.quot(i), k = i - q * P;
+        const int cx = e & 1, cy = e >> 1, lr = 2 * q + cy, j = V.jb + lr;
+        if (j < jlo || j > jhi) continue;
+        const columns3 c(k, P, cx);
+        const float4 *s = V.st + V.cls[j] * (10 * num<S>::quads);
+        const plane<S> row = V.z + lr * V.W;
+        const val2<S> bb = V.b.get(lr * V.W + c.c);
+        typename acc_of<S>::type ax, ay;
+        offdiag3<S>(s, row, V.W, c, j > 0, true, j < V.n - 1, ax, ay);
+        madd(ax, ay, s, 4, row.get(c.c));
+        const plane<S> r = V.r + (j - V.rb) * V.W;
+        r.set(c.c, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())});
+        if (cy) r.set(P + k, val2<S>{});
     }
 }
 
@@ -576,9 +584,9 @@ MGW_FN void block_restrict(const window<S, true> &V, block_walk w, int qn, int J
         for (int q = 0; q < 3; q++) {
             const int hy = row_halves(q, J, V.n);
             if (!hy) continue;
-            const typename num<S>::node *row = V.r + (2 * J + q - 1 - V.rb) * V.W;
+            const plane<S> row = V.r + (2 * J + q - 1 - V.rb) * V.W;
             const float w1 = (float)hy * 0.25f, w2 = (float)(2 * hy) * 0.25f;
-            const val2<S> l = get(row[c.l]), m = get(row[c.c]), r = get(row[c.r]);
+            const val2<S> l = row.get(c.l), m = row.get(c.c), r = row.get(c.r);
             a.x = add(a.x, scale(l.x, w1));
             a.y = add(a.y, scale(l.y, w1));
             a.x = add(a.x, scale(m.x, w2));
@@ -586,45 +594,45 @@ MGW_FN void block_restrict(const window<S, true> &V, block_walk w, int qn, int J
             a.x = add(a.x, scale(r.x, w1));
             a.y = add(a.y, scale(r.y, w1));
         }
-        out(J, w.k, put(a));
+        out(J, w.k, a);
     }
 }
 
-// Prolongation on the rows jlo..jhi: crow(J) is the child's row J (natural or
-// parity-major, col(I) its column).
-template <typename S, typename Row, typename Col>
-MGW_FN void block_prolong(const window<S, true> &V, block_walk w, int qn, int jlo, int jhi, Row crow, Col col) {
-    typedef typename num<S>::node node;
+// Prolongation on the rows jlo..jhi: crow(J) is the child's row J, col(k) and
+// next(k) the places in it of the columns under block k and right of it.
+template <typename S, typename Row, typename Col, typename Next>
+MGW_FN void block_prolong(const window<S, true> &V, block_walk w, int qn, int jlo, int jhi, Row crow, Col col,
+                          Next next) {
     jlo = imax(jlo, 0);
     jhi = imin(jhi, V.n - 1);
     for (; w.q < qn; w.next()) {
         const int je = V.jb + 2 * w.q, J = je >> 1;
         if (je > jhi || je + 1 < jlo) continue;
-        const int c0 = col(w.k), c1 = col(w.k + 1 == w.P ? 0 : w.k + 1);
+        const int c0 = col(w.k), c1 = next(w.k);
         const bool even = je >= jlo, odd = je + 1 <= jhi;
         // an even line injects its last point into the last coarse one
         const bool inject = !(V.n & 1) && je + 1 == V.n - 1;
         val2<S> a0{}, a1{}, b0{}, b1{};
         if (even || !inject) {
-            const node *r = crow(J);
-            a0 = get(r[c0]);
-            a1 = get(r[c1]);
+            const plane<S> r = crow(J);
+            a0 = r.get(c0);
+            a1 = r.get(c1);
         }
         if (odd) {
-            const node *r = crow(J + 1);
-            b0 = get(r[c0]);
-            b1 = get(r[c1]);
+            const plane<S> r = crow(J + 1);
+            b0 = r.get(c0);
+            b1 = r.get(c1);
         }
-        node *z = V.z + 2 * w.q * V.W;
+        const plane<S> z = V.z + 2 * w.q * V.W;
         if (even) {
-            const val2<S> f = get(z[w.k]), g = get(z[w.P + w.k]);
-            z[w.k] = put(val2<S>{add(f.x, a0.x), add(f.y, a0.y)});
-            z[w.P + w.k] =
-                put(val2<S>{add(g.x, scale(add(a0.x, a1.x), 0.5f)), add(g.y, scale(add(a0.y, a1.y), 0.5f))});
+            const val2<S> f = z.get(w.k), g = z.get(w.P + w.k);
+            z.set(w.k, val2<S>{add(f.x, a0.x), add(f.y, a0.y)});
+            z.set(w.P + w.k,
+                  val2<S>{add(g.x, scale(add(a0.x, a1.x), 0.5f)), add(g.y, scale(add(a0.y, a1.y), 0.5f))});
         }
         if (odd) {
-            node *y = z + V.W;
-            const val2<S> f = get(y[w.k]), g = get(y[w.P + w.k]);
+            const plane<S> y = z + V.W;
+            const val2<S> f = y.get(w.k), g = y.get(w.P + w.k);
             val2<S> u, v;
             if (inject) {
                 u = b0;
@@ -634,22 +642,22 @@ MGW_FN void block_prolong(const window<S, true> &V, block_walk w, int qn, int jl
                 v = val2<S>{add(scale(add(a0.x, a1.x), 0.25f), scale(add(b0.x, b1.x), 0.25f)),
                             add(scale(add(a0.y, a1.y), 0.25f), scale(add(b0.y, b1.y), 0.25f))};
             }
-            y[w.k] = put(val2<S>{add(f.x, u.x), add(f.y, u.y)});
-            y[w.P + w.k] = put(val2<S>{add(g.x, v.x), add(g.y, v.y)});
+            y.set(w.k, val2<S>{add(f.x, u.x), add(f.y, u.y)});
+            y.set(w.P + w.k, val2<S>{add(g.x, v.x), add(g.y, v.y)});
         }
     }
 }
 
 // Off-diagonal sums of the top level around a point (comp 0: the x equation).
 template <typename S>
-MGW_FN S top_off3(const top_consts<S> &o, const typename num<S>::node *row, int W, const columns3 &c, int comp) {
+MGW_FN S top_off3(const top_consts<S> &o, const plane<S> &row, int W, const columns3 &c, int comp) {
     if (comp == 0)
-        return three(o.Kmx, sum2(get_x(row + c.l), get_x(row + c.r)), o.my,
-                     sum2(get_x(row + c.c - W), get_x(row + c.c + W)), o.qK,
-                     cross4(get_y(row + c.l - W), get_y(row + c.r + W), get_y(row + c.r - W), get_y(row + c.l + W)));
-    return three(o.mx, sum2(get_y(row + c.l), get_y(row + c.r)), o.Kmy,
-                 sum2(get_y(row + c.c - W), get_y(row + c.c + W)), o.qK,
-                 cross4(get_x(row + c.l - W), get_x(row + c.r + W), get_x(row + c.r - W), get_x(row + c.l + W)));
+        return three(o.Kmx, sum2(row.x(c.l), row.x(c.r)), o.my,
+                     sum2(row.x(c.c - W), row.x(c.c + W)), o.qK,
+                     cross4(row.y(c.l - W), row.y(c.r + W), row.y(c.r - W), row.y(c.l + W)));
+    return three(o.mx, sum2(row.y(c.l), row.y(c.r)), o.Kmy,
+                 sum2(row.y(c.c - W), row.y(c.c + W)), o.qK,
+                 cross4(row.x(c.l - W), row.x(c.r + W), row.x(c.r - W), row.x(c.l + W)));
 }
 
 // One colour of the top level on the rows jlo..jhi: of the block's four nodes
@@ -666,20 +674,19 @@ MGW_FN void block_top_color(const top_consts<S> &o, const window<S, true> &V, bl
             if (j < jlo || j > jhi) continue;
             const bool wall = j == 0 || j == V.n - 1;
             const int cxx = (cy ^ color) & 1;  // the column whose x equation is due
-            typename num<S>::node *row = V.z + lr * V.W;
-            const typename num<S>::node *b = V.b + lr * V.W;
+            const plane<S> row = V.z + lr * V.W, b = V.b + lr * V.W;
             const columns3 cx(w.k, w.P, cxx), cyc(w.k, w.P, cxx ^ 1);
-            const S bx = get_x(b + cx.c), by = get_y(b + cyc.c);
+            const S bx = b.x(cx.c), by = b.y(cyc.c);
             if (wall) {
-                put_x(row + cx.c, mul(o.ibcxx, bx));
-                put_y(row + cyc.c, mul(o.ibcyy, by));
+                row.set_x(cx.c, mul(o.ibcxx, bx));
+                row.set_y(cyc.c, mul(o.ibcyy, by));
             } else if (from_zero) {
-                put_x(row + cx.c, mul(o.icxx, bx));
-                put_y(row + cyc.c, mul(o.icyy, by));
+                row.set_x(cx.c, mul(o.icxx, bx));
+                row.set_y(cyc.c, mul(o.icyy, by));
             } else {
                 const S ex = top_off3(o, row, V.W, cx, 0), ey = top_off3(o, row, V.W, cyc, 1);
-                put_x(row + cx.c, mul(o.icxx, sub(bx, ex)));
-                put_y(row + cyc.c, mul(o.icyy, sub(by, ey)));
+                row.set_x(cx.c, mul(o.icxx, sub(bx, ex)));
+                row.set_y(cyc.c, mul(o.icyy, sub(by, ey)));
             }
         }
     }
@@ -696,16 +703,16 @@ MGW_FN void block_top_residual(const top_consts<S> &o, const window<S, true> &V,
             const int lr = 2 * w.q + cy, j = V.jb + lr;
             if (j < jlo || j > jhi) continue;
             const bool wall = j == 0 || j == V.n - 1;
-            const typename num<S>::node *row = V.z + lr * V.W, *b = V.b + lr * V.W;
+            const plane<S> row = V.z + lr * V.W, b = V.b + lr * V.W;
             const columns3 cx(w.k, w.P, cy), cyc(w.k, w.P, cy ^ 1);
             val2<S> rx{}, ry{};
             if (!wall) {
-                rx.x = sub(sub(get_x(b + cx.c), top_off3(o, row, V.W, cx, 0)), mul(o.cxx, get_x(row + cx.c)));
-                ry.y = sub(sub(get_y(b + cyc.c), top_off3(o, row, V.W, cyc, 1)), mul(o.cyy, get_y(row + cyc.c)));
+                rx.x = sub(sub(b.x(cx.c), top_off3(o, row, V.W, cx, 0)), mul(o.cxx, row.x(cx.c)));
+                ry.y = sub(sub(b.y(cyc.c), top_off3(o, row, V.W, cyc, 1)), mul(o.cyy, row.y(cyc.c)));
             }
-            typename num<S>::node *r = V.r + (j - V.rb) * V.W;
-            r[cx.c] = put(rx);
-            r[cyc.c] = put(ry);
+            const plane<S> r = V.r + (j - V.rb) * V.W;
+            r.set(cx.c, rx);
+            r.set(cyc.c, ry);
         }
     }
 }
@@ -733,7 +740,8 @@ template <typename S> struct small_level {
     int m, n, homog, nst, ncls;
     const int *cls;     // global
     const float4 *st;   // global
-    unsigned zo, bo;    // shared offsets of the band's z and b (level d: all of them)
+    int ps;             // nodes of the band's arrays (their planes' stride)
+    unsigned zo, bo;    // shared offsets of the band's z and b (level d: all of them, b as nodes)
     unsigned ho;        // the three rows of the solution beyond the band (levels above t)
     unsigned so, co;    // stencils and row classes (kNone: read from global memory)
     node *zg;           // global z, b (level t)
@@ -743,7 +751,8 @@ template <typename S> struct small_level {
 constexpr unsigned kNone = 0xffffffffu;
 
 template <typename S> struct small_plan {
-    int t, d, blocks;
+    int t, d, blocks, shift;  // blocks = 1 << shift
+    int rs;                  // plane stride of the residual rows
     int top;                 // level t is the matrix-free top level
     int zero_start;          // its z starts from zero
     unsigned ro;             // residual rows of the level in hand
@@ -758,7 +767,7 @@ template <typename S> struct small_plan {
 // for c == blocks.
 template <typename S> MGW_BOTH int band_row(const small_plan<S> &P, int l, int c) {
     if (c >= P.blocks) return P.lv[l].n;
-    return (int)((long)c * P.lv[P.d].n / P.blocks) << (P.d - l);
+    return ((c * P.lv[P.d].n) >> P.shift) << (P.d - l);
 }
 template <typename S> MGW_BOTH int band_below(const small_plan<S> &P, int l) {
     return P.top && l == P.t ? kTopBelow : kLevBelow;
@@ -771,12 +780,11 @@ template <typename S> MGW_BOTH int band_above(const small_plan<S> &P, int l) {
 // tables in shared memory (known at compile time).
 template <bool FAST, typename S>
 MGW_FN window<S, true> band_window(const small_plan<S> &P, int l, int c, unsigned char *base) {
-    typedef typename num<S>::node node;
     const small_level<S> &L = P.lv[l];
     window<S, true> V;
-    V.z = reinterpret_cast<node *>(base + L.zo);
-    V.b = reinterpret_cast<node *>(base + L.bo);
-    V.r = reinterpret_cast<node *>(base + P.ro);
+    V.z = plane<S>{reinterpret_cast<S *>(base + L.zo), L.ps};
+    V.b = plane<S>{reinterpret_cast<S *>(base + L.bo), L.ps};
+    V.r = plane<S>{reinterpret_cast<S *>(base + P.ro), P.rs};
     V.W = V.m = L.m;
     V.He = (L.m + 1) >> 1;
     V.n = L.n;
@@ -814,22 +822,31 @@ MGW_FN ff warp_pair_sum(ff a) {
 }
 #endif
 
-// This lane's share of one row of the dense levels' product.
-template <int LANES, typename S>
-MGW_FN ff dense_share(const float4 *row, const typename num<S>::node *b, int nd, int lane) {
-    ffacc a;
+// This lane's shares of up to R rows of the dense levels' product, `stride`
+// rows apart (nr of them exist): all rows' loads are in flight together.
+template <int LANES, int R, typename S>
+MGW_FN void dense_share(const float4 *row, size_t stride, int nr, const typename num<S>::node *b, int nd, int lane,
+                        ff (&out)[R]) {
+    ffacc a[R];
+#pragma unroll 3
     for (int k = lane; k < nd; k += LANES) {
-#ifdef __CUDACC__
-        const float4 M = __ldg(row + k);
-#else
-        const float4 M = row[k];
-#endif
         const val2<S> v = get(b[k]);
-        a.mad(ff{M.x, M.y}, as_pair(v.x));
-        a.mad(ff{M.z, M.w}, as_pair(v.y));
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+            const float4 *p = row + (q < nr ? q * stride : 0) + k;
+#ifdef __CUDACC__
+            const float4 M = __ldg(p);
+#else
+            const float4 M = *p;
+#endif
+            a[q].mad(ff{M.x, M.y}, as_pair(v.x));
+            a[q].mad(ff{M.z, M.w}, as_pair(v.y));
+        }
     }
-    return a.done();
+#pragma unroll
+    for (int q = 0; q < R; q++) out[q] = a[q].done();
 }
+constexpr int kDenseRows = 3;  // 34 rows per block of sixteen warps at 17 x 16 nodes
 
 // The V-cycle on the levels of the plan.  E: the block's environment -
 // rank(), local() and base(rank) (a block's shared memory, this or another
@@ -843,7 +860,8 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
     const int me = env.rank(), nb = P.blocks;
     unsigned char *base = env.local();
     const small_level<S> &D = P.lv[P.d];
-    node *bd = reinterpret_cast<node *>(base + D.bo), *zd = reinterpret_cast<node *>(base + D.zo);
+    const node *bd = reinterpret_cast<const node *>(base + D.bo);
+    const plane<S> zd{reinterpret_cast<S *>(base + D.zo), D.ps};
     // the tables; level t's own and halo rows of b (and z)
     env.par([&](int tid, int nth) {
         for (int l = P.t; l < P.d; l++) {
@@ -866,8 +884,8 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
         const divider dv(L.m);
         for (int k = tid; k < total; k += nth) {
             const int q = dv.quot(k), j = lo + q, w = k - q * L.m;
-            V.b[V.at(j, w)] = env.ld(L.bg + (size_t)j * L.m + w);
-            if (P.top && !P.zero_start) V.z[V.at(j, w)] = env.ld(L.zg + (size_t)j * L.m + w);
+            V.b.set(V.at(j, w), get(env.ld(L.bg + (size_t)j * L.m + w)));
+            if (P.top && !P.zero_start) V.z.set(V.at(j, w), get(env.ld(L.zg + (size_t)j * L.m + w)));
         }
     });
     if (nb > 1) env.csync();  // every block runs: its shared memory may be written
@@ -896,7 +914,7 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
                         block_color(V, env.walk(w, tid, nth), qn, y0 - 2 + (c >> 1), y1 + 2 - (c >> 1), c & 1, c >> 1,
                                     true);
                     });
-                env.par([&](int tid, int nth) { block_residual(V, env.walk(w, tid, nth), qn, y0 - 1, y1 - 1); });
+                env.par([&](int tid, int nth) { block_residual(V, V.W >> 1, qn, y0 - 1, y1 - 1, tid, nth); });
             }
         } else if (top) {
             env.par([&](int tid, int nth) {
@@ -923,7 +941,7 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
             if (l + 1 < P.d) {
                 const window<S, true> CV = band_window<FAST>(P, l + 1, me, base);
                 const int He = CV.He;
-                node *to[4];  // b of the neighbours at distance -2, -1, 1, 2, shifted to absolute rows
+                S *to[4];  // b of the neighbours at distance -2, -1, 1, 2, shifted to absolute rows
                 int lo[4], hi[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
@@ -935,21 +953,22 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
                     lo[q] = band_row(P, l + 1, c) - kLevBelow;
                     hi[q] = band_row(P, l + 1, c + 1) + kLevAbove - 2;  // the last row a sweep reads
                     if (lo[q] >= J1 || hi[q] < J0) hi[q] = lo[q] - 1;
-                    else to[q] = reinterpret_cast<node *>(env.base(c) + P.lv[l + 1].bo);
+                    else to[q] = reinterpret_cast<S *>(env.base(c) + P.lv[l + 1].bo);
                 }
-                auto out = [&](int J, int I, node v) {
+                auto out = [&](int J, int I, const val2<S> &v) {
                     const int c = (I & 1) * He + (I >> 1);
-                    CV.b[(J - CV.jb) * cm + c] = v;
+                    CV.b.set((J - CV.jb) * cm + c, v);
 #pragma unroll
                     for (int q = 0; q < 4; q++)
-                        if (J >= lo[q] && J <= hi[q]) to[q][(J - lo[q]) * cm + c] = v;
+                        if (J >= lo[q] && J <= hi[q]) plane<S>{to[q], CV.b.ps}.set((J - lo[q]) * cm + c, v);
                 };
                 if (FAST) block_restrict(V, block_walk(tid, nth, V.W >> 1), qn, J0, J1 - 1, out);
                 else restrict_rows(V, J0, J1 - 1, 0, cm - 1, cm, out, tid, nth);
             } else {
-                auto out = [&](int J, int I, node v) {
+                auto out = [&](int J, int I, const val2<S> &v) {
+                    const node o = put(v);
                     for (int c = 0; c < nb; c++)
-                        reinterpret_cast<node *>((c == me ? base : env.base(c)) + D.bo)[J * cm + I] = v;
+                        reinterpret_cast<node *>((c == me ? base : env.base(c)) + D.bo)[J * cm + I] = o;
                 };
                 if (FAST) block_restrict(V, block_walk(tid, nth, V.W >> 1), qn, J0, J1 - 1, out);
                 else restrict_rows(V, J0, J1 - 1, 0, cm - 1, cm, out, tid, nth);
@@ -960,14 +979,23 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
     // level d: z = M b, a group of threads per row, the result to every block
     env.par([&](int tid, int nth) {
         const int nd = D.m * D.n, r0 = 2 * (int)((long)nd * me / nb), r1 = 2 * (int)((long)nd * (me + 1) / nb);
-        const int lane = tid % E::kLanes;
-        for (int r = r0 + tid / E::kLanes; r < r1; r += nth / E::kLanes) {
-            const float4 *row = P.dense + (size_t)r * nd;
-            const S v = from_pair(env.lane_sum(dense_share<E::kLanes, S>(row, bd, nd, lane)), S());
-            for (int c = lane; c < nb; c += E::kLanes) {
-                node *z = reinterpret_cast<node *>((c == me ? base : env.base(c)) + D.zo) + (r >> 1);
-                if (r & 1) put_y(z, v);
-                else put_x(z, v);
+        const int lane = tid % E::kLanes, groups = nth / E::kLanes;
+        for (int r = r0 + tid / E::kLanes; r < r1; r += kDenseRows * groups) {
+            const int nr = imin(kDenseRows, (r1 - r + groups - 1) / groups);
+            ff v[kDenseRows];
+            dense_share<E::kLanes, kDenseRows, S>(P.dense + (size_t)r * nd, (size_t)groups * nd, nr, bd, nd, lane, v);
+#pragma unroll
+            for (int q = 0; q < kDenseRows; q++) v[q] = env.lane_sum(v[q]);
+#pragma unroll
+            for (int q = 0; q < kDenseRows; q++) {
+                const int rr = r + q * groups;
+                if (q >= nr) break;
+                const S o = from_pair(v[q], S());
+                for (int c = lane; c < nb; c += E::kLanes) {
+                    const plane<S> z{reinterpret_cast<S *>((c == me ? base : env.base(c)) + D.zo), D.ps};
+                    if (rr & 1) z.set_y(rr >> 1, o);
+                    else z.set_x(rr >> 1, o);
+                }
             }
         }
     });
@@ -980,8 +1008,8 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
         const bool top = P.top && l == P.t, last = l + 1 == P.d;
         const window<S, true> CV = band_window<FAST>(P, l + 1, me, base);
         const int J0 = band_row(P, l + 1, me), J1 = band_row(P, l + 1, me + 1), cHe = CV.He;
-        const node *halo = last ? nullptr : reinterpret_cast<const node *>(base + P.lv[l + 1].ho);
-        auto crow = [&](int J) -> const node * {
+        const plane<S> halo{reinterpret_cast<S *>(base + (last ? 0u : P.lv[l + 1].ho)), 3 * cm};
+        auto crow = [&](int J) -> plane<S> {
             if (last) return zd + J * cm;
             if (J < J0) return halo;
             if (J >= J1) return halo + (1 + J - J1) * cm;
@@ -991,7 +1019,8 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
         if (FAST) {
             const block_walk w(env.thread(), env.threads(), V.W >> 1);
             env.par([&](int tid, int nth) {
-                block_prolong(V, env.walk(w, tid, nth), qn, y0 - (top ? 2 : 1), y1 + 1, crow, ccol);
+                block_prolong(V, env.walk(w, tid, nth), qn, y0 - (top ? 2 : 1), y1 + 1, crow, ccol,
+                              [&](int k) { return ccol(k + 1 == cm ? 0 : k + 1); });
             });
             if (top) {
                 env.par([&](int tid, int nth) {
@@ -1010,7 +1039,7 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
         } else {
             env.par([&](int tid, int nth) {
                 prolong_rows(V, y0 - (top ? 2 : 1), y1 + 1, 0, 0, cm,
-                             [&](int J, int I) -> node { return crow(J)[ccol(I)]; }, tid, nth);
+                             [&](int J, int I) { return crow(J).get(ccol(I)); }, tid, nth);
             });
             if (top) {
                 env.par([&](int tid, int nth) { top_color(P.op, V, y0 - 1, y1, 0, 0, 0, false, tid, nth); });
@@ -1032,21 +1061,23 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
                 const divider dv(V.m);
                 for (int k = tid; k < total; k += nth) {
                     const int q = dv.quot(k), w = k - q * V.m;
-                    env.store(P, (size_t)(y0 + q) * V.m + w, V.z[V.at(y0 + q, w)]);
+                    env.store(P, (size_t)(y0 + q) * V.m + w, put(V.z.get(V.at(y0 + q, w))));
                 }
             });
         } else if (nb > 1) {
             // rows next to the band's edges, for the neighbours' prolongation
             env.par([&](int tid, int nth) {
                 const int m = V.m;
-                node *lo = me > 0 ? reinterpret_cast<node *>(env.base(me - 1) + P.lv[l].ho) : nullptr;
-                node *hi = me + 1 < nb ? reinterpret_cast<node *>(env.base(me + 1) + P.lv[l].ho) : nullptr;
-                for (int k = tid; k < m; k += nth) {
+                S *lo = me > 0 ? reinterpret_cast<S *>(env.base(me - 1) + P.lv[l].ho) : nullptr;
+                S *hi = me + 1 < nb ? reinterpret_cast<S *>(env.base(me + 1) + P.lv[l].ho) : nullptr;
+                for (int k = tid; k < 2 * m; k += nth) {  // both components
+                    const int c = k < m ? k : k - m, from = k < m ? 0 : V.z.ps, to = k < m ? 0 : 3 * m;
+                    const S *z = V.z.p + from + c;
                     if (lo) {
-                        lo[m + k] = V.z[(y0 - V.jb) * m + k];
-                        lo[2 * m + k] = V.z[(y0 + 1 - V.jb) * m + k];
+                        lo[to + m + c] = z[(y0 - V.jb) * m];
+                        lo[to + 2 * m + c] = z[(y0 + 1 - V.jb) * m];
                     }
-                    if (hi) hi[k] = V.z[(y1 - 1 - V.jb) * m + k];
+                    if (hi) hi[to + c] = z[(y1 - 1 - V.jb) * m];
                 }
             });
             env.csync();
