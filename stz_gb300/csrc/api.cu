@@ -640,6 +640,7 @@ int stzg_create(const stz_params *p, const stzg_options *opt, stzg_sim **out) {
     s->sc = make_step_consts(*p);
     s->sc.track_plastic = o.track_plastic;
     s->sc.sp_increments = o.precision == STZG_MIXED && o.advection != STZG_ADV_FP64;
+    s->sc.fixed_point = o.advection != STZG_ADV_FP64;
     if (o.substep_cap > 0) s->sc.substep_cap = o.substep_cap;
     int st = STZG_OK;
     auto bail = [&](int code) {
@@ -660,9 +661,10 @@ int stzg_create(const stz_params *p, const stzg_options *opt, stzg_sim **out) {
     if ((st = dev_alloc(s, (void **)&s->F.flags, FL_COUNT * sizeof(int))) != STZG_OK) return bail(st);
     for (int k = 0; k < 4; k++)
         if ((st = dev_alloc(s, (void **)&s->F.pre[k], nc * sizeof(double))) != STZG_OK) return bail(st);
-    // cells the float-float advection hands to the FP64 plastic pass (at most all of them)
+    // cells and tiles the fixed-point advection hands on (at most all of them)
     if ((st = dev_alloc(s, (void **)&s->F.plist, (size_t)s->m * s->n * sizeof(unsigned))) != STZG_OK) return bail(st);
-    if ((st = dev_alloc(s, (void **)&s->F.pcount, sizeof(unsigned))) != STZG_OK) return bail(st);
+    if ((st = dev_alloc(s, (void **)&s->F.tlist, sizeof(unsigned) * tile_count(s->sc))) != STZG_OK) return bail(st);
+    if ((st = dev_alloc(s, (void **)&s->F.pcount, 2 * sizeof(unsigned))) != STZG_OK) return bail(st);
     s->maps = new field_maps;
     if ((st = make_field_maps(s->sc, s->F, s->maps)) != STZG_OK) return bail(st);
     if (o.extrapolate)

@@ -95,9 +95,10 @@ template <typename F> int dense_level(int ml, F nodes) {
 
 // Tile of a wide level: coarse columns and rows, threads, shared memory of one
 // launch.  top: 0 a coarse level, 1 the top level down, 2 up; bands: whole
-// rows.  A row of blocks is a warp's; 16, 8 or 4 of them per tile, the most
-// that still gives three blocks per SM (the halo of a tile of 14, 6 or 2
-// coarse rows costs 1.14, 1.33 or 2 times the rows).
+// rows.  A row of blocks is a warp's; 8 or 4 of them per tile, the most that
+// still gives three blocks per SM (the halo of a tile of 6 or 2 coarse rows
+// costs 1.33 or 2 times the rows; 16 rows, 1.14 times, took 209 us per V-cycle
+// of 1024x768 against 194: the last wave was nearly empty).
 struct tile_shape {
     int tw, th, threads;
     unsigned long bytes;
@@ -115,7 +116,7 @@ inline tile_shape shape_tile(int m, int cm, int cn, int table, int top, bool ban
         for (T.th = 4; T.th > 2 && (bytes() > max_bytes || (cn + T.th - 1) / T.th < 152); T.th >>= 1) {}
     } else {
         T.tw = top == 1 ? 29 : (top == 2 ? 30 : 28);
-        for (int rows = 16; rows >= 4; rows >>= 1) {
+        for (int rows = 8; rows >= 4; rows >>= 1) {
             T.th = rows - extra;
             T.threads = rows >= 8 ? 256 : 128;
             if ((long)((cm + T.tw - 1) / T.tw) * ((cn + T.th - 1) / T.th) >= 3 * 152) break;

@@ -56,7 +56,7 @@ struct block_env {
         P.lv[P.t].zg[k] = v;
     }
     __device__ __forceinline__ void store(const small_plan<ff> &P, size_t k, const float4 &v) const {
-        if (P.sum) add_pairs(P.sum + k, v);
+        if (P.sum) P.sum[k] = add_pairs(P.sum[k], v);
         else P.lv[P.t].zg[k] = v;
     }
 };

@@ -11,11 +11,8 @@ __device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launc
 __device__ __forceinline__ void pdl_input() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 // z += d in FP64, the pair formed as a double on the integer pipe.
-__device__ __forceinline__ void add_pairs(double2 *z, const float4 &d) {
-    double2 v = *z;
-    v.x += ff_to_d(d.x, d.z);
-    v.y += ff_to_d(d.y, d.w);
-    *z = v;
+__device__ __forceinline__ double2 add_pairs(const double2 &z, const float4 &d) {
+    return make_double2(z.x + ff_to_d(d.x, d.z), z.y + ff_to_d(d.y, d.w));
 }
 
 // ---- wide levels as tiles ------------------------------------------------------
@@ -255,7 +252,23 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_top_up(top_consts<ff> op,
     __syncthreads();
     block_top_color(op, V, w, G.qn, G.y0, G.y1 - 1, 1, false);
     __syncthreads();
-    tile_own(L, V, G, [&](size_t k, const val2<ff> &v) { add_pairs(L.sum + k, put(v)); });
+    // z += d: four nodes' iterates are on their way at a time
+    const int ow = G.x1 - G.x0, total = (G.y1 - G.y0) * ow;
+    const divider dv(ow);
+    for (int k0 = threadIdx.x; k0 < total; k0 += 4 * L.threads) {
+        double2 *at[4], z[4];
+        float4 d[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int k = min(k0 + u * L.threads, total - 1), q = dv.quot(k), w = k - q * ow;
+            at[u] = L.sum + (size_t)(G.y0 + q) * L.m + G.x0 + w;
+            z[u] = *at[u];
+            d[u] = put(V.z.get(V.at(G.y0 + q, w + G.x0 - G.xb)));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (k0 + u * L.threads < total) *at[u] = add_pairs(z[u], d[u]);
+    }
 }
 
 }  // namespace mgw

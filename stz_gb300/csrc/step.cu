@@ -4,6 +4,9 @@
 #include "step.cuh"
 #include "stz_law.cuh"
 
+#include <algorithm>
+#include <cmath>
+
 namespace stzg {
 
 // x = hi + lo as floats on the host (hi the nearest float, lo the nearest
@@ -49,6 +52,7 @@ step_consts make_step_consts(const stz_params &p) {
     c.clock = nullptr;
     c.xbc = 0;
     c.sp_increments = 0;
+    c.fixed_point = 0;
     return c;
 }
 
@@ -236,10 +240,10 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-// Bounded wait for phase 0 of bar; false when it ran out.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar) {
+// Bounded wait for a phase of bar; false when it ran out.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity = 0) {
     for (int it = 0; it < kTmaWaitIters; it++)
-        if (mbar_try_wait(bar, 0)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
 
@@ -256,33 +260,45 @@ struct adv_smem {
     uint64_t bar;
 };
 
-__global__ void __launch_bounds__(ATX * ATY) k_advect(step_consts c, advect_consts a, const __grid_constant__ field_maps maps,
-                                                      fields_dev F, int cur, double dt, double bv, int emit_source) {
+// The per-cell combinations of the advected stress (fields_dev::pre).
+__device__ __forceinline__ void write_pre(const fields_dev &F, size_t ci, double xf, double yf, double pn, double qn,
+                                          double sn, double tn) {
+    const double pq = pn + qn, Aa = pq - sn, Bb = pq + sn;
+    F.pre[0][ci] = xf * Aa + yf * tn;
+    F.pre[1][ci] = xf * Aa - yf * tn;
+    F.pre[2][ci] = xf * tn - yf * Bb;
+    F.pre[3][ci] = xf * tn + yf * Bb;
+}
+
+// One tile (bx, by) in FP64; `use`: how often the block has done this before
+// (the barrier's phase).  False when a tile copy did not arrive.
+__device__ __forceinline__ bool advect_tile(const step_consts &c, const advect_consts &a, const field_maps &maps,
+                                            const fields_dev &F, int cur, double dt, double bv, int emit_source, int bx,
+                                            int by, unsigned use) {
     extern __shared__ __align__(128) unsigned char adv_raw[];
     adv_smem &Sm = *reinterpret_cast<adv_smem *>(adv_raw + ((128 - (smem_addr(adv_raw) & 127)) & 127));
     adv_tile &T = Sm.T;
     const int m = c.m, n = c.n;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * ATX + tx;
-    const int i0 = blockIdx.x * ATX, j0 = blockIdx.y * ATY;
+    const int i0 = bx * ATX, j0 = by * ATY;
     const int i = i0 + tx, j = j0 + ty;
-    if (c.clock) cur = (int)c.clock[CLK_CUR];
     const double *__restrict__ const *A = F.f[cur];
     double *const *B = F.f[cur ^ 1];
     // One thread copies the seven field tiles (columns i0-2.., storage rows
     // j0-1..) by TMA while the block sets up the column tables.
-    if (tid == 0) mbar_init(&Sm.bar, 1);
+    if (tid == 0 && use == 0) mbar_init(&Sm.bar, 1);
     tile_columns(T, i0, m, c.lx);
     __syncthreads();
     if (tid == 0) {
         mbar_expect_tx(&Sm.bar, kTileBytes);
         for (int f = 0; f < F_COUNT; f++) tma_load_2d(&Sm.tile[f][0][0], &maps.f[cur][f], i0 - 2, j0 - 1, &Sm.bar);
     }
-    if (__syncthreads_or(!mbar_wait_bounded(&Sm.bar))) {
+    if (__syncthreads_or(!mbar_wait_bounded(&Sm.bar, use & 1))) {
         // a copy did not arrive in time: flag it, wait once more for the
         // copies in flight, and leave this tile of the next state unwritten
         if (tid == 0) atomicExch(&F.flags[FL_TMA], 1);
-        mbar_wait_bounded(&Sm.bar);
-        return;
+        mbar_wait_bounded(&Sm.bar, use & 1);
+        return false;
     }
     // Columns across the periodic seam arrive as zeros: blocks at either end
     // fetch them from their wrapped columns.
@@ -297,7 +313,7 @@ __global__ void __launch_bounds__(ATX * ATY) k_advect(step_consts c, advect_cons
     tile_differences<F_COUNT>(
         T, i0, j0, m, n, F_X, [&](int f, int row, int t) { return Sm.tile[f][row - j0 + 2][t]; },
         [](int) { return -1; });
-    if (i >= m || j >= n) return;
+    if (i >= m || j >= n) return true;
     const double hx = a.hx, hy = a.hy;
     const size_t ci = (size_t)(j + 1) * m + i;
     const int ir = T.col[tx + 3];
@@ -375,230 +391,109 @@ __global__ void __launch_bounds__(ATX * ATY) k_advect(step_consts c, advect_cons
     B[F_S][ci] = sn;
     B[F_TAU][ci] = tn;
     if (emit_source) {
-        const double pq = pn + qn, Aa = pq - sn, Bb = pq + sn;
-        F.pre[0][ci] = a.xf * Aa + a.yf * tn;
-        F.pre[1][ci] = a.xf * Aa - a.yf * tn;
-        F.pre[2][ci] = a.xf * tn - a.yf * Bb;
-        F.pre[3][ci] = a.xf * tn + a.yf * Bb;
+        write_pre(F, ci, a.xf, a.yf, pn, qn, sn, tn);
     }
+    return true;
 }
 
-// ---- float-float advection (mixed-precision handles) ------------------------
-// The same step with the ENO differences, the upwind products and the
-// increments in float-float (double-word) arithmetic on the FP32 pipe while
-// the state stays FP64.  Every staged value is split on the integer pipe
-// into a float pair hi + lo (ff_split_d, 48 of its 53 significant bits); each
-// first difference f(c+1) - f(c) is formed from the pairs by TwoSum and kept
-// as a pair (relative error ~2^-44 of the difference, plus ~2^-47 of the
-// values); the ENO value is the chosen second difference plus twice the
-// centre difference, the increment u hs eno in both directions with the
-// product errors (FMA) and the sums by TwoSum, and the spin from pair
-// differences of the node velocities.  Each field takes its increment with
-// two FP64 additions (hi, then lo), so the state carries the rounding of the
-// FP64 path plus ~2^-44 of the increment per step.  The ENO choice
-// |S(i)| > |S(i-1)| is taken on the pair second differences where the two
-// magnitudes differ by more than their error bound; near ties between
-// different values it is recomputed in FP64 from the staged tile with
-// k_advect's operations, so the choice is always the FP64 path's (a
-// different choice changes the value by the difference of two second
-// differences, which near an inflection is not small).  The yield test runs on a float-float stress norm; cells near or
-// above a cut-off take the FP64 norm and the FP64 plastic law as k_advect
-// does.  The net force is formed by k_source_ff from the stresses, so no
-// per-cell combinations are written.  GB300 issues FP64 at 1/57 of the FP32
-// rate; an elastic cell here needs two FP64 additions per field.
-// Shared memory of k_advect_ff: the split values, then the FP64 tile (the
-// TMA destination, needed only until it is split) overlaid by the first
-// differences, so that three blocks fit on an SM.
-struct adv_smem_ff {
-    float2 t2[F_COUNT][AROWS][ACOLS];  // staged values as (hi, lo) pairs: one 64-bit access each
-    union {
-        double tile[F_COUNT][AROWS][ACOLS];  // staged fields (128-byte aligned: 24192 B precede it)
-        struct {
-            float2 dx[F_COUNT][ATY][ADXW];  // first differences in x (pairs): tile columns cc, cc+1
-            float2 dy[F_COUNT][ADYH][ATX];  // first differences in y (pairs): tile rows r, r+1
-        } d;
-    } u;
-    ff nu[ATY + 1][ATX + 1];  // node velocities (i0+c, j0+r) as pairs, walls substituted
-    ff nv[ATY + 1][ATX + 1];
-    int xs[ACOLS];   // period shift of the unwrapped column: -1, 0, +1
-    int col[ACOLS];  // storage column of tile column c-2
-    uint64_t bar;
-};
-static_assert(sizeof(float) * 2 * F_COUNT * AROWS * ACOLS % 128 == 0, "the TMA tile must stay 128-byte aligned");
+__global__ void __launch_bounds__(ATX * ATY) k_advect(step_consts c, advect_consts a, const __grid_constant__ field_maps maps,
+                                                      fields_dev F, int cur, double dt, double bv, int emit_source) {
+    if (c.clock) cur = (int)c.clock[CLK_CUR];
+    advect_tile(c, a, maps, F, cur, dt, bv, emit_source, blockIdx.x, blockIdx.y, 0);
+}
+
+// ---- float pairs of the projection kernels (mixed-precision handles) ------------
 
 __device__ __forceinline__ ff split_ff(double d) {
     ff r;
     ff_split_d(d, r.hi, r.lo);
     return r;
 }
-
-// a - b for pairs a = (ah, al), b = (bh, bl): TwoSum of the high parts, the
-// low parts added to its error, renormalised.
-__device__ __forceinline__ ff ff_pair_diff(float ah, float al, float bh, float bl) {
-    const float s = ah - bh, bb = s - ah;
-    float e = (ah - (s - bb)) + (-bh - bb);
-    e += al - bl;
-    return ff_fast2sum(s, e);
-}
-__device__ __forceinline__ ff ff_x2(ff a) { return ff{2.f * a.hi, 2.f * a.lo}; }
-__device__ __forceinline__ float ffabs_hi(ff a) { return fabsf(a.hi); }
-
-// FP64 choice of k_advect in x (tile_differences with the X column
-// offsets, then eno_left / eno_right's magnitude test) from the state in
-// global memory (row: storage row, cols: the tile's storage columns, xs: the
-// tile's period shifts): true where it takes the outer second difference.
-__device__ __noinline__ bool pick_x64(const double *__restrict__ f, size_t row, const int *cols, const int *xs,
-                                      bool is_x, double lx, int tx, bool from_left) {
-    const int c0 = from_left ? tx : tx + 1;  // tile columns c0 .. c0+3
-    double g[4];
-    for (int q = 0; q < 4; q++) {
-        g[q] = f[row + cols[c0 + q]];
-        if (is_x && xs[c0 + q] != 0) g[q] += xs[c0 + q] < 0 ? -lx : lx;
-    }
-    const double da = g[1] - g[0], db = g[2] - g[1], dc = g[3] - g[2];
-    // from the left: s0 = S(i) = dc - db, s1 = S(i-1) = db - da;
-    // from the right: s0 = S(i) = db - da, s1 = S(i+1) = dc - db
-    return from_left ? mag_gt(dc - db, db - da) : mag_gt(db - da, dc - db);
-}
-// FP64 choice in y (difference r between cell rows j0+r-2 and j0+r-1, zero
-// where k_advect's tile_differences leaves it zero) at storage column i.
-__device__ __noinline__ bool pick_y64(const double *__restrict__ f, int m, int i, int ty, bool from_below, int j0,
-                                      int n) {
-    const int r0 = from_below ? ty : ty + 1;  // differences r0 .. r0+2
-    double d[3];
-    for (int q = 0; q < 3; q++) {
-        const int r = r0 + q, jj = j0 + r - 2;  // cell rows jj, jj+1 = storage rows jj+1, jj+2
-        d[q] = (jj >= -1 && jj + 1 <= n) ? f[(size_t)(jj + 2) * m + i] - f[(size_t)(jj + 1) * m + i] : 0.0;
-    }
-    return from_below ? mag_gt(d[2] - d[1], d[1] - d[0]) : mag_gt(d[1] - d[0], d[2] - d[1]);
-}
-
-// ENO2 value from three consecutive first differences Da, Db, Dc around the
-// point (Db is the upwind centre difference): from the left (outer = Db - Da)
-// 2 Db + (|Dc - Db| > |Db - Da| ? Db - Da : Dc - Db); from the right
-// (outer = Dc - Db) -2 Db + (|Db - Da| > |Dc - Db| ? Dc - Db : Db - Da).
-// The second differences are pairs; their magnitudes are compared in pairs
-// too, decided where they differ by more than the pairs' error bound (the
-// differences' ~2^-44 plus the split's ~2^-47 of the values, with room).
-// Within the margin, candidates of the same sign (equal up to the margin)
-// give values within the float-float path's own error either way; a near tie
-// of opposite signs (the candidates differ by twice their size) takes the
-// inner candidate below kEnoTieRel of the field's scale and `exact`, the
-// FP64 path's own choice, above it.
-__device__ __forceinline__ ff ff_abs(ff a) { return a.hi < 0.f ? ff_neg(a) : a; }
-constexpr float kEnoTieRel = 1e-10f;
-template <typename Exact>
-__device__ __forceinline__ ff eno_ff(ff Da, ff Db, ff Dc, bool from_left, float vmag, Exact exact) {
-    // second differences from the high parts: within |lo| parts and one
-    // float rounding of the pairs' values, themselves within ~2^-44 of the
-    // differences and ~2^-47 of the values of the exact ones
-    const float fab = Db.hi - Da.hi, fbc = Dc.hi - Db.hi;
-    const float fin = from_left ? fbc : fab, fout = from_left ? fab : fbc;
-    const float gap0 = fabsf(fin) - fabsf(fout);
-    const float big = fabsf(Da.hi) + 2.f * fabsf(Db.hi) + fabsf(Dc.hi);
-    // bounds the low parts (<= 2^-24 big), one float rounding of each second
-    // difference (<= 2.4e-7 (|fin| + |fout|) <= 2.4e-7 big) and the pairs'
-    // own error (1e-12 big + 4e-13 vmag)
-    const float m0 = 3.1e-7f * big + 4e-13f * vmag;
-    bool take_outer;
-    if (fabsf(gap0) > m0) {
-        take_outer = gap0 > 0.f;
-    } else {
-        const ff sab = ff_sub(Db, Da), sbc = ff_sub(Dc, Db);
-        const ff inner = from_left ? sbc : sab, outer = from_left ? sab : sbc;
-        const ff g = ff_sub(ff_abs(inner), ff_abs(outer));
-        const float gap = g.hi + g.lo;
-        const float margin = 1e-12f * big + 4e-13f * vmag, small = kEnoTieRel * (vmag + big);
-        if (fabsf(gap) > margin) take_outer = gap > 0.f;
-        // Within the margin the two candidates differ by at most |gap| plus
-        // its error where they have the same sign (or one is zero): either
-        // choice then moves the value by less than ~2e-12 (|value| +
-        // |differences|) times the upwind factor.  Of opposite signs they
-        // differ by twice their size: below kEnoTieRel (|value| +
-        // |differences|) that is grid-scale noise of the field at the level
-        // of the solver's tolerance, and the inner candidate is taken; above
-        // it the FP64 path's own choice.
-        else if (inner.hi * outer.hi >= 0.f || (fabsf(inner.hi) <= small && fabsf(outer.hi) <= small))
-            take_outer = false;
-        else take_outer = exact();
-    }
-    // outer: from the left Db - Da, from the right Dc - Db
-    const bool lower = from_left == take_outer;
-    const ff s = ff_sub(lower ? Db : Dc, lower ? Da : Db);
-    return ff_add(from_left ? ff_x2(Db) : ff_neg(ff_x2(Db)), s);
-}
-
-__device__ __forceinline__ ff dx_pair(const adv_smem_ff &Sm, int f, int ty, int c) {
-    const float2 v = Sm.u.d.dx[f][ty][c];
-    return ff{v.x, v.y};
-}
-__device__ __forceinline__ ff dy_pair(const adv_smem_ff &Sm, int f, int r, int tx) {
-    const float2 v = Sm.u.d.dy[f][r][tx];
-    return ff{v.x, v.y};
-}
-
-// Where the FP64 choice is needed, the state buffer read (A), the point's
-// storage row and the tile geometry.
-struct eno_ctx {
-    const double *__restrict__ const *A;
-    int m, n, j0, j;
-    double lx;
-};
-
-__device__ __forceinline__ ff eno_x_ff(const adv_smem_ff &Sm, const eno_ctx &e, int f, int ty, int tx,
-                                       bool from_left) {
-    const int c = from_left ? tx : tx + 1;  // differences c .. c+2 (tile columns c .. c+3)
-    const float vmag = fabsf(Sm.t2[f][ty + 2][tx + 2].x);
-    return eno_ff(dx_pair(Sm, f, ty, c), dx_pair(Sm, f, ty, c + 1), dx_pair(Sm, f, ty, c + 2), from_left, vmag, [&] {
-        return pick_x64(e.A[f], (size_t)(e.j + 1) * e.m, Sm.col, Sm.xs, f == F_X, e.lx, tx, from_left);
-    });
-}
-// y with the one-sided wall rows: `inner` is false on the last row before
-// the wall on the upwind side (value +-2 Db there).
-__device__ __forceinline__ ff eno_y_ff(const adv_smem_ff &Sm, const eno_ctx &e, int f, int ty, int tx,
-                                       bool from_below, bool inner) {
-    const int r = from_below ? ty : ty + 1;  // differences r .. r+2
-    const ff Db = dy_pair(Sm, f, r + 1, tx);
-    if (!inner) return from_below ? ff_x2(Db) : ff_neg(ff_x2(Db));
-    const float vmag = fabsf(Sm.t2[f][ty + 2][tx + 2].x);
-    return eno_ff(dy_pair(Sm, f, r, tx), Db, dy_pair(Sm, f, r + 2, tx), from_below, vmag, [&] {
-        return pick_y64(e.A[f], e.m, Sm.col[tx + 2], ty, from_below, e.j0, e.n);
-    });
-}
-
-// -(uh eno_x + vh eno_y)
-__device__ __forceinline__ ff upwind_inc(ff uh, ff ex, ff vh, ff ey) {
-    return ff_neg(ff_add(ff_mul(uh, ex), ff_mul(vh, ey)));
-}
 // a + inc for the FP64 state value a with one FP64 addition (the pair formed
 // as a double on the integer pipe)
 __device__ __forceinline__ double add_ff(double a, ff inc) { return a + ff_to_d(inc.hi, inc.lo); }
-// u > 0 for a finite double, on the integer pipe
-__device__ __forceinline__ bool dpos(double u) { return __double_as_longlong(u) > 0; }
 
-// Float-float pairs of the per-launch constants hx, hy and of the period lx.
-struct advect_ff_consts {
-    float hxh, hxl, hyh, hyl, lxh, lxl;
+// ---- fixed-point advection ----------------------------------------------------
+//
+// The same step with the ENO arithmetic in 64-bit integers: GB300 retires two
+// FP64 operations per clock and SM and 64 integer ones, and the ENO part of
+// the step is differences of neighbouring values, which integers form exactly.
+// Every staged field of the tile is scaled by one power of two so that its
+// largest magnitude lies in [2^58, 2^59) (a value within 2^-6 of the largest
+// keeps all of its 53 bits, a smaller one is cut at 2^-59 of the largest, 64
+// times finer than the FP64 spacing there); first and second differences, the
+// comparison of their magnitudes and the ENO value (at most 2^62) are then
+// exact, so near ties need no margin.  The products with the velocity times
+// dt/(2 dx), scaled likewise, are the high words of 64 x 64 bit products (cut
+// at about 2^-57 of the largest increment), and each field takes its increment
+// in one FP64 addition.  An update therefore carries the one rounding the FP64
+// form's last operation has.
+// Tiles with an infinity or a NaN in a field or the velocity are listed and
+// take k_advect's arithmetic in k_advect_rest, as do the cells that the yield
+// test (on the leading 24 bits, with a margin) cannot certify as elastic.
+struct fx_smem {
+    union {
+        double d[F_COUNT][AROWS][ACOLS];  // TMA destination (128-byte aligned)
+        long long v[F_COUNT][AROWS][ACOLS];
+    } t;
+    long long nu[ATY + 1][ATX + 1], nv[ATY + 1][ATX + 1];  // node velocities, walls substituted
+    unsigned top[F_COUNT + 1];  // largest high word's magnitude per field; then of the velocity
+    int xs[ACOLS], col[ACOLS];  // period shift and storage column of tile column c-2
+    uint64_t bar;
 };
 
-// Node velocity as float pairs, the walls' +-bv substituted (no FP64 work).
-struct velo_ff {
-    const double2 *vel;
-    int m, n;
-    ff bv;
-    __device__ __forceinline__ ff u(int i, int j) const {
-        return j == 0 ? ff_neg(bv) : (j == n ? bv : split_ff(vel[(size_t)j * m + i].x));
-    }
-    __device__ __forceinline__ ff v(int i, int j) const {
-        return (j == 0 || j == n) ? ff{0.f, 0.f} : split_ff(vel[(size_t)j * m + i].y);
-    }
+// hx, hy = hmx 2^he, hmy 2^he with the larger of hmx, hmy in [2^61, 2^62).
+struct advect_fx_consts {
+    long long hmx, hmy;
+    int he;
+    double xf, yf;  // 1/(2 dt dx), 1/(2 dt dy) of projection_step
 };
 
-__global__ void __launch_bounds__(ATX * ATY, 3)
-    k_advect_ff(step_consts c, advect_ff_consts h, const __grid_constant__ field_maps maps, fields_dev F, int cur,
-                double dt, double bv) {
-    extern __shared__ __align__(128) unsigned char adv_raw_ff[];
-    adv_smem_ff &Sm = *reinterpret_cast<adv_smem_ff *>(adv_raw_ff + ((128 - (smem_addr(adv_raw_ff) & 127)) & 127));
+// d 2^(1081 - E) cut to an integer; E: the biased exponent of the largest
+// magnitude of d's set, so the result is below 2^59.
+__device__ __forceinline__ long long to_fixed(double d, int E) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    const int e = (hi >> 20) & 0x7ff;
+    const unsigned long long m =
+        ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;  // below 2^63
+    const long long v = (long long)(m >> min(4 + E - e, 63));  // zero and subnormal: shifted out
+    return (int)hi < 0 ? -v : v;
+}
+
+// v 2^K as a double, rounded to nearest (ties up in magnitude).
+__device__ __forceinline__ double from_fixed(long long v, int K) {
+    const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+    const int lz = __clzll((long long)m), e = 1023 + 63 - lz + K;
+    const unsigned long long w = m << (lz & 63);
+    const unsigned long long r = (w >> 11) + ((w >> 10) & 1);
+    unsigned long long bits = ((unsigned long long)(unsigned)(e - 1) << 52) + r;  // r carries the implicit bit
+    if (m == 0 || e <= 0) bits = 0;
+    if (e >= 2047) bits = 0x7ff0000000000000ull;
+    return __longlong_as_double((long long)(bits | ((unsigned long long)v & 0x8000000000000000ull)));
+}
+
+// ENO2 value at c, upwind towards c[-d] (d: +-1 column or +-1 row): twice the
+// upwind difference plus the smaller of the two second differences;
+// `inner` false: twice the difference alone (next to a wall).
+__device__ __forceinline__ long long eno_fx(const long long *c, int d, bool inner) {
+    const long long c0 = c[0], c1 = c[-d], D3 = c[d] - c0, D2 = c0 - c1, D1 = c1 - c[-2 * d];
+    const long long S0 = D3 - D2, S1 = D2 - D1;
+    // |S0| > |S1| exactly where S0 - S1 and S0 + S1 have one sign (both not zero;
+    // equal differences may take either)
+    const long long a = S0 - S1, b = S0 + S1;
+    const bool gt = (a ^ b) >= 0 && b != 0;
+    long long s = gt ? S1 : S0;
+    if (!inner) s = 0;
+    return 2 * D2 + s;
+}
+
+// One tile.  PRE: also the combinations for k_source (FP64 handles).
+template <bool PRE>
+__global__ void __launch_bounds__(ATX * ATY, 4)
+    k_advect_fx(step_consts c, advect_fx_consts h, const __grid_constant__ field_maps maps, fields_dev F, int cur,
+                double bv) {
+    extern __shared__ __align__(128) unsigned char fx_raw[];
+    fx_smem &Sm = *reinterpret_cast<fx_smem *>(fx_raw + ((128 - (smem_addr(fx_raw) & 127)) & 127));
     const int m = c.m, n = c.n;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * ATX + tx;
     const int i0 = blockIdx.x * ATX, j0 = blockIdx.y * ATY;
@@ -614,157 +509,164 @@ __global__ void __launch_bounds__(ATX * ATY, 3)
         Sm.col[tid] = w;
         Sm.xs[tid] = u < 0 ? -1 : (u >= m ? 1 : 0);
     }
+    if (tid < F_COUNT + 1) Sm.top[tid] = 0;
     __syncthreads();
     if (tid == 0) {
         mbar_expect_tx(&Sm.bar, kTileBytes);
-        for (int f = 0; f < F_COUNT; f++) tma_load_2d(&Sm.u.tile[f][0][0], &maps.f[cur][f], i0 - 2, j0 - 1, &Sm.bar);
+        for (int f = 0; f < F_COUNT; f++) tma_load_2d(&Sm.t.d[f][0][0], &maps.f[cur][f], i0 - 2, j0 - 1, &Sm.bar);
     }
-    // node velocities of the block as pairs while the tile arrives
+    // node velocities while the tile arrives (at most two per thread)
     if (c.clock) bv = c.clock[CLK_BV_STATE];
-    {
-        const velo_ff V{F.vel, m, n, split_ff(bv)};
-        for (int p = tid; p < (ATY + 1) * (ATX + 1); p += ATX * ATY) {
-            const int r = p / (ATX + 1), cc = p - r * (ATX + 1), nj = j0 + r;
-            if (nj > n) continue;
-            const int ni = Sm.col[cc + 2];
-            Sm.nu[r][cc] = V.u(ni, nj);
-            Sm.nv[r][cc] = V.v(ni, nj);
+    constexpr int kNodes = (ATY + 1) * (ATX + 1), kPer = (kNodes + ATX * ATY - 1) / (ATX * ATY);
+    double2 vel[kPer];
+    unsigned vtop = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+        const int p = tid + q * ATX * ATY, r = p / (ATX + 1), cc = p - r * (ATX + 1), nj = j0 + r;
+        vel[q] = make_double2(0.0, 0.0);
+        if (p < kNodes && nj <= n) {
+            if (nj == 0 || nj == n) vel[q].x = nj == 0 ? -bv : bv;
+            else vel[q] = F.vel[(size_t)nj * m + Sm.col[cc + 2]];
         }
+        vtop = max(vtop, max((unsigned)__double2hiint(vel[q].x) & 0x7fffffffu,
+                             (unsigned)__double2hiint(vel[q].y) & 0x7fffffffu));
     }
     if (__syncthreads_or(!mbar_wait_bounded(&Sm.bar))) {
         if (tid == 0) atomicExch(&F.flags[FL_TMA], 1);
         mbar_wait_bounded(&Sm.bar);
         return;
     }
-    constexpr int kTileVals = F_COUNT * AROWS * ACOLS;
     // columns across the periodic seam arrive as zeros: edge blocks fetch them
     if (i0 == 0 || i0 + ACOLS - 2 > m) {
-        for (int k = tid; k < kTileVals; k += ATX * ATY) {
+        for (int k = tid; k < F_COUNT * AROWS * ACOLS; k += ATX * ATY) {
             const int f = k / (AROWS * ACOLS), rem = k - f * (AROWS * ACOLS), r = rem / ACOLS, t = rem - r * ACOLS;
             const int u = i0 + t - 2, sr = j0 - 1 + r;
-            if ((u < 0 || u >= m) && sr >= 0 && sr <= n + 1) Sm.u.tile[f][r][t] = A[f][(size_t)sr * m + Sm.col[t]];
+            if ((u < 0 || u >= m) && sr >= 0 && sr <= n + 1) Sm.t.d[f][r][t] = A[f][(size_t)sr * m + Sm.col[t]];
         }
         __syncthreads();
     }
-    // split every staged value into a float pair (one position per thread and
-    // pass, all fields: the position's index arithmetic is done once)
-    for (int p = tid; p < AROWS * ACOLS; p += ATX * ATY) {
-        const int r = p / ACOLS, t = p - r * ACOLS;
+    // the largest magnitude of every field and of the velocity
+    {
+        unsigned top[F_COUNT];
+#pragma unroll
+        for (int f = 0; f < F_COUNT; f++) top[f] = 0;
+        for (int p = tid; p < AROWS * ACOLS; p += ATX * ATY) {
+#pragma unroll
+            for (int f = 0; f < F_COUNT; f++)
+                top[f] = max(top[f], (unsigned)__double2hiint((&Sm.t.d[f][0][0])[p]) & 0x7fffffffu);
+        }
 #pragma unroll
         for (int f = 0; f < F_COUNT; f++) {
-            float hh, ll;
-            ff_split_d(Sm.u.tile[f][r][t], hh, ll);
-            Sm.t2[f][r][t] = make_float2(hh, ll);
+            const unsigned w = __reduce_max_sync(0xffffffffu, top[f]);
+            if (tx == 0) atomicMax(&Sm.top[f], w);
         }
+        vtop = __reduce_max_sync(0xffffffffu, vtop);
+        if (tx == 0) atomicMax(&Sm.top[F_COUNT], vtop);
     }
     __syncthreads();
-    // first differences: x on cell rows j0..j0+ATY-1, y on rows j0-2..j0+ATY+1;
-    // X across the periodic seam gets the period (the unwrapped difference)
-    const ff lx{h.lxh, h.lxl};
-    for (int p = tid; p < ATY * ADXW; p += ATX * ATY) {
-        const int r = p / ADXW, cc = p - r * ADXW;
-        const bool live = j0 + r < n;
-        const int sh = Sm.xs[cc + 1] - Sm.xs[cc];
+    int E[F_COUNT], Eu = max((int)(Sm.top[F_COUNT] >> 20), 128);
+    bool finite = Eu < 0x7ff;
+#pragma unroll
+    for (int f = 0; f < F_COUNT; f++) {
+        E[f] = max((int)(Sm.top[f] >> 20), 128);
+        finite = finite && E[f] < 0x7ff;
+    }
+    if (!finite) {  // the same for the whole block
+        if (tid == 0) F.tlist[atomicAdd(F.pcount + 1, 1u)] = blockIdx.y * gridDim.x + blockIdx.x;
+        return;
+    }
+    // the map's values are unwrapped across the seam: room for the period
+    E[F_X] = max(E[F_X], (int)((unsigned)__double2hiint(c.lx) >> 20)) + 1;
+    const long long lx = to_fixed(c.lx, E[F_X]);
+    for (int p = tid; p < AROWS * ACOLS; p += ATX * ATY) {
 #pragma unroll
         for (int f = 0; f < F_COUNT; f++) {
-            ff d{0.f, 0.f};
-            if (live) {
-                const float2 a = Sm.t2[f][r + 2][cc + 1], b = Sm.t2[f][r + 2][cc];
-                d = ff_pair_diff(a.x, a.y, b.x, b.y);
-                if (f == F_X && sh != 0) d = ff_add(d, sh > 0 ? lx : ff_neg(lx));
+            long long v = to_fixed((&Sm.t.d[f][0][0])[p], E[f]);
+            if (f == F_X) {
+                const int sh = Sm.xs[p % ACOLS];
+                if (sh) v += sh > 0 ? lx : -lx;
             }
-            Sm.u.d.dx[f][r][cc] = make_float2(d.hi, d.lo);
+            (&Sm.t.v[f][0][0])[p] = v;
         }
     }
-    for (int p = tid; p < ADYH * ATX; p += ATX * ATY) {
-        const int r = p / ATX, cc = p - r * ATX;
-        const int jj = j0 + r - 2;
-        const bool live = jj >= -1 && jj + 1 <= n && i0 + cc < m;
 #pragma unroll
-        for (int f = 0; f < F_COUNT; f++) {
-            ff d{0.f, 0.f};
-            if (live) {
-                const float2 a = Sm.t2[f][r + 1][cc + 2], b = Sm.t2[f][r][cc + 2];
-                d = ff_pair_diff(a.x, a.y, b.x, b.y);
-            }
-            Sm.u.d.dy[f][r][cc] = make_float2(d.hi, d.lo);
+    for (int q = 0; q < kPer; q++) {
+        const int p = tid + q * ATX * ATY;
+        if (p < kNodes) {
+            (&Sm.nu[0][0])[p] = to_fixed(vel[q].x, Eu);
+            (&Sm.nv[0][0])[p] = to_fixed(vel[q].y, Eu);
         }
     }
     __syncthreads();
     if (i >= m || j >= n) return;
-    const ff hx{h.hxh, h.hxl}, hy{h.hyh, h.hyl};
     const size_t ci = (size_t)(j + 1) * m + i;
-    const eno_ctx e{A, m, n, j0, j, c.lx};
+    const int Ku = Eu + h.he - 2039;  // an increment is its integer times 2^(E + Ku)
+    // |velocity| dt/(2 dx) from four times the velocity: below 2^62
+    auto factor = [](long long u4, long long hm) {
+        return (long long)(__umul64hi((unsigned long long)(u4 < 0 ? -u4 : u4), (unsigned long long)hm) << 3);
+    };
+    auto upwind = [&](int f, long long uh, int dx, long long vh, int dy, bool inner) {
+        const long long *q = &Sm.t.v[f][ty + 2][tx + 2];
+        return -(__mul64hi(uh, eno_fx(q, dx, true)) + __mul64hi(vh, eno_fx(q, dy, inner)));
+    };
+    const long long u00 = Sm.nu[ty][tx], v00 = Sm.nv[ty][tx];
     // reference map at node (i,j), rows 1..n-1 (shear_sim.cc:310-327)
     if (j > 0) {
-        const ff un = Sm.nu[ty][tx], vn = Sm.nv[ty][tx];
-        const bool ru = un.hi > 0.f, rv = vn.hi > 0.f;
-        const ff uh = ff_mul(un, ru ? hx : ff_neg(hx)), vh = ff_mul(vn, rv ? hy : ff_neg(hy));
-        const bool inner = rv ? j > 1 : j < n - 1;
+        const long long uh = factor(4 * u00, h.hmx), vh = factor(4 * v00, h.hmy);
+        const int dx = u00 > 0 ? 1 : -1, dy = v00 > 0 ? ACOLS : -ACOLS;
+        const bool inner = v00 > 0 ? j > 1 : j < n - 1;
 #pragma unroll
-        for (int f = F_X; f <= F_Y; f++) {
-            const ff ex = eno_x_ff(Sm, e, f, ty, tx, ru), ey = eno_y_ff(Sm, e, f, ty, tx, rv, inner);
-            B[f][ci] = add_ff(A[f][ci], upwind_inc(uh, ex, vh, ey));
-        }
+        for (int f = F_X; f <= F_Y; f++)
+            B[f][ci] = A[f][ci] + from_fixed(upwind(f, uh, dx, vh, dy, inner), E[f] + Ku);
     }
-    // staggered velocity and spin (shear_sim.cc:330-333) in pairs
-    const ff u00 = Sm.nu[ty][tx], u10 = Sm.nu[ty][tx + 1], u01 = Sm.nu[ty + 1][tx], u11 = Sm.nu[ty + 1][tx + 1];
-    const ff v00 = Sm.nv[ty][tx], v10 = Sm.nv[ty][tx + 1], v01 = Sm.nv[ty + 1][tx], v11 = Sm.nv[ty + 1][tx + 1];
-    ff uc = ff_add(ff_add(u00, u10), ff_add(u01, u11)), vc = ff_add(ff_add(v00, v10), ff_add(v01, v11));
-    uc = ff{0.25f * uc.hi, 0.25f * uc.lo};
-    vc = ff{0.25f * vc.hi, 0.25f * vc.lo};
-    const ff two_omega = ff_sub(ff_mul(hx, ff_add(ff_sub(v10, v00), ff_sub(v11, v01))),
-                                ff_mul(hy, ff_add(ff_sub(u01, u00), ff_sub(u11, u10))));
-    const bool ru = uc.hi > 0.f, rv = vc.hi > 0.f;
-    const ff uh = ff_mul(uc, ru ? hx : ff_neg(hx)), vh = ff_mul(vc, rv ? hy : ff_neg(hy));
-    const bool inner = rv ? j > 0 : j < n - 1;
-    auto inc_of = [&](int f) {
-        return upwind_inc(uh, eno_x_ff(Sm, e, f, ty, tx, ru), vh, eno_y_ff(Sm, e, f, ty, tx, rv, inner));
-    };
-    const float2 q2 = Sm.t2[F_Q][ty + 2][tx + 2], s2 = Sm.t2[F_S][ty + 2][tx + 2], t2 = Sm.t2[F_TAU][ty + 2][tx + 2];
-    const ff qf{q2.x, q2.y}, sf{s2.x, s2.y}, tf{t2.x, t2.y};
-    const double ddev = 0;
-    // chi first, then p, q, s, tau
+    // staggered velocity and spin (shear_sim.cc:330-333)
+    const long long u10 = Sm.nu[ty][tx + 1], u01 = Sm.nu[ty + 1][tx], u11 = Sm.nu[ty + 1][tx + 1];
+    const long long v10 = Sm.nv[ty][tx + 1], v01 = Sm.nv[ty + 1][tx], v11 = Sm.nv[ty + 1][tx + 1];
+    const long long u4 = (u00 + u10) + (u01 + u11), v4 = (v00 + v10) + (v01 + v11);
+    const double two_omega = from_fixed(__mul64hi((v10 - v00) + (v11 - v01), h.hmx) -
+                                            __mul64hi((u01 - u00) + (u11 - u10), h.hmy),
+                                        64 + Eu - 1081 + h.he);
+    const long long uh = factor(u4, h.hmx), vh = factor(v4, h.hmy);
+    const int dx = u4 > 0 ? 1 : -1, dy = v4 > 0 ? ACOLS : -ACOLS;
+    const bool inner = v4 > 0 ? j > 0 : j < n - 1;
+    double a[5], v[5];
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
-        const int f = k == 0 ? F_CHI : k - 1;
-        ff inc = inc_of(f);
-        if (f == F_S) inc = ff_add(inc, ff_mul(two_omega, tf));
-        else if (f == F_TAU) inc = ff_sub(inc, ff_mul(two_omega, sf));
-        const double a0 = A[f][ci];
-        double v = add_ff(a0, inc);
-        if (f == F_CHI) {
-            // Yield test: 3q^2 + s^2 + tau^2 in pairs (relative error ~2^-44);
-            // a cell clearly below the cut-offs of k_advect (1e-24, or an
-            // athermal law below yield) is elastic there too; any other cell
-            // takes k_advect's FP64 path.
-            const ff dsq = ff_add(ff_mul(ff{3.f, 0.f}, ff_mul(qf, qf)), ff_add(ff_mul(sf, sf), ff_mul(tf, tf)));
-            const float dv = dsq.hi + dsq.lo;
-            const bool athermal = c.stz_model >= 2;
-            const bool clearly_elastic = dv < 0.999e-24f * (1.f - 1e-6f) || (athermal && dv < c.yield_cut2f);
-            // the FP64 test and the plastic law run in k_plastic_ff, on the
-            // listed cells after this kernel (kept out of this one, whose
-            // registers they would otherwise set)
-            if (!clearly_elastic) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
-            F.ddev[ci] = ddev;
-        }
-        B[f][ci] = v;
+    for (int f = 0; f < 5; f++) a[f] = A[f][ci];
+#pragma unroll
+    for (int f = 0; f < 5; f++) {
+        double inc = from_fixed(upwind(f, uh, dx, vh, dy, inner), E[f] + Ku);
+        if (f == F_S) inc = fma(two_omega, a[F_TAU], inc);
+        else if (f == F_TAU) inc = fma(-two_omega, a[F_S], inc);
+        v[f] = a[f] + inc;
+        B[f][ci] = v[f];
     }
+    // Yield test on the leading 24 bits: 3q^2 + s^2 + tau^2 within 5e-7; a cell
+    // clearly below the cut-offs of k_advect (1e-24, or an athermal law below
+    // yield) is elastic there too, any other one takes the FP64 test and law.
+    const float qf = ff_hi(a[F_Q]), sf = ff_hi(a[F_S]), tf = ff_hi(a[F_TAU]);
+    const float dv = 3.f * qf * qf + sf * sf + tf * tf;
+    const bool elastic = dv < 0.999e-24f * (1.f - 1e-6f) || (c.stz_model >= 2 && dv < c.yield_cut2f);
+    if (!elastic) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
+    F.ddev[ci] = 0;
+    if (PRE) write_pre(F, ci, h.xf, h.yf, v[F_P], v[F_Q], v[F_S], v[F_TAU]);
 }
 
-// The plastic part of the float-float step for the cells k_advect_ff listed:
-// k_advect's FP64 yield test and, above the cut-offs, the FP64 plastic law
-// (adaptive_plastic_term, shear_sim.cc:513-548) on the advected chi, then
-// q, s, tau -= dtmp times their old values, ddev and the plastic strain.  The
-// same operations in the same order as k_advect, so the cell ends where the
-// one-pass form would take it.
-__global__ void k_plastic_ff(step_consts c, fields_dev F, int cur, double dt) {
+// What k_advect_fx left: the listed cells' plastic part (k_advect's FP64 yield
+// test and, above the cut-offs, the FP64 plastic law,
+// adaptive_plastic_term, shear_sim.cc:513-548, on the advected chi, then
+// q, s, tau -= dtmp times their old values, ddev and the plastic strain: the
+// same operations in the same order, so the cell ends where the one-pass form
+// would take it) and the listed tiles, with k_advect's arithmetic.
+__global__ void __launch_bounds__(ATX * ATY)
+    k_advect_rest(step_consts c, advect_consts a, const __grid_constant__ field_maps maps, fields_dev F, int cur,
+                  double dt, double bv, int emit_source, int tiles_x) {
     if (c.clock) cur = (int)c.clock[CLK_CUR];
-    const unsigned cnt = *F.pcount;
+    const unsigned cnt = F.pcount[0], tiles = F.pcount[1];
     const double *__restrict__ const *A = F.f[cur];
     double *const *B = F.f[cur ^ 1];
     const bool athermal = c.stz_model >= 2;
-    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
+    const int tid = threadIdx.y * ATX + threadIdx.x;
+    for (unsigned k = blockIdx.x * (ATX * ATY) + tid; k < cnt; k += gridDim.x * (ATX * ATY)) {
         const size_t ci = F.plist[k];
         const double q = A[F_Q][ci], s = A[F_S][ci], t = A[F_TAU][ci];
         const double devsq = 3 * q * q + s * s + t * t;
@@ -784,10 +686,17 @@ __global__ void k_plastic_ff(step_consts c, fields_dev F, int cur, double dt) {
             F.eps_pl[(size_t)j * m + i] += ddev / (2 * c.mu);
         }
         if (dtmp != 0) {
-            B[F_Q][ci] -= dtmp * q;
-            B[F_S][ci] -= dtmp * s;
-            B[F_TAU][ci] -= dtmp * t;
+            const double qn = B[F_Q][ci] - dtmp * q, sn = B[F_S][ci] - dtmp * s, tn = B[F_TAU][ci] - dtmp * t;
+            B[F_Q][ci] = qn;
+            B[F_S][ci] = sn;
+            B[F_TAU][ci] = tn;
+            if (emit_source) write_pre(F, ci, a.xf, a.yf, B[F_P][ci], qn, sn, tn);
         }
+    }
+    for (unsigned k = blockIdx.x, it = 0; k < tiles; k += gridDim.x, it++) {
+        const unsigned tile = F.tlist[k];
+        if (!advect_tile(c, a, maps, F, cur, dt, bv, emit_source, tile % tiles_x, tile / tiles_x, it)) return;
+        __syncthreads();  // the next tile reuses the shared memory
     }
 }
 
@@ -1160,6 +1069,8 @@ inline dim3 g2(int m, int n, dim3 b) { return dim3(ceil_div(m, b.x), ceil_div(n,
 
 }  // namespace
 
+size_t tile_count(const step_consts &c) { return (size_t)ceil_div(c.m, ATX) * ceil_div(c.n, ATY); }
+
 cudaError_t prepare_step_kernels() {
     static unsigned long long done = 0;  // per device ordinal
     int dev = 0;
@@ -1168,8 +1079,8 @@ cudaError_t prepare_step_kernels() {
     if (dev < 64 && (done >> dev & 1)) return cudaSuccess;
     e = cudaFuncSetAttribute(k_advect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(adv_smem) + 128));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_advect_ff, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(adv_smem_ff) + 128));
+        e = cudaFuncSetAttribute(k_advect_rest, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(adv_smem) + 128));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(direct_tile));
     if (e == cudaSuccess && dev < 64) done |= 1ull << dev;
@@ -1216,15 +1127,25 @@ void advection(const step_consts &c, const field_maps &maps, fields_dev &F, int 
     a.xf = 0.5 / dt * c.xsp;
     a.yf = 0.5 / dt * c.ysp;
     const dim3 grid(ceil_div(c.m, ATX), ceil_div(c.n, ATY));
-    if (c.sp_increments) {
-        advect_ff_consts h;
-        split_host(a.hx, &h.hxh, &h.hxl);
-        split_host(a.hy, &h.hyh, &h.hyl);
-        split_host(c.lx, &h.lxh, &h.lxl);
-        cudaMemsetAsync(F.pcount, 0, sizeof(unsigned), st);
-        k_advect_ff<<<grid, dim3(ATX, ATY), sizeof(adv_smem_ff) + 128, st>>>(c, h, maps, F, cur, dt, bv);
+    if (c.fixed_point) {
+        advect_fx_consts h;
+        int ex, ey;
+        std::frexp(a.hx, &ex);
+        std::frexp(a.hy, &ey);
+        h.he = std::max(ex, ey) - 62;
+        h.hmx = (long long)std::ldexp(a.hx, -h.he);
+        h.hmy = (long long)std::ldexp(a.hy, -h.he);
+        h.xf = a.xf;
+        h.yf = a.yf;
+        const int pre = !c.sp_increments;
+        cudaMemsetAsync(F.pcount, 0, 2 * sizeof(unsigned), st);
+        if (pre)
+            k_advect_fx<true><<<grid, dim3(ATX, ATY), sizeof(fx_smem) + 128, st>>>(c, h, maps, F, cur, bv);
+        else
+            k_advect_fx<false><<<grid, dim3(ATX, ATY), sizeof(fx_smem) + 128, st>>>(c, h, maps, F, cur, bv);
         note_launch();
-        k_plastic_ff<<<2 * 152, 256, 0, st>>>(c, F, cur, dt);
+        k_advect_rest<<<2 * 152, dim3(ATX, ATY), sizeof(adv_smem) + 128, st>>>(c, a, maps, F, cur, dt, bv, pre,
+                                                                              (int)grid.x);
     } else {
         k_advect<<<grid, dim3(ATX, ATY), sizeof(adv_smem) + 128, st>>>(c, a, maps, F, cur, dt, bv, 1);
     }

@@ -43,9 +43,10 @@ struct fields_dev {
     // U = xf A + yf tau, W = xf A - yf tau, Y1 = xf tau - yf B,
     // Y2 = xf tau + yf B, A = p+q-s, B = p+q+s (xf, yf of projection_step).
     double *pre[4];
-    // Float-float advection: cells that the pair yield test cannot certify as
-    // elastic (their index, then their count), for the FP64 plastic pass.
+    // Fixed-point advection: cells that its yield test cannot certify as elastic,
+    // tiles with a value that is not finite, and their counts (two words).
     unsigned *plist;
+    unsigned *tlist;
     unsigned *pcount;
 };
 
@@ -60,14 +61,17 @@ struct step_consts {
     int track_plastic;
     int substep_cap;
     double yield_cut2;  // s_y^2 (1 - 1e-12): athermal cells below it skip the plastic loop
-    float yield_cut2f;  // the same lowered by 1e-6, for the float-float path's test
+    float yield_cut2f;  // the same lowered by 1e-6, for the fixed-point path's test
     // Device clock of a graph-driven run (nullptr: wall quantities come as
     // kernel arguments from the host).  Layout: CLK_* below.
     const double *clock;
     double xbc;  // bcs*cxx of the projection operator (wall source = -+xbc*bv)
-    // advection, projection source and stress correction in float-float on
-    // the FP64 state (mixed-precision handles); 0: all FP64, bit-exact
+    // projection source and stress correction in float-float on the FP64 state
+    // (mixed-precision handles); 0: FP64
     int sp_increments;
+    // advection in 64-bit fixed point (k_advect_fx); 0: FP64, bit-exact with the
+    // per-point ENO2
+    int fixed_point;
 };
 
 // Device clock slots: time, wall speed of the stored state, wall speed and
@@ -75,6 +79,8 @@ struct step_consts {
 // CLK_CUR holds the state buffer index at the start of the step.
 enum { CLK_TIME = 0, CLK_BV_STATE = 1, CLK_BV = 2, CLK_BP = 3, CLK_CUR = 4, CLK_COUNT = 5 };
 
+// Tiles of the advection kernels.
+size_t tile_count(const step_consts &c);
 step_consts make_step_consts(const stz_params &p);
 // x as a float pair hi + lo (host).
 void split_host(double x, float *hi, float *lo);
