@@ -272,7 +272,7 @@ __device__ __forceinline__ void write_pre(const fields_dev &F, size_t ci, double
 
 // One tile (bx, by) in FP64; `use`: how often the block has done this before
 // (the barrier's phase).  False when a tile copy did not arrive.
-__device__ __forceinline__ bool advect_tile(const step_consts &c, const advect_consts &a, const field_maps &maps,
+__device__ __forceinline__ bool advect_tile(const step_consts &c, const advect_consts &a, const field_boxes &maps,
                                             const fields_dev &F, int cur, double dt, double bv, int emit_source, int bx,
                                             int by, unsigned use) {
     extern __shared__ __align__(128) unsigned char adv_raw[];
@@ -396,7 +396,7 @@ __device__ __forceinline__ bool advect_tile(const step_consts &c, const advect_c
     return true;
 }
 
-__global__ void __launch_bounds__(ATX * ATY) k_advect(step_consts c, advect_consts a, const __grid_constant__ field_maps maps,
+__global__ void __launch_bounds__(ATX * ATY) k_advect(step_consts c, advect_consts a, const __grid_constant__ field_boxes maps,
                                                       fields_dev F, int cur, double dt, double bv, int emit_source) {
     if (c.clock) cur = (int)c.clock[CLK_CUR];
     advect_tile(c, a, maps, F, cur, dt, bv, emit_source, blockIdx.x, blockIdx.y, 0);
@@ -431,12 +431,17 @@ __device__ __forceinline__ double add_ff(double a, ff inc) { return a + ff_to_d(
 // Tiles with an infinity or a NaN in a field or the velocity are listed and
 // take k_advect's arithmetic in k_advect_rest, as do the cells that the yield
 // test (on the leading 24 bits, with a margin) cannot certify as elastic.
+// A block takes 32 x 16 cells, two rows of eight threads after one another: the
+// staged halo is 1.4 times the cells (1.7 at 32 x 8, where converting it was a
+// fifth of the kernel).
+constexpr int FXY = 2 * ATY, FROWS = FXY + 4;
+constexpr unsigned kFxBytes = F_COUNT * FROWS * ACOLS * sizeof(double);
 struct fx_smem {
     union {
-        double d[F_COUNT][AROWS][ACOLS];  // TMA destination (128-byte aligned)
-        long long v[F_COUNT][AROWS][ACOLS];
+        double d[F_COUNT][FROWS][ACOLS];  // TMA destination (128-byte aligned)
+        long long v[F_COUNT][FROWS][ACOLS];
     } t;
-    long long nu[ATY + 1][ATX + 1], nv[ATY + 1][ATX + 1];  // node velocities, walls substituted
+    long long nu[FXY + 1][ATX + 1], nv[FXY + 1][ATX + 1];  // node velocities, walls substituted
     unsigned top[F_COUNT + 1];  // largest high word's magnitude per field; then of the velocity
     int xs[ACOLS], col[ACOLS];  // period shift and storage column of tile column c-2
     uint64_t bar;
@@ -460,44 +465,57 @@ __device__ __forceinline__ long long to_fixed(double d, int E) {
     return (int)hi < 0 ? -v : v;
 }
 
-// v 2^K as a double, rounded to nearest (ties up in magnitude).
-__device__ __forceinline__ double from_fixed(long long v, int K) {
-    const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
-    const int lz = __clzll((long long)m), e = 1023 + 63 - lz + K;
-    const unsigned long long w = m << (lz & 63);
-    const unsigned long long r = (w >> 11) + ((w >> 10) & 1);
-    unsigned long long bits = ((unsigned long long)(unsigned)(e - 1) << 52) + r;  // r carries the implicit bit
-    if (m == 0 || e <= 0) bits = 0;
-    if (e >= 2047) bits = 0x7ff0000000000000ull;
-    return __longlong_as_double((long long)(bits | ((unsigned long long)v & 0x8000000000000000ull)));
+// 2^K as a double (0 below the normal range, infinity above).
+__device__ __forceinline__ double power_of_two(int K) {
+    const int e = min(max(K + 1023, 0), 0x7ff);
+    return __hiloint2double(e << 20, 0);
 }
 
 // ENO2 value at c, upwind towards c[-d] (d: +-1 column or +-1 row): twice the
 // upwind difference plus the smaller of the two second differences;
 // `inner` false: twice the difference alone (next to a wall).
 __device__ __forceinline__ long long eno_fx(const long long *c, int d, bool inner) {
-    const long long c0 = c[0], c1 = c[-d], D3 = c[d] - c0, D2 = c0 - c1, D1 = c1 - c[-2 * d];
-    const long long S0 = D3 - D2, S1 = D2 - D1;
+    const long long c0 = c[0], c1 = c[-d], D2 = c0 - c1;
+    const long long S0 = c[d] - c0 - D2, S1 = D2 - c1 + c[-2 * d];
     // |S0| > |S1| exactly where S0 - S1 and S0 + S1 have one sign (both not zero;
     // equal differences may take either)
     const long long a = S0 - S1, b = S0 + S1;
     const bool gt = (a ^ b) >= 0 && b != 0;
     long long s = gt ? S1 : S0;
     if (!inner) s = 0;
-    return 2 * D2 + s;
+    return D2 + D2 + s;
+}
+
+// |velocity| dt/(2 dx) from four times the velocity, below 2^60, in two words
+// whose lower one is halved (its last bit is dropped), so that the products
+// below are signed 32 x 32 bit ones.
+struct fx_factor {
+    int hi, lo;
+    __device__ __forceinline__ fx_factor(long long u4, long long hm) {
+        const unsigned long long w =
+            __umul64hi((unsigned long long)(u4 < 0 ? -u4 : u4), (unsigned long long)hm) << 1;
+        hi = (int)(w >> 32);
+        lo = (int)((unsigned)w >> 1);
+    }
+};
+// (u a + v b) / 2^64 within three units: |a|, |b| <= 2^62.
+__device__ __forceinline__ long long fx_products(const fx_factor &u, long long a, const fx_factor &v, long long b) {
+    const int a1 = (int)(a >> 32), b1 = (int)(b >> 32), a0 = (int)((unsigned)a >> 1), b0 = (int)((unsigned)b >> 1);
+    const long long mid = (long long)u.lo * a1 + (long long)u.hi * a0 + (long long)v.lo * b1 + (long long)v.hi * b0;
+    return (long long)u.hi * a1 + (long long)v.hi * b1 + (mid >> 31);
 }
 
 // One tile.  PRE: also the combinations for k_source (FP64 handles).
 template <bool PRE>
 __global__ void __launch_bounds__(ATX * ATY, 4)
-    k_advect_fx(step_consts c, advect_fx_consts h, const __grid_constant__ field_maps maps, fields_dev F, int cur,
+    k_advect_fx(step_consts c, advect_fx_consts h, const __grid_constant__ field_boxes maps, fields_dev F, int cur,
                 double bv) {
     extern __shared__ __align__(128) unsigned char fx_raw[];
     fx_smem &Sm = *reinterpret_cast<fx_smem *>(fx_raw + ((128 - (smem_addr(fx_raw) & 127)) & 127));
     const int m = c.m, n = c.n;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * ATX + tx;
-    const int i0 = blockIdx.x * ATX, j0 = blockIdx.y * ATY;
-    const int i = i0 + tx, j = j0 + ty;
+    const int i0 = blockIdx.x * ATX, j0 = blockIdx.y * FXY;
+    const int i = i0 + tx;
     if (c.clock) cur = (int)c.clock[CLK_CUR];
     const double *__restrict__ const *A = F.f[cur];
     double *const *B = F.f[cur ^ 1];
@@ -512,12 +530,12 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
     if (tid < F_COUNT + 1) Sm.top[tid] = 0;
     __syncthreads();
     if (tid == 0) {
-        mbar_expect_tx(&Sm.bar, kTileBytes);
+        mbar_expect_tx(&Sm.bar, kFxBytes);
         for (int f = 0; f < F_COUNT; f++) tma_load_2d(&Sm.t.d[f][0][0], &maps.f[cur][f], i0 - 2, j0 - 1, &Sm.bar);
     }
-    // node velocities while the tile arrives (at most two per thread)
+    // node velocities while the tile arrives (at most three per thread)
     if (c.clock) bv = c.clock[CLK_BV_STATE];
-    constexpr int kNodes = (ATY + 1) * (ATX + 1), kPer = (kNodes + ATX * ATY - 1) / (ATX * ATY);
+    constexpr int kNodes = (FXY + 1) * (ATX + 1), kPer = (kNodes + ATX * ATY - 1) / (ATX * ATY);
     double2 vel[kPer];
     unsigned vtop = 0;
 #pragma unroll
@@ -538,8 +556,8 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
     }
     // columns across the periodic seam arrive as zeros: edge blocks fetch them
     if (i0 == 0 || i0 + ACOLS - 2 > m) {
-        for (int k = tid; k < F_COUNT * AROWS * ACOLS; k += ATX * ATY) {
-            const int f = k / (AROWS * ACOLS), rem = k - f * (AROWS * ACOLS), r = rem / ACOLS, t = rem - r * ACOLS;
+        for (int k = tid; k < F_COUNT * FROWS * ACOLS; k += ATX * ATY) {
+            const int f = k / (FROWS * ACOLS), rem = k - f * (FROWS * ACOLS), r = rem / ACOLS, t = rem - r * ACOLS;
             const int u = i0 + t - 2, sr = j0 - 1 + r;
             if ((u < 0 || u >= m) && sr >= 0 && sr <= n + 1) Sm.t.d[f][r][t] = A[f][(size_t)sr * m + Sm.col[t]];
         }
@@ -550,7 +568,7 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         unsigned top[F_COUNT];
 #pragma unroll
         for (int f = 0; f < F_COUNT; f++) top[f] = 0;
-        for (int p = tid; p < AROWS * ACOLS; p += ATX * ATY) {
+        for (int p = tid; p < FROWS * ACOLS; p += ATX * ATY) {
 #pragma unroll
             for (int f = 0; f < F_COUNT; f++)
                 top[f] = max(top[f], (unsigned)__double2hiint((&Sm.t.d[f][0][0])[p]) & 0x7fffffffu);
@@ -572,13 +590,15 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         finite = finite && E[f] < 0x7ff;
     }
     if (!finite) {  // the same for the whole block
-        if (tid == 0) F.tlist[atomicAdd(F.pcount + 1, 1u)] = blockIdx.y * gridDim.x + blockIdx.x;
+        // two of k_advect's tiles
+        if (tid < 2 && j0 + tid * ATY < n)
+            F.tlist[atomicAdd(F.pcount + 1, 1u)] = (2 * blockIdx.y + tid) * gridDim.x + blockIdx.x;
         return;
     }
     // the map's values are unwrapped across the seam: room for the period
     E[F_X] = max(E[F_X], (int)((unsigned)__double2hiint(c.lx) >> 20)) + 1;
     const long long lx = to_fixed(c.lx, E[F_X]);
-    for (int p = tid; p < AROWS * ACOLS; p += ATX * ATY) {
+    for (int p = tid; p < FROWS * ACOLS; p += ATX * ATY) {
 #pragma unroll
         for (int f = 0; f < F_COUNT; f++) {
             long long v = to_fixed((&Sm.t.d[f][0][0])[p], E[f]);
@@ -598,57 +618,58 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         }
     }
     __syncthreads();
-    if (i >= m || j >= n) return;
-    const size_t ci = (size_t)(j + 1) * m + i;
-    const int Ku = Eu + h.he - 2039;  // an increment is its integer times 2^(E + Ku)
-    // |velocity| dt/(2 dx) from four times the velocity: below 2^62
-    auto factor = [](long long u4, long long hm) {
-        return (long long)(__umul64hi((unsigned long long)(u4 < 0 ? -u4 : u4), (unsigned long long)hm) << 3);
-    };
-    auto upwind = [&](int f, long long uh, int dx, long long vh, int dy, bool inner) {
-        const long long *q = &Sm.t.v[f][ty + 2][tx + 2];
-        return -(__mul64hi(uh, eno_fx(q, dx, true)) + __mul64hi(vh, eno_fx(q, dy, inner)));
-    };
-    const long long u00 = Sm.nu[ty][tx], v00 = Sm.nv[ty][tx];
-    // reference map at node (i,j), rows 1..n-1 (shear_sim.cc:310-327)
-    if (j > 0) {
-        const long long uh = factor(4 * u00, h.hmx), vh = factor(4 * v00, h.hmy);
-        const int dx = u00 > 0 ? 1 : -1, dy = v00 > 0 ? ACOLS : -ACOLS;
-        const bool inner = v00 > 0 ? j > 1 : j < n - 1;
+    if (i >= m) return;
+    const int Ku = Eu + h.he - 2037;  // an increment is its integer times -2^(E + Ku)
+#pragma unroll 1
+    for (int row = ty; row < FXY; row += ATY) {
+        const int j = j0 + row;
+        if (j >= n) return;
+        const size_t ci = (size_t)(j + 1) * m + i;
+        auto upwind = [&](int f, const fx_factor &uh, int dx, const fx_factor &vh, int dy, bool inner) {
+            const long long *q = &Sm.t.v[f][row + 2][tx + 2];
+            return fx_products(uh, eno_fx(q, dx, true), vh, eno_fx(q, dy, inner));
+        };
+        const long long u00 = Sm.nu[row][tx], v00 = Sm.nv[row][tx];
+        // reference map at node (i,j), rows 1..n-1 (shear_sim.cc:310-327)
+        if (j > 0) {
+            const fx_factor uh(4 * u00, h.hmx), vh(4 * v00, h.hmy);
+            const int dx = u00 > 0 ? 1 : -1, dy = v00 > 0 ? ACOLS : -ACOLS;
+            const bool inner = v00 > 0 ? j > 1 : j < n - 1;
 #pragma unroll
-        for (int f = F_X; f <= F_Y; f++)
-            B[f][ci] = A[f][ci] + from_fixed(upwind(f, uh, dx, vh, dy, inner), E[f] + Ku);
+            for (int f = F_X; f <= F_Y; f++)
+                B[f][ci] = fma((double)upwind(f, uh, dx, vh, dy, inner), -power_of_two(E[f] + Ku), A[f][ci]);
+        }
+        // staggered velocity and spin (shear_sim.cc:330-333)
+        const long long u10 = Sm.nu[row][tx + 1], u01 = Sm.nu[row + 1][tx], u11 = Sm.nu[row + 1][tx + 1];
+        const long long v10 = Sm.nv[row][tx + 1], v01 = Sm.nv[row + 1][tx], v11 = Sm.nv[row + 1][tx + 1];
+        const long long u4 = (u00 + u10) + (u01 + u11), v4 = (v00 + v10) + (v01 + v11);
+        const double two_omega = (double)(__mul64hi((v10 - v00) + (v11 - v01), h.hmx) -
+                                          __mul64hi((u01 - u00) + (u11 - u10), h.hmy)) *
+                                 power_of_two(64 + Eu - 1081 + h.he);
+        const fx_factor uh(u4, h.hmx), vh(v4, h.hmy);
+        const int dx = u4 > 0 ? 1 : -1, dy = v4 > 0 ? ACOLS : -ACOLS;
+        const bool inner = v4 > 0 ? j > 0 : j < n - 1;
+        double a[5], v[5];
+#pragma unroll
+        for (int f = 0; f < 5; f++) a[f] = A[f][ci];
+#pragma unroll
+        for (int f = 0; f < 5; f++) {
+            const double inc = (double)upwind(f, uh, dx, vh, dy, inner), sc = -power_of_two(E[f] + Ku);
+            if (f == F_S) v[f] = a[f] + fma(inc, sc, two_omega * a[F_TAU]);
+            else if (f == F_TAU) v[f] = a[f] + fma(inc, sc, -two_omega * a[F_S]);
+            else v[f] = fma(inc, sc, a[f]);
+            B[f][ci] = v[f];
+        }
+        // Yield test on the leading 24 bits: 3q^2 + s^2 + tau^2 within 5e-7; a cell
+        // clearly below the cut-offs of k_advect (1e-24, or an athermal law below
+        // yield) is elastic there too, any other one takes the FP64 test and law.
+        const float qf = ff_hi(a[F_Q]), sf = ff_hi(a[F_S]), tf = ff_hi(a[F_TAU]);
+        const float dv = 3.f * qf * qf + sf * sf + tf * tf;
+        const bool elastic = dv < 0.999e-24f * (1.f - 1e-6f) || (c.stz_model >= 2 && dv < c.yield_cut2f);
+        if (!elastic) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
+        F.ddev[ci] = 0;
+        if (PRE) write_pre(F, ci, h.xf, h.yf, v[F_P], v[F_Q], v[F_S], v[F_TAU]);
     }
-    // staggered velocity and spin (shear_sim.cc:330-333)
-    const long long u10 = Sm.nu[ty][tx + 1], u01 = Sm.nu[ty + 1][tx], u11 = Sm.nu[ty + 1][tx + 1];
-    const long long v10 = Sm.nv[ty][tx + 1], v01 = Sm.nv[ty + 1][tx], v11 = Sm.nv[ty + 1][tx + 1];
-    const long long u4 = (u00 + u10) + (u01 + u11), v4 = (v00 + v10) + (v01 + v11);
-    const double two_omega = from_fixed(__mul64hi((v10 - v00) + (v11 - v01), h.hmx) -
-                                            __mul64hi((u01 - u00) + (u11 - u10), h.hmy),
-                                        64 + Eu - 1081 + h.he);
-    const long long uh = factor(u4, h.hmx), vh = factor(v4, h.hmy);
-    const int dx = u4 > 0 ? 1 : -1, dy = v4 > 0 ? ACOLS : -ACOLS;
-    const bool inner = v4 > 0 ? j > 0 : j < n - 1;
-    double a[5], v[5];
-#pragma unroll
-    for (int f = 0; f < 5; f++) a[f] = A[f][ci];
-#pragma unroll
-    for (int f = 0; f < 5; f++) {
-        double inc = from_fixed(upwind(f, uh, dx, vh, dy, inner), E[f] + Ku);
-        if (f == F_S) inc = fma(two_omega, a[F_TAU], inc);
-        else if (f == F_TAU) inc = fma(-two_omega, a[F_S], inc);
-        v[f] = a[f] + inc;
-        B[f][ci] = v[f];
-    }
-    // Yield test on the leading 24 bits: 3q^2 + s^2 + tau^2 within 5e-7; a cell
-    // clearly below the cut-offs of k_advect (1e-24, or an athermal law below
-    // yield) is elastic there too, any other one takes the FP64 test and law.
-    const float qf = ff_hi(a[F_Q]), sf = ff_hi(a[F_S]), tf = ff_hi(a[F_TAU]);
-    const float dv = 3.f * qf * qf + sf * sf + tf * tf;
-    const bool elastic = dv < 0.999e-24f * (1.f - 1e-6f) || (c.stz_model >= 2 && dv < c.yield_cut2f);
-    if (!elastic) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
-    F.ddev[ci] = 0;
-    if (PRE) write_pre(F, ci, h.xf, h.yf, v[F_P], v[F_Q], v[F_S], v[F_TAU]);
 }
 
 // What k_advect_fx left: the listed cells' plastic part (k_advect's FP64 yield
@@ -658,7 +679,7 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
 // same operations in the same order, so the cell ends where the one-pass form
 // would take it) and the listed tiles, with k_advect's arithmetic.
 __global__ void __launch_bounds__(ATX * ATY)
-    k_advect_rest(step_consts c, advect_consts a, const __grid_constant__ field_maps maps, fields_dev F, int cur,
+    k_advect_rest(step_consts c, advect_consts a, const __grid_constant__ field_boxes maps, fields_dev F, int cur,
                   double dt, double bv, int emit_source, int tiles_x) {
     if (c.clock) cur = (int)c.clock[CLK_CUR];
     const unsigned cnt = F.pcount[0], tiles = F.pcount[1];
@@ -1079,6 +1100,12 @@ cudaError_t prepare_step_kernels() {
     if (dev < 64 && (done >> dev & 1)) return cudaSuccess;
     e = cudaFuncSetAttribute(k_advect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(adv_smem) + 128));
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_advect_fx<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(fx_smem) + 128));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_advect_fx<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(fx_smem) + 128));
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_advect_rest, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(adv_smem) + 128));
     if (e == cudaSuccess)
@@ -1105,16 +1132,18 @@ int make_field_maps(const step_consts &c, const fields_dev &F, field_maps *out) 
     if ((c.m * sizeof(double)) % 16 != 0) return fail(STZG_EINVAL, "tile copies need an even m");
     const cuuint64_t dims[2] = {(cuuint64_t)c.m, (cuuint64_t)c.n + 2};
     const cuuint64_t strides[1] = {(cuuint64_t)c.m * sizeof(double)};
-    const cuuint32_t box[2] = {ACOLS, AROWS};
     const cuuint32_t estr[2] = {1, 1};
-    for (int b = 0; b < 2; b++)
-        for (int f = 0; f < F_COUNT; f++) {
-            if (((uintptr_t)F.f[b][f]) % 16 != 0) return fail(STZG_EINVAL, "field not 16-byte aligned");
-            const CUresult r = encode(&out->f[b][f], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void *)F.f[b][f], dims,
-                                      strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return fail(STZG_ECUDA, "cuTensorMapEncodeTiled failed");
-        }
+    for (int k = 0; k < 4 * F_COUNT; k++) {
+        const int b = k & 1, f = k / 4;
+        const bool tall = k & 2;
+        const cuuint32_t box[2] = {ACOLS, (cuuint32_t)(tall ? FROWS : AROWS)};
+        if (((uintptr_t)F.f[b][f]) % 16 != 0) return fail(STZG_EINVAL, "field not 16-byte aligned");
+        const CUresult r =
+            encode(tall ? &out->tall.f[b][f] : &out->f[b][f], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void *)F.f[b][f],
+                   dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(STZG_ECUDA, "cuTensorMapEncodeTiled failed");
+    }
     return STZG_OK;
 }
 
@@ -1138,11 +1167,12 @@ void advection(const step_consts &c, const field_maps &maps, fields_dev &F, int 
         h.xf = a.xf;
         h.yf = a.yf;
         const int pre = !c.sp_increments;
+        const dim3 fgrid(grid.x, ceil_div(c.n, FXY));
         cudaMemsetAsync(F.pcount, 0, 2 * sizeof(unsigned), st);
         if (pre)
-            k_advect_fx<true><<<grid, dim3(ATX, ATY), sizeof(fx_smem) + 128, st>>>(c, h, maps, F, cur, bv);
+            k_advect_fx<true><<<fgrid, dim3(ATX, ATY), sizeof(fx_smem) + 128, st>>>(c, h, maps.tall, F, cur, bv);
         else
-            k_advect_fx<false><<<grid, dim3(ATX, ATY), sizeof(fx_smem) + 128, st>>>(c, h, maps, F, cur, bv);
+            k_advect_fx<false><<<fgrid, dim3(ATX, ATY), sizeof(fx_smem) + 128, st>>>(c, h, maps.tall, F, cur, bv);
         note_launch();
         k_advect_rest<<<2 * 152, dim3(ATX, ATY), sizeof(adv_smem) + 128, st>>>(c, a, maps, F, cur, dt, bv, pre,
                                                                               (int)grid.x);

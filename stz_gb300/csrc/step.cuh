@@ -115,8 +115,11 @@ __device__ __forceinline__ double eno2(double p0, double p1, double p2, double p
 // FP64 tensors of m x (n+2) (rows -1..n), box of the advection tile (36
 // columns x 12 rows).  Built once per simulation; the pointers of F must not
 // change afterwards.
-struct field_maps {
+struct field_boxes {
     CUtensorMap f[2][F_COUNT];
+};
+struct field_maps : field_boxes {
+    field_boxes tall;  // the fixed-point kernel's boxes, 36 columns x 20 rows
 };
 int make_field_maps(const step_consts &c, const fields_dev &F, field_maps *out);
 // F.flags[FL_TMA] is set when a tile's copy wait runs out (status, no fault); that
