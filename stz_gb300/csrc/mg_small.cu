@@ -17,6 +17,7 @@
 #include "mg.cuh"
 #include "mg_device.cuh"
 #include "mg_plan.h"
+#include "mg_env.cuh"
 #include "mg_tiles.cuh"
 
 namespace stzg {
@@ -24,42 +25,6 @@ namespace stzg {
 using namespace mgw;
 
 namespace {
-
-// The environment of small_vcycle on the GPU.
-struct block_env {
-    static constexpr int kLanes = 32;
-    unsigned char *mem;
-    int r;
-    __device__ __forceinline__ int rank() const { return r; }
-    __device__ __forceinline__ unsigned char *local() const { return mem; }
-    __device__ __forceinline__ unsigned char *base(int k) const {
-        unsigned long long a;
-        asm("mapa.u64 %0, %1, %2;\n" : "=l"(a) : "l"((unsigned long long)mem), "r"(k));
-        return (unsigned char *)a;
-    }
-    __device__ __forceinline__ int thread() const { return (int)threadIdx.x; }
-    __device__ __forceinline__ int threads() const { return (int)blockDim.x; }
-    __device__ __forceinline__ const block_walk &walk(const block_walk &w, int, int) const { return w; }
-    template <typename F> __device__ __forceinline__ void par(F f) {
-        f((int)threadIdx.x, (int)blockDim.x);
-        __syncthreads();
-    }
-    __device__ __forceinline__ void csync() {
-        asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-    }
-    __device__ __forceinline__ ff lane_sum(ff a) const { return warp_pair_sum(a); }
-    __device__ __forceinline__ float2 ld(const float2 *p) const { return __ldcg(p); }
-    __device__ __forceinline__ float4 ld(const float4 *p) const { return __ldcg(p); }
-    __device__ __forceinline__ void wait_input() const { pdl_input(); }
-    __device__ __forceinline__ void store(const small_plan<float> &P, size_t k, const float2 &v) const {
-        P.lv[P.t].zg[k] = v;
-    }
-    __device__ __forceinline__ void store(const small_plan<ff> &P, size_t k, const float4 &v) const {
-        if (P.sum) P.sum[k] = add_pairs(P.sum[k], v);
-        else P.lv[P.t].zg[k] = v;
-    }
-};
 
 // The small levels of one V-cycle.  Bound by the latency of its dependent
 // phases (three to six per level and direction, 0.3 to 0.5 us each) and of the
@@ -70,34 +35,14 @@ struct block_env {
 // 512^2, FP32: 47 / - / 79 us with one launch per level, 20 / 29 / 67 us with
 // this kernel; FP64 handles: 201 / 293 / 512 us with one FP64 launch per colour,
 // 35 / 51 / 122 us in pairs.
-constexpr int kSmallThreads = 512;
-constexpr unsigned kSmallMax = 227 * 1024;
 
 template <typename S, bool FAST>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constant__ small_plan<S> P) {
     extern __shared__ __align__(16) unsigned char small_raw[];
     pdl_start();
     block_env env{small_raw, (int)blockIdx.x};  // one cluster: its rank is the block index
-    small_vcycle<FAST>(P, env);
+    small_vcycle<FAST, false>(P, env);
 }
-
-// Column c of the matrix of the V-cycle from level t on: block c runs it on
-// the right-hand side that is one at unknown c.
-struct column_env : block_env {
-    const float4 *b0;
-    float2 *out;
-    int col, n;
-    __device__ __forceinline__ int rank() const { return 0; }
-    __device__ __forceinline__ float4 ld(const float4 *p) const {
-        const int k = 2 * (int)(p - b0);
-        return make_float4(k == col ? 1.f : 0.f, k + 1 == col ? 1.f : 0.f, 0.f, 0.f);
-    }
-    __device__ __forceinline__ void wait_input() const {}
-    __device__ __forceinline__ void store(const small_plan<ff> &, size_t k, const float4 &v) const {
-        out[(2 * k) * n + col] = make_float2(v.x, v.z);
-        out[(2 * k + 1) * n + col] = make_float2(v.y, v.w);
-    }
-};
 
 __global__ void __launch_bounds__(kSmallThreads, 1)
     k_dense_columns(const __grid_constant__ small_plan<ff> P, float2 *out) {
@@ -109,7 +54,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     env.out = out;
     env.col = blockIdx.x;
     env.n = gridDim.x;
-    small_vcycle<false>(P, env);
+    small_vcycle<false, false>(P, env);
 }
 
 // r = b - A z of the top level in FP64 as float pairs; with partials, the sums
@@ -170,38 +115,20 @@ template <typename T> struct scalar_of;
 template <> struct scalar_of<float> { typedef float type; };
 template <> struct scalar_of<double> { typedef ff type; };
 
-// Largest cluster the device takes for the small-level kernel (16 where the
-// non-portable size is allowed, else 8; probed once per device).
+// Largest cluster the device takes for the small-level kernels (probed once
+// per device; at least 1).
 int max_blocks() {
     static int known[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
-    return known[dev] ? known[dev] : (known[dev] = [] {
+    if (!known[dev]) {
         const void *k[4] = {(const void *)k_small<float, true>, (const void *)k_small<float, false>,
                             (const void *)k_small<ff, true>, (const void *)k_small<ff, false>};
-        for (const void *f : k)
-            if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMax) != cudaSuccess ||
-                cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-                cudaGetLastError();
-                return 1;
-            }
-        for (int c = 16; c >= 2; c >>= 1) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(c);
-            cfg.blockDim = dim3(kSmallThreads);
-            cfg.dynamicSmemBytes = kSmallMax;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = c;
-            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, k_small<ff, false>, &cfg) == cudaSuccess && n > 0) return c;
-        }
-        cudaGetLastError();
-        return 1;
-    }());
+        int c = 16;
+        for (const void *f : k) c = std::min(c, cluster_limit(f));
+        known[dev] = std::max(c, 1);
+    }
+    return known[dev];
 }
 
 // Levels t..d of h as a plan (not yet laid out).
@@ -258,19 +185,9 @@ bool choose_small(const hierarchy<T> &h, bool zero_start, small_plan<typename sc
 }
 
 template <typename S> void launch_small(const small_plan<S> &P, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(P.blocks);
-    cfg.blockDim = dim3(kSmallThreads);
-    cfg.dynamicSmemBytes = P.bytes;
-    cfg.stream = st;
+    cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = P.blocks;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = P.blocks > 1 ? 2 : 1;
+    cluster_config(cfg, at, P.blocks, P.bytes, st);
     if (block_phases(P)) cudaLaunchKernelEx(&cfg, k_small<S, true>, P);
     else cudaLaunchKernelEx(&cfg, k_small<S, false>, P);
     note_launch();
@@ -350,7 +267,6 @@ template <typename T> int build_dense(hierarchy<T> &h, const std::vector<double>
     const int ml = h.nl - 1;
     if (ml < 1 || inverse.empty()) return STZG_OK;
     h.dense_from = dense_level(ml, [&](int l) { return (long)h.lv[l].m * h.lv[l].n; });
-    if (max_blocks() < 1) return STZG_OK;
     STZG_CUDA(cudaFuncSetAttribute(k_dense_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMax));
     const float4 *next = nullptr;
     for (int l = ml; l >= h.dense_from; l--) {

@@ -1,0 +1,196 @@
+// The small levels of the general 2x2-block multigrid in one launch
+// (mg_small.h).
+#include "mg_small.h"
+
+#include <algorithm>
+#include <cstring>
+
+#include "common.cuh"
+#include "mg_env.cuh"
+
+namespace stzg {
+
+using namespace mgw;
+
+namespace {
+
+// b and z of the first level are FP64 vectors of the size of a node.
+struct io_env : block_env {
+    __device__ __forceinline__ float4 ld(const float4 *p) const {
+        const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+        float4 o;
+        ff_split_d(v.x, o.x, o.z);
+        ff_split_d(v.y, o.y, o.w);
+        return o;
+    }
+    __device__ __forceinline__ void store(const small_plan<ff> &P, size_t k, const float4 &v) const {
+        reinterpret_cast<double2 *>(P.lv[P.t].zg)[k] = make_double2(ff_to_d(v.x, v.z), ff_to_d(v.y, v.w));
+    }
+};
+
+// FP64 V-cycle of a 512 x 256 grid of 2x2 blocks, y periodic: 520 us with one
+// FP64 launch per colour and a single-block FP64 tail of 215 us.
+template <bool FAST, bool YP>
+__global__ void __launch_bounds__(kSmallThreads, 1) k_small_blocks(const __grid_constant__ small_plan<ff> P) {
+    extern __shared__ __align__(16) unsigned char small_raw[];
+    pdl_start();
+    io_env env;
+    env.mem = small_raw;
+    env.r = (int)blockIdx.x;
+    small_vcycle<FAST, YP>(P, env);
+}
+
+template <bool YP>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+    k_block_columns(const __grid_constant__ small_plan<ff> P, float2 *out) {
+    extern __shared__ __align__(16) unsigned char small_raw[];
+    column_env env;
+    env.mem = small_raw;
+    env.r = 0;
+    env.b0 = P.lv[P.t].bg;
+    env.out = out;
+    env.col = blockIdx.x;
+    env.n = gridDim.x;
+    small_vcycle<false, YP>(P, env);
+}
+
+int max_blocks() {
+    static int known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (!known[dev]) {
+        const void *k[4] = {(const void *)k_small_blocks<true, true>, (const void *)k_small_blocks<true, false>,
+                            (const void *)k_small_blocks<false, true>, (const void *)k_small_blocks<false, false>};
+        int c = 16;
+        for (const void *f : k) c = std::min(c, cluster_limit(f));
+        if (cudaFuncSetAttribute(k_block_columns<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMax) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(k_block_columns<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kSmallMax) != cudaSuccess)
+            c = 0;
+        known[dev] = c + 1;
+    }
+    return known[dev] - 1;
+}
+
+// Levels of at most this many nodes: the alternative is eleven FP64 launches
+// of about 7 us per level.
+constexpr long kBlockPoints = 33000;
+
+}  // namespace
+
+small_cycle::~small_cycle() {
+    for (int l = 0; l < 17; l++) {
+        cudaFree(tab_[l].p);
+        cudaFree(cls_[l].p);
+        cudaFree(dense_[l].p);
+    }
+}
+
+int small_cycle::need(buffer &b, size_t bytes, bool *moved) {
+    if (b.cap >= bytes) return STZG_OK;
+    if (b.p) cudaFree(b.p);
+    b = buffer();
+    const cudaError_t e = cudaMalloc(&b.p, bytes);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(small levels)");
+    b.cap = bytes;
+    *moved = true;
+    return STZG_OK;
+}
+
+int small_cycle::setup(const std::vector<small_desc> &desc, int yp, const std::vector<double> &bottom, cudaStream_t st,
+                       bool *moved) {
+    const int was = t_, ml = (int)desc.size() - 1, cap = max_blocks();
+    t_ = 0;
+    yp_ = yp;
+    auto done = [&](const small_plan<ff> *P) {
+        std::vector<unsigned char> now(sizeof(small_plan<ff>));
+        if (P) std::memcpy(now.data(), P, sizeof(*P));
+        if (t_ != was || now != plan_) *moved = true;
+        plan_.swap(now);
+        return STZG_OK;
+    };
+    if (ml < 2 || ml > 16 || cap < 1 || bottom.empty()) return done(nullptr);
+    const int d = std::max(2, dense_level(ml, [&](int l) { return (long)desc[l].m * desc[l].n; }));
+    // a periodic y line is even on every level that is swept here
+    int t = d;
+    while (t > 1 && (long)desc[t - 1].m * desc[t - 1].n <= kBlockPoints && !(yp && (desc[t - 1].n & 1))) t--;
+    for (int l = d; l < ml; l++)
+        if (yp && (desc[l].n & 1)) return done(nullptr);
+    small_plan<ff> P;
+    std::memset(&P, 0, sizeof(P));
+    for (int l = t; l <= ml; l++) {
+        const small_desc &D = desc[l];
+        const int nst = (int)D.table.size() / 40;
+        pairs_[l].resize(20 * (size_t)nst);
+        for (int c = 0; c < nst; c++)
+            for (int e = 0; e < 10; e++) {
+                float h[4], o[4];
+                for (int q = 0; q < 4; q++) {
+                    const double v = D.table[(size_t)c * 40 + 4 * e + q];
+                    h[q] = (float)v;
+                    o[q] = (float)(v - (double)h[q]);
+                }
+                pairs_[l][20 * c + 2 * e] = make_float4(h[0], h[1], h[2], h[3]);
+                pairs_[l][20 * c + 2 * e + 1] = make_float4(o[0], o[1], o[2], o[3]);
+            }
+        STZG_CHECK(need(tab_[l], pairs_[l].size() * sizeof(float4), moved));
+        STZG_CHECK(need(cls_[l], D.ids.size() * sizeof(int), moved));
+        STZG_CUDA(cudaMemcpyAsync(tab_[l].p, pairs_[l].data(), pairs_[l].size() * sizeof(float4),
+                                  cudaMemcpyHostToDevice, st));
+        STZG_CUDA(cudaMemcpyAsync(cls_[l].p, D.ids.data(), D.ids.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+        small_level<ff> &S = P.lv[l];
+        S.m = D.m;
+        S.n = D.n;
+        S.homog = D.rows;
+        S.nst = nst;
+        S.ncls = (int)D.ids.size();
+        S.cls = (const int *)cls_[l].p;
+        S.st = (const float4 *)tab_[l].p;
+    }
+    // the matrices from the coarsest level's up to level d's
+    for (int l = ml; l >= d; l--) {
+        const size_t N = 2 * (size_t)desc[l].m * desc[l].n;
+        STZG_CHECK(need(dense_[l], N * N * sizeof(float2), moved));
+        if (l == ml) {
+            bottom_.resize(N * N);
+            for (size_t k = 0; k < N * N; k++) {
+                const float h = (float)bottom[k];
+                bottom_[k] = make_float2(h, (float)(bottom[k] - (double)h));
+            }
+            STZG_CUDA(cudaMemcpyAsync(dense_[l].p, bottom_.data(), N * N * sizeof(float2), cudaMemcpyHostToDevice, st));
+            continue;
+        }
+        small_plan<ff> Q = P;
+        Q.dense = (const float4 *)dense_[l + 1].p;
+        if (!layout_small(Q, l, l + 1, 1, kSmallMax)) return done(nullptr);
+        if (yp) k_block_columns<true><<<(unsigned)N, kSmallThreads, Q.bytes, st>>>(Q, (float2 *)dense_[l].p);
+        else k_block_columns<false><<<(unsigned)N, kSmallThreads, Q.bytes, st>>>(Q, (float2 *)dense_[l].p);
+        STZG_CUDA(cudaGetLastError());
+    }
+    P.dense = (const float4 *)dense_[d].p;
+    P.zero_start = 1;
+    for (; t < d; t++)
+        for (int c = cap; c >= 1; c >>= 1)
+            if (layout_small(P, t, d, c, kSmallMax)) {
+                t_ = t;
+                return done(&P);
+            }
+    return done(nullptr);
+}
+
+void small_cycle::launch(const double2 *b, double2 *z, cudaStream_t st) const {
+    small_plan<ff> P;
+    std::memcpy(&P, plan_.data(), sizeof(P));
+    P.lv[P.t].bg = reinterpret_cast<const float4 *>(b);
+    P.lv[P.t].zg = reinterpret_cast<float4 *>(z);
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[2];
+    cluster_config(cfg, at, P.blocks, P.bytes, st);
+    const bool fast = block_phases(P);
+    if (yp_) fast ? cudaLaunchKernelEx(&cfg, k_small_blocks<true, true>, P) : cudaLaunchKernelEx(&cfg, k_small_blocks<false, true>, P);
+    else fast ? cudaLaunchKernelEx(&cfg, k_small_blocks<true, false>, P) : cudaLaunchKernelEx(&cfg, k_small_blocks<false, false>, P);
+    note_launch();
+}
+
+}  // namespace stzg

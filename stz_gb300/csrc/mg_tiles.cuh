@@ -2,18 +2,10 @@
 #pragma once
 
 #include "ff.cuh"
-#include "mg_window.cuh"
+#include "mg_env.cuh"
 
 namespace stzg {
 namespace mgw {
-
-__device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_input() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
-// z += d in FP64, the pair formed as a double on the integer pipe.
-__device__ __forceinline__ double2 add_pairs(const double2 &z, const float4 &d) {
-    return make_double2(z.x + ff_to_d(d.x, d.z), z.y + ff_to_d(d.y, d.w));
-}
 
 // ---- wide levels as tiles ------------------------------------------------------
 //

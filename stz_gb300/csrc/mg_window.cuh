@@ -129,7 +129,9 @@ MGW_FN ff three(ff k1, ff s1, ff k2, ff s2, ff k3, ff s3) {
 
 // ---- windows -----------------------------------------------------------------
 
-template <typename S, bool WRAP> struct window {
+// YP: y is periodic too; rows are unwrapped (a band's halo rows continue below
+// 0 and beyond n), lines in y are even.
+template <typename S, bool WRAP, bool YP = false> struct window {
     plane<S> z, b, r;
     int W, He;          // columns; even ones
     int jb, rb;         // rows of local row 0 of z and b; of r
@@ -138,6 +140,29 @@ template <typename S, bool WRAP> struct window {
     const float4 *st;   // stencils: 10 blocks each
     const int *cls;     // class per row (homog) or per point
     int homog;
+    MGW_FN int lo(int j) const { return YP || j > 0 ? j : 0; }          // first row of a range from j on
+    MGW_FN int hi(int j) const { return YP || j < n - 1 ? j : n - 1; }  // last row of a range up to j
+    MGW_FN bool has_below(int j) const { return YP || j > 0; }
+    MGW_FN bool has_above(int j) const { return YP || j < n - 1; }
+    MGW_FN int wrapped(int j) const { return !YP ? j : (j < 0 ? j + n : (j >= n ? j - n : j)); }
+    // halves_of(2J + q - 1, n, yp, J), q = 0, 1, 2
+    MGW_FN int halves(int q, int J) const {
+        if (YP) return q == 1 ? 2 : 1;
+        const int fy = 2 * J + q - 1;
+        if (fy < 0 || fy >= n) return 0;
+        if (q == 1) return 2;
+        if ((n & 1) || fy != n - 1) return 1;
+        return q == 0 ? 2 : 0;
+    }
+    // the coarse rows (unwrapped) that feed row j and their halves
+    MGW_FN int feeds(int j, int *c, int *h) const {
+        if (!YP) return p1d_halves(j, n, 0, c, h);
+        c[0] = j >> 1;
+        c[1] = c[0] + 1;
+        h[0] = j & 1 ? 1 : 2;
+        h[1] = 1;
+        return 1 + (j & 1);
+    }
     MGW_FN int col(int w) const { return (w & 1) * He + (w >> 1); }
     MGW_FN int at(int j, int w) const { return (j - jb) * W + col(w); }
     MGW_FN int rat(int j, int w) const { return (j - rb) * W + col(w); }
@@ -149,7 +174,7 @@ template <typename S, bool WRAP> struct window {
         return g < 0 ? g + m : (g >= m ? g % m : g);
     }
     MGW_FN const float4 *sten(int j, int w) const {
-        const int c = homog ? cls[j] : cls[(size_t)j * m + gcol(w)];
+        const int c = homog ? cls[wrapped(j)] : cls[(size_t)wrapped(j) * m + gcol(w)];
         return st + (size_t)c * (10 * num<S>::quads);
     }
 };
@@ -193,11 +218,11 @@ MGW_FN val2<ff> apply(const float4 *s, int e, const val2<ff> &v) {
 // tgmg.in.cc:536-547).  rows: whether the rows below and above take part;
 // mid: whether the neighbours in the row do (a sweep that starts from zero
 // skips what is still zero: adding exact zeros changes nothing).
-template <typename S, bool WRAP>
-MGW_FN void offdiag(const window<S, WRAP> &V, const float4 *s, int j, int w, bool rows, bool mid,
+template <typename S, bool WRAP, bool YP>
+MGW_FN void offdiag(const window<S, WRAP, YP> &V, const float4 *s, int j, int w, bool rows, bool mid,
                     typename acc_of<S>::type &ax, typename acc_of<S>::type &ay) {
     const int wl = V.left(w), wr = V.right(w);
-    if (rows && j > 0) {
+    if (rows && V.has_below(j)) {
         madd(ax, ay, s, 0, V.z.get(V.at(j - 1, wl)));
         madd(ax, ay, s, 1, V.z.get(V.at(j - 1, w)));
         madd(ax, ay, s, 2, V.z.get(V.at(j - 1, wr)));
@@ -206,7 +231,7 @@ MGW_FN void offdiag(const window<S, WRAP> &V, const float4 *s, int j, int w, boo
         madd(ax, ay, s, 3, V.z.get(V.at(j, wl)));
         madd(ax, ay, s, 5, V.z.get(V.at(j, wr)));
     }
-    if (rows && j < V.n - 1) {
+    if (rows && V.has_above(j)) {
         madd(ax, ay, s, 6, V.z.get(V.at(j + 1, wl)));
         madd(ax, ay, s, 7, V.z.get(V.at(j + 1, w)));
         madd(ax, ay, s, 8, V.z.get(V.at(j + 1, wr)));
@@ -219,11 +244,11 @@ MGW_FN int imin(int a, int b) { return a < b ? a : b; }
 // Colours of a sweep: rows of parity cy, columns of parity cx (cx == 2: the
 // last column of an odd line), rows jlo..jhi and window columns wlo..whi (all
 // when WRAP).
-template <typename S, bool WRAP>
-MGW_FN void lev_color(const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int cx, int cy, bool from_zero,
+template <typename S, bool WRAP, bool YP>
+MGW_FN void lev_color(const window<S, WRAP, YP> &V, int jlo, int jhi, int wlo, int whi, int cx, int cy, bool from_zero,
                       int tid, int nth) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     const int j0 = jlo + ((jlo ^ cy) & 1);
     if (j0 > jhi) return;
     int w0, nw;
@@ -252,10 +277,10 @@ MGW_FN void lev_color(const window<S, WRAP> &V, int jlo, int jhi, int wlo, int w
 
 // z = 0 on the last column of an odd line (the third colour, read before its
 // first update in a sweep from zero).
-template <typename S, bool WRAP>
-MGW_FN void lev_clear_last(const window<S, WRAP> &V, int jlo, int jhi, int tid, int nth) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+template <typename S, bool WRAP, bool YP>
+MGW_FN void lev_clear_last(const window<S, WRAP, YP> &V, int jlo, int jhi, int tid, int nth) {
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     for (int j = jlo + tid; j <= jhi; j += nth) {
         val2<S> o{};
         V.z.set(V.at(j, V.W - 1), o);
@@ -264,10 +289,10 @@ MGW_FN void lev_clear_last(const window<S, WRAP> &V, int jlo, int jhi, int tid, 
 
 // r = b - A z after a sweep.  On an even line the odd columns of odd rows took
 // the last colour: their residual is zero up to rounding and set to zero.
-template <typename S, bool WRAP>
-MGW_FN void lev_residual(const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int tid, int nth) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+template <typename S, bool WRAP, bool YP>
+MGW_FN void lev_residual(const window<S, WRAP, YP> &V, int jlo, int jhi, int wlo, int whi, int tid, int nth) {
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     if (jlo > jhi) return;
     if (WRAP) {
         wlo = 0;
@@ -293,16 +318,16 @@ MGW_FN void lev_residual(const window<S, WRAP> &V, int jlo, int jhi, int wlo, in
 }
 
 // Off-diagonal sums of the top level (qs_multi::mul_a, qs_multi.hh:41-50).
-template <typename S, bool WRAP>
-MGW_FN S top_off_x(const top_consts<S> &o, const window<S, WRAP> &V, int j, int w) {
+template <typename S, bool WRAP, bool YP>
+MGW_FN S top_off_x(const top_consts<S> &o, const window<S, WRAP, YP> &V, int j, int w) {
     const int wl = V.left(w), wr = V.right(w);
     return three(o.Kmx, sum2(V.z.x(V.at(j, wl)), V.z.x(V.at(j, wr))), o.my,
                  sum2(V.z.x(V.at(j - 1, w)), V.z.x(V.at(j + 1, w))), o.qK,
                  cross4(V.z.y(V.at(j - 1, wl)), V.z.y(V.at(j + 1, wr)), V.z.y(V.at(j - 1, wr)),
                         V.z.y(V.at(j + 1, wl))));
 }
-template <typename S, bool WRAP>
-MGW_FN S top_off_y(const top_consts<S> &o, const window<S, WRAP> &V, int j, int w) {
+template <typename S, bool WRAP, bool YP>
+MGW_FN S top_off_y(const top_consts<S> &o, const window<S, WRAP, YP> &V, int j, int w) {
     const int wl = V.left(w), wr = V.right(w);
     return three(o.mx, sum2(V.z.y(V.at(j, wl)), V.z.y(V.at(j, wr))), o.Kmy,
                  sum2(V.z.y(V.at(j - 1, w)), V.z.y(V.at(j + 1, w))), o.qK,
@@ -313,11 +338,11 @@ MGW_FN S top_off_y(const top_consts<S> &o, const window<S, WRAP> &V, int j, int 
 // One colour of the top level: a thread takes a pair of columns, the x
 // equation at one and the y equation at the other, so that lanes do not
 // diverge on the component.  from_zero: z is zero, so only b counts.
-template <typename S, bool WRAP>
-MGW_FN void top_color(const top_consts<S> &o, const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int color,
+template <typename S, bool WRAP, bool YP>
+MGW_FN void top_color(const top_consts<S> &o, const window<S, WRAP, YP> &V, int jlo, int jhi, int wlo, int whi, int color,
                       bool from_zero, int tid, int nth) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     if (jlo > jhi) return;
     if (WRAP) {
         wlo = 0;
@@ -349,11 +374,11 @@ MGW_FN void top_color(const top_consts<S> &o, const window<S, WRAP> &V, int jlo,
 
 // Residual of the colour-0 equations after a sweep (the colour-1 ones, whose
 // unknowns were updated last, and the wall rows are zero up to rounding).
-template <typename S, bool WRAP>
-MGW_FN void top_residual(const top_consts<S> &o, const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int tid,
+template <typename S, bool WRAP, bool YP>
+MGW_FN void top_residual(const top_consts<S> &o, const window<S, WRAP, YP> &V, int jlo, int jhi, int wlo, int whi, int tid,
                          int nth) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     if (jlo > jhi) return;
     if (WRAP) {
         wlo = 0;
@@ -380,19 +405,10 @@ MGW_FN void top_residual(const top_consts<S> &o, const window<S, WRAP> &V, int j
     }
 }
 
-// halves_of(2J + q - 1, n, 0, J), q = 0, 1, 2 on a bounded line of n points.
-MGW_FN int row_halves(int q, int J, int n) {
-    const int fy = 2 * J + q - 1;
-    if (fy < 0 || fy >= n) return 0;
-    if (q == 1) return 2;
-    if ((n & 1) || fy != n - 1) return 1;
-    return q == 0 ? 2 : 0;
-}
-
 // Full weighting of r at the coarse points of rows Jlo..Jhi, columns
 // Ilo..Ihi (global): out(J, I, value).
-template <typename S, bool WRAP, typename Out>
-MGW_FN void restrict_rows(const window<S, WRAP> &V, int Jlo, int Jhi, int Ilo, int Ihi, int cm, Out out, int tid,
+template <typename S, bool WRAP, bool YP, typename Out>
+MGW_FN void restrict_rows(const window<S, WRAP, YP> &V, int Jlo, int Jhi, int Ilo, int Ihi, int cm, Out out, int tid,
                           int nth) {
     const int nI = Ihi - Ilo + 1, total = (Jhi - Jlo + 1) * nI;
     if (Jhi < Jlo || nI <= 0) return;
@@ -406,7 +422,7 @@ MGW_FN void restrict_rows(const window<S, WRAP> &V, int Jlo, int Jhi, int Ilo, i
         val2<S> a{};
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            const int hy = row_halves(q, J, V.n);
+            const int hy = V.halves(q, J);
             if (!hy) continue;
             const int fy = 2 * J + q - 1;
             const float w1 = (float)hy * 0.25f, w2 = (float)(2 * hy) * 0.25f;
@@ -431,11 +447,11 @@ MGW_FN void restrict_rows(const window<S, WRAP> &V, int Jlo, int Jhi, int Ilo, i
 // z += P zc on rows jlo..jhi, window columns wlo..whi: zc(J, I) is the child's
 // value at row J and the coarse column I of window column 2 (I - x0/2) (WRAP:
 // 0 <= I < cm; else unwrapped).
-template <typename S, bool WRAP, typename Child>
-MGW_FN void prolong_rows(const window<S, WRAP> &V, int jlo, int jhi, int wlo, int whi, int cm, Child zc, int tid,
+template <typename S, bool WRAP, bool YP, typename Child>
+MGW_FN void prolong_rows(const window<S, WRAP, YP> &V, int jlo, int jhi, int wlo, int whi, int cm, Child zc, int tid,
                          int nth) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     if (jlo > jhi) return;
     if (WRAP) {
         wlo = 0;
@@ -446,7 +462,7 @@ MGW_FN void prolong_rows(const window<S, WRAP> &V, int jlo, int jhi, int wlo, in
     for (int k = tid; k < total; k += nth) {
         const int qk = dv.quot(k), j = jlo + qk, w = wlo + (k - qk * nw);
         int cy[2], hy[2];
-        const int ny = p1d_halves(j, V.n, 0, cy, hy);
+        const int ny = V.feeds(j, cy, hy);
         const int I = (V.x0 + w) >> 1;  // floor: x0 is even
         val2<S> a{};
         if (w & 1) {
@@ -527,31 +543,31 @@ MGW_FN void offdiag3(const float4 *s, const plane<S> &row, int W, const columns3
 }
 
 // Colour (cx, cy) on the rows jlo..jhi of the band (qn block rows).
-template <typename S>
-MGW_FN void block_color(const window<S, true> &V, block_walk w, int qn, int jlo, int jhi, int cx, int cy,
+template <typename S, bool YP>
+MGW_FN void block_color(const window<S, true, YP> &V, block_walk w, int qn, int jlo, int jhi, int cx, int cy,
                         bool from_zero) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     for (; w.q < qn; w.next()) {
         const int lr = 2 * w.q + cy, j = V.jb + lr;
         if (j < jlo || j > jhi) continue;
-        const float4 *s = V.st + V.cls[j] * (10 * num<S>::quads);
+        const float4 *s = V.st + V.cls[V.wrapped(j)] * (10 * num<S>::quads);
         const columns3 c(w.k, w.P, cx);
         const plane<S> row = V.z + lr * V.W;
         const bool rows = !(from_zero && cy == 0);
         const val2<S> bb = V.b.get(lr * V.W + c.c);
         typename acc_of<S>::type ax, ay;
-        offdiag3<S>(s, row, V.W, c, rows && j > 0, !(from_zero && cx == 0), rows && j < V.n - 1, ax, ay);
+        offdiag3<S>(s, row, V.W, c, rows && V.has_below(j), !(from_zero && cx == 0), rows && V.has_above(j), ax, ay);
         row.set(c.c, apply(s, 9, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())}));
     }
 }
 
 // Residual of the rows jlo..jhi (the odd columns of odd rows: zero): the three
 // points of a block on different threads.
-template <typename S>
-MGW_FN void block_residual(const window<S, true> &V, int P, int qn, int jlo, int jhi, int tid, int nth) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+template <typename S, bool YP>
+MGW_FN void block_residual(const window<S, true, YP> &V, int P, int qn, int jlo, int jhi, int tid, int nth) {
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     const int blocks = P * qn;
     const divider dv(P);
     for (int t = tid; t < 3 * blocks; t += nth) {
@@ -559,11 +575,11 @@ MGW_FN void block_residual(const window<S, true> &V, int P, int qn, int jlo, int
         const int cx = e & 1, cy = e >> 1, lr = 2 * q + cy, j = V.jb + lr;
         if (j < jlo || j > jhi) continue;
         const columns3 c(k, P, cx);
-        const float4 *s = V.st + V.cls[j] * (10 * num<S>::quads);
+        const float4 *s = V.st + V.cls[V.wrapped(j)] * (10 * num<S>::quads);
         const plane<S> row = V.z + lr * V.W;
         const val2<S> bb = V.b.get(lr * V.W + c.c);
         typename acc_of<S>::type ax, ay;
-        offdiag3<S>(s, row, V.W, c, j > 0, true, j < V.n - 1, ax, ay);
+        offdiag3<S>(s, row, V.W, c, V.has_below(j), true, V.has_above(j), ax, ay);
         madd(ax, ay, s, 4, row.get(c.c));
         const plane<S> r = V.r + (j - V.rb) * V.W;
         r.set(c.c, val2<S>{sub(bb.x, ax.done()), sub(bb.y, ay.done())});
@@ -573,8 +589,8 @@ MGW_FN void block_residual(const window<S, true> &V, int P, int qn, int jlo, int
 
 // Restriction to the coarse rows Jlo..Jhi: coarse point (J, k) under block
 // (J - jb/2, k).
-template <typename S, typename Out>
-MGW_FN void block_restrict(const window<S, true> &V, block_walk w, int qn, int Jlo, int Jhi, Out out) {
+template <typename S, bool YP, typename Out>
+MGW_FN void block_restrict(const window<S, true, YP> &V, block_walk w, int qn, int Jlo, int Jhi, Out out) {
     for (; w.q < qn; w.next()) {
         const int J = (V.jb >> 1) + w.q;
         if (J < Jlo || J > Jhi) continue;
@@ -582,7 +598,7 @@ MGW_FN void block_restrict(const window<S, true> &V, block_walk w, int qn, int J
         val2<S> a{};
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            const int hy = row_halves(q, J, V.n);
+            const int hy = V.halves(q, J);
             if (!hy) continue;
             const plane<S> row = V.r + (2 * J + q - 1 - V.rb) * V.W;
             const float w1 = (float)hy * 0.25f, w2 = (float)(2 * hy) * 0.25f;
@@ -600,18 +616,18 @@ MGW_FN void block_restrict(const window<S, true> &V, block_walk w, int qn, int J
 
 // Prolongation on the rows jlo..jhi: crow(J) is the child's row J, col(k) and
 // next(k) the places in it of the columns under block k and right of it.
-template <typename S, typename Row, typename Col, typename Next>
-MGW_FN void block_prolong(const window<S, true> &V, block_walk w, int qn, int jlo, int jhi, Row crow, Col col,
+template <typename S, bool YP, typename Row, typename Col, typename Next>
+MGW_FN void block_prolong(const window<S, true, YP> &V, block_walk w, int qn, int jlo, int jhi, Row crow, Col col,
                           Next next) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     for (; w.q < qn; w.next()) {
         const int je = V.jb + 2 * w.q, J = je >> 1;
         if (je > jhi || je + 1 < jlo) continue;
         const int c0 = col(w.k), c1 = next(w.k);
         const bool even = je >= jlo, odd = je + 1 <= jhi;
         // an even line injects its last point into the last coarse one
-        const bool inject = !(V.n & 1) && je + 1 == V.n - 1;
+        const bool inject = !YP && !(V.n & 1) && je + 1 == V.n - 1;
         val2<S> a0{}, a1{}, b0{}, b1{};
         if (even || !inject) {
             const plane<S> r = crow(J);
@@ -662,11 +678,11 @@ MGW_FN S top_off3(const top_consts<S> &o, const plane<S> &row, int W, const colu
 
 // One colour of the top level on the rows jlo..jhi: of the block's four nodes
 // the x equation at the two with (i + j) & 1 == color, the y one at the others.
-template <typename S>
-MGW_FN void block_top_color(const top_consts<S> &o, const window<S, true> &V, block_walk w, int qn, int jlo, int jhi,
+template <typename S, bool YP>
+MGW_FN void block_top_color(const top_consts<S> &o, const window<S, true, YP> &V, block_walk w, int qn, int jlo, int jhi,
                             int color, bool from_zero) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     for (; w.q < qn; w.next()) {
 #pragma unroll
         for (int cy = 0; cy < 2; cy++) {
@@ -692,11 +708,11 @@ MGW_FN void block_top_color(const top_consts<S> &o, const window<S, true> &V, bl
     }
 }
 
-template <typename S>
-MGW_FN void block_top_residual(const top_consts<S> &o, const window<S, true> &V, block_walk w, int qn, int jlo,
+template <typename S, bool YP>
+MGW_FN void block_top_residual(const top_consts<S> &o, const window<S, true, YP> &V, block_walk w, int qn, int jlo,
                                int jhi) {
-    jlo = imax(jlo, 0);
-    jhi = imin(jhi, V.n - 1);
+    jlo = V.lo(jlo);
+    jhi = V.hi(jhi);
     for (; w.q < qn; w.next()) {
 #pragma unroll
         for (int cy = 0; cy < 2; cy++) {
@@ -778,10 +794,10 @@ template <typename S> MGW_BOTH int band_above(const small_plan<S> &P, int l) {
 
 // FAST: every level t .. d-1 is an even line with one class per row and its
 // tables in shared memory (known at compile time).
-template <bool FAST, typename S>
-MGW_FN window<S, true> band_window(const small_plan<S> &P, int l, int c, unsigned char *base) {
+template <bool FAST, bool YP, typename S>
+MGW_FN window<S, true, YP> band_window(const small_plan<S> &P, int l, int c, unsigned char *base) {
     const small_level<S> &L = P.lv[l];
-    window<S, true> V;
+    window<S, true, YP> V;
     V.z = plane<S>{reinterpret_cast<S *>(base + L.zo), L.ps};
     V.b = plane<S>{reinterpret_cast<S *>(base + L.bo), L.ps};
     V.r = plane<S>{reinterpret_cast<S *>(base + P.ro), P.rs};
@@ -855,7 +871,7 @@ constexpr int kDenseRows = 3;  // 34 rows per block of sixteen warps at 17 x 16 
 // product row and the sum over them), ld(p) (a global load), store(P, k, v)
 // (the result of level t at its node k), wait_input() (before the first read
 // of what an earlier kernel wrote).
-template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const small_plan<S> &P, E &env) {
+template <bool FAST, bool YP, typename S, typename E> MGW_FN void small_vcycle(const small_plan<S> &P, E &env) {
     typedef typename num<S>::node node;
     const int me = env.rank(), nb = P.blocks;
     unsigned char *base = env.local();
@@ -877,21 +893,21 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
         }
         env.wait_input();
         const small_level<S> &L = P.lv[P.t];
-        const window<S, true> V = band_window<FAST>(P, P.t, me, base);
+        const window<S, true, YP> V = band_window<FAST, YP>(P, P.t, me, base);
         const int y1 = band_row(P, P.t, me + 1);
-        const int lo = imax(0, V.jb), hi = imin(L.n, y1 + band_above(P, P.t));
+        const int lo = V.lo(V.jb), hi = V.hi(y1 + band_above(P, P.t) - 1) + 1;
         const int total = (hi - lo) * L.m;
         const divider dv(L.m);
         for (int k = tid; k < total; k += nth) {
             const int q = dv.quot(k), j = lo + q, w = k - q * L.m;
-            V.b.set(V.at(j, w), get(env.ld(L.bg + (size_t)j * L.m + w)));
-            if (P.top && !P.zero_start) V.z.set(V.at(j, w), get(env.ld(L.zg + (size_t)j * L.m + w)));
+            V.b.set(V.at(j, w), get(env.ld(L.bg + (size_t)V.wrapped(j) * L.m + w)));
+            if (P.top && !P.zero_start) V.z.set(V.at(j, w), get(env.ld(L.zg + (size_t)V.wrapped(j) * L.m + w)));
         }
     });
     if (nb > 1) env.csync();  // every block runs: its shared memory may be written
     // down
     for (int l = P.t; l < P.d; l++) {
-        const window<S, true> V = band_window<FAST>(P, l, me, base);
+        const window<S, true, YP> V = band_window<FAST, YP>(P, l, me, base);
         const int y0 = band_row(P, l, me), y1 = band_row(P, l, me + 1), cm = P.lv[l + 1].m;
         const int qn = (y1 - V.jb + band_above(P, l) + 1) >> 1;
         const bool top = P.top && l == P.t;
@@ -939,21 +955,25 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
         const int J0 = band_row(P, l + 1, me), J1 = band_row(P, l + 1, me + 1);
         env.par([&](int tid, int nth) {
             if (l + 1 < P.d) {
-                const window<S, true> CV = band_window<FAST>(P, l + 1, me, base);
+                const window<S, true, YP> CV = band_window<FAST, YP>(P, l + 1, me, base);
                 const int He = CV.He;
                 S *to[4];  // b of the neighbours at distance -2, -1, 1, 2, shifted to absolute rows
                 int lo[4], hi[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const int c = me + (q < 2 ? q - 2 : q - 1);
+                    int c = me + (q < 2 ? q - 2 : q - 1), turn = 0;
                     lo[q] = 1;
                     hi[q] = 0;
                     to[q] = nullptr;
+                    if (YP) {  // the bands go round
+                        while (c < 0) c += nb, turn -= P.lv[l + 1].n;
+                        while (c >= nb) c -= nb, turn += P.lv[l + 1].n;
+                    }
                     if (c < 0 || c >= nb) continue;
-                    lo[q] = band_row(P, l + 1, c) - kLevBelow;
-                    hi[q] = band_row(P, l + 1, c + 1) + kLevAbove - 2;  // the last row a sweep reads
+                    lo[q] = band_row(P, l + 1, c) - kLevBelow + turn;
+                    hi[q] = band_row(P, l + 1, c + 1) + kLevAbove - 2 + turn;  // the last row a sweep reads
                     if (lo[q] >= J1 || hi[q] < J0) hi[q] = lo[q] - 1;
-                    else to[q] = reinterpret_cast<S *>(env.base(c) + P.lv[l + 1].bo);
+                    else to[q] = reinterpret_cast<S *>((c == me ? base : env.base(c)) + P.lv[l + 1].bo);
                 }
                 auto out = [&](int J, int I, const val2<S> &v) {
                     const int c = (I & 1) * He + (I >> 1);
@@ -1002,15 +1022,15 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
     if (nb > 1) env.csync();
     // up
     for (int l = P.d - 1; l >= P.t; l--) {
-        const window<S, true> V = band_window<FAST>(P, l, me, base);
+        const window<S, true, YP> V = band_window<FAST, YP>(P, l, me, base);
         const int y0 = band_row(P, l, me), y1 = band_row(P, l, me + 1), cm = P.lv[l + 1].m;
         const int qn = (y1 - V.jb + band_above(P, l) + 1) >> 1;
         const bool top = P.top && l == P.t, last = l + 1 == P.d;
-        const window<S, true> CV = band_window<FAST>(P, l + 1, me, base);
+        const window<S, true, YP> CV = band_window<FAST, YP>(P, l + 1, me, base);
         const int J0 = band_row(P, l + 1, me), J1 = band_row(P, l + 1, me + 1), cHe = CV.He;
         const plane<S> halo{reinterpret_cast<S *>(base + (last ? 0u : P.lv[l + 1].ho)), 3 * cm};
         auto crow = [&](int J) -> plane<S> {
-            if (last) return zd + J * cm;
+            if (last) return zd + CV.wrapped(J) * cm;
             if (J < J0) return halo;
             if (J >= J1) return halo + (1 + J - J1) * cm;
             return CV.z + (J - CV.jb) * cm;
@@ -1064,12 +1084,13 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
                     env.store(P, (size_t)(y0 + q) * V.m + w, put(V.z.get(V.at(y0 + q, w))));
                 }
             });
-        } else if (nb > 1) {
+        } else if (nb > 1 || YP) {
             // rows next to the band's edges, for the neighbours' prolongation
             env.par([&](int tid, int nth) {
                 const int m = V.m;
-                S *lo = me > 0 ? reinterpret_cast<S *>(env.base(me - 1) + P.lv[l].ho) : nullptr;
-                S *hi = me + 1 < nb ? reinterpret_cast<S *>(env.base(me + 1) + P.lv[l].ho) : nullptr;
+                const int below = YP && me == 0 ? nb - 1 : me - 1, above = YP && me + 1 == nb ? 0 : me + 1;
+                S *lo = below >= 0 ? reinterpret_cast<S *>((below == me ? base : env.base(below)) + P.lv[l].ho) : nullptr;
+                S *hi = above < nb ? reinterpret_cast<S *>((above == me ? base : env.base(above)) + P.lv[l].ho) : nullptr;
                 for (int k = tid; k < 2 * m; k += nth) {  // both components
                     const int c = k < m ? k : k - m, from = k < m ? 0 : V.z.ps, to = k < m ? 0 : 3 * m;
                     const S *z = V.z.p + from + c;
@@ -1080,7 +1101,7 @@ template <bool FAST, typename S, typename E> MGW_FN void small_vcycle(const smal
                     if (hi) hi[to + c] = z[(y1 - 1 - V.jb) * m];
                 }
             });
-            env.csync();
+            if (nb > 1) env.csync();
         }
     }
 }
