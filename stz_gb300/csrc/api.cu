@@ -1209,7 +1209,7 @@ int stzg_time_kernel(stzg_sim *s, double dt, int kernel, int reps, double *ms) {
 // array, then set_boundaries at the new time.
 static int do_direct(stzg_sim *s, double dt) {
     s->time += dt;
-    direct_step(s->sc, s->P.viscosity, s->F, s->cur, dt, s->bv_state, s->st);
+    direct_step(s->sc, *s->maps, s->P.viscosity, s->F, s->cur, dt, s->bv_state, s->st);
     const size_t m = s->m;
     if (s->n > 1)
         STZG_CUDA(cudaMemcpyAsync(s->F.vel + m, s->F.src + m, (size_t)(s->n - 1) * m * sizeof(double2),

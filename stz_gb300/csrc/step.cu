@@ -505,6 +505,15 @@ __device__ __forceinline__ long long fx_products(const fx_factor &u, long long a
     return (long long)u.hi * a1 + (long long)v.hi * b1 + (mid >> 31);
 }
 
+// Yield test on the leading 24 bits: 3q^2 + s^2 + tau^2 within 5e-7; a cell
+// clearly below the cut-offs of k_advect (1e-24, or an athermal law below
+// yield) is elastic there too, any other one takes the FP64 test and law.
+__device__ __forceinline__ bool surely_elastic(const step_consts &c, double q, double s, double t) {
+    const float qf = ff_hi(q), sf = ff_hi(s), tf = ff_hi(t);
+    const float dv = 3.f * qf * qf + sf * sf + tf * tf;
+    return dv < 0.999e-24f * (1.f - 1e-6f) || (c.stz_model >= 2 && dv < c.yield_cut2f);
+}
+
 // One tile.  PRE: also the combinations for k_source (FP64 handles).
 template <bool PRE>
 __global__ void __launch_bounds__(ATX * ATY, 4)
@@ -660,13 +669,7 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
             else v[f] = fma(inc, sc, a[f]);
             B[f][ci] = v[f];
         }
-        // Yield test on the leading 24 bits: 3q^2 + s^2 + tau^2 within 5e-7; a cell
-        // clearly below the cut-offs of k_advect (1e-24, or an athermal law below
-        // yield) is elastic there too, any other one takes the FP64 test and law.
-        const float qf = ff_hi(a[F_Q]), sf = ff_hi(a[F_S]), tf = ff_hi(a[F_TAU]);
-        const float dv = 3.f * qf * qf + sf * sf + tf * tf;
-        const bool elastic = dv < 0.999e-24f * (1.f - 1e-6f) || (c.stz_model >= 2 && dv < c.yield_cut2f);
-        if (!elastic) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
+        if (!surely_elastic(c, a[F_Q], a[F_S], a[F_TAU])) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
         F.ddev[ci] = 0;
         if (PRE) write_pre(F, ci, h.xf, h.yf, v[F_P], v[F_Q], v[F_S], v[F_TAU]);
     }
@@ -741,13 +744,14 @@ struct direct_consts {
 enum { DF_U = F_COUNT, DF_V, DF_COUNT };
 typedef eno_tile<DF_COUNT> direct_tile;
 
-__global__ void __launch_bounds__(ATX * ATY) k_direct(step_consts c, direct_consts d, fields_dev F, int cur,
-                                                      double dt, double bv) {
+// One tile (bx, by) in FP64.
+__device__ __forceinline__ void direct_tile_step(const step_consts &c, const direct_consts &d, const fields_dev &F,
+                                                 int cur, double dt, double bv, int bx, int by) {
     extern __shared__ __align__(16) unsigned char dir_smem[];
     direct_tile &TT = *reinterpret_cast<direct_tile *>(dir_smem);
     const int m = c.m, n = c.n;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i0 = blockIdx.x * ATX, j0 = blockIdx.y * ATY;
+    const int i0 = bx * ATX, j0 = by * ATY;
     const int i = i0 + tx, j = j0 + ty;
     const double *__restrict__ const *A = F.f[cur];
     double *const *B = F.f[cur ^ 1];
@@ -830,6 +834,261 @@ __global__ void __launch_bounds__(ATX * ATY) k_direct(step_consts c, direct_cons
     B[F_Q][ci] = q + (fma(-vh, f2[1], -uh * f1[1]) - c.mu * third * (ux + vy) - dtmp * q);
     B[F_S][ci] = s + (fma(-vh, f2[2], -uh * f1[2]) + two_omega * t + c.mu * (ux - vy) - dtmp * s);
     B[F_TAU][ci] = t + (fma(-vh, f2[3], -uh * f1[3]) - two_omega * s + c.mu * (vx + uy) - dtmp * t);
+}
+
+__global__ void __launch_bounds__(ATX * ATY) k_direct(step_consts c, direct_consts d, fields_dev F, int cur,
+                                                      double dt, double bv) {
+    direct_tile_step(c, d, F, cur, dt, bv, blockIdx.x, blockIdx.y);
+}
+
+// The explicit step with the arithmetic of k_advect_fx: the nine advected
+// fields (the node velocity among them) in 64-bit fixed point, and with them
+// the exact sums of the net force (the four stresses share one scale), the
+// velocity gradient and the viscous term.  k_direct was bound by its ~160 FP64
+// operations per cell.  Tiles with a value that is not finite and cells near
+// yield are listed for k_direct_rest.
+struct fxd_smem {
+    union {
+        double d[DF_COUNT][FROWS][ACOLS];  // TMA destination of the first seven (128-byte aligned)
+        long long v[DF_COUNT][FROWS][ACOLS];
+    } t;
+    unsigned top[DF_COUNT];  // largest high word's magnitude per field
+    int xs[ACOLS], col[ACOLS];
+    // -hx, -hy times the scale of the stresses' sums; hx, hy, hxxv, hyyv times that of the velocities
+    double xfs, yfs, hx[2], hy[2], vx[2], vy[2];
+    uint64_t bar;
+};
+
+__global__ void __launch_bounds__(ATX * ATY, 4)
+    k_direct_fx(step_consts c, direct_consts d, advect_fx_consts h, const __grid_constant__ field_boxes maps,
+                fields_dev F, int cur, double bv) {
+    extern __shared__ __align__(128) unsigned char fxd_raw[];
+    fxd_smem &Sm = *reinterpret_cast<fxd_smem *>(fxd_raw + ((128 - (smem_addr(fxd_raw) & 127)) & 127));
+    const int m = c.m, n = c.n;
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * ATX + tx;
+    const int i0 = blockIdx.x * ATX, j0 = blockIdx.y * FXY;
+    const int i = i0 + tx;
+    const double *__restrict__ const *A = F.f[cur];
+    double *const *B = F.f[cur ^ 1];
+    if (tid == 0) mbar_init(&Sm.bar, 1);
+    if (tid < ACOLS) {
+        const int u = i0 + tid - 2;
+        int w = u % m;
+        if (w < 0) w += m;
+        Sm.col[tid] = w;
+        Sm.xs[tid] = u < 0 ? -1 : (u >= m ? 1 : 0);
+    }
+    if (tid < DF_COUNT) Sm.top[tid] = 0;
+    __syncthreads();
+    if (tid == 0) {
+        mbar_expect_tx(&Sm.bar, kFxBytes);
+        for (int f = 0; f < F_COUNT; f++) tma_load_2d(&Sm.t.d[f][0][0], &maps.f[cur][f], i0 - 2, j0 - 1, &Sm.bar);
+    }
+    // node velocities of the tile's rows while it arrives
+    constexpr int kTile = FROWS * ACOLS, kPer = (kTile + ATX * ATY - 1) / (ATX * ATY);
+    unsigned utop = 0, vtop = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+        const int p = tid + q * ATX * ATY, r = p / ACOLS, t = p - r * ACOLS, nj = j0 - 2 + r;
+        double2 v = make_double2(0.0, 0.0);
+        if (p >= kTile) break;
+        if (nj >= 0 && nj <= n) {
+            if (nj == 0 || nj == n) v.x = nj == 0 ? -bv : bv;
+            else v = F.vel[(size_t)nj * m + Sm.col[t]];
+        }
+        (&Sm.t.d[DF_U][0][0])[p] = v.x;
+        (&Sm.t.d[DF_V][0][0])[p] = v.y;
+        utop = max(utop, (unsigned)__double2hiint(v.x) & 0x7fffffffu);
+        vtop = max(vtop, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
+    }
+    if (__syncthreads_or(!mbar_wait_bounded(&Sm.bar))) {
+        if (tid == 0) atomicExch(&F.flags[FL_TMA], 1);
+        mbar_wait_bounded(&Sm.bar);
+        return;
+    }
+    if (i0 == 0 || i0 + ACOLS - 2 > m) {
+        for (int k = tid; k < F_COUNT * kTile; k += ATX * ATY) {
+            const int f = k / kTile, rem = k - f * kTile, r = rem / ACOLS, t = rem - r * ACOLS;
+            const int u = i0 + t - 2, sr = j0 - 1 + r;
+            if ((u < 0 || u >= m) && sr >= 0 && sr <= n + 1) Sm.t.d[f][r][t] = A[f][(size_t)sr * m + Sm.col[t]];
+        }
+        __syncthreads();
+    }
+    {
+        unsigned top[F_COUNT];
+#pragma unroll
+        for (int f = 0; f < F_COUNT; f++) top[f] = 0;
+        for (int p = tid; p < kTile; p += ATX * ATY) {
+#pragma unroll
+            for (int f = 0; f < F_COUNT; f++)
+                top[f] = max(top[f], (unsigned)__double2hiint((&Sm.t.d[f][0][0])[p]) & 0x7fffffffu);
+        }
+#pragma unroll
+        for (int f = 0; f < F_COUNT; f++) {
+            const unsigned w = __reduce_max_sync(0xffffffffu, top[f]);
+            if (tx == 0) atomicMax(&Sm.top[f], w);
+        }
+        utop = __reduce_max_sync(0xffffffffu, utop);
+        vtop = __reduce_max_sync(0xffffffffu, vtop);
+        if (tx == 0) {
+            atomicMax(&Sm.top[DF_U], utop);
+            atomicMax(&Sm.top[DF_V], vtop);
+        }
+    }
+    __syncthreads();
+    int E[DF_COUNT];
+    bool finite = true;
+#pragma unroll
+    for (int f = 0; f < DF_COUNT; f++) {
+        E[f] = max((int)(Sm.top[f] >> 20), 128);
+        finite = finite && E[f] < 0x7ff;
+    }
+    if (!finite) {  // the same for the whole block: two of k_direct's tiles
+        if (tid < 2 && j0 + tid * ATY < n)
+            F.tlist[atomicAdd(F.pcount + 1, 1u)] = (2 * blockIdx.y + tid) * gridDim.x + blockIdx.x;
+        return;
+    }
+    E[F_X] = max(E[F_X], (int)((unsigned)__double2hiint(c.lx) >> 20)) + 1;
+    const long long lx = to_fixed(c.lx, E[F_X]);
+    // the stresses at one scale, and both velocities at one (cut to it)
+    const int Es = max(max(E[F_P], E[F_Q]), max(E[F_S], E[F_TAU])), Eu = max(E[DF_U], E[DF_V]);
+    auto cut = [](long long v, int by) { return v >> min(by, 63); };
+    if (tid == 0) {
+        const double ss = power_of_two(Es - 1081);
+        Sm.xfs = -d.hx * ss;
+        Sm.yfs = -d.hy * ss;
+    }
+    if (tid < 2) {
+        const double su = power_of_two((tid ? E[DF_V] : E[DF_U]) - 1081);
+        Sm.hx[tid] = d.hx * su;
+        Sm.hy[tid] = d.hy * su;
+        Sm.vx[tid] = d.hxxv * su;
+        Sm.vy[tid] = d.hyyv * su;
+    }
+    for (int p = tid; p < kTile; p += ATX * ATY) {
+#pragma unroll
+        for (int f = 0; f < DF_COUNT; f++) {
+            long long v = to_fixed((&Sm.t.d[f][0][0])[p], E[f]);
+            if (f == F_X) {
+                const int sh = Sm.xs[p % ACOLS];
+                if (sh) v += sh > 0 ? lx : -lx;
+            }
+            (&Sm.t.v[f][0][0])[p] = v;
+        }
+    }
+    __syncthreads();
+    if (i >= m) return;
+    const int Ku = Eu + h.he - 2037;
+#pragma unroll 1
+    for (int row = ty; row < FXY; row += ATY) {
+        const int j = j0 + row;
+        if (j >= n) return;
+        const size_t ci = (size_t)(j + 1) * m + i;
+        const int at = (row + 2) * ACOLS + tx + 2;
+        auto fld = [&](int f) { return &Sm.t.v[f][0][0] + at; };
+        auto upwind = [&](int f, const fx_factor &uh, int dx, const fx_factor &vh, int dy, bool inner) {
+            return -(double)fx_products(uh, eno_fx(fld(f), dx, true), vh, eno_fx(fld(f), dy, inner)) *
+                   power_of_two(E[f] + Ku);
+        };
+        const long long *U = fld(DF_U), *V = fld(DF_V);
+        if (j > 0) {
+            const long long u0 = U[0], v0 = V[0];
+            const fx_factor uh(4 * cut(u0, Eu - E[DF_U]), h.hmx), vh(4 * cut(v0, Eu - E[DF_V]), h.hmy);
+            const int dx = u0 > 0 ? 1 : -1, dy = v0 > 0 ? ACOLS : -ACOLS;
+            const bool inner = v0 > 0 ? j > 1 : j < n - 1;
+            // net force from the cells (i-1,j-1), (i,j-1), (i-1,j), (i,j)
+            long long a[4], b[4], t[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int o = (k & 1) - 1 + ((k >> 1) - 1) * ACOLS;
+                const long long pq = cut(fld(F_P)[o], Es - E[F_P]) + cut(fld(F_Q)[o], Es - E[F_Q]);
+                const long long sv = cut(fld(F_S)[o], Es - E[F_S]);
+                a[k] = pq - sv;
+                b[k] = pq + sv;
+                t[k] = cut(fld(F_TAU)[o], Es - E[F_TAU]);
+            }
+            const double xfs = Sm.xfs, yfs = Sm.yfs;
+            const double fx = fma(xfs, (double)((a[1] - a[0]) + (a[3] - a[2])),
+                                  yfs * (double)((t[0] - t[2]) + (t[1] - t[3])));
+            const double fy = fma(xfs, (double)((t[0] - t[1]) + (t[2] - t[3])),
+                                  yfs * (double)((b[2] - b[0]) + (b[3] - b[1])));
+            const double uvisc = fma(Sm.vx[0], (double)((U[1] - u0) + (U[-1] - u0)),
+                                     Sm.vy[0] * (double)((U[ACOLS] - u0) + (U[-ACOLS] - u0)));
+            const double vvisc = fma(Sm.vx[1], (double)((V[1] - v0) + (V[-1] - v0)),
+                                     Sm.vy[1] * (double)((V[ACOLS] - v0) + (V[-ACOLS] - v0)));
+            const double2 w = F.vel[(size_t)j * m + i];
+            F.src[(size_t)j * m + i] =
+                make_double2(w.x + fma(d.mu_inv, fx + uvisc, upwind(DF_U, uh, dx, vh, dy, inner)),
+                             w.y + fma(d.mu_inv, fy + vvisc, upwind(DF_V, uh, dx, vh, dy, inner)));
+#pragma unroll
+            for (int f = F_X; f <= F_Y; f++) B[f][ci] = A[f][ci] + upwind(f, uh, dx, vh, dy, inner);
+        }
+        // deformation rate, staggered velocity and spin
+        const long long u00 = U[0], u10 = U[1], u01 = U[ACOLS], u11 = U[ACOLS + 1];
+        const long long v00 = V[0], v10 = V[1], v01 = V[ACOLS], v11 = V[ACOLS + 1];
+        const long long u4 = (u00 + u10) + (u01 + u11), v4 = (v00 + v10) + (v01 + v11);
+        const double ux = Sm.hx[0] * (double)((u10 - u00) + (u11 - u01));
+        const double uy = Sm.hy[0] * (double)((u01 - u00) + (u11 - u10));
+        const double vx = Sm.hx[1] * (double)((v10 - v00) + (v11 - v01));
+        const double vy = Sm.hy[1] * (double)((v01 - v00) + (v11 - v10));
+        const double two_omega = vx - uy, div = ux + vy;
+        const fx_factor uh(cut(u4, Eu - E[DF_U]), h.hmx), vh(cut(v4, Eu - E[DF_V]), h.hmy);
+        const int dx = u4 > 0 ? 1 : -1, dy = v4 > 0 ? ACOLS : -ACOLS;
+        const bool inner = v4 > 0 ? j > 0 : j < n - 1;
+        auto inc = [&](int f) { return upwind(f, uh, dx, vh, dy, inner); };
+        const double q = A[F_Q][ci], s = A[F_S][ci], t = A[F_TAU][ci];
+        B[F_P][ci] = A[F_P][ci] + (inc(F_P) - c.K * div);
+        B[F_Q][ci] = q + (inc(F_Q) - c.mu * (1 / 3.0) * div);
+        B[F_S][ci] = s + (fma(two_omega, t, inc(F_S)) + c.mu * (ux - vy));
+        B[F_TAU][ci] = t + (fma(-two_omega, s, inc(F_TAU)) + c.mu * (vx + uy));
+        double cchi = A[F_CHI][ci] + inc(F_CHI);
+        if (d.hccd != 0) {
+            const long long *H = fld(F_CHI);
+            cchi += power_of_two(E[F_CHI] - 1081) *
+                    fma(d.hxxcd, (double)((H[1] - H[0]) + (H[-1] - H[0])),
+                        d.hyycd * (double)((H[ACOLS] - H[0]) + (H[-ACOLS] - H[0])));
+        }
+        B[F_CHI][ci] = cchi;
+        if (!surely_elastic(c, q, s, t)) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
+        F.ddev[ci] = 0;
+    }
+}
+
+// What k_direct_fx left: the listed cells' plastic part and the listed tiles.
+__global__ void __launch_bounds__(ATX * ATY)
+    k_direct_rest(step_consts c, direct_consts d, fields_dev F, int cur, double dt, double bv, int tiles_x) {
+    const unsigned cnt = F.pcount[0], tiles = F.pcount[1];
+    const double *__restrict__ const *A = F.f[cur];
+    double *const *B = F.f[cur ^ 1];
+    const int tid = threadIdx.y * ATX + threadIdx.x;
+    for (unsigned k = blockIdx.x * (ATX * ATY) + tid; k < cnt; k += gridDim.x * (ATX * ATY)) {
+        const size_t ci = F.plist[k];
+        const double q = A[F_Q][ci], s = A[F_S][ci], t = A[F_TAU][ci];
+        const double devsq = 3 * q * q + s * s + t * t;
+        if (devsq < 0.999e-24 || (c.stz_model >= 2 && devsq < c.yield_cut2)) continue;
+        int iters;
+        double chi = B[F_CHI][ci], ddev = 0;
+        const stz_law_params<double> lp = law_params(c);
+        const double sbar = sqrt(devsq), dtmp = adaptive_plastic(lp, sbar, chi, ddev, dt, iters);
+        if (iters >= c.substep_cap) atomicExch(&F.flags[FL_SUBSTEP_CAP], 1);
+        if (iters > 1) atomicMax(&F.flags[FL_SUBSTEP_MAX], iters);
+        B[F_CHI][ci] = chi;
+        F.ddev[ci] = ddev * sbar;
+        if (c.track_plastic && ddev != 0) {
+            const int m = c.m, j = (int)(ci / (size_t)m) - 1, i = (int)(ci - (size_t)(j + 1) * m);
+            F.eps_pl[(size_t)j * m + i] += ddev / (2 * c.mu);
+        }
+        if (dtmp != 0) {
+            B[F_Q][ci] -= dtmp * q;
+            B[F_S][ci] -= dtmp * s;
+            B[F_TAU][ci] -= dtmp * t;
+        }
+    }
+    for (unsigned k = blockIdx.x; k < tiles; k += gridDim.x) {
+        const unsigned tile = F.tlist[k];
+        direct_tile_step(c, d, F, cur, dt, bv, tile % tiles_x, tile / tiles_x);
+        __syncthreads();  // the next tile reuses the shared memory
+    }
 }
 
 __global__ void k_precombine(step_consts c, fields_dev F, int cur, double xf, double yf) {
@@ -1109,6 +1368,11 @@ cudaError_t prepare_step_kernels() {
         e = cudaFuncSetAttribute(k_advect_rest, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(adv_smem) + 128));
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_direct_fx, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(fxd_smem) + 128));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_direct_rest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(direct_tile));
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(direct_tile));
     if (e == cudaSuccess && dev < 64) done |= 1ull << dev;
     return e;
@@ -1147,6 +1411,18 @@ int make_field_maps(const step_consts &c, const fields_dev &F, field_maps *out) 
     return STZG_OK;
 }
 
+static advect_fx_consts fx_consts(double hx, double hy) {
+    advect_fx_consts h;
+    int ex, ey;
+    std::frexp(hx, &ex);
+    std::frexp(hy, &ey);
+    h.he = std::max(ex, ey) - 62;
+    h.hmx = (long long)std::ldexp(hx, -h.he);
+    h.hmy = (long long)std::ldexp(hy, -h.he);
+    h.xf = h.yf = 0;
+    return h;
+}
+
 void advection(const step_consts &c, const field_maps &maps, fields_dev &F, int cur, double dt, double bv,
                cudaStream_t st) {
     dim3 blk(32, 8);
@@ -1157,13 +1433,7 @@ void advection(const step_consts &c, const field_maps &maps, fields_dev &F, int 
     a.yf = 0.5 / dt * c.ysp;
     const dim3 grid(ceil_div(c.m, ATX), ceil_div(c.n, ATY));
     if (c.fixed_point) {
-        advect_fx_consts h;
-        int ex, ey;
-        std::frexp(a.hx, &ex);
-        std::frexp(a.hy, &ey);
-        h.he = std::max(ex, ey) - 62;
-        h.hmx = (long long)std::ldexp(a.hx, -h.he);
-        h.hmy = (long long)std::ldexp(a.hy, -h.he);
+        advect_fx_consts h = fx_consts(a.hx, a.hy);
         h.xf = a.xf;
         h.yf = a.yf;
         const int pre = !c.sp_increments;
@@ -1186,8 +1456,8 @@ void advection(const step_consts &c, const field_maps &maps, fields_dev &F, int 
     }
 }
 
-void direct_step(const step_consts &c, double viscosity, fields_dev &F, int cur, double dt, double bv,
-                 cudaStream_t st) {
+void direct_step(const step_consts &c, const field_maps &maps, double viscosity, fields_dev &F, int cur, double dt,
+                 double bv, cudaStream_t st) {
     const double hx = 0.5 * c.xsp * dt, hy = 0.5 * c.ysp * dt;
     direct_consts d;
     d.hx = hx;
@@ -1200,7 +1470,17 @@ void direct_step(const step_consts &c, double viscosity, fields_dev &F, int cur,
     d.hyycd = 2 * c.ysp * hy * c.chi_diff;
     d.hccd = 2 * (d.hxxcd + d.hyycd);
     dim3 blk(ATX, ATY);
-    k_direct<<<g2(c.m, c.n, blk), blk, sizeof(direct_tile), st>>>(c, d, F, cur, dt, bv);
+    const dim3 grid = g2(c.m, c.n, blk);
+    if (c.fixed_point) {
+        const advect_fx_consts h = fx_consts(hx, hy);
+        cudaMemsetAsync(F.pcount, 0, 2 * sizeof(unsigned), st);
+        k_direct_fx<<<dim3(grid.x, ceil_div(c.n, FXY)), blk, sizeof(fxd_smem) + 128, st>>>(c, d, h, maps.tall, F, cur,
+                                                                                          bv);
+        note_launch();
+        k_direct_rest<<<2 * 152, blk, sizeof(direct_tile), st>>>(c, d, F, cur, dt, bv, (int)grid.x);
+    } else {
+        k_direct<<<grid, blk, sizeof(direct_tile), st>>>(c, d, F, cur, dt, bv);
+    }
     note_launch();
     if (c.chi_diff != 0 || c.chi_len != 0) {
         k_chi_diffusion<<<g2(c.m, c.n, blk), blk, 0, st>>>(c, F, cur, dt);

@@ -132,8 +132,8 @@ cudaError_t prepare_step_kernels();
 // shear_sim::step_forward (shear_sim.cc:185-276) up to set_boundaries:
 // explicit update of buffer cur into cur^1, new interior node velocities in
 // F.src (rows 1..n-1), chi diffusion.  bv is the wall speed of the state.
-void direct_step(const step_consts &c, double viscosity, fields_dev &F, int cur, double dt, double bv,
-                 cudaStream_t st);
+void direct_step(const step_consts &c, const field_maps &maps, double viscosity, fields_dev &F, int cur, double dt,
+                 double bv, cudaStream_t st);
 // The per-cell combinations above from the current stress (used when the
 // projection runs without the advection kernel in front of it).
 void precombine(const step_consts &c, fields_dev &F, int cur, double dt, cudaStream_t st);
