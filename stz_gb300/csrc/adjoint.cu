@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(128) k_adj_advect(step_consts c, adj_fields A,
             lp.Omegaeps0 = dual::var(c.Omegaeps0, 3);
             lp.chi_inf = dual::var(c.chi_inf, 4);
             lp.s_y = dual::var(c.s_y, 5);
+            lp.derive();
             dual sbar = dual::var(::sqrt(devsq), 0), chiv = dual::var(cchi, 1), dd;
             int iters;
             dual dt_ = adaptive_plastic(lp, sbar, chiv, dd, dt, iters);

@@ -962,6 +962,7 @@ int stzg_ct_create(const stzg_ct_params *p, int device, stzg_ct **out) {
     L.Omegaeps0 = p->Omegaeps0;
     L.chi_inf = p->chi_inf;
     L.s_y = 1;  // s0 of this variant's stz_dynamics (stz_model.hh:20)
+    L.derive();
     if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&s->ev0) != cudaSuccess || cudaEventCreate(&s->ev1) != cudaSuccess)
         return bail(fail(STZG_ECUDA, "stream/event creation failed"));

@@ -690,6 +690,8 @@ __global__ void __launch_bounds__(ATX * ATY)
     double *const *B = F.f[cur ^ 1];
     const bool athermal = c.stz_model >= 2;
     const int tid = threadIdx.y * ATX + threadIdx.x;
+    const stz_law_params<double> lp = law_params(c);
+    const double strain = 1 / (2 * c.mu);
     for (unsigned k = blockIdx.x * (ATX * ATY) + tid; k < cnt; k += gridDim.x * (ATX * ATY)) {
         const size_t ci = F.plist[k];
         const double q = A[F_Q][ci], s = A[F_S][ci], t = A[F_TAU][ci];
@@ -699,7 +701,6 @@ __global__ void __launch_bounds__(ATX * ATY)
             continue;
         int iters;
         double chi = B[F_CHI][ci], ddev = 0;
-        const stz_law_params<double> lp = law_params(c);
         const double dtmp = adaptive_plastic(lp, sqrt(devsq), chi, ddev, dt, iters);
         if (iters >= c.substep_cap) atomicExch(&F.flags[FL_SUBSTEP_CAP], 1);
         if (iters > 1) atomicMax(&F.flags[FL_SUBSTEP_MAX], iters);
@@ -707,7 +708,7 @@ __global__ void __launch_bounds__(ATX * ATY)
         F.ddev[ci] = ddev;
         if (c.track_plastic && ddev != 0) {
             const int m = c.m, j = (int)(ci / (size_t)m) - 1, i = (int)(ci - (size_t)(j + 1) * m);
-            F.eps_pl[(size_t)j * m + i] += ddev / (2 * c.mu);
+            F.eps_pl[(size_t)j * m + i] += ddev * strain;
         }
         if (dtmp != 0) {
             const double qn = B[F_Q][ci] - dtmp * q, sn = B[F_S][ci] - dtmp * s, tn = B[F_TAU][ci] - dtmp * t;
@@ -1061,6 +1062,8 @@ __global__ void __launch_bounds__(ATX * ATY)
     const double *__restrict__ const *A = F.f[cur];
     double *const *B = F.f[cur ^ 1];
     const int tid = threadIdx.y * ATX + threadIdx.x;
+    const stz_law_params<double> lp = law_params(c);
+    const double strain = 1 / (2 * c.mu);
     for (unsigned k = blockIdx.x * (ATX * ATY) + tid; k < cnt; k += gridDim.x * (ATX * ATY)) {
         const size_t ci = F.plist[k];
         const double q = A[F_Q][ci], s = A[F_S][ci], t = A[F_TAU][ci];
@@ -1068,7 +1071,6 @@ __global__ void __launch_bounds__(ATX * ATY)
         if (devsq < 0.999e-24 || (c.stz_model >= 2 && devsq < c.yield_cut2)) continue;
         int iters;
         double chi = B[F_CHI][ci], ddev = 0;
-        const stz_law_params<double> lp = law_params(c);
         const double sbar = sqrt(devsq), dtmp = adaptive_plastic(lp, sbar, chi, ddev, dt, iters);
         if (iters >= c.substep_cap) atomicExch(&F.flags[FL_SUBSTEP_CAP], 1);
         if (iters > 1) atomicMax(&F.flags[FL_SUBSTEP_MAX], iters);
@@ -1076,7 +1078,7 @@ __global__ void __launch_bounds__(ATX * ATY)
         F.ddev[ci] = ddev * sbar;
         if (c.track_plastic && ddev != 0) {
             const int m = c.m, j = (int)(ci / (size_t)m) - 1, i = (int)(ci - (size_t)(j + 1) * m);
-            F.eps_pl[(size_t)j * m + i] += ddev / (2 * c.mu);
+            F.eps_pl[(size_t)j * m + i] += ddev * strain;
         }
         if (dtmp != 0) {
             B[F_Q][ci] -= dtmp * q;

@@ -16,6 +16,15 @@ template <typename S> struct stz_law_params {
     int stz_model, t_model, substep_cap;
     double t_scale, adapt_fac, theta, Delta, tau0, kappa, rho, mu;
     S c0, Omegaeps0, chi_inf, s_y;
+    double Delta_theta, half_rate;  // Delta/theta, 1/(2 tau0)
+    S Omega_theta, gain;            // Omega eps0/theta, 2/(s_y c0)
+    // what the laws use of the parameters above, once they are set
+    __host__ __device__ void derive() {
+        Delta_theta = Delta / theta;
+        half_rate = 0.5 / tau0;
+        Omega_theta = Omegaeps0 / S(theta);
+        gain = S(2) / (s_y * c0);
+    }
 };
 
 __host__ __device__ inline stz_law_params<double> law_params(const step_consts &c) {
@@ -35,6 +44,7 @@ __host__ __device__ inline stz_law_params<double> law_params(const step_consts &
     p.Omegaeps0 = c.Omegaeps0;
     p.chi_inf = c.chi_inf;
     p.s_y = c.s_y;
+    p.derive();
     return p;
 }
 
@@ -73,6 +83,20 @@ __device__ __forceinline__ S dplastic(const stz_law_params<S> &c, S sbar, S chi,
     if (value(sbar) < value(s0)) {
         dchi1 = S(0);
         return S(0);
+    }
+    // stz_model.hh:103-151 far from the backward jumps: with x = Om sbar/theta
+    // above 20, exp(-2x) is below half a unit in the last place of 1, so tanh(x)
+    // is 1 and the rate is one exponential times 1 - s0/sbar.  Two more
+    // exponentials, a tanh and four divisions of the general form below are FP64
+    // work that bounded every kernel that evaluates it (175 FP64 operations a
+    // cell, now about 90).
+    if (c.stz_model == 2 && (c.t_model == -1 || De >= value(Om * sbar))) {
+        const S x = c.Omega_theta * sbar;
+        if (value(x) > 20) {
+            const S Dpl = c.half_rate * exp(x - c.Delta_theta - 1 / chi) * (1 - s0 / sbar);
+            dchi1 = c.gain * Dpl * sbar;
+            return Dpl;
+        }
     }
     S sC, sT;
     if (c.stz_model == 3) {  // stz_model.hh:179-206
