@@ -11,9 +11,11 @@
 // costs 10 to 20 issue slots on the FP32 pipe where an FP64 one blocks its
 // quarter of the SM for 64 clocks.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "ff.cuh"
+#include "fixed.cuh"
 #include "mg.cuh"
 #include "mg_device.cuh"
 #include "mg_plan.h"
@@ -57,31 +59,132 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     small_vcycle<false, false>(P, env);
 }
 
-// r = b - A z of the top level in FP64 as float pairs; with partials, the sums
-// of r^2 and b^2 per block (as k_top_sqnorm).
-constexpr int kResThreads = 256;
-__global__ void __launch_bounds__(kResThreads) k_res_pairs(top_op<double> op, const double2 *__restrict__ z,
-                                                           const double2 *__restrict__ b, int m, int n,
-                                                           float4 *__restrict__ r, double *partials) {
+// r = b - A z of the top level as float pairs; with partials, the sums of r^2
+// and b^2 per block (as k_top_sqnorm).
+// A z is evaluated on second differences of z, exact in 64-bit fixed point
+// (fixed.cuh, one scale per tile), and integer products with the
+// coefficients; only b - A z and the norms are FP64.  The rounding is 0.6
+// units of 2^-55 max|z| times the largest coefficient, an eighth of the
+// plain FP64 sum's.  FP64 operations per node: 31 in the plain form, which was
+// bound by them (56 us at 1024^2), four here.
+// A block walks tiles of 32 x 8 RPT nodes (RPT rows per thread) with the next
+// tile's loads in flight: two rows per thread where that still gives each SM
+// two tiles, else one (latency).  Tiles with an infinity or a NaN take the FP64 form.
+constexpr int kResThreads = 256, RX = 32, RC = RX + 2, kResRows = kResThreads / RX;
+
+// A coefficient over 2^ke, in two words, the lower one halved.
+struct res_factor {
+    int hi, lo;
+};
+struct res_consts {
+    res_factor Kmx, Kmy, mx, my, qK, dxx, dyy;  // dxx = cxx + 2 (Kmx + my), dyy = cyy + 2 (mx + Kmy)
+    int ke;
+};
+struct res_sum {
+    long long H, M;
+    __device__ __forceinline__ void add(const res_factor &w, long long a) {
+        const int a1 = (int)(a >> 32), a0 = (int)((unsigned)a >> 1);
+        H += (long long)w.hi * a1;
+        M += (long long)w.lo * a1 + (long long)w.hi * a0;
+    }
+    // sum / 2^64; the 1 is the mean of the parts dropped
+    __device__ __forceinline__ double value() const { return (double)(H + (M >> 31) + 1); }
+};
+
+template <int RPT>
+__global__ void __launch_bounds__(kResThreads, 4)
+    k_res_pairs(top_op<double> op, res_consts C, const double2 *__restrict__ z, const double2 *__restrict__ b, int m,
+                int n, int tiles_x, int tiles, float4 *__restrict__ r, double *partials) {
+    constexpr int RY = kResRows * RPT, RR = RY + 2;
+    __shared__ long long X[RR][RC], Y[RR][RC];
+    __shared__ unsigned top[2];
     __shared__ double sh[32];
-    const unsigned total = (unsigned)m * (unsigned)n;
+    constexpr int kPer = (RR * RC + kResThreads - 1) / kResThreads;
+    const int tid = threadIdx.x, tx = tid & (RX - 1), ty = tid / RX;
     double sr = 0, sb = 0;
-    for (unsigned k = blockIdx.x * kResThreads + threadIdx.x; k < total; k += gridDim.x * kResThreads) {
-        const int j = (int)(k / (unsigned)m), i = (int)k - j * m;
-        const double2 v = top_res<double>(op, z, b, m, n, i, j);
-        float4 o;
-        ff_split_d(v.x, o.x, o.z);
-        ff_split_d(v.y, o.y, o.w);
-        r[k] = o;
-        if (partials) {
-            const double2 bb = b[k];
-            sr += v.x * v.x + v.y * v.y;
-            sb += bb.x * bb.x + bb.y * bb.y;
+    double2 v[kPer];
+    auto load = [&](int tile) {
+        const int i0 = (tile % tiles_x) * RX, j0 = (tile / tiles_x) * RY;
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+            const int p = tid + q * kResThreads, row = p / RC, t = p - row * RC, j = j0 + row - 1;
+            int i = i0 + t - 1;
+            v[q] = make_double2(0.0, 0.0);
+            if (p >= RR * RC || j < 0 || j >= n || i > m) continue;
+            if (i < 0) i += m;
+            if (i == m) i = 0;
+            v[q] = z[(size_t)j * m + i];
         }
+    };
+    if (tid < 2) top[tid] = 0;
+    if ((int)blockIdx.x < tiles) load(blockIdx.x);
+    __syncthreads();
+    int it = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, it ^= 1) {
+        const int i = (tile % tiles_x) * RX + tx, j0 = (tile / tiles_x) * RY;
+        double2 g[RPT];
+#pragma unroll
+        for (int q = 0; q < RPT; q++) {
+            const int j = j0 + ty * RPT + q;
+            g[q] = i < m && j < n ? b[(size_t)j * m + i] : make_double2(0.0, 0.0);
+        }
+        unsigned w = 0;
+#pragma unroll
+        for (int q = 0; q < kPer; q++)
+            w = max(w, max((unsigned)__double2hiint(v[q].x) & 0x7fffffffu, (unsigned)__double2hiint(v[q].y) & 0x7fffffffu));
+        w = __reduce_max_sync(0xffffffffu, w);
+        if (tx == 0) atomicMax(&top[it], w);
+        __syncthreads();
+        const int E = max((int)(top[it] >> 20), 128);
+        const bool finite = E < 0x7ff;
+        if (tid == 0) top[it ^ 1] = 0;
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+            const int p = tid + q * kResThreads;
+            if (p < RR * RC && finite) {
+                (&X[0][0])[p] = to_fixed(v[q].x, E);
+                (&Y[0][0])[p] = to_fixed(v[q].y, E);
+            }
+        }
+        if (tile + (int)gridDim.x < tiles) load(tile + gridDim.x);
+        __syncthreads();
+        const double unit = power_of_two(64 + C.ke + E - 1081);
+#pragma unroll
+        for (int q = 0; q < RPT; q++) {
+            const int row = ty * RPT + q, j = j0 + row;
+            if (i >= m || j >= n) continue;
+            const size_t k = (size_t)j * m + i;
+            double2 e;
+            if (j == 0 || j == n - 1 || !finite) {
+                e = top_res<double>(op, z, b, m, n, i, j);
+            } else {
+                const long long *x = &X[row + 1][tx + 1], *y = &Y[row + 1][tx + 1];
+                const long long x0 = x[0], y0 = y[0];
+                res_sum ax{0, 0}, ay{0, 0};
+                ax.add(C.Kmx, (x[-1] - x0) + (x[1] - x0));
+                ax.add(C.my, (x[-RC] - x0) + (x[RC] - x0));
+                ax.add(C.qK, (y[-RC - 1] - y[-RC + 1]) + (y[RC + 1] - y[RC - 1]));
+                ax.add(C.dxx, x0);
+                ay.add(C.mx, (y[-1] - y0) + (y[1] - y0));
+                ay.add(C.Kmy, (y[-RC] - y0) + (y[RC] - y0));
+                ay.add(C.qK, (x[-RC - 1] - x[-RC + 1]) + (x[RC + 1] - x[RC - 1]));
+                ay.add(C.dyy, y0);
+                e = make_double2(fma(-unit, ax.value(), g[q].x), fma(-unit, ay.value(), g[q].y));
+            }
+            float4 o;
+            ff_split_d(e.x, o.x, o.z);
+            ff_split_d(e.y, o.y, o.w);
+            r[k] = o;
+            if (partials) {
+                sr += e.x * e.x + e.y * e.y;
+                sb += g[q].x * g[q].x + g[q].y * g[q].y;
+            }
+        }
+        __syncthreads();  // the next tile reuses the planes
     }
     if (!partials) return;
     const double a = block_sum(sr, sh), c = block_sum(sb, sh);
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         partials[2 * blockIdx.x] = a;
         partials[2 * blockIdx.x + 1] = c;
     }
@@ -318,9 +421,34 @@ bool pair_cycle_supported(const hierarchy<double> &h) {
 
 void pair_residual(const hierarchy<double> &h, double *partials, int npart, cudaStream_t st) {
     const level_view<double> &T0 = h.lv[0];
-    const int blocks = partials ? npart : std::min(npart, ceil_div((long)T0.m * T0.n, kResThreads));
-    k_res_pairs<<<blocks, kResThreads, 0, st>>>(h.op, T0.z, T0.b, T0.m, T0.n, reinterpret_cast<float4 *>(T0.r),
-                                                partials);
+    const top_op<double> &o = h.op;
+    res_consts C;
+    std::frexp(std::max(std::max(std::fabs(o.Kmx), std::fabs(o.Kmy)),
+                        std::max(std::max(std::fabs(o.mx), std::fabs(o.my)), std::fabs(o.qK))), &C.ke);
+    C.ke -= 61;  // the largest magnitude is in [2^60, 2^61)
+    auto factor = [&](double d) {
+        const long long w = (long long)std::ldexp(d, -C.ke);
+        return res_factor{(int)(w >> 32), (int)((unsigned)w >> 1)};
+    };
+    C.Kmx = factor(o.Kmx);
+    C.Kmy = factor(o.Kmy);
+    C.mx = factor(o.mx);
+    C.my = factor(o.my);
+    C.qK = factor(o.qK);
+    // with the rounding error of the sums, so that the operator is h.op's exactly
+    auto excess = [](double c, double p, double q) {
+        const double s = p + q, t = s - p, e = (p - (s - t)) + (q - t);
+        return (c + 2 * s) + 2 * e;
+    };
+    C.dxx = factor(excess(o.cxx, o.Kmx, o.my));
+    C.dyy = factor(excess(o.cyy, o.mx, o.Kmy));
+    auto run = [&](auto kernel, int rows) {
+        const int tiles_x = ceil_div(T0.m, RX), tiles = tiles_x * ceil_div(T0.n, rows);
+        kernel<<<partials ? npart : std::min(npart, tiles), kResThreads, 0, st>>>(
+            o, C, T0.z, T0.b, T0.m, T0.n, tiles_x, tiles, reinterpret_cast<float4 *>(T0.r), partials);
+    };
+    if (ceil_div(T0.m, RX) * ceil_div(T0.n, 2 * kResRows) < 2 * 152) run(k_res_pairs<1>, kResRows);
+    else run(k_res_pairs<2>, 2 * kResRows);
     note_launch();
 }
 
