@@ -137,6 +137,9 @@ int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, 
     // cluster a single simulation takes (24 instances of 64^2 to 512^2, graph
     // time at 16 / 8 / 4 / 2 / 1 blocks: 21.8 / 20.1 / 20.0 / 21.5 / 25.4 ms)
     s->h64.small_blocks = s->h32.small_blocks = b->sims.size() > 8 ? 4 : 16;
+    // and the top level's long marches, whose halo is smaller (graph time 18.9
+    // ms; 19.9 with the short ones)
+    s->h32.crowded = b->sims.size() > 8;
     double *clk = b->dclock + (size_t)k * CLK_COUNT;
     int *ctr = b->dctr + (size_t)k * CTR_COUNT;
     // the captured step kernels read time, wall data and buffer index from the clock

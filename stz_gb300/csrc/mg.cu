@@ -955,8 +955,7 @@ __device__ __forceinline__ int wrapx(int x, int m) { return x < 0 ? x + m : (x >
 constexpr int kFusedThreads = 256;     // blockDim of the coarse tile kernels
 constexpr int kFusedMinWidth = 80;     // narrowest even periodic line of the tile and strip kernels
 constexpr int kMarchWarps = 4;         // warps (row tiles) per block of the top-level kernels
-constexpr int kDownRows = 8;  // coarse rows per warp tile (down)
-constexpr int kUpRows = 8;      // coarse rows per warp tile (up)
+constexpr int kTopRows = 8;            // most coarse rows per warp tile of the top-level kernels
 constexpr int kMarchMinWidth = 64;     // narrowest even periodic line of the streaming kernels
 constexpr int kDownCols = 28;          // coarse columns per strip (down): fine [xs + 4, xs + 60)
 constexpr int kUpCols = 30;            // coarse columns per strip (up):   fine [xs + 2, xs + 62)
@@ -1203,7 +1202,7 @@ struct top_march {
 // One row step of the down march: row k arrives, colour 0 on row k-1,
 // colour 1 on row k-2 (stored when owned), the residual on row k-3, and the
 // restriction to coarse row (k-4)/2 when k-3 is odd.
-template <int U>
+template <int U, int TCH>
 __device__ __forceinline__ void top_down_step(const top_march &t, int k, float4 (&Z)[kRing], float4 (&B)[kRing],
                                               float2 (&R)[kRing]) {
     constexpr int P1 = (U + 5) % 6, P2 = (U + 4) % 6, P3 = (U + 3) % 6, P4 = (U + 2) % 6, P5 = (U + 1) % 6;
@@ -1219,7 +1218,7 @@ __device__ __forceinline__ void top_down_step(const top_march &t, int k, float4 
     if (j0 >= t.y0 - 3 && j0 >= 0 && j0 < n) march_color<E0>(t.op, Z[P2], Z[P1], Z[U], B[P1], j0, n);
     if (j1 >= t.y0 - 2 && j1 >= 0 && j1 < n) {
         march_color<E1>(t.op, Z[P3], Z[P2], Z[P1], B[P2], j1, n);
-        if (j1 >= t.y0 && j1 < t.y0 + 2 * kDownRows && t.own)
+        if (j1 >= t.y0 && j1 < t.y0 + 2 * TCH && t.own)
             *reinterpret_cast<float4 *>(t.zout + (size_t)j1 * t.m + t.gx) = Z[P2];
     }
     if (j2 >= t.y0 - 1) {
@@ -1234,6 +1233,8 @@ __device__ __forceinline__ void top_down_step(const top_march &t, int k, float4 
 
 // Pre-smooth + residual + restriction of the top level (apply_r after one
 // gauss_seidel, tgmg.in.cc:313-320): z_out = one sweep of z_in, bc = R(b - A z_out).
+// TCH: coarse rows per warp.
+template <int TCH>
 __global__ void __launch_bounds__(32 * kMarchWarps) k_top_down(top_op<float> op, const float2 *__restrict__ zin,
                                                                const float2 *__restrict__ b, int m, int n,
                                                                float2 *__restrict__ zout, float2 *__restrict__ bc,
@@ -1241,7 +1242,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps) k_top_down(top_op<float> op,
     __shared__ __align__(16) float4 ring[kMarchWarps][kRing][2][32];
     pdl_trigger();
     const int lane = threadIdx.x & 31;
-    const int J0 = (blockIdx.y * kMarchWarps + (threadIdx.x >> 5)) * kDownRows;
+    const int J0 = (blockIdx.y * kMarchWarps + (threadIdx.x >> 5)) * TCH;
     if (J0 >= cn) return;
     const int I0 = blockIdx.x * kDownCols;
     top_march t;
@@ -1256,7 +1257,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps) k_top_down(top_op<float> op,
     t.cn = cn;
     t.y0 = 2 * J0;
     t.kb = t.y0 - 4;
-    t.ke = t.y0 + 2 * kDownRows + 2;
+    t.ke = t.y0 + 2 * TCH + 2;
     const int xs = 2 * I0 - 4;
     t.gx = wrapx(xs + 2 * lane, m);
     t.lane = lane;
@@ -1275,17 +1276,17 @@ __global__ void __launch_bounds__(32 * kMarchWarps) k_top_down(top_op<float> op,
     pdl_wait();
     for (int d = 0; d < kRing - 1; d++) ring_issue(t.rg, d, zin, b, t.kb + d, m, n, t.gx, lane);
     for (int k = t.kb; k <= t.ke; k += kRing) {
-        top_down_step<0>(t, k, Z, B, R);
+        top_down_step<0, TCH>(t, k, Z, B, R);
         if (k + 1 > t.ke) break;
-        top_down_step<1>(t, k + 1, Z, B, R);
+        top_down_step<1, TCH>(t, k + 1, Z, B, R);
         if (k + 2 > t.ke) break;
-        top_down_step<2>(t, k + 2, Z, B, R);
+        top_down_step<2, TCH>(t, k + 2, Z, B, R);
         if (k + 3 > t.ke) break;
-        top_down_step<3>(t, k + 3, Z, B, R);
+        top_down_step<3, TCH>(t, k + 3, Z, B, R);
         if (k + 4 > t.ke) break;
-        top_down_step<4>(t, k + 4, Z, B, R);
+        top_down_step<4, TCH>(t, k + 4, Z, B, R);
         if (k + 5 > t.ke) break;
-        top_down_step<5>(t, k + 5, Z, B, R);
+        top_down_step<5, TCH>(t, k + 5, Z, B, R);
     }
 }
 
@@ -1315,15 +1316,17 @@ __device__ __forceinline__ void top_up_step(const top_march &t, const float2 (*c
 // up_gs_iterations, tgmg.in.cc:323-327): z_out = one sweep of z_in + P zc.
 // Fine node i takes coarse i/2 (even) or the mean of (i-1)/2 and (i+1)/2
 // (odd, wrapping on the even periodic line); rows through p1d_halves.
+// TCH: coarse rows per warp.
+template <int TCH>
 __global__ void __launch_bounds__(32 * kMarchWarps) k_top_up(top_op<float> op, const float2 *__restrict__ zin,
                                                              const float2 *__restrict__ b, int m, int n,
                                                              const float2 *__restrict__ zc, int cm, int cn,
                                                              float2 *__restrict__ zout) {
     __shared__ __align__(16) float4 ring[kMarchWarps][kRing][2][32];
-    __shared__ float2 czs[kMarchWarps][kUpRows + 3][33];
+    __shared__ float2 czs[kMarchWarps][TCH + 3][33];
     pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int J0 = (blockIdx.y * kMarchWarps + w) * kUpRows;
+    const int J0 = (blockIdx.y * kMarchWarps + w) * TCH;
     if (J0 >= cn) return;
     const int I0 = blockIdx.x * kUpCols;
     const int xs = 2 * I0 - 2;
@@ -1339,7 +1342,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps) k_top_up(top_op<float> op, c
     t.cn = cn;
     t.y0 = 2 * J0;
     t.kb = t.y0 - 2;
-    t.ke = t.y0 + 2 * kUpRows + 1;
+    t.ke = t.y0 + 2 * TCH + 1;
     t.gx = wrapx(xs + 2 * lane, m);
     t.lane = lane;
     t.I = 0;
@@ -1354,7 +1357,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps) k_top_up(top_op<float> op, c
     }
     pdl_wait();
     for (int d = 0; d < kRing - 1; d++) ring_issue(t.rg, d, zin, b, t.kb + d, m, n, t.gx, lane);
-    stage_coarse<kUpRows + 3>(czs[w], zc, cm, cn, xs / 2, J0 - 1, lane);
+    stage_coarse<TCH + 3>(czs[w], zc, cm, cn, xs / 2, J0 - 1, lane);
     for (int k = t.kb; k <= t.ke; k += kRing) {
         top_up_step<0>(t, czs[w], J0, k, Z, B);
         if (k + 1 > t.ke) break;
@@ -2534,15 +2537,30 @@ template <typename T> void launch_lev_up(level_view<T> &F, level_view<T> &C, cud
     note_launch();
 }
 
+// Coarse rows per warp of the top-level kernels, as in march_rows but at most
+// 8.  A march of 8 coarse rows is 23 row steps (down) or 20 (up) one after
+// another, at 2 rows 11 and 8, and below 2048^2 there are too few warps to
+// hide them: V-cycle at 256^2 / 512^2 / 1024^2 with 8 rows 45 / 62 / 84 us, so
+// 36 / 54 / 73 us (2048^2 keeps 8).
+template <typename T> static int top_rows(const hierarchy<T> &h, int strips, int cn) {
+    return h.crowded ? kTopRows : std::min(march_rows(strips, cn), kTopRows);
+}
+
 // The streaming top-level kernels (single precision only): the swept z goes
 // to the level's r array on the way down and back to z on the way up.
 template <typename T> void launch_top_down(hierarchy<T> &h, cudaStream_t st, bool zero_start) {
     if constexpr (sizeof(T) == 4) {
         level_view<T> &T0 = h.lv[0], &C = h.lv[1];
-        dim3 g(ceil_div(C.m, kDownCols), ceil_div(ceil_div(C.n, kDownRows), kMarchWarps));
-        launch_pdl(k_top_down, g, dim3(32 * kMarchWarps), 0, st, h.op,
-                   zero_start ? (const float2 *)nullptr : (const float2 *)T0.z, (const float2 *)T0.b,
-                   T0.m, T0.n, T0.r, C.b, C.m, C.n);
+        const int strips = ceil_div(C.m, kDownCols), t = top_rows(h, strips, C.n);
+        const dim3 g(strips, ceil_div(ceil_div(C.n, t), kMarchWarps));
+        auto go = [&](auto kernel) {
+            launch_pdl(kernel, g, dim3(32 * kMarchWarps), 0, st, h.op,
+                       zero_start ? (const float2 *)nullptr : (const float2 *)T0.z, (const float2 *)T0.b, T0.m, T0.n,
+                       T0.r, C.b, C.m, C.n);
+        };
+        if (t == 8) go(k_top_down<8>);
+        else if (t == 4) go(k_top_down<4>);
+        else go(k_top_down<2>);
         note_launch();
     }
 }
@@ -2550,9 +2568,15 @@ template <typename T> void launch_top_down(hierarchy<T> &h, cudaStream_t st, boo
 template <typename T> void launch_top_up(hierarchy<T> &h, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) {
         level_view<T> &T0 = h.lv[0], &C = h.lv[1];
-        dim3 g(ceil_div(C.m, kUpCols), ceil_div(ceil_div(C.n, kUpRows), kMarchWarps));
-        launch_pdl(k_top_up, g, dim3(32 * kMarchWarps), 0, st, h.op, (const float2 *)T0.r, (const float2 *)T0.b,
-                   T0.m, T0.n, (const float2 *)C.z, C.m, C.n, T0.z);
+        const int strips = ceil_div(C.m, kUpCols), t = top_rows(h, strips, C.n);
+        const dim3 g(strips, ceil_div(ceil_div(C.n, t), kMarchWarps));
+        auto go = [&](auto kernel) {
+            launch_pdl(kernel, g, dim3(32 * kMarchWarps), 0, st, h.op, (const float2 *)T0.r, (const float2 *)T0.b, T0.m,
+                       T0.n, (const float2 *)C.z, C.m, C.n, T0.z);
+        };
+        if (t == 8) go(k_top_up<8>);
+        else if (t == 4) go(k_top_up<4>);
+        else go(k_top_up<2>);
         note_launch();
     }
 }

@@ -97,6 +97,7 @@ template <typename T> class hierarchy {
     int fuse = 1;
     // most blocks of the small-level kernel's cluster (mg_small.cu)
     int small_blocks = 16;
+    bool crowded = false;  // many cycles at the same time: work counts, not latency
     // single precision: the coarse levels at most 512 wide and the tail in
     // one cooperative persistent kernel (set by the owner once
     // coarse_persist_supported() holds; bar: two zeroed device words for its
