@@ -605,7 +605,7 @@ int adjoint_solve(stzg_sim *s, stzg_adjoint *a) {
     hierarchy<double> &h = a->h;
     const size_t nn = (size_t)s->m * (s->n + 1);
     for (int it = 0; it < 200; it++) {
-        top_residual_sqnorm(h, s->partials, s->npart, s->dnorm, s->dnorm + 1, s->st);
+        top_residual_sqnorm(h, norm_sink{s->partials, s->npart, s->dnorm, {}}, s->st);
         STZG_CUDA(cudaMemcpyAsync(s->hnorm, s->dnorm, 16, cudaMemcpyDeviceToHost, s->st));
         STZG_CUDA(cudaStreamSynchronize(s->st));
         const double r2 = s->hnorm[0], b2 = s->hnorm[1];
@@ -705,7 +705,7 @@ int stzg_adjoint_backward(stzg_sim *s, double dloss, double *grad_params, double
     {
         STZG_CUDA(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
         const long c0 = launch_count();
-        vcycle<double>(a->h, s->st, 10, 1);
+        vcycle<double>(a->h, s->st, 10, 1, false, true);  // adjoint_solve has just taken the residual
         vcycle<double>(a->h, s->st, 10, 1);
         a->n_vc = launch_count() - c0;
         discount_launches(a->n_vc);

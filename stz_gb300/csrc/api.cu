@@ -127,13 +127,13 @@ int ensure_ops(stzg_sim *s, double dt) {
 // Residual norms of the current vel/src (FP64) into dnorm = [r.r, b.b];
 // the mixed variant also leaves r in FP32 as the right-hand side of the
 // next FP32 V-cycles.
-void launch_norms(stzg_sim *s, bool mixed) {
+void launch_norms(stzg_sim *s, bool mixed, const loop_rule &rule) {
     const int M = s->m, N = s->n + 1;
+    const norm_sink sink{s->partials, s->npart, s->dnorm, rule};
     if (mixed)
-        ff_residual(s->q.op<double>(), s->zhi, s->zlo, s->bhi, s->blo, M, N, s->h32.lv[0].b, s->partials, s->npart,
-                    s->dnorm, s->dnorm + 1, s->st);
+        ff_residual(s->q.op<double>(), s->zhi, s->zlo, s->bhi, s->blo, M, N, s->h32.lv[0].b, sink, s->st);
     else
-        top_residual_sqnorm(s->h64, s->partials, s->npart, s->dnorm, s->dnorm + 1, s->st);
+        top_residual_sqnorm(s->h64, sink, s->st);
 }
 
 void mixed_begin(stzg_sim *s) {
@@ -282,35 +282,8 @@ int solve_mixed(stzg_sim *s, int *ncyc) {
 // V-cycles) ends a solve that does not converge, with an error flag.
 // h_ran: the IF node after the loop (the float-float merge of the mixed
 // solve), taken only when a pass ran: otherwise the FP64 velocity is still
-// the solution and stays as it is.
-__global__ void k_loop_start(const double *dnorm, int *flags, double tol2, cudaGraphConditionalHandle h,
-                             cudaGraphConditionalHandle h_ran, int has_ran) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const double r2 = dnorm[0], b2 = dnorm[1];
-        const bool conv = b2 > 0 ? r2 <= tol2 * b2 : r2 == 0;
-        const bool nan = isnan(r2);
-        flags[FL_PASSES] = 0;
-        flags[FL_LOOP_ERR] = nan ? 2 : 0;
-        if (nan && !flags[FL_ERR_FIRST]) flags[FL_ERR_FIRST] = 2;
-        cudaGraphSetConditional(h, (!conv && !nan) ? 1u : 0u);
-        if (has_ran) cudaGraphSetConditional(h_ran, (!conv && !nan) ? 1u : 0u);
-    }
-}
-
-__global__ void k_loop_check(const double *dnorm, int *flags, double tol2, int cap, cudaGraphConditionalHandle h) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const double r2 = dnorm[0], b2 = dnorm[1];
-        const bool conv = b2 > 0 ? r2 <= tol2 * b2 : r2 == 0;
-        const bool nan = isnan(r2);
-        const int it = ++flags[FL_PASSES];
-        ++flags[FL_PASSES_SUM];
-        if (nan) flags[FL_LOOP_ERR] = 2;
-        else if (!conv && it >= cap) flags[FL_LOOP_ERR] = 1;
-        if (flags[FL_LOOP_ERR] && !flags[FL_ERR_FIRST]) flags[FL_ERR_FIRST] = flags[FL_LOOP_ERR];
-        cudaGraphSetConditional(h, (!conv && !nan && it < cap) ? 1u : 0u);
-    }
-}
-
+// the solution and stays as it is.  The tests are part of the residual
+// kernels (loop_rule).
 static int loop_cap(const stzg_sim *s, int per_pass) {
     return std::max(1, s->max_thresh / s->mult / per_pass);
 }
@@ -363,9 +336,13 @@ static int build_loop_graph(stzg_sim *s, bool mixed, int inner, bool fused_extra
         extrap_split(s->F.vel, s->vel_prev, s->F.src, s->zhi, s->zlo, s->bhi, s->blo, count, s->st);
     else if (mixed)
         mixed_begin(s);
-    launch_norms(s, mixed);
-    k_loop_start<<<1, 32, 0, s->st>>>(s->dnorm, s->F.flags, tol2, h, h_ran, mixed && mixed_extra == 0 ? 1 : 0);
-    note_launch();
+    loop_rule rule;
+    rule.flags = s->F.flags;
+    rule.tol2 = tol2;
+    rule.has_ran = mixed && mixed_extra == 0 ? 1 : 0;
+    rule.h = h;
+    rule.h_ran = h_ran;
+    launch_norms(s, mixed, rule);
     {
         cudaStreamCaptureStatus cs;
         cudaGraph_t cg;
@@ -416,7 +393,7 @@ static int build_loop_graph(stzg_sim *s, bool mixed, int inner, bool fused_extra
             return abandon_capture(s, cuda_fail(e, "conditional node"));
         }
     } else {
-        for (int c = 0; c < s->extra_iters; c++) vcycle<double>(s->h64, s->st, 10, 1);
+        for (int c = 0; c < s->extra_iters; c++) vcycle<double>(s->h64, s->st, 10, 1, false, c == 0);
     }
     cudaGraph_t got = nullptr;
     e = cudaStreamEndCapture(s->st, &got);
@@ -451,11 +428,11 @@ static int build_loop_graph(stzg_sim *s, bool mixed, int inner, bool fused_extra
         for (int c = 0; c < inner; c++) vcycle<float>(s->h32, s->st, 10, 1, c == 0);
         ff_correct(s->zhi, s->zlo, s->h32.lv[0].z, count, s->st);
     } else {
-        vcycle<double>(s->h64, s->st, 10, 1);
+        vcycle<double>(s->h64, s->st, 10, 1, false, true);
     }
-    launch_norms(s, mixed);
-    k_loop_check<<<1, 32, 0, s->st>>>(s->dnorm, s->F.flags, tol2, loop_cap(s, per_pass), h);
-    note_launch();
+    rule.cap = loop_cap(s, per_pass);
+    rule.has_ran = 0;
+    launch_norms(s, mixed, rule);
     e = cudaStreamEndCapture(s->st, &got);
     if (e != cudaSuccess) {
         cudaGraphDestroy(root);
@@ -672,7 +649,9 @@ int stzg_create(const stz_params *p, const stzg_options *opt, stzg_sim **out) {
     if (o.extrapolate >= 2)
         if ((st = dev_alloc(s, (void **)&s->vel_prev2, nn * sizeof(double2))) != STZG_OK) return bail(st);
     s->npart = reduction_blocks();
-    if ((st = dev_alloc(s, (void **)&s->partials, 2 * s->npart * sizeof(double))) != STZG_OK) return bail(st);
+    if ((st = dev_alloc(s, (void **)&s->partials, (2 * s->npart + 1) * sizeof(double))) != STZG_OK) return bail(st);
+    if (cudaMemsetAsync(s->partials + 2 * s->npart, 0, sizeof(double), s->st) != cudaSuccess)
+        return bail(fail(STZG_ECUDA, "memset"));
     if ((st = dev_alloc(s, (void **)&s->dnorm, 2 * sizeof(double))) != STZG_OK) return bail(st);
     if (cudaMallocHost(&s->hnorm, 2 * sizeof(double)) != cudaSuccess) return bail(fail(STZG_ENOMEM, "pinned alloc"));
     if (cudaMallocHost(&s->hflags, FL_COUNT * sizeof(int)) != cudaSuccess)
@@ -1310,7 +1289,7 @@ int stzg_mg_l2_error(stzg_sim *s, double dt, const double *src, const double *ve
     const size_t nn = (size_t)s->m * (s->n + 1);
     STZG_CUDA(cudaMemcpyAsync(s->F.src, src, nn * sizeof(double2), cudaMemcpyHostToDevice, s->st));
     STZG_CUDA(cudaMemcpyAsync(s->F.vel, vel, nn * sizeof(double2), cudaMemcpyHostToDevice, s->st));
-    top_residual_sqnorm(s->h64, s->partials, s->npart, s->dnorm, s->dnorm + 1, s->st);
+    launch_norms(s, false);
     STZG_CUDA(cudaMemcpyAsync(s->hnorm, s->dnorm, 2 * sizeof(double), cudaMemcpyDeviceToHost, s->st));
     STZG_CUDA(cudaStreamSynchronize(s->st));
     *err = s->hnorm[0] / (double)nn;

@@ -170,10 +170,8 @@ int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, 
     advection(sc, *s->maps, s->F, 0, dt, 0.0, s->st);
     projection_source(sc, s->F, 0, dt, 0.0, s->st);
     if (s->O.extrapolate) extrapolate_guess(s->F.vel, s->vel_prev, count, s->st);
-    if (mixed) {
-        mixed_begin(s);
-        launch_norms(s, true);
-    }
+    if (mixed) mixed_begin(s);
+    launch_norms(s, mixed);
     k_solve_reset<<<1, 32, 0, s->st>>>(ctr, hsolve);
     note_launch();
     cudaStreamCaptureStatus cs;
@@ -207,7 +205,7 @@ int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, 
         ff_correct(s->zhi, s->zlo, s->h32.lv[0].z, count, s->st);
         launch_norms(s, true);
     } else {
-        vcycle<double>(s->h64, s->st, 10, 1);
+        vcycle<double>(s->h64, s->st, 10, 1, false, true);
         launch_norms(s, false);
     }
     const int relative = s->O.tol_mode == STZG_TOL_RELATIVE;

@@ -680,7 +680,7 @@ constexpr int kRedThreads = 256;
 
 template <typename T>
 __global__ void k_top_sqnorm(top_op<T> op, const typename vec2_t<T>::type *__restrict__ z,
-                             const typename vec2_t<T>::type *__restrict__ b, int m, int n, double *partials) {
+                             const typename vec2_t<T>::type *__restrict__ b, int m, int n, norm_sink sink) {
     typedef typename vec2_t<T>::type V;
     __shared__ double sh[32];
     // 32-bit indices (grids are limited to 2^30 points): the division by m
@@ -696,57 +696,7 @@ __global__ void k_top_sqnorm(top_op<T> op, const typename vec2_t<T>::type *__res
     }
     double a = block_sum(sr, sh);
     double c = block_sum(sb, sh);
-    if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = a;
-        partials[2 * blockIdx.x + 1] = c;
-    }
-}
-
-// Sums the per-block partials with one block in a fixed order.
-__global__ void k_final_sum(const double *partials, int npart, double *out, double *out_b) {
-    __shared__ double sh[32];
-    double a = 0, c = 0;
-    for (int k = threadIdx.x; k < npart; k += blockDim.x) {
-        a += partials[2 * k];
-        c += partials[2 * k + 1];
-    }
-    a = block_sum(a, sh);
-    c = block_sum(c, sh);
-    if (threadIdx.x == 0) {
-        *out = a;
-        if (out_b) *out_b = c;
-    }
-}
-
-__global__ void k_mixed_residual(top_op<double> op, const double2 *__restrict__ z, const double2 *__restrict__ b,
-                                 int m, int n, float2 *__restrict__ r32, double *partials) {
-    __shared__ double sh[32];
-    const unsigned total = (unsigned)m * (unsigned)n;
-    double sr = 0, sb = 0;
-    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
-        const int j = (int)(k / (unsigned)m), i = (int)k - j * m;
-        double2 r = top_res<double>(op, z, b, m, n, i, j);
-        r32[k] = make_float2((float)r.x, (float)r.y);
-        sr += r.x * r.x + r.y * r.y;
-        double2 bb = b[k];
-        sb += bb.x * bb.x + bb.y * bb.y;
-    }
-    double a = block_sum(sr, sh);
-    double c = block_sum(sb, sh);
-    if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = a;
-        partials[2 * blockIdx.x + 1] = c;
-    }
-}
-
-__global__ void k_mixed_correct(double2 *__restrict__ z, const float2 *__restrict__ e, long count) {
-    for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (long)gridDim.x * blockDim.x) {
-        float2 d = e[k];
-        double2 v = z[k];
-        v.x += (double)d.x;
-        v.y += (double)d.y;
-        z[k] = v;
-    }
+    finish_norms(a, c, sink, sh);
 }
 
 // Quadratic extrapolation through the last three solutions:
@@ -860,11 +810,11 @@ struct ff_op {
 };
 
 // r = b - A z (qs_multi::mul_a + a_cc) in float-float; r is stored in FP32
-// as the next right-hand side; sum r^2 and sum b^2 go to the partials
-// (FP32 per thread, FP64 across threads).
+// as the next right-hand side; sum r^2 and sum b^2 go to the sink (FP32 per
+// thread, FP64 across threads).
 __global__ void k_ff_residual(ff_op op, const float2 *__restrict__ zh, const float2 *__restrict__ zl,
                               const float2 *__restrict__ bh, const float2 *__restrict__ bl, int m, int n,
-                              float2 *__restrict__ r32, double *partials) {
+                              float2 *__restrict__ r32, norm_sink sink) {
     __shared__ double sh[32];
     const unsigned total = (unsigned)m * (unsigned)n;
     float sr = 0.f, sb = 0.f;
@@ -917,10 +867,7 @@ __global__ void k_ff_residual(ff_op op, const float2 *__restrict__ zh, const flo
     }
     const double a = block_sum((double)sr, sh);
     const double c = block_sum((double)sb, sh);
-    if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = a;
-        partials[2 * blockIdx.x + 1] = c;
-    }
+    finish_norms(a, c, sink, sh);
 }
 
 // ---------------------------------------------------------------------------
@@ -2723,7 +2670,8 @@ bool coarse_persist_supported() {
 
 bool coarse_persist_active(const hierarchy<float> &h) { return persist_start(h, tail_start(h)) > 0; }
 
-template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64, bool zero_start) {
+template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64, bool zero_start,
+                                  bool residual_known) {
     typedef typename vec2_t<T>::type V;
     dim3 blk(32, 8);
     const int ml = h.nl - 1;
@@ -2739,7 +2687,7 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
     if constexpr (sizeof(T) == 8) {
         if (pair_cycle_supported(h)) {
             if (zero_start) cudaMemsetAsync(T0.z, 0, sizeof(V) * (size_t)T0.m * T0.n, st);
-            pair_residual(h, nullptr, reduction_blocks(), st);
+            if (!residual_known) pair_residual(h, nullptr, st);
             pair_cycle(h, st);
             return;
         }
@@ -2844,26 +2792,15 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
     }
 }
 
-template <typename T>
-void top_residual_sqnorm(hierarchy<T> &h, double *partials, int npart, double *out, double *out_b,
-                         cudaStream_t st) {
+template <typename T> void top_residual_sqnorm(hierarchy<T> &h, const norm_sink &sink, cudaStream_t st) {
     level_view<T> &L = h.lv[0];
     if constexpr (sizeof(T) == 8) {
         if (pair_cycle_supported(h)) {
-            pair_residual(h, partials, npart, st);
-            k_final_sum<<<1, 256, 0, st>>>(partials, npart, out, out_b);
-            note_launch();
+            pair_residual(h, &sink, st);
             return;
         }
     }
-    k_top_sqnorm<T><<<npart, kRedThreads, 0, st>>>(h.op, L.z, L.b, L.m, L.n, partials); note_launch();
-    k_final_sum<<<1, 256, 0, st>>>(partials, npart, out, out_b); note_launch();
-}
-
-void mixed_residual(const top_op<double> &op64, const double2 *z64, const double2 *b64, int m, int n, float2 *r32,
-                    double *partials, int npart, double *out, double *out_b, cudaStream_t st) {
-    k_mixed_residual<<<npart, kRedThreads, 0, st>>>(op64, z64, b64, m, n, r32, partials); note_launch();
-    k_final_sum<<<1, 256, 0, st>>>(partials, npart, out, out_b); note_launch();
+    k_top_sqnorm<T><<<sink.npart, kRedThreads, 0, st>>>(h.op, L.z, L.b, L.m, L.n, sink); note_launch();
 }
 
 static ff ff_of(double d) {
@@ -2894,18 +2831,13 @@ void ff_correct_merge(const float2 *hi, const float2 *lo, const float2 *e32, dou
 }
 
 void ff_residual(const top_op<double> &o, const float2 *zhi, const float2 *zlo, const float2 *bhi, const float2 *blo,
-                 int m, int n, float2 *r32, double *partials, int npart, double *out, double *out_b, cudaStream_t st) {
+                 int m, int n, float2 *r32, const norm_sink &sink, cudaStream_t st) {
     ff_op f;
     f.Kmx = ff_of(o.Kmx); f.Kmy = ff_of(o.Kmy); f.mx = ff_of(o.mx); f.my = ff_of(o.my); f.qK = ff_of(o.qK);
     f.bcxx = ff_of(o.bcxx); f.bcyy = ff_of(o.bcyy);
     f.dxx = ff_of(o.cxx + 2 * (o.Kmx + o.my));
     f.dyy = ff_of(o.cyy + 2 * (o.mx + o.Kmy));
-    k_ff_residual<<<npart, kRedThreads, 0, st>>>(f, zhi, zlo, bhi, blo, m, n, r32, partials); note_launch();
-    k_final_sum<<<1, 256, 0, st>>>(partials, npart, out, out_b); note_launch();
-}
-
-void mixed_correct(double2 *z64, const float2 *e32, long count, cudaStream_t st) {
-    k_mixed_correct<<<4 * 152, 256, 0, st>>>(z64, e32, count); note_launch();
+    k_ff_residual<<<sink.npart, kRedThreads, 0, st>>>(f, zhi, zlo, bhi, blo, m, n, r32, sink); note_launch();
 }
 
 void extrapolate_guess2(double2 *z, double2 *prev, double2 *prev2, long count, cudaStream_t st) {
@@ -2926,11 +2858,11 @@ bool top_level_kernel(hierarchy<float> &h, int which, cudaStream_t st) {
     return true;
 }
 
-template void vcycle<double>(hierarchy<double> &, cudaStream_t, int, int, bool);
-template void vcycle<float>(hierarchy<float> &, cudaStream_t, int, int, bool);
+template void vcycle<double>(hierarchy<double> &, cudaStream_t, int, int, bool, bool);
+template void vcycle<float>(hierarchy<float> &, cudaStream_t, int, int, bool, bool);
 template void top_sweep<double>(hierarchy<double> &, cudaStream_t);
 template void top_sweep<float>(hierarchy<float> &, cudaStream_t);
-template void top_residual_sqnorm<double>(hierarchy<double> &, double *, int, double *, double *, cudaStream_t);
-template void top_residual_sqnorm<float>(hierarchy<float> &, double *, int, double *, double *, cudaStream_t);
+template void top_residual_sqnorm<double>(hierarchy<double> &, const norm_sink &, cudaStream_t);
+template void top_residual_sqnorm<float>(hierarchy<float> &, const norm_sink &, cudaStream_t);
 
 }  // namespace stzg

@@ -127,19 +127,39 @@ template <typename T> class hierarchy {
     double *inv_dev_ = nullptr;
 };
 
+// Where a residual kernel leaves [r.r, b.b]: per-block sums, which the last
+// block to arrive adds up in block order (deterministic), and, where the
+// solve loop runs on the device, its stopping rule on them.
+struct loop_rule {
+    int *flags = nullptr;  // F.flags; null: sums only
+    double tol2 = 0;       // go on while r.r > tol2 b.b
+    int cap = 0;           // passes at most; 0: the test before the first pass
+    int has_ran = 0;       // before the first pass: h_ran takes the same decision
+    cudaGraphConditionalHandle h = 0, h_ran = 0;
+};
+struct norm_sink {
+    double *partials;  // 2 npart sums, then the arrival count (zero between launches)
+    int npart;
+    double *out;  // [r.r, b.b]
+    loop_rule rule;
+};
+
 // Kernel-level building blocks (mg.cu).
 // zero_start: the top-level z is taken as zero (the first cycle of a pass);
-// the V-cycle then clears it itself or never reads it.
+// the V-cycle then clears it itself or never reads it.  residual_known: the
+// last launch that touched h's top z, b and r was top_residual_sqnorm, whose r
+// a cycle in correction form (FP64) starts from.
 template <typename T>
-void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64, bool zero_start = false);
+void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64, bool zero_start = false,
+            bool residual_known = false);
 template <typename T> void top_sweep(hierarchy<T> &h, cudaStream_t st);
 // FP64 V-cycles in correction form (mg_small.cu): pair_residual leaves
-// r = b - A z of the top level as float pairs in its r array (and, with
-// partials, the per-block sums of r^2 and b^2 for k_final_sum); pair_cycle
+// r = b - A z of the top level as float pairs in its r array (and, with a
+// sink, its norms); pair_cycle
 // adds one V-cycle on A d = r to z.  Where supported, vcycle<double> is the
 // two of them.
 bool pair_cycle_supported(const hierarchy<double> &h);
-void pair_residual(const hierarchy<double> &h, double *partials, int npart, cudaStream_t st);
+void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream_t st);
 void pair_cycle(const hierarchy<double> &h, cudaStream_t st);
 // Lays out the matrix of the levels from dense_from on (inverse: of the
 // coarsest level); own and caps: the hierarchy's allocations and their sizes.
@@ -160,18 +180,10 @@ bool coarse_persist_supported();
 // Whether a V-cycle of h would use the persistent coarse kernel.
 bool coarse_persist_active(const hierarchy<float> &h);
 
-// Sum of squared residuals of the top level into *out (device), optional
-// sum of squared b into *out_b.  Deterministic: fixed grid, ordered final sum.
+// Residual norms of the top level.
 template <typename T>
-void top_residual_sqnorm(hierarchy<T> &h, double *partials, int npart, double *out, double *out_b,
-                         cudaStream_t st);
+void top_residual_sqnorm(hierarchy<T> &h, const norm_sink &sink, cudaStream_t st);
 
-// Mixed precision: r32 = b64 - A64 z64 (FP64 arithmetic) stored in h32's top
-// b, with squared norms of r and b accumulated like top_residual_sqnorm.
-void mixed_residual(const top_op<double> &op64, const double2 *z64, const double2 *b64, int m, int n,
-                    float2 *r32, double *partials, int npart, double *out, double *out_b, cudaStream_t st);
-// z64 += e32
-void mixed_correct(double2 *z64, const float2 *e32, long count, cudaStream_t st);
 // Float-float iterates (hi + lo pairs of FP32 vectors) of the mixed solve:
 // split FP64 vectors (a, and a2 unless null), merge back, add an FP32
 // correction, and the residual r32 = b - A z in float-float arithmetic with
@@ -186,8 +198,7 @@ void extrap_split(const double2 *v, double2 *prev, const double2 *b, float2 *hi,
 // a = (hi, lo) + e32 as doubles (the last correction and the merge in one pass)
 void ff_correct_merge(const float2 *hi, const float2 *lo, const float2 *e32, double2 *a, long count, cudaStream_t st);
 void ff_residual(const top_op<double> &op64, const float2 *zhi, const float2 *zlo, const float2 *bhi,
-                 const float2 *blo, int m, int n, float2 *r32, double *partials, int npart, double *out,
-                 double *out_b, cudaStream_t st);
+                 const float2 *blo, int m, int n, float2 *r32, const norm_sink &sink, cudaStream_t st);
 // Linear extrapolation of the initial guess: z <- 2 z - prev, prev <- old z.
 void extrapolate_guess(double2 *z, double2 *prev, long count, cudaStream_t st);
 // Quadratic: z <- 3 z - 3 prev + prev2, prev2 <- prev, prev <- old z.

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "mg.cuh"
+#include "step.cuh"
 
 namespace stzg {
 
@@ -41,6 +42,53 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     }
     __syncthreads();
     return t;
+}
+
+// The end of a residual kernel: a and c are the block's sums of r^2 and b^2
+// (valid in thread 0), sh 32 doubles of shared memory.  The sums and the
+// stopping rule used to be two more launches of one block each per pass (2 to
+// 3 us each inside the solve's graph).
+__device__ __forceinline__ void finish_norms(double a, double c, const norm_sink &s, double *sh) {
+    __shared__ int last;
+    unsigned *arrived = reinterpret_cast<unsigned *>(s.partials + 2 * s.npart);
+    if (threadIdx.x == 0) {
+        s.partials[2 * blockIdx.x] = a;
+        s.partials[2 * blockIdx.x + 1] = c;
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    a = c = 0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+        a += __ldcg(s.partials + 2 * k);
+        c += __ldcg(s.partials + 2 * k + 1);
+    }
+    a = block_sum(a, sh);
+    c = block_sum(c, sh);
+    if (threadIdx.x != 0) return;
+    *arrived = 0;
+    s.out[0] = a;
+    s.out[1] = c;
+    const loop_rule &r = s.rule;
+    if (!r.flags) return;
+    const bool conv = c > 0 ? a <= r.tol2 * c : a == 0;
+    const bool nan = isnan(a);
+    int it = 0;
+    if (r.cap == 0) {
+        r.flags[FL_PASSES] = 0;
+        r.flags[FL_LOOP_ERR] = nan ? 2 : 0;
+    } else {
+        it = ++r.flags[FL_PASSES];
+        ++r.flags[FL_PASSES_SUM];
+        if (nan) r.flags[FL_LOOP_ERR] = 2;
+        else if (!conv && it >= r.cap) r.flags[FL_LOOP_ERR] = 1;
+    }
+    if (r.flags[FL_LOOP_ERR] && !r.flags[FL_ERR_FIRST]) r.flags[FL_ERR_FIRST] = r.flags[FL_LOOP_ERR];
+    const unsigned on = !conv && !nan && (r.cap == 0 || it < r.cap) ? 1u : 0u;
+    cudaGraphSetConditional(r.h, on);
+    if (r.has_ran) cudaGraphSetConditional(r.h_ran, on);
 }
 
 }  // namespace stzg

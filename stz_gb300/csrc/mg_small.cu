@@ -59,8 +59,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     small_vcycle<false, false>(P, env);
 }
 
-// r = b - A z of the top level as float pairs; with partials, the sums of r^2
-// and b^2 per block (as k_top_sqnorm).
+// r = b - A z of the top level as float pairs; with a sink, the norms (as
+// k_top_sqnorm).
 // A z is evaluated on second differences of z, exact in 64-bit fixed point
 // (fixed.cuh, one scale per tile), and integer products with the
 // coefficients; only b - A z and the norms are FP64.  The rounding is 0.6
@@ -94,7 +94,7 @@ struct res_sum {
 template <int RPT>
 __global__ void __launch_bounds__(kResThreads, 4)
     k_res_pairs(top_op<double> op, res_consts C, const double2 *__restrict__ z, const double2 *__restrict__ b, int m,
-                int n, int tiles_x, int tiles, float4 *__restrict__ r, double *partials) {
+                int n, int tiles_x, int tiles, float4 *__restrict__ r, norm_sink sink) {
     constexpr int RY = kResRows * RPT, RR = RY + 2;
     __shared__ long long X[RR][RC], Y[RR][RC];
     __shared__ unsigned top[2];
@@ -175,19 +175,16 @@ __global__ void __launch_bounds__(kResThreads, 4)
             ff_split_d(e.x, o.x, o.z);
             ff_split_d(e.y, o.y, o.w);
             r[k] = o;
-            if (partials) {
+            if (sink.partials) {
                 sr += e.x * e.x + e.y * e.y;
                 sb += g[q].x * g[q].x + g[q].y * g[q].y;
             }
         }
         __syncthreads();  // the next tile reuses the planes
     }
-    if (!partials) return;
+    if (!sink.partials) return;
     const double a = block_sum(sr, sh), c = block_sum(sb, sh);
-    if (tid == 0) {
-        partials[2 * blockIdx.x] = a;
-        partials[2 * blockIdx.x + 1] = c;
-    }
+    finish_norms(a, c, sink, sh);
 }
 
 // ---- host ----------------------------------------------------------------------
@@ -419,7 +416,7 @@ bool pair_cycle_supported(const hierarchy<double> &h) {
     return true;
 }
 
-void pair_residual(const hierarchy<double> &h, double *partials, int npart, cudaStream_t st) {
+void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream_t st) {
     const level_view<double> &T0 = h.lv[0];
     const top_op<double> &o = h.op;
     res_consts C;
@@ -444,8 +441,9 @@ void pair_residual(const hierarchy<double> &h, double *partials, int npart, cuda
     C.dyy = factor(excess(o.cyy, o.mx, o.Kmy));
     auto run = [&](auto kernel, int rows) {
         const int tiles_x = ceil_div(T0.m, RX), tiles = tiles_x * ceil_div(T0.n, rows);
-        kernel<<<partials ? npart : std::min(npart, tiles), kResThreads, 0, st>>>(
-            o, C, T0.z, T0.b, T0.m, T0.n, tiles_x, tiles, reinterpret_cast<float4 *>(T0.r), partials);
+        kernel<<<std::min(reduction_blocks(), tiles), kResThreads, 0, st>>>(
+            o, C, T0.z, T0.b, T0.m, T0.n, tiles_x, tiles, reinterpret_cast<float4 *>(T0.r),
+            sink ? *sink : norm_sink{nullptr, 0, nullptr, {}});
     };
     if (ceil_div(T0.m, RX) * ceil_div(T0.n, 2 * kResRows) < 2 * 152) run(k_res_pairs<1>, kResRows);
     else run(k_res_pairs<2>, 2 * kResRows);

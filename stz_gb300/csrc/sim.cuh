@@ -77,7 +77,7 @@ double bdry_pos(const stzg_sim *s, double t);
 int validate(const stz_params *p);
 void drop_graphs(stzg_sim *s);
 int ensure_ops(stzg_sim *s, double dt);
-void launch_norms(stzg_sim *s, bool mixed);
+void launch_norms(stzg_sim *s, bool mixed, const loop_rule &rule = loop_rule());
 // Mixed solve: vel, src -> float-float iterate and right-hand side, and back.
 void mixed_begin(stzg_sim *s);
 void mixed_end(stzg_sim *s);
