@@ -738,6 +738,7 @@ __global__ void k_extrapolate(double2 *__restrict__ z, double2 *__restrict__ pre
 __global__ void k_extrap_split(const double2 *__restrict__ v, double2 *__restrict__ prev,
                                const double2 *__restrict__ b, float2 *__restrict__ hi, float2 *__restrict__ lo,
                                float2 *__restrict__ bhi, float2 *__restrict__ blo, long count) {
+    pdl_wait();
     for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (long)gridDim.x * blockDim.x) {
         const double2 a = v[k], p = prev[k], w = b[k];
         prev[k] = a;
@@ -757,6 +758,7 @@ __global__ void k_extrap_split(const double2 *__restrict__ v, double2 *__restric
 __global__ void k_ff_split(const double2 *__restrict__ a, float2 *__restrict__ hi, float2 *__restrict__ lo,
                            const double2 *__restrict__ a2, float2 *__restrict__ hi2, float2 *__restrict__ lo2,
                            long count) {
+    pdl_wait();
     for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (long)gridDim.x * blockDim.x) {
         float2 h, l;
         const double2 v = a[k];
@@ -784,6 +786,7 @@ __global__ void k_ff_merge(const float2 *__restrict__ hi, const float2 *__restri
 
 __global__ void k_ff_correct(float2 *__restrict__ hi, float2 *__restrict__ lo, const float2 *__restrict__ e,
                              long count) {
+    pdl_wait();
     for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (long)gridDim.x * blockDim.x) {
         const float2 h = hi[k], l = lo[k], d = e[k];
         const ff x = ff_add_f(ff{h.x, l.x}, d.x), y = ff_add_f(ff{h.y, l.y}, d.y);
@@ -796,6 +799,7 @@ __global__ void k_ff_correct(float2 *__restrict__ hi, float2 *__restrict__ lo, c
 // double, without writing the pairs back (the solve ends here).
 __global__ void k_ff_correct_merge(const float2 *__restrict__ hi, const float2 *__restrict__ lo,
                                    const float2 *__restrict__ e, double2 *__restrict__ a, long count) {
+    pdl_wait();
     for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (long)gridDim.x * blockDim.x) {
         const float2 h = hi[k], l = lo[k], d = e[k];
         const ff x = ff_add_f(ff{h.x, l.x}, d.x), y = ff_add_f(ff{h.y, l.y}, d.y);
@@ -815,6 +819,7 @@ struct ff_op {
 __global__ void k_ff_residual(ff_op op, const float2 *__restrict__ zh, const float2 *__restrict__ zl,
                               const float2 *__restrict__ bh, const float2 *__restrict__ bl, int m, int n,
                               float2 *__restrict__ r32, norm_sink sink) {
+    pdl_wait();
     __shared__ double sh[32];
     const unsigned total = (unsigned)m * (unsigned)n;
     float sr = 0.f, sb = 0.f;
@@ -1081,31 +1086,6 @@ __device__ __forceinline__ void prolong_staged(float4 &z, const float2 (*cz)[33]
 __device__ __forceinline__ void madd4(float2 &acc, const float4 &A, float zx, float zy) {
     acc.x = fmaf(A.y, zy, fmaf(A.x, zx, acc.x));
     acc.y = fmaf(A.w, zy, fmaf(A.z, zx, acc.y));
-}
-
-// Programmatic dependent launch within the FP32 V-cycle: each streaming
-// kernel lets the next one be scheduled as soon as it starts
-// (griddepcontrol.launch_dependents) and waits for its predecessor's results
-// (griddepcontrol.wait) only after the set-up that needs none, so launch
-// latency and set-up overlap the previous level's work.  Kernels launched
-// with the attribute all execute the wait before touching data another
-// kernel writes.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
-template <typename... K, typename... A>
-void launch_pdl(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 // Per-warp ring of rows of z and b for the top-level kernels, filled by
@@ -2808,14 +2788,21 @@ static ff ff_of(double d) {
     return ff{hi, (float)(d - (double)hi)};
 }
 
+// Blocks of the one-pass kernels of the pair iterate.
+static int blocks_for(long count) { return std::min(4 * 152, ceil_div(count, 256)); }
+
 void ff_split(const double2 *a, float2 *hi, float2 *lo, const double2 *a2, float2 *hi2, float2 *lo2, long count,
               cudaStream_t st) {
-    k_ff_split<<<4 * 152, 256, 0, st>>>(a, hi, lo, a2, hi2, lo2, count); note_launch();
+    launch_early(count <= kEarlyPoints, k_ff_split, dim3(blocks_for(count)), dim3(256), 0, st,
+                 a, hi, lo, a2, hi2, lo2, count);
+    note_launch();
 }
 
 void extrap_split(const double2 *v, double2 *prev, const double2 *b, float2 *hi, float2 *lo, float2 *bhi,
                   float2 *blo, long count, cudaStream_t st) {
-    k_extrap_split<<<4 * 152, 256, 0, st>>>(v, prev, b, hi, lo, bhi, blo, count); note_launch();
+    launch_early(count <= kEarlyPoints, k_extrap_split, dim3(blocks_for(count)), dim3(256), 0, st,
+                 v, prev, b, hi, lo, bhi, blo, count);
+    note_launch();
 }
 
 void ff_merge(const float2 *hi, const float2 *lo, double2 *a, long count, cudaStream_t st) {
@@ -2823,11 +2810,15 @@ void ff_merge(const float2 *hi, const float2 *lo, double2 *a, long count, cudaSt
 }
 
 void ff_correct(float2 *hi, float2 *lo, const float2 *e32, long count, cudaStream_t st) {
-    k_ff_correct<<<4 * 152, 256, 0, st>>>(hi, lo, e32, count); note_launch();
+    launch_early(count <= kEarlyPoints, k_ff_correct, dim3(blocks_for(count)), dim3(256), 0, st,
+                 hi, lo, e32, count);
+    note_launch();
 }
 
 void ff_correct_merge(const float2 *hi, const float2 *lo, const float2 *e32, double2 *a, long count, cudaStream_t st) {
-    k_ff_correct_merge<<<4 * 152, 256, 0, st>>>(hi, lo, e32, a, count); note_launch();
+    launch_early(count <= kEarlyPoints, k_ff_correct_merge, dim3(blocks_for(count)), dim3(256), 0, st,
+                 hi, lo, e32, a, count);
+    note_launch();
 }
 
 void ff_residual(const top_op<double> &o, const float2 *zhi, const float2 *zlo, const float2 *bhi, const float2 *blo,
@@ -2837,7 +2828,10 @@ void ff_residual(const top_op<double> &o, const float2 *zhi, const float2 *zlo, 
     f.bcxx = ff_of(o.bcxx); f.bcyy = ff_of(o.bcyy);
     f.dxx = ff_of(o.cxx + 2 * (o.Kmx + o.my));
     f.dyy = ff_of(o.cyy + 2 * (o.mx + o.Kmy));
-    k_ff_residual<<<sink.npart, kRedThreads, 0, st>>>(f, zhi, zlo, bhi, blo, m, n, r32, sink); note_launch();
+    launch_early((long)m * n <= kEarlyPoints, k_ff_residual,
+                 dim3(std::min(sink.npart, ceil_div((long)m * n, kRedThreads))), dim3(kRedThreads), 0, st, f, zhi, zlo,
+                 bhi, blo, m, n, r32, sink);
+    note_launch();
 }
 
 void extrapolate_guess2(double2 *z, double2 *prev, double2 *prev2, long count, cudaStream_t st) {

@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kResThreads, 4)
         }
     };
     if (tid < 2) top[tid] = 0;
+    pdl_wait();
     if ((int)blockIdx.x < tiles) load(blockIdx.x);
     __syncthreads();
     int it = 0;
@@ -441,8 +442,9 @@ void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream
     C.dyy = factor(excess(o.cyy, o.mx, o.Kmy));
     auto run = [&](auto kernel, int rows) {
         const int tiles_x = ceil_div(T0.m, RX), tiles = tiles_x * ceil_div(T0.n, rows);
-        kernel<<<std::min(reduction_blocks(), tiles), kResThreads, 0, st>>>(
-            o, C, T0.z, T0.b, T0.m, T0.n, tiles_x, tiles, reinterpret_cast<float4 *>(T0.r),
+        launch_early(
+            (long)T0.m * T0.n <= kEarlyPoints, kernel, dim3(std::min(reduction_blocks(), tiles)), dim3(kResThreads), 0, st, o, C, (const double2 *)T0.z,
+            (const double2 *)T0.b, T0.m, T0.n, tiles_x, tiles, reinterpret_cast<float4 *>(T0.r),
             sink ? *sink : norm_sink{nullptr, 0, nullptr, {}});
     };
     if (ceil_div(T0.m, RX) * ceil_div(T0.n, 2 * kResRows) < 2 * 152) run(k_res_pairs<1>, kResRows);
