@@ -649,8 +649,8 @@ int stzg_create(const stz_params *p, const stzg_options *opt, stzg_sim **out) {
     if (o.extrapolate >= 2)
         if ((st = dev_alloc(s, (void **)&s->vel_prev2, nn * sizeof(double2))) != STZG_OK) return bail(st);
     s->npart = reduction_blocks();
-    if ((st = dev_alloc(s, (void **)&s->partials, (2 * s->npart + 1) * sizeof(double))) != STZG_OK) return bail(st);
-    if (cudaMemsetAsync(s->partials + 2 * s->npart, 0, sizeof(double), s->st) != cudaSuccess)
+    if ((st = dev_alloc(s, (void **)&s->partials, (2 * s->npart + 1) * sizeof(double) + FL_COUNT * sizeof(int))) != STZG_OK) return bail(st);
+    if (cudaMemsetAsync(s->partials + 2 * s->npart, 0, sizeof(double) + FL_COUNT * sizeof(int), s->st) != cudaSuccess)
         return bail(fail(STZG_ECUDA, "memset"));
     if ((st = dev_alloc(s, (void **)&s->dnorm, 2 * sizeof(double))) != STZG_OK) return bail(st);
     if (cudaMallocHost(&s->hnorm, 2 * sizeof(double)) != cudaSuccess) return bail(fail(STZG_ENOMEM, "pinned alloc"));

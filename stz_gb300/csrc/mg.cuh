@@ -135,6 +135,7 @@ struct loop_rule {
     double tol2 = 0;       // go on while r.r > tol2 b.b
     int cap = 0;           // passes at most; 0: the test before the first pass
     int has_ran = 0;       // before the first pass: h_ran takes the same decision
+    int zero_ends = 0;     // b = 0 ends the loop whatever r is
     cudaGraphConditionalHandle h = 0, h_ran = 0;
 };
 struct norm_sink {

@@ -106,7 +106,7 @@ __device__ __forceinline__ void finish_norms(double a, double c, const norm_sink
     s.out[1] = c;
     const loop_rule &r = s.rule;
     if (!r.flags) return;
-    const bool conv = c > 0 ? a <= r.tol2 * c : a == 0;
+    const bool conv = c > 0 ? a <= r.tol2 * c : a == 0 || (c == 0 && r.zero_ends);
     const bool nan = isnan(a);
     int it = 0;
     if (r.cap == 0) {

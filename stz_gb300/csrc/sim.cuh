@@ -27,7 +27,7 @@ struct stzg_sim {
     std::vector<stzg::level_ops> ops;
     stzg::hierarchy<double> h64;
     stzg::hierarchy<float> h32;
-    double *partials = nullptr;  // device, 2 per block
+    double *partials = nullptr;  // device, 2 per block, the arrival count, the adjoint solve's flags
     double *dnorm = nullptr;     // device: [r2, b2]
     double *hnorm = nullptr;     // pinned host copy
     int npart = 0;
