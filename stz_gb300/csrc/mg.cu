@@ -829,10 +829,10 @@ __global__ void k_ff_residual(ff_op op, const float2 *__restrict__ zh, const flo
         const ff bx{b0h.x, b0l.x}, by{b0h.y, b0l.y};
         const float2 ch = zh[k], cl = zl[k];
         const ff cx{ch.x, cl.x}, cy{ch.y, cl.y};
-        ff rx, ry;
+        float2 r;
         if (j == 0 || j == n - 1) {
-            rx = ff_sub(bx, ff_mul(op.bcxx, cx));
-            ry = ff_sub(by, ff_mul(op.bcyy, cy));
+            const ff rx = ff_sub(bx, ff_mul(op.bcxx, cx)), ry = ff_sub(by, ff_mul(op.bcyy, cy));
+            r = make_float2(rx.hi + rx.lo, ry.hi + ry.lo);
         } else {
             const int il = i == 0 ? m - 1 : i - 1, ir = i == m - 1 ? 0 : i + 1;
             const unsigned rd = k - (unsigned)m, ru = k + (unsigned)m;
@@ -854,18 +854,13 @@ __global__ void k_ff_residual(ff_op op, const float2 *__restrict__ zh, const flo
             // (qs_multi.cc:31-55), so A z is evaluated on differences from
             // the centre value, which are small for smooth z: the float-float
             // rounding then scales with them rather than with z itself.
-            const ff axx = ff_add(
-                ff_add(ff_mul(op.Kmx, ff_add(ff_sub(lx, cx), ff_sub(rrx, cx))),
-                       ff_mul(op.my, ff_add(ff_sub(dx, cx), ff_sub(ux, cx)))),
-                ff_add(ff_mul(op.qK, ff_add(ff_sub(dly, dry), ff_sub(ury, uly))), ff_mul(op.dxx, cx)));
-            const ff ayy = ff_add(
-                ff_add(ff_mul(op.mx, ff_add(ff_sub(ly, cy), ff_sub(rry, cy))),
-                       ff_mul(op.Kmy, ff_add(ff_sub(dy, cy), ff_sub(uy, cy)))),
-                ff_add(ff_mul(op.qK, ff_add(ff_sub(dlx, drx), ff_sub(urx, ulx))), ff_mul(op.dyy, cy)));
-            rx = ff_sub(bx, axx);
-            ry = ff_sub(by, ayy);
+            // The sum of the products stays unnormalised: 140 FP32 operations a component
+            // (171 with each product and sum normalised, which bound this kernel).
+            r.x = ff_residual(bx, op.Kmx, ff_diffs(lx, cx, rrx, cx), op.my, ff_diffs(dx, cx, ux, cx), op.qK,
+                              ff_diffs(dly, dry, ury, uly), op.dxx, cx);
+            r.y = ff_residual(by, op.mx, ff_diffs(ly, cy, rry, cy), op.Kmy, ff_diffs(dy, cy, uy, cy), op.qK,
+                              ff_diffs(dlx, drx, urx, ulx), op.dyy, cy);
         }
-        const float2 r = make_float2(rx.hi + rx.lo, ry.hi + ry.lo);
         r32[k] = r;
         sr = fmaf(r.x, r.x, fmaf(r.y, r.y, sr));
         sb = fmaf(b0h.x, b0h.x, fmaf(b0h.y, b0h.y, sb));
