@@ -131,13 +131,14 @@ void launch_norms(stzg_sim *s, bool mixed, const loop_rule &rule) {
     const int M = s->m, N = s->n + 1;
     const norm_sink sink{s->partials, s->npart, s->dnorm, rule};
     if (mixed)
-        ff_residual(s->q.op<double>(), s->zhi, s->zlo, s->bhi, s->blo, M, N, s->h32.lv[0].b, sink, s->st);
+        ff_residual(s->q.op<double>(), s->zhi, s->zlo, s->bhi, s->blo, M, N, s->h32.lv[0].b, sink,
+                    !s->h32.crowded, s->st);
     else
         top_residual_sqnorm(s->h64, sink, s->st);
 }
 
 void mixed_begin(stzg_sim *s) {
-    ff_split(s->F.vel, s->zhi, s->zlo, s->F.src, s->bhi, s->blo, (long)s->m * (s->n + 1), s->st);
+    ff_split(s->F.vel, s->zhi, s->zlo, s->F.src, s->bhi, s->blo, (long)s->m * (s->n + 1), !s->h32.crowded, s->st);
 }
 
 void mixed_end(stzg_sim *s) { ff_merge(s->zhi, s->zlo, s->F.vel, (long)s->m * (s->n + 1), s->st); }
@@ -219,7 +220,7 @@ int run_passes(stzg_sim *s, int k) {
     const int inner = s->g_inner;
     auto pass = [&] {
         for (int c = 0; c < inner; c++) vcycle<float>(s->h32, s->st, 10, 1, c == 0);
-        ff_correct(s->zhi, s->zlo, s->h32.lv[0].z, count, s->st);
+        ff_correct(s->zhi, s->zlo, s->h32.lv[0].z, count, !s->h32.crowded, s->st);
         launch_norms(s, true);
     };
     if (k <= 0) return STZG_OK;
@@ -426,7 +427,7 @@ static int build_loop_graph(stzg_sim *s, bool mixed, int inner, bool fused_extra
     }
     if (mixed) {
         for (int c = 0; c < inner; c++) vcycle<float>(s->h32, s->st, 10, 1, c == 0);
-        ff_correct(s->zhi, s->zlo, s->h32.lv[0].z, count, s->st);
+        ff_correct(s->zhi, s->zlo, s->h32.lv[0].z, count, !s->h32.crowded, s->st);
     } else {
         vcycle<double>(s->h64, s->st, 10, 1, false, true);
     }

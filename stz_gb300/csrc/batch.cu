@@ -133,13 +133,16 @@ int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, 
     s->h64.fuse = tn.fuse;
     s->h32.tail_limit = tn.tail_limit;
     s->h32.fuse = tn.fuse;
-    // Many instances share the chip: their small levels take a quarter of the
-    // cluster a single simulation takes (24 instances of 64^2 to 512^2, graph
-    // time at 16 / 8 / 4 / 2 / 1 blocks: 21.8 / 20.1 / 20.0 / 21.5 / 25.4 ms)
-    s->h64.small_blocks = s->h32.small_blocks = b->sims.size() > 8 ? 4 : 16;
-    // and the top level's long marches, whose halo is smaller (graph time 18.9
-    // ms; 19.9 with the short ones)
-    s->h32.crowded = b->sims.size() > 8;
+    // The instances share the chip.  None of their kernels starts early, whose
+    // waiting blocks would hold slots the others need (24 mixed instances of
+    // 64^2 to 512^2, graph time: 18.9 ms with early launches, 13.6 without; 6
+    // of them: 8.6, 7.8).  Many of them take smaller clusters for their small
+    // levels (16 / 8 / 4 / 2 blocks, 12 instances: 9.1 / 9.5 / 10.3 / 11.4 ms;
+    // 24: 15.4 / 13.8 / 13.6 / 14.9; 32: 12.7 / 11.1 / 10.3 / 11.1) and the top
+    // level's long marches, whose halo is smaller (32: 10.3 ms, short 10.8).
+    const size_t together = b->sims.size();
+    s->h64.crowded = s->h32.crowded = together > 1;
+    s->h64.small_blocks = s->h32.small_blocks = together > 20 ? 4 : (together > 12 ? 8 : 16);
     double *clk = b->dclock + (size_t)k * CLK_COUNT;
     int *ctr = b->dctr + (size_t)k * CTR_COUNT;
     // the captured step kernels read time, wall data and buffer index from the clock
@@ -202,7 +205,7 @@ int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, 
     if (mixed) {
         per_pass = tn.inner;
         for (int c = 0; c < tn.inner; c++) vcycle<float>(s->h32, s->st, 10, 1, c == 0);
-        ff_correct(s->zhi, s->zlo, s->h32.lv[0].z, count, s->st);
+        ff_correct(s->zhi, s->zlo, s->h32.lv[0].z, count, !s->h32.crowded, s->st);
         launch_norms(s, true);
     } else {
         vcycle<double>(s->h64, s->st, 10, 1, false, true);

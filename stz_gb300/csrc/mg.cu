@@ -2401,31 +2401,31 @@ inline int march_rows(int strips, int cn) {
     return 2;
 }
 
-template <typename T> void launch_lev_down_m(level_view<T> &L, level_view<T> &C, cudaStream_t st) {
+template <typename T> void launch_lev_down_m(level_view<T> &L, level_view<T> &C, bool early, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) {
         const int strips = ceil_div(C.m, kLevDownCols);
         const int t = march_rows(strips, C.n);
         const dim3 g(strips, ceil_div(ceil_div(C.n, t), kMarchWarps)), blk(32 * kMarchWarps);
         switch (t) {
-            case 16: launch_pdl(k_lev_down_m<16>, g, blk, 0, st, L, C); break;
-            case 8: launch_pdl(k_lev_down_m<8>, g, blk, 0, st, L, C); break;
-            case 4: launch_pdl(k_lev_down_m<4>, g, blk, 0, st, L, C); break;
-            default: launch_pdl(k_lev_down_m<2>, g, blk, 0, st, L, C);
+            case 16: launch_early(early, k_lev_down_m<16>, g, blk, 0, st, L, C); break;
+            case 8: launch_early(early, k_lev_down_m<8>, g, blk, 0, st, L, C); break;
+            case 4: launch_early(early, k_lev_down_m<4>, g, blk, 0, st, L, C); break;
+            default: launch_early(early, k_lev_down_m<2>, g, blk, 0, st, L, C);
         }
         note_launch();
     }
 }
 
-template <typename T> void launch_lev_up_m(level_view<T> &F, level_view<T> &C, cudaStream_t st) {
+template <typename T> void launch_lev_up_m(level_view<T> &F, level_view<T> &C, bool early, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) {
         const int strips = ceil_div(C.m, kLevUpCols);
         const int t = march_rows(strips, C.n);
         const dim3 g(strips, ceil_div(ceil_div(C.n, t), kMarchWarps)), blk(32 * kMarchWarps);
         switch (t) {
-            case 16: launch_pdl(k_lev_up_m<16>, g, blk, 0, st, F, C); break;
-            case 8: launch_pdl(k_lev_up_m<8>, g, blk, 0, st, F, C); break;
-            case 4: launch_pdl(k_lev_up_m<4>, g, blk, 0, st, F, C); break;
-            default: launch_pdl(k_lev_up_m<2>, g, blk, 0, st, F, C);
+            case 16: launch_early(early, k_lev_up_m<16>, g, blk, 0, st, F, C); break;
+            case 8: launch_early(early, k_lev_up_m<8>, g, blk, 0, st, F, C); break;
+            case 4: launch_early(early, k_lev_up_m<4>, g, blk, 0, st, F, C); break;
+            default: launch_early(early, k_lev_up_m<2>, g, blk, 0, st, F, C);
         }
         note_launch();
     }
@@ -2465,7 +2465,7 @@ template <typename T> void launch_lev_up(level_view<T> &F, level_view<T> &C, cud
 // hide them: V-cycle at 256^2 / 512^2 / 1024^2 with 8 rows 45 / 62 / 84 us, so
 // 36 / 54 / 73 us (2048^2 keeps 8).
 template <typename T> static int top_rows(const hierarchy<T> &h, int strips, int cn) {
-    return h.crowded ? kTopRows : std::min(march_rows(strips, cn), kTopRows);
+    return h.small_blocks < 16 ? kTopRows : std::min(march_rows(strips, cn), kTopRows);
 }
 
 // The streaming top-level kernels (single precision only): the swept z goes
@@ -2476,7 +2476,7 @@ template <typename T> void launch_top_down(hierarchy<T> &h, cudaStream_t st, boo
         const int strips = ceil_div(C.m, kDownCols), t = top_rows(h, strips, C.n);
         const dim3 g(strips, ceil_div(ceil_div(C.n, t), kMarchWarps));
         auto go = [&](auto kernel) {
-            launch_pdl(kernel, g, dim3(32 * kMarchWarps), 0, st, h.op,
+            launch_early(!h.crowded, kernel, g, dim3(32 * kMarchWarps), 0, st, h.op,
                        zero_start ? (const float2 *)nullptr : (const float2 *)T0.z, (const float2 *)T0.b, T0.m, T0.n,
                        T0.r, C.b, C.m, C.n);
         };
@@ -2493,7 +2493,7 @@ template <typename T> void launch_top_up(hierarchy<T> &h, cudaStream_t st) {
         const int strips = ceil_div(C.m, kUpCols), t = top_rows(h, strips, C.n);
         const dim3 g(strips, ceil_div(ceil_div(C.n, t), kMarchWarps));
         auto go = [&](auto kernel) {
-            launch_pdl(kernel, g, dim3(32 * kMarchWarps), 0, st, h.op, (const float2 *)T0.r, (const float2 *)T0.b, T0.m,
+            launch_early(!h.crowded, kernel, g, dim3(32 * kMarchWarps), 0, st, h.op, (const float2 *)T0.r, (const float2 *)T0.b, T0.m,
                        T0.n, (const float2 *)C.z, C.m, C.n, T0.z);
         };
         if (t == 8) go(k_top_up<8>);
@@ -2693,7 +2693,7 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
         level_view<T> &L = h.lv[i];
         level_view<T> &C = h.lv[i + 1];
         if (march_level(h, L)) {
-            launch_lev_down_m(L, C, st);
+            launch_lev_down_m(L, C, !h.crowded, st);
             continue;
         }
         if (tile_level(h, L)) {
@@ -2723,7 +2723,7 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
         if (sizeof(T) == 4 && pair_tail(h, t)) smem = pair_tail_smem(h, t, &tl.inv_off);
         if constexpr (sizeof(T) == 4) {
             if (pair_tail(h, t))
-                launch_pdl(k_tail_pairs, dim3(1), dim3(32, STZG_TAIL_WARPS), smem, st, tl, hv);
+                launch_early(!h.crowded, k_tail_pairs, dim3(1), dim3(32, STZG_TAIL_WARPS), smem, st, tl, hv);
             else
                 k_tail<T><<<1, dim3(32, 32), smem, st>>>(tl, hv);
         } else {
@@ -2746,7 +2746,7 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
     for (int i = up_from; i >= 2; i--) {
         level_view<T> &C = h.lv[i], &F = h.lv[i - 1];
         if (march_level(h, F)) {
-            launch_lev_up_m(F, C, st);
+            launch_lev_up_m(F, C, !h.crowded, st);
             continue;
         }
         if (tile_level(h, F)) {
@@ -2787,8 +2787,8 @@ static ff ff_of(double d) {
 static int blocks_for(long count) { return std::min(4 * 152, ceil_div(count, 256)); }
 
 void ff_split(const double2 *a, float2 *hi, float2 *lo, const double2 *a2, float2 *hi2, float2 *lo2, long count,
-              cudaStream_t st) {
-    launch_early(count <= kEarlyPoints, k_ff_split, dim3(blocks_for(count)), dim3(256), 0, st,
+              bool early, cudaStream_t st) {
+    launch_early(early && count <= kEarlyPoints, k_ff_split, dim3(blocks_for(count)), dim3(256), 0, st,
                  a, hi, lo, a2, hi2, lo2, count);
     note_launch();
 }
@@ -2804,8 +2804,8 @@ void ff_merge(const float2 *hi, const float2 *lo, double2 *a, long count, cudaSt
     k_ff_merge<<<4 * 152, 256, 0, st>>>(hi, lo, a, count); note_launch();
 }
 
-void ff_correct(float2 *hi, float2 *lo, const float2 *e32, long count, cudaStream_t st) {
-    launch_early(count <= kEarlyPoints, k_ff_correct, dim3(blocks_for(count)), dim3(256), 0, st,
+void ff_correct(float2 *hi, float2 *lo, const float2 *e32, long count, bool early, cudaStream_t st) {
+    launch_early(early && count <= kEarlyPoints, k_ff_correct, dim3(blocks_for(count)), dim3(256), 0, st,
                  hi, lo, e32, count);
     note_launch();
 }
@@ -2817,13 +2817,13 @@ void ff_correct_merge(const float2 *hi, const float2 *lo, const float2 *e32, dou
 }
 
 void ff_residual(const top_op<double> &o, const float2 *zhi, const float2 *zlo, const float2 *bhi, const float2 *blo,
-                 int m, int n, float2 *r32, const norm_sink &sink, cudaStream_t st) {
+                 int m, int n, float2 *r32, const norm_sink &sink, bool early, cudaStream_t st) {
     ff_op f;
     f.Kmx = ff_of(o.Kmx); f.Kmy = ff_of(o.Kmy); f.mx = ff_of(o.mx); f.my = ff_of(o.my); f.qK = ff_of(o.qK);
     f.bcxx = ff_of(o.bcxx); f.bcyy = ff_of(o.bcyy);
     f.dxx = ff_of(o.cxx + 2 * (o.Kmx + o.my));
     f.dyy = ff_of(o.cyy + 2 * (o.mx + o.Kmy));
-    launch_early((long)m * n <= kEarlyPoints, k_ff_residual,
+    launch_early(early && (long)m * n <= kEarlyPoints, k_ff_residual,
                  dim3(std::min(sink.npart, ceil_div((long)m * n, kRedThreads))), dim3(kRedThreads), 0, st, f, zhi, zlo,
                  bhi, blo, m, n, r32, sink);
     note_launch();

@@ -95,9 +95,13 @@ template <typename T> class hierarchy {
     // and whether wide single-precision levels use the fused tile kernels
     long tail_limit = -1;
     int fuse = 1;
-    // most blocks of the small-level kernel's cluster (mg_small.cu)
+    // most blocks of the small-level kernel's cluster (mg_small.cu); fewer than
+    // 16 where so many cycles run at the same time that their work counts, not
+    // their latency
     int small_blocks = 16;
-    bool crowded = false;  // many cycles at the same time: work counts, not latency
+    // other cycles run at the same time: no early launches, whose waiting
+    // blocks take the others' slots
+    bool crowded = false;
     // single precision: the coarse levels at most 512 wide and the tail in
     // one cooperative persistent kernel (set by the owner once
     // coarse_persist_supported() holds; bar: two zeroed device words for its
@@ -188,18 +192,19 @@ void top_residual_sqnorm(hierarchy<T> &h, const norm_sink &sink, cudaStream_t st
 // Float-float iterates (hi + lo pairs of FP32 vectors) of the mixed solve:
 // split FP64 vectors (a, and a2 unless null), merge back, add an FP32
 // correction, and the residual r32 = b - A z in float-float arithmetic with
-// squared norms like top_residual_sqnorm.
+// squared norms like top_residual_sqnorm.  early: the launch may overlap the
+// one before it.
 void ff_split(const double2 *a, float2 *hi, float2 *lo, const double2 *a2, float2 *hi2, float2 *lo2, long count,
-              cudaStream_t st);
+              bool early, cudaStream_t st);
 void ff_merge(const float2 *hi, const float2 *lo, double2 *a, long count, cudaStream_t st);
-void ff_correct(float2 *hi, float2 *lo, const float2 *e32, long count, cudaStream_t st);
+void ff_correct(float2 *hi, float2 *lo, const float2 *e32, long count, bool early, cudaStream_t st);
 // prev = v; (hi, lo) = split(2 v - prev_old); (bhi, blo) = split(b)
 void extrap_split(const double2 *v, double2 *prev, const double2 *b, float2 *hi, float2 *lo, float2 *bhi,
                   float2 *blo, long count, cudaStream_t st);
 // a = (hi, lo) + e32 as doubles (the last correction and the merge in one pass)
 void ff_correct_merge(const float2 *hi, const float2 *lo, const float2 *e32, double2 *a, long count, cudaStream_t st);
 void ff_residual(const top_op<double> &op64, const float2 *zhi, const float2 *zlo, const float2 *bhi,
-                 const float2 *blo, int m, int n, float2 *r32, const norm_sink &sink, cudaStream_t st);
+                 const float2 *blo, int m, int n, float2 *r32, const norm_sink &sink, bool early, cudaStream_t st);
 // Linear extrapolation of the initial guess: z <- 2 z - prev, prev <- old z.
 void extrapolate_guess(double2 *z, double2 *prev, long count, cudaStream_t st);
 // Quadratic: z <- 3 z - 3 prev + prev2, prev2 <- prev, prev <- old z.

@@ -74,14 +74,15 @@ struct column_env : block_env {
 
 // Attributes of a launch of `blocks` blocks as one cluster, with programmatic
 // dependent launch; at: room for two.
-inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int blocks, unsigned bytes, cudaStream_t st) {
+inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int blocks, unsigned bytes, cudaStream_t st,
+                           bool early = true) {
     cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(kSmallThreads);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = st;
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].val.programmaticStreamSerializationAllowed = early;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = blocks;
     at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;

@@ -285,10 +285,10 @@ bool choose_small(const hierarchy<T> &h, bool zero_start, small_plan<typename sc
     return false;
 }
 
-template <typename S> void launch_small(const small_plan<S> &P, cudaStream_t st) {
+template <typename S> void launch_small(const small_plan<S> &P, bool early, cudaStream_t st) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[2];
-    cluster_config(cfg, at, P.blocks, P.bytes, st);
+    cluster_config(cfg, at, P.blocks, P.bytes, st, early);
     if (block_phases(P)) cudaLaunchKernelEx(&cfg, k_small<S, true>, P);
     else cudaLaunchKernelEx(&cfg, k_small<S, false>, P);
     note_launch();
@@ -326,7 +326,8 @@ tile_level plan_tile(const hierarchy<double> &h, int l, bool up, bool &bands, si
 }
 
 template <typename... K, typename... A>
-void launch_tile(void (*kern)(K...), const tile_level &L, bool bands, size_t smem, cudaStream_t st, A... args) {
+void launch_tile(void (*kern)(K...), const tile_level &L, bool bands, size_t smem, bool early, cudaStream_t st,
+                 A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(bands ? 1 : ceil_div(L.cm, L.tw), ceil_div(L.cn, L.th));
     cfg.blockDim = dim3(L.threads);
@@ -334,7 +335,7 @@ void launch_tile(void (*kern)(K...), const tile_level &L, bool bands, size_t sme
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].val.programmaticStreamSerializationAllowed = early;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kern, args...);
@@ -443,7 +444,7 @@ void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream
     auto run = [&](auto kernel, int rows) {
         const int tiles_x = ceil_div(T0.m, RX), tiles = tiles_x * ceil_div(T0.n, rows);
         launch_early(
-            (long)T0.m * T0.n <= kEarlyPoints, kernel, dim3(std::min(reduction_blocks(), tiles)), dim3(kResThreads), 0, st, o, C, (const double2 *)T0.z,
+            !h.crowded && (long)T0.m * T0.n <= kEarlyPoints, kernel, dim3(std::min(reduction_blocks(), tiles)), dim3(kResThreads), 0, st, o, C, (const double2 *)T0.z,
             (const double2 *)T0.b, T0.m, T0.n, tiles_x, tiles, reinterpret_cast<float4 *>(T0.r),
             sink ? *sink : norm_sink{nullptr, 0, nullptr, {}});
     };
@@ -460,22 +461,22 @@ void pair_cycle(const hierarchy<double> &h, cudaStream_t st) {
         bool bands;
         size_t bytes;
         const tile_level L = plan_tile(h, l, false, bands, bytes);
-        if (l == 0) launch_tile(k_pair_top_down, L, false, bytes, st, op, L);
-        else if (bands) launch_tile(k_pair_lev_down<true>, L, true, bytes, st, L);
-        else launch_tile(k_pair_lev_down<false>, L, false, bytes, st, L);
+        if (l == 0) launch_tile(k_pair_top_down, L, false, bytes, !h.crowded, st, op, L);
+        else if (bands) launch_tile(k_pair_lev_down<true>, L, true, bytes, !h.crowded, st, L);
+        else launch_tile(k_pair_lev_down<false>, L, false, bytes, !h.crowded, st, L);
     }
     if (P.t == 0) {
         P.lv[0].bg = reinterpret_cast<const float4 *>(h.lv[0].r);
         P.sum = h.lv[0].z;
     }
-    launch_small(P, st);
+    launch_small(P, !h.crowded, st);
     for (int l = P.t - 1; l >= 0; l--) {
         bool bands;
         size_t bytes;
         const tile_level L = plan_tile(h, l, true, bands, bytes);
-        if (l == 0) launch_tile(k_pair_top_up, L, false, bytes, st, op, L);
-        else if (bands) launch_tile(k_pair_lev_up<true>, L, true, bytes, st, L);
-        else launch_tile(k_pair_lev_up<false>, L, false, bytes, st, L);
+        if (l == 0) launch_tile(k_pair_top_up, L, false, bytes, !h.crowded, st, op, L);
+        else if (bands) launch_tile(k_pair_lev_up<true>, L, true, bytes, !h.crowded, st, L);
+        else launch_tile(k_pair_lev_up<false>, L, false, bytes, !h.crowded, st, L);
     }
 }
 
@@ -486,7 +487,7 @@ int small_first(const hierarchy<float> &h) {
 
 void small_levels(const hierarchy<float> &h, bool zero_start, cudaStream_t st) {
     small_plan<float> P;
-    if (choose_small(h, zero_start, P)) launch_small(P, st);
+    if (choose_small(h, zero_start, P)) launch_small(P, !h.crowded, st);
 }
 
 }  // namespace stzg
