@@ -119,7 +119,7 @@ int ensure_ops(stzg_sim *s, double dt) {
     s->ops = build_coarse_ops(s->q, s->m, s->n + 1);
     top_op<double> o = s->q.op<double>();
     STZG_CHECK(s->h64.upload_ops(s->ops, o));
-    if (s->O.precision == STZG_MIXED) STZG_CHECK(s->h32.upload_ops(s->ops, o));
+    if (s->O.precision == STZG_MIXED) STZG_CHECK(s->h32.upload_ops(s->ops, o, &s->h64));
     s->viscdt = viscdt;
     return STZG_OK;
 }

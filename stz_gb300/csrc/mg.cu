@@ -329,7 +329,8 @@ static void split_stencil(const stencil9<double> &s, float4 *out) {
 
 template <typename T> cudaError_t prepare_tail_kernel();
 
-template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> &ops, const top_op<double> &o) {
+template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> &ops, const top_op<double> &o,
+                                                   const hierarchy<double> *same) {
     op.Kmx = (T)o.Kmx; op.Kmy = (T)o.Kmy; op.mx = (T)o.mx; op.my = (T)o.my; op.qK = (T)o.qK;
     op.cxx = (T)o.cxx; op.cyy = (T)o.cyy; op.icxx = (T)o.icxx; op.icyy = (T)o.icyy;
     op.bcxx = (T)o.bcxx; op.bcyy = (T)o.bcyy; op.ibcxx = (T)o.ibcxx; op.ibcyy = (T)o.ibcyy;
@@ -349,21 +350,29 @@ template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> 
         D.ncls = (int)L.cls.size();
         STZG_CUDA(cudaMemcpy((void *)D.st, tab.data(), sizeof(stencil9<T>) * tab.size(), cudaMemcpyHostToDevice));
         STZG_CUDA(cudaMemcpy((void *)D.cls, L.cls.data(), sizeof(int) * L.cls.size(), cudaMemcpyHostToDevice));
-        {
-            std::vector<float4> pairs(20 * L.table.size());
-            for (size_t k = 0; k < L.table.size(); k++) split_stencil(L.table[k], pairs.data() + 20 * k);
-            if (L.table.size() > pair_cap_[l]) {
-                void *p;
-                cudaError_t e = cudaMalloc(&p, sizeof(float4) * pairs.size());
-                if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(stencil pairs)");
-                owned_.push_back(p);
-                bytes_ += sizeof(float4) * pairs.size();
-                st_pairs[l] = (const float4 *)p;
-                pair_cap_[l] = L.table.size();
-            }
-            STZG_CUDA(cudaMemcpy((void *)st_pairs[l], pairs.data(), sizeof(float4) * pairs.size(),
-                                 cudaMemcpyHostToDevice));
+    }
+    if (!same) {
+        // every level's stencils as float pairs, in one copy
+        std::vector<float4> pairs;
+        size_t at[17] = {0};
+        for (int l = 1; l < nl; l++) {
+            at[l] = pairs.size();
+            pairs.resize(at[l] + 20 * ops[l - 1].table.size());
+            for (size_t k = 0; k < ops[l - 1].table.size(); k++)
+                split_stencil(ops[l - 1].table[k], pairs.data() + at[l] + 20 * k);
         }
+        if (pairs.size() > pair_cap_) {
+            void *p;
+            cudaError_t e = cudaMalloc(&p, sizeof(float4) * pairs.size());
+            if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(stencil pairs)");
+            owned_.push_back(p);
+            bytes_ += sizeof(float4) * pairs.size();
+            pairs_dev_ = (float4 *)p;
+            pair_cap_ = pairs.size();
+        }
+        if (!pairs.empty())
+            STZG_CUDA(cudaMemcpy(pairs_dev_, pairs.data(), sizeof(float4) * pairs.size(), cudaMemcpyHostToDevice));
+        for (int l = 1; l < nl; l++) st_pairs[l] = pairs_dev_ + at[l];
     }
     STZG_CUDA(prepare_tail_kernel<T>());
     bottom_inv = nullptr;
@@ -384,7 +393,12 @@ template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> 
             bottom_inv = inv_dev_;
             bottom_unknowns = 2 * ops.back().m * ops.back().n;
         }
-        STZG_CHECK(build_dense(*this, inv, owned_, dense_cap_));
+        if (same) {
+            dense = same->dense;
+            dense_from = same->dense_from;
+        } else {
+            STZG_CHECK(build_dense(*this, inv, owned_, &dense_cap_));
+        }
     }
     return STZG_OK;
 }
@@ -414,13 +428,14 @@ template <typename T> int hierarchy<T>::grow(int l, size_t st_need, size_t cls_n
 
 template <typename T> void hierarchy<T>::release() {
     for (int l = 0; l < 17; l++) {
-        st_cap_[l] = cls_cap_[l] = pair_cap_[l] = dense_cap_[l] = 0;
+        st_cap_[l] = cls_cap_[l] = 0;
         st_pairs[l] = nullptr;
-        dense_buf[l] = nullptr;
     }
     top_pairs = nullptr;
     dense = nullptr;
-    inv_cap_ = 0;
+    dense_buf = nullptr;
+    pairs_dev_ = nullptr;
+    pair_cap_ = dense_cap_ = inv_cap_ = 0;
     inv_dev_ = nullptr;
     bottom_inv = nullptr;
     for (void *p : owned_) cudaFree(p);

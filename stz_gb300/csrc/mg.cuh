@@ -86,7 +86,10 @@ template <typename T> class hierarchy {
     top_op<T> op;
     // allocation: top z/b may be external (FP64 path uses vel/src directly)
     int allocate(int m, int n, V *top_z, V *top_b);
-    int upload_ops(const std::vector<level_ops> &ops, const top_op<double> &op64);
+    // same: an FP64 hierarchy with these operators, whose matrix of the coarse
+    // levels serves this one too (it must outlive it).
+    int upload_ops(const std::vector<level_ops> &ops, const top_op<double> &op64,
+                   const hierarchy<double> *same = nullptr);
     // exact coarsest solve z = A^-1 b in FP64 (nullptr: Gauss-Seidel sweeps)
     const double *bottom_inv = nullptr;
     int bottom_unknowns = 0;
@@ -118,7 +121,7 @@ template <typename T> class hierarchy {
     const float4 *st_pairs[17] = {nullptr};
     const float4 *dense = nullptr;
     int dense_from = 0;
-    float2 *dense_buf[17] = {nullptr};
+    float2 *dense_buf = nullptr;
     float4 *top_pairs = nullptr;
     void release();
     ~hierarchy() { release(); }
@@ -126,7 +129,8 @@ template <typename T> class hierarchy {
   private:
     std::vector<void *> owned_;
     size_t bytes_ = 0;
-    size_t st_cap_[17] = {0}, cls_cap_[17] = {0}, pair_cap_[17] = {0}, dense_cap_[17] = {0}, inv_cap_ = 0;
+    size_t st_cap_[17] = {0}, cls_cap_[17] = {0}, pair_cap_ = 0, dense_cap_ = 0, inv_cap_ = 0;
+    float4 *pairs_dev_ = nullptr;  // every level's st_pairs
     int grow(int l, size_t st_need, size_t cls_need);
     double *inv_dev_ = nullptr;
 };
@@ -169,7 +173,7 @@ void pair_cycle(const hierarchy<double> &h, cudaStream_t st);
 // Lays out the matrix of the levels from dense_from on (inverse: of the
 // coarsest level); own and caps: the hierarchy's allocations and their sizes.
 template <typename T>
-int build_dense(hierarchy<T> &h, const std::vector<double> &inverse, std::vector<void *> &own, size_t *caps);
+int build_dense(hierarchy<T> &h, const std::vector<double> &inverse, std::vector<void *> &own, size_t *cap);
 // FP32: the levels from small_first (-1: none) on in one launch, from and to
 // that level's global b and z.
 int small_first(const hierarchy<float> &h);

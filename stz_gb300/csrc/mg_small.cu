@@ -364,39 +364,45 @@ bool prepare_tiles() {
 // level's is its inverse; a finer one's columns are the V-cycle's results on
 // unit right-hand sides, one block each, with the next matrix at its bottom.
 template <typename T> int build_dense(hierarchy<T> &h, const std::vector<double> &inverse, std::vector<void *> &own,
-                                      size_t *caps) {
+                                      size_t *cap) {
     h.dense = nullptr;
     const int ml = h.nl - 1;
     if (ml < 1 || inverse.empty()) return STZG_OK;
     h.dense_from = dense_level(ml, [&](int l) { return (long)h.lv[l].m * h.lv[l].n; });
     STZG_CUDA(cudaFuncSetAttribute(k_dense_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMax));
+    size_t at[17] = {0}, all = 0;
+    for (int l = ml; l >= h.dense_from; l--) {
+        at[l] = all;
+        all += 4 * (size_t)h.lv[l].m * h.lv[l].n * h.lv[l].m * h.lv[l].n;
+    }
+    if (*cap < all) {
+        void *p = nullptr;
+        cudaError_t e = cudaMalloc(&p, all * sizeof(float2));
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(dense levels)");
+        own.push_back(p);
+        h.dense_buf = (float2 *)p;
+        *cap = all;
+    }
     const float4 *next = nullptr;
     for (int l = ml; l >= h.dense_from; l--) {
         const size_t N = 2 * (size_t)h.lv[l].m * h.lv[l].n, bytes = N * N * sizeof(float2);
-        if (caps[l] < bytes) {
-            void *p = nullptr;
-            cudaError_t e = cudaMalloc(&p, bytes);
-            if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(dense levels)");
-            own.push_back(p);
-            h.dense_buf[l] = (float2 *)p;
-            caps[l] = bytes;
-        }
+        float2 *const M = h.dense_buf + at[l];
         if (l == ml) {
             std::vector<float2> pairs(N * N);
             for (size_t k = 0; k < N * N; k++) {
                 const ff v = pair_of(inverse[k]);
                 pairs[k] = make_float2(v.hi, v.lo);
             }
-            STZG_CUDA(cudaMemcpy(h.dense_buf[l], pairs.data(), bytes, cudaMemcpyHostToDevice));
+            STZG_CUDA(cudaMemcpy(M, pairs.data(), bytes, cudaMemcpyHostToDevice));
         } else {
             small_plan<ff> P;
             plan_levels(h, l, l + 1, P);
             P.dense = next;
             if (!layout_small(P, l, l + 1, 1, kSmallMax)) return STZG_OK;  // the older kernels serve it
-            k_dense_columns<<<(unsigned)N, kSmallThreads, P.bytes>>>(P, h.dense_buf[l]);
+            k_dense_columns<<<(unsigned)N, kSmallThreads, P.bytes>>>(P, M);
             STZG_CUDA(cudaGetLastError());
         }
-        next = reinterpret_cast<const float4 *>(h.dense_buf[l]);
+        next = reinterpret_cast<const float4 *>(M);
     }
     STZG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the handle's streams do not wait for this one
     h.dense = next;
