@@ -64,15 +64,14 @@ typedef struct {
                           2 = quadratic, 3v(n) - 3v(n-1) + v(n-2) */
     int substep_cap;   /* iteration cap of the plastic sub-stepping per cell and step
                           (0: 4194304); reaching it returns STZG_ESUBSTEP */
-    int advection;     /* Mixed-precision handles: STZG_ADV_AUTO (0) or STZG_ADV_SPLIT run the
-                          advection, the projection source and the stress correction in
-                          float-float arithmetic (pairs of floats, ~2^-44 relative) on the
-                          FP64 state, each field updated by one FP64 addition, with the ENO
-                          choices of the FP64 path wherever the two candidates differ by
-                          more than 1e-10 of the field's scale; STZG_ADV_FP64 keeps them
-                          FP64.  FP64
-                          handles always run them in FP64, bit-exact with the per-point
-                          ENO2. */
+    int advection;     /* STZG_ADV_AUTO (0) or STZG_ADV_SPLIT: the advection (and the explicit
+                          step) takes its increments from 64-bit fixed-point copies of the
+                          FP64 fields, with exact differences and ENO choices and one FP64
+                          rounding per updated value; mixed-precision handles also run the
+                          projection source and the stress correction in float-float
+                          arithmetic (pairs of floats, ~2^-44 relative) on the FP64 state.
+                          STZG_ADV_FP64 keeps all of them in FP64, bit-exact with the
+                          per-point ENO2. */
     int reserved[5];
 } stzg_options;
 
@@ -226,9 +225,9 @@ int stzg_time_kernel(stzg_sim *s, double dt, int kernel, int reps, double *ms);
  * columns and its single-block tail in one persistent cooperative kernel
  * with grid barriers between the level phases, where the device allows.
  * Off by default: on GB300 at 2048^2 the FP32 V-cycle takes 0.178 ms with
- * it against 0.145 ms with one launch per level chained by programmatic
- * dependent launch (0.166 ms with the persistent kernel from 128 columns
- * down); on = 0 restores the per-level launches.  on = 2 is a test of the kernel's
+ * it against 0.135 ms with the wide levels as launches chained by
+ * programmatic dependent launch and the small ones in one cluster launch
+ * (0.166 ms with the persistent kernel from 128 columns down); on = 0 restores the per-level launches.  on = 2 is a test of the kernel's
  * bounded grid barrier: as 1, and the barrier's arrival count is set so that
  * the next launch's first barrier never completes; each block gives up after
  * about a second, the step reports STZG_ECUDA and the handle must be

@@ -80,17 +80,6 @@ __device__ __forceinline__ double ff_to_d(float hi, float lo) {
     return __longlong_as_double((long long)H);
 }
 
-// a - b for a = ah + al, b = bh + bl (pairs from ff_split_d), rounded to a
-// float: the difference of the high parts by TwoSum (exact) plus the
-// difference of the low parts, so the result carries the float rounding of
-// a - b itself however close a and b are (~2^-24 relative to |a - b|, plus
-// ~2^-48 of |a| and |b| from the split).
-__device__ __forceinline__ float ff_diff(float ah, float al, float bh, float bl) {
-    const float s = ah - bh, bb = s - ah;
-    const float e = (ah - (s - bb)) + (-bh - bb);
-    return s + (e + (al - bl));
-}
-
 // Leading 24 bits of a double as a float (sign, exponent and truncated
 // significand), on the integer pipe: relative error below 2^-23.
 __device__ __forceinline__ float ff_hi(double d) {

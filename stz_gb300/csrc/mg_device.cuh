@@ -72,10 +72,6 @@ void launch_early(bool early, void (*kern)(K...), dim3 grid, dim3 block, size_t 
     cfg.numAttrs = early ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kern, args...);
 }
-template <typename... K, typename... A>
-void launch_pdl(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
-    launch_early(true, kern, grid, block, smem, st, args...);
-}
 
 // The end of a residual kernel: a and c are the block's sums of r^2 and b^2
 // (valid in thread 0), sh 32 doubles of shared memory.  The sums and the

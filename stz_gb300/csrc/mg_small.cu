@@ -34,9 +34,9 @@ namespace {
 // work of a phase is a few microseconds of one SM at most.  Hence bands with
 // halo rows (a level needs no exchange inside), a thread per 2 x 2 block, and
 // the matrix in place of the levels below 450 nodes.  V-cycle at 64^2 / 128^2 /
-// 512^2, FP32: 47 / - / 79 us with one launch per level, 20 / 29 / 67 us with
+// 512^2, FP32: 47 / - / 79 us with one launch per level, 17 / 23 / 54 us with
 // this kernel; FP64 handles: 201 / 293 / 512 us with one FP64 launch per colour,
-// 35 / 51 / 122 us in pairs.
+// 31 / 43 / 93 us in pairs.
 
 template <typename S, bool FAST>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constant__ small_plan<S> P) {

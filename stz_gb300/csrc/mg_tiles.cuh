@@ -17,7 +17,8 @@ namespace mgw {
 // reads beyond the window's edge is wrong and stays in the halo.
 // Bound by instruction issue (a block product in pairs is about 48 operations
 // per neighbour); with nodes as (x, y) words instead of planes the top level's
-// kernels were bound by shared-memory bank conflicts (41 and 51 us at 1024^2).
+// kernels were bound by shared-memory bank conflicts (41 and 51 us at 1024^2,
+// now 26 and 39 with cold caches).
 // BANDS: whole periodic rows, for odd lines and levels whose stencils differ
 // along a row.
 

@@ -238,7 +238,6 @@ MGW_FN void offdiag(const window<S, WRAP, YP> &V, const float4 *s, int j, int w,
     }
 }
 
-MGW_FN int imax(int a, int b) { return a > b ? a : b; }
 MGW_FN int imin(int a, int b) { return a < b ? a : b; }
 
 // Colours of a sweep: rows of parity cy, columns of parity cx (cx == 2: the

@@ -434,7 +434,9 @@ __device__ __forceinline__ double add_ff(double a, ff inc) { return a + ff_to_d(
 // test (on the leading 24 bits, with a margin) cannot certify as elastic.
 // A block takes 32 x 16 cells, two rows of eight threads after one another: the
 // staged halo is 1.4 times the cells (1.7 at 32 x 8, where converting it was a
-// fifth of the kernel).
+// fifth of the kernel).  At 2048^2: 290 us on FP64 handles (1390 with k_advect),
+// 254 us on mixed ones (456 with float pairs); FP64 pipe 62 % busy (21 FP64
+// instructions a cell, the integers' conversions among them).
 constexpr int FXY = 2 * ATY, FROWS = FXY + 4;
 constexpr unsigned kFxBytes = F_COUNT * FROWS * ACOLS * sizeof(double);
 struct fx_smem {
@@ -829,8 +831,9 @@ __global__ void __launch_bounds__(ATX * ATY) k_direct(step_consts c, direct_cons
 // The explicit step with the arithmetic of k_advect_fx: the nine advected
 // fields (the node velocity among them) in 64-bit fixed point, and with them
 // the exact sums of the net force (the four stresses share one scale), the
-// velocity gradient and the viscous term.  k_direct was bound by its ~160 FP64
-// operations per cell.  Tiles with a value that is not finite and cells near
+// velocity gradient and the viscous term.  k_direct is bound by its ~160 FP64
+// operations per cell (0.70 ms a step at 1024 x 768 with flow everywhere; 0.11
+// this kernel, 0.14 the plastic law in k_direct_rest).  Tiles with a value that is not finite and cells near
 // yield are listed for k_direct_rest.
 struct fxd_smem {
     union {
@@ -1140,8 +1143,8 @@ __global__ void k_source(step_consts c, fields_dev F, double xbc_bv) {
     F.src[(size_t)j * m + i] = f;
 }
 
-// The projection source of the float-float path (k_advect_ff writes no
-// per-cell combinations): net_force (shear_sim.cc:447-453) at the interior
+// The projection source of the float-float path (mixed handles, whose
+// advection writes no per-cell combinations): net_force (shear_sim.cc:447-453) at the interior
 // nodes from the stresses of the four surrounding cells.  A block of 32 x 32
 // nodes (four rows per thread) first forms, for each of the 33 x 33 cells
 // around it, the pairs
