@@ -2074,10 +2074,32 @@ __device__ __forceinline__ void tail_inv_prefetch(const tail_levels &tl, unsigne
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
+// Rows first, first + step .. of the coarse levels' matrix times b (nd nodes),
+// a warp per pair of rows (both rows' loads in flight), into z.
+__device__ __forceinline__ void dense_rows(const float4 *M, const float2 *b, float2 *z, int nd, int first, int step,
+                                           int lane) {
+    for (int r = first; r < 2 * nd; r += 2 * step) {
+        ff share[2];
+        mgw::dense_share<32, 2, float>(M + (size_t)r * nd, (size_t)step * nd, r + step < 2 * nd ? 2 : 1, b, nd, lane,
+                                       share);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const ff v = mgw::warp_pair_sum(share[q]);
+            const int k = r + q * step;
+            if (lane == 0 && k < 2 * nd) {
+                if (k & 1) z[k >> 1].y = v.hi + v.lo;
+                else z[k >> 1].x = v.hi + v.lo;
+            }
+        }
+    }
+}
+
 // The pair tail on one block of 32 x nw threads (lane, warp w): levels t ..
 // ml-1 down, the coarsest solve, back up to t; level t's b is read from and
-// its z written to global memory.  S, offs: the caller's shared views.
-__device__ void tail_pairs_body(const tail_levels &tl, const hierarchy_view<float> &H, unsigned char *tail_raw,
+// its z written to global memory.  S, offs: the caller's shared views;
+// dense(b, z, nd): the product with the matrix of the levels from tl.d on.
+template <typename D>
+__device__ void tail_pairs_body(const D &dense, const tail_levels &tl, const hierarchy_view<float> &H, unsigned char *tail_raw,
                                 level_view<float> *S, unsigned (*offs)[5], int lane, int w, int nw) {
     double *tsh = (double *)tail_raw;
     const int tid = w * 32 + lane, nth = 32 * nw;
@@ -2120,16 +2142,7 @@ __device__ void tail_pairs_body(const tail_levels &tl, const hierarchy_view<floa
     }
     if (tl.dense) {
         const pair_level B = pair_view(tail_raw, offs, tl.d);
-        const int nd = S[tl.d].m * S[tl.d].n;
-        for (int r = w; r < 2 * nd; r += nw) {
-            ff share[1];
-            mgw::dense_share<32, 1, float>(tl.dense + (size_t)r * nd, 0, 1, B.b2, nd, lane, share);
-            const ff v = mgw::warp_pair_sum(share[0]);
-            if (lane == 0) {
-                if (r & 1) B.z2[r >> 1].y = v.hi + v.lo;
-                else B.z2[r >> 1].x = v.hi + v.lo;
-            }
-        }
+        dense(B.b2, B.z2, S[tl.d].m * S[tl.d].n);
         __syncthreads();
     } else if (tl.inv_off >= 0) {
         asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -2181,7 +2194,9 @@ __global__ void __launch_bounds__(1024) k_tail_pairs(tail_levels tl, hierarchy_v
     tail_inv_prefetch(tl, tail_raw, w * 32 + lane, 32 * nw);
     pdl_trigger();
     pdl_wait();
-    tail_pairs_body(tl, H, tail_raw, S, offs, lane, w, nw);
+    tail_pairs_body(
+        [&](const float2 *b, float2 *z, int nd) { dense_rows(tl.dense, b, z, nd, threadIdx.y, blockDim.y, threadIdx.x); },
+        tl, H, tail_raw, S, offs, lane, w, nw);
 }
 
 // ---------------------------------------------------------------------------
@@ -2286,7 +2301,30 @@ __global__ void __launch_bounds__(32 * kPersistWarps, 1)
         }
         if (!grid_barrier(cp, gen, &s_ok)) return;
     }
-    if (blockIdx.x == 0) tail_pairs_body(cp.tl, H, tail_raw, S, offs, lane, w, kPersistWarps);
+    // The product with the matrix of the levels from tl.d on is the whole
+    // grid's: the right-hand side and the result go through that level's global
+    // arrays (V-cycle at 2048^2: 0.18 ms; 0.27 with the product in block 0).
+    if (blockIdx.x == 0) {
+        tail_pairs_body(
+            [&](const float2 *b, float2 *z, int nd) {
+                const level_view<float> &L = H.lv[cp.tl.d];
+                for (int k = tid; k < nd; k += nth) L.b[k] = b[k];
+                if (!grid_barrier(cp, gen, &s_ok)) return;
+                dense_rows(cp.tl.dense, b, L.z, nd, gw, nwarps, lane);
+                if (!grid_barrier(cp, gen, &s_ok)) return;
+                for (int k = tid; k < nd; k += nth) z[k] = __ldcg(L.z + k);
+            },
+            cp.tl, H, tail_raw, S, offs, lane, w, kPersistWarps);
+    } else if (cp.tl.dense) {
+        if (!grid_barrier(cp, gen, &s_ok)) return;
+        const level_view<float> &L = H.lv[cp.tl.d];
+        const int nd = L.m * L.n;
+        float2 *b = reinterpret_cast<float2 *>(tail_raw);
+        for (int k = tid; k < nd; k += nth) b[k] = __ldcg(L.b + k);
+        __syncthreads();
+        dense_rows(cp.tl.dense, b, L.z, nd, gw, nwarps, lane);
+        if (!grid_barrier(cp, gen, &s_ok)) return;
+    }
     if (!grid_barrier(cp, gen, &s_ok)) return;
     // the up marches stage the child's strip per warp where the tail was
     float2 (*czs)[33] = reinterpret_cast<float2 (*)[33]>(tail_raw) + w * (kPersistRows + 3);
