@@ -723,6 +723,7 @@ int stzg_adjoint_forward(stzg_sim *s, double dt, int nsteps, int every, const do
         a->every = every;
     }
     if (!a->h_ready) {
+        a->h.pair_cycles = true;
         STZG_CHECK(a->h.allocate(s->m, s->n + 1, nullptr, nullptr));
         a->h_ready = true;
     }

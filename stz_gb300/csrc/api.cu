@@ -658,6 +658,7 @@ int stzg_create(const stz_params *p, const stzg_options *opt, stzg_sim **out) {
     if (cudaMallocHost(&s->hflags, FL_COUNT * sizeof(int)) != cudaSuccess)
         return bail(fail(STZG_ENOMEM, "pinned alloc"));
     // FP64 hierarchy over vel/src; FP32 hierarchy with its own top arrays
+    s->h64.pair_cycles = o.precision != STZG_MIXED;
     if ((st = s->h64.allocate(s->m, s->n + 1, s->F.vel, s->F.src)) != STZG_OK) return bail(st);
     if (o.precision == STZG_MIXED) {
         if ((st = s->h32.allocate(s->m, s->n + 1, nullptr, nullptr)) != STZG_OK) return bail(st);

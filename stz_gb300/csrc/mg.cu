@@ -301,7 +301,7 @@ template <typename T> int hierarchy<T>::allocate(int m, int n, V *top_z, V *top_
         L.b = p[1];
         L.r = p[2];
     }
-    if (sizeof(T) == 8) {
+    if (pair_cycles) {
         const size_t bytes = sizeof(float4) * (size_t)m * n;
         void *p = nullptr;
         cudaError_t e = cudaMalloc(&p, bytes);
@@ -351,7 +351,7 @@ template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> 
         STZG_CUDA(cudaMemcpy((void *)D.st, tab.data(), sizeof(stencil9<T>) * tab.size(), cudaMemcpyHostToDevice));
         STZG_CUDA(cudaMemcpy((void *)D.cls, L.cls.data(), sizeof(int) * L.cls.size(), cudaMemcpyHostToDevice));
     }
-    if (!same) {
+    if constexpr (sizeof(T) == 8) {
         // every level's stencils as float pairs, in one copy
         std::vector<float4> pairs;
         size_t at[17] = {0};
@@ -393,11 +393,11 @@ template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> 
             bottom_inv = inv_dev_;
             bottom_unknowns = 2 * ops.back().m * ops.back().n;
         }
-        if (same) {
+        if constexpr (sizeof(T) == 8) {
+            STZG_CHECK(build_dense(*this, inv, owned_, &dense_cap_));
+        } else {
             dense = same->dense;
             dense_from = same->dense_from;
-        } else {
-            STZG_CHECK(build_dense(*this, inv, owned_, &dense_cap_));
         }
     }
     return STZG_OK;

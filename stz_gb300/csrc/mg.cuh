@@ -86,8 +86,8 @@ template <typename T> class hierarchy {
     top_op<T> op;
     // allocation: top z/b may be external (FP64 path uses vel/src directly)
     int allocate(int m, int n, V *top_z, V *top_b);
-    // same: an FP64 hierarchy with these operators, whose matrix of the coarse
-    // levels serves this one too (it must outlive it).
+    // same (every FP32 hierarchy): an FP64 hierarchy with these operators, whose
+    // matrix of the coarse levels serves this one too (it must outlive it).
     int upload_ops(const std::vector<level_ops> &ops, const top_op<double> &op64,
                    const hierarchy<double> *same = nullptr);
     // exact coarsest solve z = A^-1 b in FP64 (nullptr: Gauss-Seidel sweeps)
@@ -114,10 +114,17 @@ template <typename T> class hierarchy {
     int persist = 0;
     unsigned *bar = nullptr;
     int *bar_err = nullptr;
+    // FP64 hierarchies whose owner runs V-cycles on them, set before allocate:
+    // the top level's correction is allocated and the cycles run in correction
+    // form (pair_cycle_supported).  Off for the FP64 hierarchy of a
+    // mixed-precision handle, whose solves run FP32 cycles (16 bytes a node,
+    // 67 MB at 2048^2).
+    bool pair_cycles = false;
     // the coarse stencils as float pairs (20 float4 each: per block the high
-    // parts, then the low ones; FP32 hierarchies: from dense_from on), the
-    // V-cycle from level dense_from on as one matrix of float pairs (null: none),
-    // and for FP64 hierarchies the top level's correction
+    // parts, then the low ones; none in an FP32 hierarchy), the V-cycle from
+    // level dense_from on as one matrix of float pairs (null: none; an FP32
+    // hierarchy borrows its FP64 sibling's), and the top level's correction
+    // (pair_cycles)
     const float4 *st_pairs[17] = {nullptr};
     const float4 *dense = nullptr;
     int dense_from = 0;
@@ -172,8 +179,7 @@ void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream
 void pair_cycle(const hierarchy<double> &h, cudaStream_t st);
 // Lays out the matrix of the levels from dense_from on (inverse: of the
 // coarsest level); own and caps: the hierarchy's allocations and their sizes.
-template <typename T>
-int build_dense(hierarchy<T> &h, const std::vector<double> &inverse, std::vector<void *> &own, size_t *cap);
+int build_dense(hierarchy<double> &h, const std::vector<double> &inverse, std::vector<void *> &own, size_t *cap);
 // FP32: the levels from small_first (-1: none) on in one launch, from and to
 // that level's global b and z.
 int small_first(const hierarchy<float> &h);

@@ -363,8 +363,7 @@ bool prepare_tiles() {
 // The matrices of the V-cycle from each level ml, ml-1 .. d on: the coarsest
 // level's is its inverse; a finer one's columns are the V-cycle's results on
 // unit right-hand sides, one block each, with the next matrix at its bottom.
-template <typename T> int build_dense(hierarchy<T> &h, const std::vector<double> &inverse, std::vector<void *> &own,
-                                      size_t *cap) {
+int build_dense(hierarchy<double> &h, const std::vector<double> &inverse, std::vector<void *> &own, size_t *cap) {
     h.dense = nullptr;
     const int ml = h.nl - 1;
     if (ml < 1 || inverse.empty()) return STZG_OK;
@@ -408,8 +407,6 @@ template <typename T> int build_dense(hierarchy<T> &h, const std::vector<double>
     h.dense = next;
     return STZG_OK;
 }
-template int build_dense<float>(hierarchy<float> &, const std::vector<double> &, std::vector<void *> &, size_t *);
-template int build_dense<double>(hierarchy<double> &, const std::vector<double> &, std::vector<void *> &, size_t *);
 
 bool pair_cycle_supported(const hierarchy<double> &h) {
     if (!h.fuse || h.tail_limit >= 0 || h.nl < 2 || !h.dense || !h.top_pairs || !prepare_tiles()) return false;
