@@ -40,6 +40,15 @@ __device__ __forceinline__ void ff_split_d(double d, float &hi, float &lo) {
     }
 }
 
+// d 2^k on the integer pipe; 0 where d or the result is below the normal range,
+// infinity and NaN as they are.  The result must stay below 2^1024.
+__device__ __forceinline__ double shift_exponent(double d, int k) {
+    const int hi = __double2hiint(d), e = (hi >> 20) & 0x7ff;
+    if (e == 0x7ff) return d;
+    if (e == 0 || e + k <= 0) return 0.0;
+    return __hiloint2double(hi + (k << 20), __double2loint(d));
+}
+
 // float -> double bits on the integer pipe (exact for normal floats; zero
 // and subnormal floats give a signed zero, infinity and NaN keep their class
 // and payload).

@@ -309,14 +309,22 @@ template <typename T> int hierarchy<T>::allocate(int m, int n, V *top_z, V *top_
         owned_.push_back(p);
         bytes_ += bytes;
         top_pairs = (float4 *)p;
+        e = cudaMalloc(&p, 3 * sizeof(unsigned));
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(residual scale)");
+        owned_.push_back(p);
+        cudaMemset(p, 0, 3 * sizeof(unsigned));
+        peak = (unsigned *)p;
     }
     return STZG_OK;
 }
 
-// A stencil as float pairs: per block the high parts, then the low ones.
-static void split_stencil(const stencil9<double> &s, float4 *out) {
+// The stencil of A 2^-unit as float pairs: per block the high parts, then the
+// low ones (the last block is the inverse of the centre).
+static void split_stencil(const stencil9<double> &s, int unit, float4 *out) {
     for (int e = 0; e < 10; e++) {
-        const double v[4] = {s.e[e].a, s.e[e].b, s.e[e].c, s.e[e].d};
+        const int k = e < 9 ? -unit : unit;
+        const double v[4] = {std::ldexp(s.e[e].a, k), std::ldexp(s.e[e].b, k), std::ldexp(s.e[e].c, k),
+                             std::ldexp(s.e[e].d, k)};
         float h[4], l[4];
         for (int q = 0; q < 4; q++) {
             h[q] = (float)v[q];
@@ -335,6 +343,8 @@ template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> 
     op.cxx = (T)o.cxx; op.cyy = (T)o.cyy; op.icxx = (T)o.icxx; op.icyy = (T)o.icyy;
     op.bcxx = (T)o.bcxx; op.bcyy = (T)o.bcyy; op.ibcxx = (T)o.ibcxx; op.ibcyy = (T)o.ibcyy;
     if ((int)ops.size() != nl - 1) return fail(STZG_EINVAL, "hierarchy/operator level mismatch");
+    unit = 0;
+    if (pair_cycles) std::frexp(std::max(std::fabs(o.cxx), std::fabs(o.cyy)), &unit);
     for (int l = 1; l < nl; l++) {
         const level_ops &L = ops[l - 1];
         level_view<T> &D = lv[l];
@@ -359,7 +369,7 @@ template <typename T> int hierarchy<T>::upload_ops(const std::vector<level_ops> 
             at[l] = pairs.size();
             pairs.resize(at[l] + 20 * ops[l - 1].table.size());
             for (size_t k = 0; k < ops[l - 1].table.size(); k++)
-                split_stencil(ops[l - 1].table[k], pairs.data() + at[l] + 20 * k);
+                split_stencil(ops[l - 1].table[k], unit, pairs.data() + at[l] + 20 * k);
         }
         if (pairs.size() > pair_cap_) {
             void *p;
@@ -432,6 +442,7 @@ template <typename T> void hierarchy<T>::release() {
         st_pairs[l] = nullptr;
     }
     top_pairs = nullptr;
+    peak = nullptr;
     dense = nullptr;
     dense_buf = nullptr;
     pairs_dev_ = nullptr;

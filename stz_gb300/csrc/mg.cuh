@@ -130,6 +130,14 @@ template <typename T> class hierarchy {
     int dense_from = 0;
     float2 *dense_buf = nullptr;
     float4 *top_pairs = nullptr;
+    // Float pairs have FP32's exponents, the problems FP64's: with pair_cycles
+    // the tables are those of A 2^-unit (its largest coefficient between 1/2 and
+    // 1), and a cycle takes the residual times the power of two that brings its
+    // largest value to [1, 2).  peak: the high word of that value's magnitude as
+    // the last residual kernel left it, its running maximum and its blocks'
+    // arrival count (both zero between launches).
+    int unit = 0;
+    unsigned *peak = nullptr;
     void release();
     ~hierarchy() { release(); }
     size_t device_bytes() const { return bytes_; }
@@ -170,10 +178,9 @@ void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64
             bool residual_known = false);
 template <typename T> void top_sweep(hierarchy<T> &h, cudaStream_t st);
 // FP64 V-cycles in correction form (mg_small.cu): pair_residual leaves
-// r = b - A z of the top level as float pairs in its r array (and, with a
-// sink, its norms); pair_cycle
-// adds one V-cycle on A d = r to z.  Where supported, vcycle<double> is the
-// two of them.
+// r = b - A z of the top level in its r array, its largest magnitude in peak
+// (and, with a sink, its norms); pair_cycle adds one V-cycle on A d = r, in
+// float pairs, to z.  Where supported, vcycle<double> is the two of them.
 bool pair_cycle_supported(const hierarchy<double> &h);
 void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream_t st);
 void pair_cycle(const hierarchy<double> &h, cudaStream_t st);

@@ -6,7 +6,9 @@
 // of the FP64 iterate in FP64, one V-cycle from zero on A d = r in float
 // pairs (~48 significant bits), z += d in FP64.  That is the reference's
 // V-cycle (the cycle is linear in z and b) with the rounding of d at 2^-48
-// of d itself, so the iterate keeps FP64 accuracy.  What bounds the cycle on
+// of d itself, so the iterate keeps FP64 accuracy.  Powers of two on r and on
+// the operator's tables (pair_scale, hierarchy::unit), exact both ways, keep
+// the pairs inside FP32's exponents whatever the problem's magnitude.  What bounds the cycle on
 // GB300 is the FP64 pipe, two results per clock and SM: a pair operation
 // costs 10 to 20 issue slots on the FP32 pipe where an FP64 one blocks its
 // quarter of the SM for 64 clocks.
@@ -59,8 +61,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     small_vcycle<false, false>(P, env);
 }
 
-// r = b - A z of the top level as float pairs; with a sink, the norms (as
-// k_top_sqnorm).
+// r = b - A z of the top level and its largest magnitude (hierarchy::peak);
+// with a sink, the norms (as k_top_sqnorm).
 // A z is evaluated on second differences of z, exact in 64-bit fixed point
 // (fixed.cuh, one scale per tile), and integer products with the
 // coefficients; only b - A z and the norms are FP64.  The rounding is 0.6
@@ -94,14 +96,15 @@ struct res_sum {
 template <int RPT>
 __global__ void __launch_bounds__(kResThreads, 4)
     k_res_pairs(top_op<double> op, res_consts C, const double2 *__restrict__ z, const double2 *__restrict__ b, int m,
-                int n, int tiles_x, int tiles, float4 *__restrict__ r, norm_sink sink) {
+                int n, int tiles_x, int tiles, double2 *__restrict__ r, unsigned *peak, norm_sink sink) {
     constexpr int RY = kResRows * RPT, RR = RY + 2;
     __shared__ long long X[RR][RC], Y[RR][RC];
-    __shared__ unsigned top[2];
+    __shared__ unsigned top[2], rtop;
     __shared__ double sh[32];
     constexpr int kPer = (RR * RC + kResThreads - 1) / kResThreads;
     const int tid = threadIdx.x, tx = tid & (RX - 1), ty = tid / RX;
     double sr = 0, sb = 0;
+    unsigned rw = 0;
     double2 v[kPer];
     auto load = [&](int tile) {
         const int i0 = (tile % tiles_x) * RX, j0 = (tile / tiles_x) * RY;
@@ -117,6 +120,7 @@ __global__ void __launch_bounds__(kResThreads, 4)
         }
     };
     if (tid < 2) top[tid] = 0;
+    if (tid == 0) rtop = 0;
     pdl_wait();
     if ((int)blockIdx.x < tiles) load(blockIdx.x);
     __syncthreads();
@@ -172,10 +176,8 @@ __global__ void __launch_bounds__(kResThreads, 4)
                 ay.add(C.dyy, y0);
                 e = make_double2(fma(-unit, ax.value(), g[q].x), fma(-unit, ay.value(), g[q].y));
             }
-            float4 o;
-            ff_split_d(e.x, o.x, o.z);
-            ff_split_d(e.y, o.y, o.w);
-            r[k] = o;
+            r[k] = e;
+            rw = max(rw, max((unsigned)__double2hiint(e.x) & 0x7fffffffu, (unsigned)__double2hiint(e.y) & 0x7fffffffu));
             if (sink.partials) {
                 sr += e.x * e.x + e.y * e.y;
                 sb += g[q].x * g[q].x + g[q].y * g[q].y;
@@ -183,9 +185,21 @@ __global__ void __launch_bounds__(kResThreads, 4)
         }
         __syncthreads();  // the next tile reuses the planes
     }
-    if (!sink.partials) return;
+    rw = __reduce_max_sync(0xffffffffu, rw);
+    if (tx == 0) atomicMax(&rtop, rw);
+    __syncthreads();
+    if (tid == 0) atomicMax(peak + 1, rtop);
+    if (!sink.partials) {
+        if (tid != 0) return;
+        __threadfence();
+        if (atomicAdd(peak + 2, 1u) != gridDim.x - 1) return;
+        __threadfence();
+        peak[2] = 0;
+        peak[0] = atomicExch(peak + 1, 0u);
+        return;
+    }
     const double a = block_sum(sr, sh), c = block_sum(sb, sh);
-    finish_norms(a, c, sink, sh);
+    finish_norms(a, c, sink, sh, peak);
 }
 
 // ---- host ----------------------------------------------------------------------
@@ -197,14 +211,16 @@ ff pair_of(double d) {
     return r;
 }
 
-top_consts<ff> consts_of(const top_op<double> &o) {
+top_consts<ff> consts_of(const top_op<double> &o, int unit) {
+    auto coef = [&](double d) { return pair_of(std::ldexp(d, -unit)); };
+    auto inverse = [&](double d) { return pair_of(std::ldexp(d, unit)); };
     top_consts<ff> c;
-    c.Kmx = pair_of(o.Kmx); c.Kmy = pair_of(o.Kmy); c.mx = pair_of(o.mx); c.my = pair_of(o.my); c.qK = pair_of(o.qK);
-    c.cxx = pair_of(o.cxx); c.cyy = pair_of(o.cyy); c.icxx = pair_of(o.icxx); c.icyy = pair_of(o.icyy);
-    c.bcxx = pair_of(o.bcxx); c.bcyy = pair_of(o.bcyy); c.ibcxx = pair_of(o.ibcxx); c.ibcyy = pair_of(o.ibcyy);
+    c.Kmx = coef(o.Kmx); c.Kmy = coef(o.Kmy); c.mx = coef(o.mx); c.my = coef(o.my); c.qK = coef(o.qK);
+    c.cxx = coef(o.cxx); c.cyy = coef(o.cyy); c.icxx = inverse(o.icxx); c.icyy = inverse(o.icyy);
+    c.bcxx = coef(o.bcxx); c.bcyy = coef(o.bcyy); c.ibcxx = inverse(o.ibcxx); c.ibcyy = inverse(o.ibcyy);
     return c;
 }
-top_consts<float> consts_of(const top_op<float> &o) {
+top_consts<float> consts_of(const top_op<float> &o, int) {
     return top_consts<float>{o.Kmx, o.Kmy, o.mx, o.my, o.qK, o.cxx, o.cyy, o.icxx, o.icyy, o.bcxx, o.bcyy, o.ibcxx, o.ibcyy};
 }
 
@@ -257,7 +273,8 @@ bool plan_small(const hierarchy<T> &h, int t, int blocks, bool zero_start, small
     P.top = t == 0;
     P.zero_start = zero_start;
     P.dense = h.dense;
-    P.op = consts_of(h.op);
+    P.op = consts_of(h.op, h.unit);
+    P.unit = h.unit;
     P.lv[t].zg = reinterpret_cast<node *>(h.lv[t].z);
     P.lv[t].bg = reinterpret_cast<const node *>(h.lv[t].b);
     return layout_small(P, t, h.dense_from, blocks, kSmallMax);
@@ -310,12 +327,17 @@ tile_level plan_tile(const hierarchy<double> &h, int l, bool up, bool &bands, si
     L.cls = A.cls;
     L.st = l ? h.st_pairs[l] : nullptr;
     L.staged = l && A.homog && A.nst * 320 <= 16384;
-    L.b = reinterpret_cast<const float4 *>(l ? A.b : A.r);
+    L.b = reinterpret_cast<const float4 *>(A.b);
     L.zdown = l ? reinterpret_cast<float4 *>(A.r) : h.top_pairs;
     L.zup = reinterpret_cast<float4 *>(A.z);
     L.bc = reinterpret_cast<float4 *>(C.b);
     L.zc = reinterpret_cast<const float4 *>(C.z);
-    if (!l) L.sum = h.lv[0].z;
+    if (!l) {
+        L.res = A.r;
+        L.peak = h.peak;
+        L.unit = h.unit;
+        L.sum = A.z;
+    }
     bands = l && ((A.m & 1) || !A.homog);
     const tile_shape T = shape_tile(L.m, L.cm, L.cn, L.staged ? A.nst * 320 : 0, l ? 0 : (up ? 2 : 1), bands, kTileMax);
     L.tw = T.tw;
@@ -389,7 +411,7 @@ int build_dense(hierarchy<double> &h, const std::vector<double> &inverse, std::v
         if (l == ml) {
             std::vector<float2> pairs(N * N);
             for (size_t k = 0; k < N * N; k++) {
-                const ff v = pair_of(inverse[k]);
+                const ff v = pair_of(std::ldexp(inverse[k], h.unit));
                 pairs[k] = make_float2(v.hi, v.lo);
             }
             STZG_CUDA(cudaMemcpy(M, pairs.data(), bytes, cudaMemcpyHostToDevice));
@@ -448,7 +470,7 @@ void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream
         const int tiles_x = ceil_div(T0.m, RX), tiles = tiles_x * ceil_div(T0.n, rows);
         launch_early(
             !h.crowded && (long)T0.m * T0.n <= kEarlyPoints, kernel, dim3(std::min(reduction_blocks(), tiles)), dim3(kResThreads), 0, st, o, C, (const double2 *)T0.z,
-            (const double2 *)T0.b, T0.m, T0.n, tiles_x, tiles, reinterpret_cast<float4 *>(T0.r),
+            (const double2 *)T0.b, T0.m, T0.n, tiles_x, tiles, T0.r, h.peak,
             sink ? *sink : norm_sink{nullptr, 0, nullptr, {}});
     };
     if (ceil_div(T0.m, RX) * ceil_div(T0.n, 2 * kResRows) < 2 * 152) run(k_res_pairs<1>, kResRows);
@@ -459,7 +481,7 @@ void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream
 void pair_cycle(const hierarchy<double> &h, cudaStream_t st) {
     small_plan<ff> P;
     if (!choose_small(h, true, P)) return;
-    const top_consts<ff> op = consts_of(h.op);
+    const top_consts<ff> op = consts_of(h.op, h.unit);
     for (int l = 0; l < P.t; l++) {
         bool bands;
         size_t bytes;
@@ -471,6 +493,7 @@ void pair_cycle(const hierarchy<double> &h, cudaStream_t st) {
     if (P.t == 0) {
         P.lv[0].bg = reinterpret_cast<const float4 *>(h.lv[0].r);
         P.sum = h.lv[0].z;
+        P.peak = h.peak;
     }
     launch_small(P, !h.crowded, st);
     for (int l = P.t - 1; l >= 0; l--) {

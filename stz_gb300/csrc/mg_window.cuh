@@ -773,7 +773,10 @@ template <typename S> struct small_plan {
     unsigned ro;             // residual rows of the level in hand
     unsigned bytes;
     const float4 *dense;     // row-major, per column node (x.hi, x.lo, y.hi, y.lo)
-    double2 *sum;            // not null: the top level's result is added to this iterate
+    double2 *sum;            // not null: level t is the top one, its b the FP64 residual
+                             // (magnitude: peak), and its result is added to this iterate
+    const unsigned *peak;
+    int unit;                // the tables are those of A 2^-unit
     top_consts<S> op;
     small_level<S> lv[kMaxLevels];
 };
@@ -868,7 +871,7 @@ constexpr int kDenseRows = 3;  // 34 rows per block of sixteen warps at 17 x 16 
 // one's), par(f) (f(thread, threads) on every thread, then a block barrier),
 // csync() (a barrier of all blocks), kLanes and lane_sum(v) (threads of a
 // product row and the sum over them), ld(p) (a global load), store(P, k, v)
-// (the result of level t at its node k), wait_input() (before the first read
+// (the result of level t at its node k), wait_input(P) (before the first read
 // of what an earlier kernel wrote).
 template <bool FAST, bool YP, typename S, typename E> MGW_FN void small_vcycle(const small_plan<S> &P, E &env) {
     typedef typename num<S>::node node;
@@ -890,7 +893,7 @@ template <bool FAST, bool YP, typename S, typename E> MGW_FN void small_vcycle(c
                 for (int k = tid; k < L.ncls; k += nth) d[k] = L.cls[k];
             }
         }
-        env.wait_input();
+        env.wait_input(P);
         const small_level<S> &L = P.lv[P.t];
         const window<S, true, YP> V = band_window<FAST, YP>(P, P.t, me, base);
         const int y1 = band_row(P, P.t, me + 1);
