@@ -520,7 +520,7 @@ struct stzg_adjoint {
     // the solve: residual, then two V-cycles of h and the residual until the
     // tolerance is met; captured per backward call
     cudaGraphExec_t g_vc = nullptr;
-    long n_vc = 0;  // kernels of one pass
+    long n_vc = 0, n_begin = 0;  // kernels of one pass, and before the first one
     void drop_graph() {
         if (g_vc) cudaGraphExecDestroy(g_vc);
         g_vc = nullptr;
@@ -622,6 +622,7 @@ int capture_solve(stzg_sim *s, stzg_adjoint *a) {
         if (e != cudaSuccess) return e;
         e = cudaStreamBeginCaptureToGraph(s->st, root, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
+        pair_begin(a->h, s->st);
         top_residual_sqnorm(a->h, sink, s->st);
         c1 = launch_count();
         cudaStreamCaptureStatus cs;
@@ -654,6 +655,7 @@ int capture_solve(stzg_sim *s, stzg_adjoint *a) {
     };
     const cudaError_t e = build();
     a->n_vc = launch_count() - c1;
+    a->n_begin = c1 - c0;
     discount_launches(launch_count() - c0);  // graph nodes, counted when they execute
     cudaGraphDestroy(root);
     if (e != cudaSuccess) {
@@ -672,7 +674,7 @@ int adjoint_solve(stzg_sim *s, stzg_adjoint *a) {
     STZG_CUDA(cudaMemcpyAsync(s->hflags, solve_flags(s), FL_COUNT * sizeof(int), cudaMemcpyDeviceToHost, s->st));
     STZG_CUDA(cudaMemcpyAsync(s->hnorm, s->dnorm, 16, cudaMemcpyDeviceToHost, s->st));
     STZG_CUDA(cudaStreamSynchronize(s->st));
-    for (long k = 0; k < 1 + s->hflags[FL_PASSES] * a->n_vc; k++) note_launch();
+    for (long k = 0; k < a->n_begin + s->hflags[FL_PASSES] * a->n_vc; k++) note_launch();
     const double r2 = s->hnorm[0], b2 = s->hnorm[1];
     if (std::isnan(r2) || std::isnan(b2)) return fail(STZG_ENAN, "NaN in the adjoint solve");
     if (b2 == 0) {

@@ -184,6 +184,7 @@ int run_vcycles(stzg_sim *s, int k) {
 // tgmg::solve(4, tgmg_predict&) (tgmg.in.cc:266-301) in FP64.
 int solve_fp64(stzg_sim *s, int *ncyc) {
     int nc = s->lim / s->mult;
+    pair_begin(s->h64, s->st);
     STZG_CHECK(run_vcycles(s, nc));
     double err;
     bool ok;
@@ -343,6 +344,7 @@ static int build_loop_graph(stzg_sim *s, bool mixed, int inner, bool fused_extra
     rule.has_ran = mixed && mixed_extra == 0 ? 1 : 0;
     rule.h = h;
     rule.h_ran = h_ran;
+    if (!mixed) pair_begin(s->h64, s->st);
     launch_norms(s, mixed, rule);
     {
         cudaStreamCaptureStatus cs;
@@ -1279,6 +1281,7 @@ int stzg_mg_vcycle(stzg_sim *s, double dt, const double *src, double *vel) {
     const size_t nn = (size_t)s->m * (s->n + 1);
     STZG_CUDA(cudaMemcpyAsync(s->F.src, src, nn * sizeof(double2), cudaMemcpyHostToDevice, s->st));
     STZG_CUDA(cudaMemcpyAsync(s->F.vel, vel, nn * sizeof(double2), cudaMemcpyHostToDevice, s->st));
+    pair_begin(s->h64, s->st);
     STZG_CHECK(run_vcycles(s, 1));
     STZG_CUDA(cudaMemcpyAsync(vel, s->F.vel, nn * sizeof(double2), cudaMemcpyDeviceToHost, s->st));
     STZG_CUDA(cudaStreamSynchronize(s->st));

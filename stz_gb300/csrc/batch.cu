@@ -174,6 +174,7 @@ int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, 
     projection_source(sc, s->F, 0, dt, 0.0, s->st);
     if (s->O.extrapolate) extrapolate_guess(s->F.vel, s->vel_prev, count, s->st);
     if (mixed) mixed_begin(s);
+    else pair_begin(s->h64, s->st);
     launch_norms(s, mixed);
     k_solve_reset<<<1, 32, 0, s->st>>>(ctr, hsolve);
     note_launch();

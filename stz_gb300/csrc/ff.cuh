@@ -40,13 +40,20 @@ __device__ __forceinline__ void ff_split_d(double d, float &hi, float &lo) {
     }
 }
 
-// d 2^k on the integer pipe; 0 where d or the result is below the normal range,
-// infinity and NaN as they are.  The result must stay below 2^1024.
-__device__ __forceinline__ double shift_exponent(double d, int k) {
-    const int hi = __double2hiint(d), e = (hi >> 20) & 0x7ff;
-    if (e == 0x7ff) return d;
-    if (e == 0 || e + k <= 0) return 0.0;
-    return __hiloint2double(hi + (k << 20), __double2loint(d));
+// d 2^k as a pair in the same way (d's own subnormal numbers count as 0).
+__device__ __forceinline__ void ff_split_shifted(double d, int k, float &hi, float &lo) {
+    const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d), sign = dh & 0x80000000u;
+    // exponent field of the float above the high word's 20 bits of significand
+    const unsigned at = (dh ^ sign) + ((unsigned)(k - 1023 + 127) << 20);
+    if (at - (1u << 20) < (254u << 20) && (dh & 0x7ff00000u) != 0) {
+        hi = __uint_as_float(__funnelshift_l(dl, at, 3) | sign);
+        lo = __uint2float_rn(dl & 0x1fffffffu) * __uint_as_float((unsigned)max((int)(at >> 20) - 52, 0) << 23 | sign);
+        return;
+    }
+    const int e = (dh >> 20) & 0x7ff, ef = e + k - 1023 + 127;
+    const bool nan = e == 0x7ff && ((dh & 0xfffffu) | dl);
+    hi = __uint_as_float(ef < 255 || e == 0 ? sign : (sign | 0x7f800000u | (nan ? 0x400000u : 0u)));
+    lo = 0.f;
 }
 
 // float -> double bits on the integer pipe (exact for normal floats; zero

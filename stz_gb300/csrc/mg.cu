@@ -302,18 +302,15 @@ template <typename T> int hierarchy<T>::allocate(int m, int n, V *top_z, V *top_
         L.r = p[2];
     }
     if (pair_cycles) {
-        const size_t bytes = sizeof(float4) * (size_t)m * n;
+        const size_t bytes = sizeof(float4) * (size_t)m * n + sizeof(pair_range);
         void *p = nullptr;
         cudaError_t e = cudaMalloc(&p, bytes);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(top correction)");
         owned_.push_back(p);
         bytes_ += bytes;
         top_pairs = (float4 *)p;
-        e = cudaMalloc(&p, 3 * sizeof(unsigned));
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(residual scale)");
-        owned_.push_back(p);
-        cudaMemset(p, 0, 3 * sizeof(unsigned));
-        peak = (unsigned *)p;
+        range = reinterpret_cast<pair_range *>(top_pairs + (size_t)m * n);
+        cudaMemset(range, 0, sizeof(pair_range));
     }
     return STZG_OK;
 }
@@ -442,7 +439,7 @@ template <typename T> void hierarchy<T>::release() {
         st_pairs[l] = nullptr;
     }
     top_pairs = nullptr;
-    peak = nullptr;
+    range = nullptr;
     dense = nullptr;
     dense_buf = nullptr;
     pairs_dev_ = nullptr;

@@ -77,6 +77,14 @@ std::vector<std::pair<int, int>> coarse_sizes(int m, int n);
 // Galerkin products for the whole hierarchy below the top operator.
 std::vector<level_ops> build_coarse_ops(const qs_constants &q, int m, int n);
 
+// The power of two 2^next by which the next residual of an FP64 hierarchy
+// becomes float pairs, 2^used of the last one, and the magnitude and the
+// arrival count of pair_begin's blocks (zero between launches).
+struct pair_range {
+    int next, used;
+    unsigned top, arrived;
+};
+
 // Device hierarchy in precision T.
 template <typename T> class hierarchy {
   public:
@@ -132,12 +140,9 @@ template <typename T> class hierarchy {
     float4 *top_pairs = nullptr;
     // Float pairs have FP32's exponents, the problems FP64's: with pair_cycles
     // the tables are those of A 2^-unit (its largest coefficient between 1/2 and
-    // 1), and a cycle takes the residual times the power of two that brings its
-    // largest value to [1, 2).  peak: the high word of that value's magnitude as
-    // the last residual kernel left it, its running maximum and its blocks'
-    // arrival count (both zero between launches).
+    // 1), and residuals become pairs times a power of two (range).
     int unit = 0;
-    unsigned *peak = nullptr;
+    pair_range *range = nullptr;
     void release();
     ~hierarchy() { release(); }
     size_t device_bytes() const { return bytes_; }
@@ -178,12 +183,15 @@ void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64
             bool residual_known = false);
 template <typename T> void top_sweep(hierarchy<T> &h, cudaStream_t st);
 // FP64 V-cycles in correction form (mg_small.cu): pair_residual leaves
-// r = b - A z of the top level in its r array, its largest magnitude in peak
-// (and, with a sink, its norms); pair_cycle adds one V-cycle on A d = r, in
-// float pairs, to z.  Where supported, vcycle<double> is the two of them.
+// r = b - A z of the top level as float pairs in its r array (and, with a
+// sink, its norms); pair_cycle
+// adds one V-cycle on A d = r to z.  Where supported, vcycle<double> is the
+// two of them.  pair_begin, before the first of them on a new b or z, takes the
+// range of the residuals from b and z; every residual with norms adapts it.
 bool pair_cycle_supported(const hierarchy<double> &h);
 void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream_t st);
 void pair_cycle(const hierarchy<double> &h, cudaStream_t st);
+void pair_begin(const hierarchy<double> &h, cudaStream_t st);
 // Lays out the matrix of the levels from dense_from on (inverse: of the
 // coarsest level); own and caps: the hierarchy's allocations and their sizes.
 int build_dense(hierarchy<double> &h, const std::vector<double> &inverse, std::vector<void *> &own, size_t *cap);

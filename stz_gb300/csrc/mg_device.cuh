@@ -74,12 +74,14 @@ void launch_early(bool early, void (*kern)(K...), dim3 grid, dim3 block, size_t 
 }
 
 // The end of a residual kernel: a and c are the block's sums of r^2 and b^2
-// (valid in thread 0), sh 32 doubles of shared memory; peak (or null): the
-// launch's running maximum in peak[1], whose final value goes to peak[0].  The sums and the
+// (valid in thread 0), sh 32 doubles of shared memory; range (or null): the
+// residual's power of two was `used`.  While a solve converges its residual
+// leaves the pairs' exponents downwards (or, from a bad guess, upwards): the
+// next one is brought back to 1 once it is 2^30 below or 2^40 above.  The sums and the
 // stopping rule used to be two more launches of one block each per pass (2 to
 // 3 us each inside the solve's graph).
 __device__ __forceinline__ void finish_norms(double a, double c, const norm_sink &s, double *sh,
-                                             unsigned *peak = nullptr) {
+                                             pair_range *range = nullptr, int used = 0) {
     __shared__ int last;
     unsigned *arrived = reinterpret_cast<unsigned *>(s.partials + 2 * s.npart);
     if (threadIdx.x == 0) {
@@ -100,7 +102,11 @@ __device__ __forceinline__ void finish_norms(double a, double c, const norm_sink
     c = block_sum(c, sh);
     if (threadIdx.x != 0) return;
     *arrived = 0;
-    if (peak) peak[0] = atomicExch(peak + 1, 0u);
+    if (range) {
+        range->used = used;
+        const int e = (__double2hiint(a) >> 20) & 0x7ff, at = (e - 1023) >> 1;  // |r| is about 2^at
+        if (e > 0 && e < 0x7ff && (at + used < -30 || at + used > 40)) range->next = min(max(-at, -1000), 1000);
+    }
     s.out[0] = a;
     s.out[1] = c;
     const loop_rule &r = s.rule;

@@ -3,6 +3,7 @@
 
 #include "ff.cuh"
 #include "fixed.cuh"
+#include "mg.cuh"
 #include "mg_plan.h"
 
 namespace stzg {
@@ -15,34 +16,18 @@ __device__ __forceinline__ void pdl_input() { asm volatile("griddepcontrol.wait;
 __device__ __forceinline__ double2 add_pairs(const double2 &z, const float4 &d, double back) {
     return make_double2(fma(ff_to_d(d.x, d.z), back, z.x), fma(ff_to_d(d.y, d.w), back, z.y));
 }
-
-// The powers of two between FP64 vectors and the pairs of a cycle on
-// A 2^-unit: peak is the high word of the vector's largest magnitude, which
-// 2^shift brings to [1, 2) (not finite: left alone); a solution returns by back.
-struct pair_scale {
-    int shift = 0;
-    double back = 1;
-    __device__ __forceinline__ pair_scale() {}
-    __device__ __forceinline__ pair_scale(unsigned peak, int unit) {
-        const int e = (int)(peak >> 20);
-        shift = e >= 0x7ff ? 0 : 1023 - max(e, 1);
-        back = power_of_two(min(max(-shift - unit, -1022), 1023));
-    }
-    __device__ __forceinline__ float4 split(const double2 &v) const {
-        float4 o;
-        ff_split_d(shift_exponent(v.x, shift), o.x, o.z);
-        ff_split_d(shift_exponent(v.y, shift), o.y, o.w);
-        return o;
-    }
-};
+// The power of two that takes a solution of the system in pairs back: the
+// residual was multiplied by 2^used, the operator by 2^-unit.
+__device__ __forceinline__ double pair_back(int used, int unit) {
+    return power_of_two(min(max(-used - unit, -1022), 1023));
+}
 
 // The environment of small_vcycle on the GPU.
 struct block_env {
     static constexpr int kLanes = 32;
     unsigned char *mem;
     int r;
-    bool fp64 = false;  // level t's b is FP64
-    pair_scale scale;
+    int used = 0;  // pair_range::used
     __device__ __forceinline__ int rank() const { return r; }
     __device__ __forceinline__ unsigned char *local() const { return mem; }
     __device__ __forceinline__ unsigned char *base(int k) const {
@@ -63,20 +48,17 @@ struct block_env {
     }
     __device__ __forceinline__ ff lane_sum(ff a) const { return warp_pair_sum(a); }
     __device__ __forceinline__ float2 ld(const float2 *p) const { return __ldcg(p); }
-    __device__ __forceinline__ float4 ld(const float4 *p) const {
-        return fp64 ? scale.split(__ldcg(reinterpret_cast<const double2 *>(p))) : __ldcg(p);
-    }
+    __device__ __forceinline__ float4 ld(const float4 *p) const { return __ldcg(p); }
     __device__ __forceinline__ void wait_input(const small_plan<float> &) { pdl_input(); }
     __device__ __forceinline__ void wait_input(const small_plan<ff> &P) {
         pdl_input();
-        fp64 = P.sum != nullptr;
-        if (fp64) scale = pair_scale(__ldcg(P.peak), P.unit);
+        if (P.sum) used = __ldcg(&P.range->used);
     }
     __device__ __forceinline__ void store(const small_plan<float> &P, size_t k, const float2 &v) const {
         P.lv[P.t].zg[k] = v;
     }
     __device__ __forceinline__ void store(const small_plan<ff> &P, size_t k, const float4 &v) const {
-        if (P.sum) P.sum[k] = add_pairs(P.sum[k], v, scale.back);
+        if (P.sum) P.sum[k] = add_pairs(P.sum[k], v, pair_back(used, P.unit));
         else P.lv[P.t].zg[k] = v;
     }
 };

@@ -6,9 +6,11 @@
 // of the FP64 iterate in FP64, one V-cycle from zero on A d = r in float
 // pairs (~48 significant bits), z += d in FP64.  That is the reference's
 // V-cycle (the cycle is linear in z and b) with the rounding of d at 2^-48
-// of d itself, so the iterate keeps FP64 accuracy.  Powers of two on r and on
-// the operator's tables (pair_scale, hierarchy::unit), exact both ways, keep
-// the pairs inside FP32's exponents whatever the problem's magnitude.  What bounds the cycle on
+// of d itself, so the iterate keeps FP64 accuracy.  Powers of two on r
+// (pair_range) and on the operator's tables (hierarchy::unit), exact both ways,
+// keep the pairs inside FP32's exponents whatever the problem's magnitude; r's
+// is taken once per solve, from b and z, since a maximum over r in front of
+// every cycle cost 3 to 5 percent of it.  What bounds the cycle on
 // GB300 is the FP64 pipe, two results per clock and SM: a pair operation
 // costs 10 to 20 issue slots on the FP32 pipe where an FP64 one blocks its
 // quarter of the SM for 64 clocks.
@@ -61,8 +63,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     small_vcycle<false, false>(P, env);
 }
 
-// r = b - A z of the top level and its largest magnitude (hierarchy::peak);
-// with a sink, the norms (as k_top_sqnorm).
+// r = b - A z of the top level, times 2^range->next, as float pairs; with a sink, the norms (as
+// k_top_sqnorm).
 // A z is evaluated on second differences of z, exact in 64-bit fixed point
 // (fixed.cuh, one scale per tile), and integer products with the
 // coefficients; only b - A z and the norms are FP64.  The rounding is 0.6
@@ -96,15 +98,14 @@ struct res_sum {
 template <int RPT>
 __global__ void __launch_bounds__(kResThreads, 4)
     k_res_pairs(top_op<double> op, res_consts C, const double2 *__restrict__ z, const double2 *__restrict__ b, int m,
-                int n, int tiles_x, int tiles, double2 *__restrict__ r, unsigned *peak, norm_sink sink) {
+                int n, int tiles_x, int tiles, float4 *__restrict__ r, pair_range *range, norm_sink sink) {
     constexpr int RY = kResRows * RPT, RR = RY + 2;
     __shared__ long long X[RR][RC], Y[RR][RC];
-    __shared__ unsigned top[2], rtop;
+    __shared__ unsigned top[2];
     __shared__ double sh[32];
     constexpr int kPer = (RR * RC + kResThreads - 1) / kResThreads;
     const int tid = threadIdx.x, tx = tid & (RX - 1), ty = tid / RX;
     double sr = 0, sb = 0;
-    unsigned rw = 0;
     double2 v[kPer];
     auto load = [&](int tile) {
         const int i0 = (tile % tiles_x) * RX, j0 = (tile / tiles_x) * RY;
@@ -120,8 +121,8 @@ __global__ void __launch_bounds__(kResThreads, 4)
         }
     };
     if (tid < 2) top[tid] = 0;
-    if (tid == 0) rtop = 0;
     pdl_wait();
+    const int shift = __ldcg(&range->next);
     if ((int)blockIdx.x < tiles) load(blockIdx.x);
     __syncthreads();
     int it = 0;
@@ -176,8 +177,10 @@ __global__ void __launch_bounds__(kResThreads, 4)
                 ay.add(C.dyy, y0);
                 e = make_double2(fma(-unit, ax.value(), g[q].x), fma(-unit, ay.value(), g[q].y));
             }
-            r[k] = e;
-            rw = max(rw, max((unsigned)__double2hiint(e.x) & 0x7fffffffu, (unsigned)__double2hiint(e.y) & 0x7fffffffu));
+            float4 o;
+            ff_split_shifted(e.x, shift, o.x, o.z);
+            ff_split_shifted(e.y, shift, o.y, o.w);
+            r[k] = o;
             if (sink.partials) {
                 sr += e.x * e.x + e.y * e.y;
                 sb += g[q].x * g[q].x + g[q].y * g[q].y;
@@ -185,21 +188,43 @@ __global__ void __launch_bounds__(kResThreads, 4)
         }
         __syncthreads();  // the next tile reuses the planes
     }
-    rw = __reduce_max_sync(0xffffffffu, rw);
-    if (tx == 0) atomicMax(&rtop, rw);
-    __syncthreads();
-    if (tid == 0) atomicMax(peak + 1, rtop);
     if (!sink.partials) {
-        if (tid != 0) return;
-        __threadfence();
-        if (atomicAdd(peak + 2, 1u) != gridDim.x - 1) return;
-        __threadfence();
-        peak[2] = 0;
-        peak[0] = atomicExch(peak + 1, 0u);
+        if (tid == 0 && blockIdx.x == 0) range->used = shift;
         return;
     }
     const double a = block_sum(sr, sh), c = block_sum(sb, sh);
-    finish_norms(a, c, sink, sh, peak);
+    finish_norms(a, c, sink, sh, range, shift);
+}
+
+// The power of two that brings the largest of |b| and 4 2^unit |z|, a bound on
+// A z and so (with b) on the residual up to a factor of 2, to [1, 2); 1 where a
+// value is not finite.
+__global__ void __launch_bounds__(kResThreads)
+    k_pair_begin(const double2 *__restrict__ z, const double2 *__restrict__ b, unsigned count, int unit,
+                 pair_range *range) {
+    __shared__ unsigned top;
+    if (threadIdx.x == 0) top = 0;
+    __syncthreads();
+    int e = 0;
+#pragma unroll 4
+    for (unsigned k = blockIdx.x * kResThreads + threadIdx.x; k < count; k += gridDim.x * kResThreads) {
+        const double2 v = z[k], w = b[k];
+        const int ez = max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff) >> 20;
+        const int eb = max(__double2hiint(w.x) & 0x7fffffff, __double2hiint(w.y) & 0x7fffffff) >> 20;
+        if (ez == 0x7ff || eb == 0x7ff) e = 1 << 16;
+        else e = max(e, max(eb, ez ? ez + unit + 2 : 0));
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    if ((threadIdx.x & 31) == 0) atomicMax(&top, (unsigned)e);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    atomicMax(&range->top, top);
+    __threadfence();
+    if (atomicAdd(&range->arrived, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const int all = (int)atomicExch(&range->top, 0u);
+    range->arrived = 0;
+    range->next = all == 0 || all >= 1 << 16 ? 0 : min(max(1023 - all, -1000), 1000);
 }
 
 // ---- host ----------------------------------------------------------------------
@@ -275,6 +300,7 @@ bool plan_small(const hierarchy<T> &h, int t, int blocks, bool zero_start, small
     P.dense = h.dense;
     P.op = consts_of(h.op, h.unit);
     P.unit = h.unit;
+    P.range = h.range;
     P.lv[t].zg = reinterpret_cast<node *>(h.lv[t].z);
     P.lv[t].bg = reinterpret_cast<const node *>(h.lv[t].b);
     return layout_small(P, t, h.dense_from, blocks, kSmallMax);
@@ -327,16 +353,15 @@ tile_level plan_tile(const hierarchy<double> &h, int l, bool up, bool &bands, si
     L.cls = A.cls;
     L.st = l ? h.st_pairs[l] : nullptr;
     L.staged = l && A.homog && A.nst * 320 <= 16384;
-    L.b = reinterpret_cast<const float4 *>(A.b);
+    L.b = reinterpret_cast<const float4 *>(l ? A.b : A.r);
     L.zdown = l ? reinterpret_cast<float4 *>(A.r) : h.top_pairs;
     L.zup = reinterpret_cast<float4 *>(A.z);
     L.bc = reinterpret_cast<float4 *>(C.b);
     L.zc = reinterpret_cast<const float4 *>(C.z);
     if (!l) {
-        L.res = A.r;
-        L.peak = h.peak;
-        L.unit = h.unit;
         L.sum = A.z;
+        L.range = h.range;
+        L.unit = h.unit;
     }
     bands = l && ((A.m & 1) || !A.homog);
     const tile_shape T = shape_tile(L.m, L.cm, L.cn, L.staged ? A.nst * 320 : 0, l ? 0 : (up ? 2 : 1), bands, kTileMax);
@@ -470,11 +495,20 @@ void pair_residual(const hierarchy<double> &h, const norm_sink *sink, cudaStream
         const int tiles_x = ceil_div(T0.m, RX), tiles = tiles_x * ceil_div(T0.n, rows);
         launch_early(
             !h.crowded && (long)T0.m * T0.n <= kEarlyPoints, kernel, dim3(std::min(reduction_blocks(), tiles)), dim3(kResThreads), 0, st, o, C, (const double2 *)T0.z,
-            (const double2 *)T0.b, T0.m, T0.n, tiles_x, tiles, T0.r, h.peak,
+            (const double2 *)T0.b, T0.m, T0.n, tiles_x, tiles, reinterpret_cast<float4 *>(T0.r), h.range,
             sink ? *sink : norm_sink{nullptr, 0, nullptr, {}});
     };
     if (ceil_div(T0.m, RX) * ceil_div(T0.n, 2 * kResRows) < 2 * 152) run(k_res_pairs<1>, kResRows);
     else run(k_res_pairs<2>, 2 * kResRows);
+    note_launch();
+}
+
+void pair_begin(const hierarchy<double> &h, cudaStream_t st) {
+    if (!pair_cycle_supported(h)) return;
+    const level_view<double> &T0 = h.lv[0];
+    const long count = (long)T0.m * T0.n;
+    k_pair_begin<<<std::min(4 * 152, ceil_div(count, kResThreads)), kResThreads, 0, st>>>(T0.z, T0.b, (unsigned)count,
+                                                                                          h.unit, h.range);
     note_launch();
 }
 
@@ -493,7 +527,6 @@ void pair_cycle(const hierarchy<double> &h, cudaStream_t st) {
     if (P.t == 0) {
         P.lv[0].bg = reinterpret_cast<const float4 *>(h.lv[0].r);
         P.sum = h.lv[0].z;
-        P.peak = h.peak;
     }
     launch_small(P, !h.crowded, st);
     for (int l = P.t - 1; l >= 0; l--) {

@@ -34,12 +34,11 @@ struct tile_level {
     float4 *zup;            // written on the way up (coarse level)
     float4 *bc;             // the child's right-hand side
     const float4 *zc;       // the child's solution
-    // top level: the FP64 residual, the high word of its largest magnitude, the
-    // tables' exponent, and the iterate that takes the correction
-    const double2 *res;
-    const unsigned *peak;
-    int unit;
+    // top level: the iterate that takes the correction, the residual's power of
+    // two and the tables'
     double2 *sum;
+    const pair_range *range;
+    int unit;
 };
 
 constexpr int kTileThreads = 256;  // most threads of a tile
@@ -85,11 +84,9 @@ __device__ __forceinline__ window<ff, true> tile_window(const tile_level &L, uns
     return V;
 }
 
-// Rows jlo..jhi of a level into a plane of the window (its column 0 at xb);
-// src(k): the value at node k.
-template <typename F>
-__device__ __forceinline__ void tile_load(const tile_level &L, const window<ff, true> &V, const plane<ff> &dst, F src,
-                                          int jlo, int jhi, int xb) {
+// Rows jlo..jhi of a level into a plane of the window (its column 0 at xb).
+__device__ __forceinline__ void tile_load(const tile_level &L, const window<ff, true> &V, const plane<ff> &dst,
+                                          const float4 *__restrict__ src, int jlo, int jhi, int xb) {
     jlo = max(jlo, 0);
     jhi = min(jhi, V.n - 1);
     const int total = (jhi - jlo + 1) * V.W;
@@ -99,22 +96,9 @@ __device__ __forceinline__ void tile_load(const tile_level &L, const window<ff, 
         int g = xb + w;
         g = g < 0 ? g % L.m + L.m : g;
         g = g >= L.m ? g % L.m : g;
-        dst.set(V.at(j, w), get(src((size_t)j * L.m + g)));
+        dst.set(V.at(j, w), get(__ldcg(src + (size_t)j * L.m + g)));
     }
 }
-
-struct pairs_at {
-    const float4 *p;
-    __device__ __forceinline__ explicit pairs_at(const float4 *q) : p(q) {}
-    __device__ __forceinline__ float4 operator()(size_t k) const { return __ldcg(p + k); }
-};
-// The top level's residual as the pairs of the cycle.
-struct residual_at {
-    const double2 *p;
-    pair_scale s;
-    __device__ __forceinline__ residual_at(const tile_level &L, const pair_scale &q) : p(L.res), s(q) {}
-    __device__ __forceinline__ float4 operator()(size_t k) const { return s.split(__ldcg(p + k)); }
-};
 
 __device__ __forceinline__ void tile_table(const tile_level &L, const float4 *dst) {
     if (!L.staged) return;
@@ -165,7 +149,7 @@ template <bool BANDS> __global__ void __launch_bounds__(kTileThreads) k_pair_lev
     const window<ff, true> V = tile_window(L, tile_raw, W, 2 * (L.th + kLevExtra), G.y0 - kLevRows);
     tile_table(L, V.st);
     pdl_input();
-    tile_load(L, V, V.b, pairs_at(L.b), G.y0 - 2, G.y1, G.xb);
+    tile_load(L, V, V.b, L.b, G.y0 - 2, G.y1, G.xb);
     if (BANDS && (L.m & 1)) lev_clear_last(V, G.y0 - 2, G.y1, tid, nth);
     __syncthreads();
     const block_walk w(tid, nth, W >> 1);
@@ -200,8 +184,8 @@ template <bool BANDS> __global__ void __launch_bounds__(kTileThreads) k_pair_lev
     ff *cs = reinterpret_cast<ff *>(tile_raw + (size_t)W * rows * 4 * sizeof(ff) + (L.staged ? L.nst * 320 : 0));
     tile_table(L, V.st);
     pdl_input();
-    tile_load(L, V, V.z, pairs_at(L.zdown), G.y0 - 1, G.y1 + 1, G.xb);
-    tile_load(L, V, V.b, pairs_at(L.b), G.y0, G.y1, G.xb);
+    tile_load(L, V, V.z, L.zdown, G.y0 - 1, G.y1 + 1, G.xb);
+    tile_load(L, V, V.b, L.b, G.y0, G.y1, G.xb);
     const child_tile C = tile_child(L, G, cs, G.xb >> 1, BANDS ? L.cm : kTileCols / 2 + 1);
     __syncthreads();
     const block_walk w(tid, nth, W >> 1);
@@ -229,7 +213,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_top_down(top_consts<ff> o
     const tile_geom G(L, false, kTopDownCols, kTopDownExtra);
     const window<ff, true> V = tile_window(L, tile_raw, kTileCols, 2 * (L.th + kTopDownExtra), G.y0 - kTopDownRows);
     pdl_input();
-    tile_load(L, V, V.b, residual_at(L, pair_scale(__ldcg(L.peak), L.unit)), G.y0 - 3, G.y1 + 1, G.xb);
+    tile_load(L, V, V.b, L.b, G.y0 - 3, G.y1 + 1, G.xb);
     __syncthreads();
     const block_walk w(threadIdx.x, L.threads, kTileCols / 2);
     block_top_color(op, V, w, G.qn, G.y0 - 3, G.y1 + 1, 0, true);
@@ -253,9 +237,9 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_top_up(top_consts<ff> op,
     const window<ff, true> V = tile_window(L, tile_raw, kTileCols, rows, G.y0 - kTopUpRows);
     ff *cs = reinterpret_cast<ff *>(tile_raw + (size_t)kTileCols * rows * 4 * sizeof(ff));
     pdl_input();
-    const pair_scale scale(__ldcg(L.peak), L.unit);
-    tile_load(L, V, V.z, pairs_at(L.zdown), G.y0 - 2, G.y1 + 1, G.xb);
-    tile_load(L, V, V.b, residual_at(L, scale), G.y0 - 1, G.y1, G.xb);
+    const int used = __ldcg(&L.range->used);
+    tile_load(L, V, V.z, L.zdown, G.y0 - 2, G.y1 + 1, G.xb);
+    tile_load(L, V, V.b, L.b, G.y0 - 1, G.y1, G.xb);
     const child_tile C = tile_child(L, G, cs, G.xb >> 1, kTileCols / 2 + 1);
     __syncthreads();
     const block_walk w(threadIdx.x, L.threads, kTileCols / 2);
@@ -266,6 +250,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_top_up(top_consts<ff> op,
     __syncthreads();
     block_top_color(op, V, w, G.qn, G.y0, G.y1 - 1, 1, false);
     __syncthreads();
+    const double back = pair_back(used, L.unit);
     // z += d: four nodes' iterates are on their way at a time
     const int ow = G.x1 - G.x0, total = (G.y1 - G.y0) * ow;
     const divider dv(ow);
@@ -281,7 +266,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_top_up(top_consts<ff> op,
         }
 #pragma unroll
         for (int u = 0; u < 4; u++)
-            if (k0 + u * L.threads < total) *at[u] = add_pairs(z[u], d[u], scale.back);
+            if (k0 + u * L.threads < total) *at[u] = add_pairs(z[u], d[u], back);
     }
 }
 

@@ -28,6 +28,7 @@
 #include "ffnum.cuh"
 
 namespace stzg {
+struct pair_range;
 namespace mgw {
 
 // ---- numbers -----------------------------------------------------------------
@@ -773,9 +774,9 @@ template <typename S> struct small_plan {
     unsigned ro;             // residual rows of the level in hand
     unsigned bytes;
     const float4 *dense;     // row-major, per column node (x.hi, x.lo, y.hi, y.lo)
-    double2 *sum;            // not null: level t is the top one, its b the FP64 residual
-                             // (magnitude: peak), and its result is added to this iterate
-    const unsigned *peak;
+    double2 *sum;            // not null: the top level's result, times a power of
+                             // two, is added to this iterate
+    const pair_range *range;
     int unit;                // the tables are those of A 2^-unit
     top_consts<S> op;
     small_level<S> lv[kMaxLevels];
