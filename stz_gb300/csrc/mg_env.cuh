@@ -25,6 +25,7 @@ __device__ __forceinline__ double pair_back(int used, int unit) {
 // The environment of small_vcycle on the GPU.
 struct block_env {
     static constexpr int kLanes = 32;
+    static constexpr bool kMeasured = false;
     unsigned char *mem;
     int r;
     int used = 0;  // pair_range::used
@@ -35,6 +36,9 @@ struct block_env {
         asm("mapa.u64 %0, %1, %2;\n" : "=l"(a) : "l"((unsigned long long)mem), "r"(k));
         return (unsigned char *)a;
     }
+    template <typename N> __device__ __forceinline__ void measure(const N *) {}
+    __device__ __forceinline__ void measured() {}
+    __device__ __forceinline__ void share(int, int) {}
     __device__ __forceinline__ int thread() const { return (int)threadIdx.x; }
     __device__ __forceinline__ int threads() const { return (int)blockDim.x; }
     __device__ __forceinline__ const block_walk &walk(const block_walk &w, int, int) const { return w; }
@@ -103,9 +107,9 @@ inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int
 }
 
 // Largest cluster (a power of two up to 16) the device takes for a small-level
-// kernel with all of the shared memory; 0 where its attributes are refused.
-inline int cluster_limit(const void *kernel) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMax) != cudaSuccess ||
+// kernel with that much dynamic shared memory; 0 where its attributes are refused.
+inline int cluster_limit(const void *kernel, unsigned bytes = kSmallMax) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -113,7 +117,7 @@ inline int cluster_limit(const void *kernel) {
     for (int c = 16; c >= 2; c >>= 1) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute at[2];
-        cluster_config(cfg, at, c, kSmallMax, nullptr);
+        cluster_config(cfg, at, c, bytes, nullptr);
         cfg.attrs = at + 1;
         cfg.numAttrs = 1;
         int n = 0;

@@ -3,6 +3,7 @@
 #include "mg_small.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -14,19 +15,52 @@ using namespace mgw;
 
 namespace {
 
-// b and z of the first level are FP64 vectors of the size of a node.
+// b and z of the first level are FP64 vectors of the size of a node.  Pairs have
+// FP32's exponents, so b is taken times the power of two that brings its
+// largest value to [1, 2), and z back (the tables are those of A 2^-unit).
+// That value is a maximum over the cluster: one more barrier and a second
+// look at b.
 struct io_env : block_env {
+    static constexpr bool kMeasured = true;
+    unsigned *words;  // shared: the block's largest high word, the cluster's
+    unsigned mine = 0;
+    __device__ __forceinline__ double2 raw(const float4 *p) const {
+        return __ldcg(reinterpret_cast<const double2 *>(p));
+    }
+    __device__ __forceinline__ void measure(const float4 *p) {
+        const double2 v = raw(p);
+        mine = max(mine, max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu));
+    }
+    __device__ __forceinline__ void measured() {
+        mine = __reduce_max_sync(0xffffffffu, mine);
+        if ((threadIdx.x & 31) == 0) atomicMax(&words[0], mine);
+    }
+    __device__ __forceinline__ void share(int tid, int nb) {
+        if (tid >= nb) return;
+        unsigned long long a;
+        asm("mapa.u64 %0, %1, %2;\n" : "=l"(a) : "l"((unsigned long long)(words + 1)), "r"(tid));
+        atomicMax((unsigned *)a, words[0]);
+    }
+    __device__ __forceinline__ int shift() const {
+        const int e = (int)(words[1] >> 20);
+        return e == 0x7ff ? 0 : 1023 - max(e, 1);
+    }
     __device__ __forceinline__ float4 ld(const float4 *p) const {
-        const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+        const double2 v = raw(p);
+        const int s = shift();
         float4 o;
-        ff_split_d(v.x, o.x, o.z);
-        ff_split_d(v.y, o.y, o.w);
+        ff_split_shifted(v.x, s, o.x, o.z);
+        ff_split_shifted(v.y, s, o.y, o.w);
         return o;
     }
     __device__ __forceinline__ void store(const small_plan<ff> &P, size_t k, const float4 &v) const {
-        reinterpret_cast<double2 *>(P.lv[P.t].zg)[k] = make_double2(ff_to_d(v.x, v.z), ff_to_d(v.y, v.w));
+        const double back = pair_back(shift(), P.unit);
+        reinterpret_cast<double2 *>(P.lv[P.t].zg)[k] =
+            make_double2(ff_to_d(v.x, v.z) * back, ff_to_d(v.y, v.w) * back);
     }
 };
+
+constexpr unsigned kBlockMax = kSmallMax - 256;  // the rest for io_env's words
 
 // FP64 V-cycle of a 512 x 256 grid of 2x2 blocks, y periodic: 520 us with one
 // FP64 launch per colour and a single-block FP64 tail of 215 us; the four steps
@@ -35,9 +69,12 @@ template <bool FAST, bool YP>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_small_blocks(const __grid_constant__ small_plan<ff> P) {
     extern __shared__ __align__(16) unsigned char small_raw[];
     pdl_start();
+    __shared__ unsigned words[2];
+    if (threadIdx.x < 2) words[threadIdx.x] = 0;  // seen by all from the first barrier on
     io_env env;
     env.mem = small_raw;
     env.r = (int)blockIdx.x;
+    env.words = words;
     small_vcycle<FAST, YP>(P, env);
 }
 
@@ -63,7 +100,7 @@ int max_blocks() {
         const void *k[4] = {(const void *)k_small_blocks<true, true>, (const void *)k_small_blocks<true, false>,
                             (const void *)k_small_blocks<false, true>, (const void *)k_small_blocks<false, false>};
         int c = 16;
-        for (const void *f : k) c = std::min(c, cluster_limit(f));
+        for (const void *f : k) c = std::min(c, cluster_limit(f, kBlockMax));
         if (cudaFuncSetAttribute(k_block_columns<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMax) !=
                 cudaSuccess ||
             cudaFuncSetAttribute(k_block_columns<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -120,6 +157,11 @@ int small_cycle::setup(const std::vector<small_desc> &desc, int yp, const std::v
         if (yp && (desc[l].n & 1)) return done(nullptr);
     small_plan<ff> P;
     std::memset(&P, 0, sizeof(P));
+    double top = 0;
+    for (int l = t; l <= ml; l++)
+        for (size_t k = 0; k < desc[l].table.size(); k++)
+            if (k % 40 < 36) top = std::max(top, std::fabs(desc[l].table[k]));
+    if (top > 0 && std::isfinite(top)) std::frexp(top, &P.unit);
     for (int l = t; l <= ml; l++) {
         const small_desc &D = desc[l];
         const int nst = (int)D.table.size() / 40;
@@ -128,7 +170,7 @@ int small_cycle::setup(const std::vector<small_desc> &desc, int yp, const std::v
             for (int e = 0; e < 10; e++) {
                 float h[4], o[4];
                 for (int q = 0; q < 4; q++) {
-                    const double v = D.table[(size_t)c * 40 + 4 * e + q];
+                    const double v = std::ldexp(D.table[(size_t)c * 40 + 4 * e + q], e < 9 ? -P.unit : P.unit);
                     h[q] = (float)v;
                     o[q] = (float)(v - (double)h[q]);
                 }
@@ -156,8 +198,9 @@ int small_cycle::setup(const std::vector<small_desc> &desc, int yp, const std::v
         if (l == ml) {
             bottom_.resize(N * N);
             for (size_t k = 0; k < N * N; k++) {
-                const float h = (float)bottom[k];
-                bottom_[k] = make_float2(h, (float)(bottom[k] - (double)h));
+                const double v = std::ldexp(bottom[k], P.unit);
+                const float h = (float)v;
+                bottom_[k] = make_float2(h, (float)(v - (double)h));
             }
             STZG_CUDA(cudaMemcpyAsync(dense_[l].p, bottom_.data(), N * N * sizeof(float2), cudaMemcpyHostToDevice, st));
             continue;
@@ -173,7 +216,7 @@ int small_cycle::setup(const std::vector<small_desc> &desc, int yp, const std::v
     P.zero_start = 1;
     for (; t < d; t++)
         for (int c = cap; c >= 1; c >>= 1)
-            if (layout_small(P, t, d, c, kSmallMax)) {
+            if (layout_small(P, t, d, c, kBlockMax)) {
                 t_ = t;
                 return done(&P);
             }

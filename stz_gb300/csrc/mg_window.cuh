@@ -873,7 +873,9 @@ constexpr int kDenseRows = 3;  // 34 rows per block of sixteen warps at 17 x 16 
 // csync() (a barrier of all blocks), kLanes and lane_sum(v) (threads of a
 // product row and the sum over them), ld(p) (a global load), store(P, k, v)
 // (the result of level t at its node k), wait_input(P) (before the first read
-// of what an earlier kernel wrote).
+// of what an earlier kernel wrote).  kMeasured: the largest magnitude of level
+// t's b is taken before b is loaded, each thread with measure(p), each block
+// with measured() and, on one thread per block of the cluster, share(thread, nb).
 template <bool FAST, bool YP, typename S, typename E> MGW_FN void small_vcycle(const small_plan<S> &P, E &env) {
     typedef typename num<S>::node node;
     const int me = env.rank(), nb = P.blocks;
@@ -881,7 +883,21 @@ template <bool FAST, bool YP, typename S, typename E> MGW_FN void small_vcycle(c
     const small_level<S> &D = P.lv[P.d];
     const node *bd = reinterpret_cast<const node *>(base + D.bo);
     const plane<S> zd{reinterpret_cast<S *>(base + D.zo), D.ps};
-    // the tables; level t's own and halo rows of b (and z)
+    // level t's own and halo rows of b (and z)
+    auto load = [&](int tid, int nth) {
+        const small_level<S> &L = P.lv[P.t];
+        const window<S, true, YP> V = band_window<FAST, YP>(P, P.t, me, base);
+        const int y1 = band_row(P, P.t, me + 1);
+        const int lo = V.lo(V.jb), hi = V.hi(y1 + band_above(P, P.t) - 1) + 1;
+        const int total = (hi - lo) * L.m;
+        const divider dv(L.m);
+        for (int k = tid; k < total; k += nth) {
+            const int q = dv.quot(k), j = lo + q, w = k - q * L.m;
+            V.b.set(V.at(j, w), get(env.ld(L.bg + (size_t)V.wrapped(j) * L.m + w)));
+            if (P.top && !P.zero_start) V.z.set(V.at(j, w), get(env.ld(L.zg + (size_t)V.wrapped(j) * L.m + w)));
+        }
+    };
+    // the tables
     env.par([&](int tid, int nth) {
         for (int l = P.t; l < P.d; l++) {
             const small_level<S> &L = P.lv[l];
@@ -895,19 +911,20 @@ template <bool FAST, bool YP, typename S, typename E> MGW_FN void small_vcycle(c
             }
         }
         env.wait_input(P);
-        const small_level<S> &L = P.lv[P.t];
-        const window<S, true, YP> V = band_window<FAST, YP>(P, P.t, me, base);
-        const int y1 = band_row(P, P.t, me + 1);
-        const int lo = V.lo(V.jb), hi = V.hi(y1 + band_above(P, P.t) - 1) + 1;
-        const int total = (hi - lo) * L.m;
-        const divider dv(L.m);
-        for (int k = tid; k < total; k += nth) {
-            const int q = dv.quot(k), j = lo + q, w = k - q * L.m;
-            V.b.set(V.at(j, w), get(env.ld(L.bg + (size_t)V.wrapped(j) * L.m + w)));
-            if (P.top && !P.zero_start) V.z.set(V.at(j, w), get(env.ld(L.zg + (size_t)V.wrapped(j) * L.m + w)));
-        }
+        if (!E::kMeasured) load(tid, nth);
     });
     if (nb > 1) env.csync();  // every block runs: its shared memory may be written
+    if (E::kMeasured) {
+        env.par([&](int tid, int nth) {
+            const int m = P.lv[P.t].m, y0 = band_row(P, P.t, me), y1 = band_row(P, P.t, me + 1);
+            const node *b = P.lv[P.t].bg + (size_t)y0 * m;
+            for (int k = tid; k < (y1 - y0) * m; k += nth) env.measure(b + k);
+            env.measured();
+        });
+        env.par([&](int tid, int nth) { env.share(tid, nb); });
+        if (nb > 1) env.csync();
+        env.par(load);
+    }
     // down
     for (int l = P.t; l < P.d; l++) {
         const window<S, true, YP> V = band_window<FAST, YP>(P, l, me, base);

@@ -54,6 +54,16 @@ def test_moduli(m, n, k):
         np.testing.assert_array_equal(zk, z / s)
 
 
+@pytest.mark.parametrize("m,n", SIZES)
+def test_zero_right_hand_side(m, n):
+    """From a guess to zero: the stopping rule asks for a residual whose squares
+    vanish, 150 decades below the first one."""
+    g = _src(m, n)
+    with _sim(simple_shear(m, n, viscosity=0.02)) as sim:
+        z, cycles, _ = sim.mg_solve(0.01, 0 * g, g)
+        assert np.abs(z).max() < 1e-150 and cycles > 0
+
+
 def test_reference_rule():
     """The absolute stopping rule, whose threshold follows the moduli."""
     P, b, s = simple_shear(64, 64, viscosity=0.02), _src(64, 64), 2.0 ** 200
