@@ -66,7 +66,10 @@ int stzg_tgmg_destroy(stzg_tgmg *g);
  * correction added to z in FP64; the predictor, l2_error and acc count and
  * test passes and FP64 residuals as they do V-cycles.  Residuals must stay
  * inside FP32's range (1e-38..3e38).  The other solver types, and precision 0
- * (STZG_FP64, the default), run in FP64. */
+ * (STZG_FP64, the default), run in FP64; inside V-cycle and full-multigrid
+ * solves of 2x2-block operators periodic in x, whose residual is tested, the
+ * small levels work on the correction in pairs of floats (48 bits of it,
+ * scaled: FP64's range).  stzg_tgmg_iterate runs every level in FP64. */
 int stzg_tgmg_set_precision(stzg_tgmg *g, int precision);
 
 /* The source b and solution z (block*m*n doubles, row-major), copied in and out. */

@@ -1281,8 +1281,8 @@ int stzg_mg_vcycle(stzg_sim *s, double dt, const double *src, double *vel) {
     const size_t nn = (size_t)s->m * (s->n + 1);
     STZG_CUDA(cudaMemcpyAsync(s->F.src, src, nn * sizeof(double2), cudaMemcpyHostToDevice, s->st));
     STZG_CUDA(cudaMemcpyAsync(s->F.vel, vel, nn * sizeof(double2), cudaMemcpyHostToDevice, s->st));
-    pair_begin(s->h64, s->st);
-    STZG_CHECK(run_vcycles(s, 1));
+    vcycle<double>(s->h64, s->st, 10, 1, false, false, true);
+    STZG_CUDA(cudaGetLastError());
     STZG_CUDA(cudaMemcpyAsync(vel, s->F.vel, nn * sizeof(double2), cudaMemcpyDeviceToHost, s->st));
     STZG_CUDA(cudaStreamSynchronize(s->st));
     return STZG_OK;

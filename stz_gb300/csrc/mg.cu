@@ -2707,7 +2707,7 @@ bool coarse_persist_supported() {
 bool coarse_persist_active(const hierarchy<float> &h) { return persist_start(h, tail_start(h)) > 0; }
 
 template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64, bool zero_start,
-                                  bool residual_known) {
+                                  bool residual_known, bool plain) {
     typedef typename vec2_t<T>::type V;
     dim3 blk(32, 8);
     const int ml = h.nl - 1;
@@ -2721,7 +2721,7 @@ template <typename T> void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_s
     int t = tail_start(h);
     int small = -1;  // first level of the small-level kernel (-1: none)
     if constexpr (sizeof(T) == 8) {
-        if (pair_cycle_supported(h)) {
+        if (!plain && pair_cycle_supported(h)) {
             if (zero_start) cudaMemsetAsync(T0.z, 0, sizeof(V) * (size_t)T0.m * T0.n, st);
             if (!residual_known) pair_residual(h, nullptr, st);
             pair_cycle(h, st);
@@ -2908,8 +2908,8 @@ bool top_level_kernel(hierarchy<float> &h, int which, cudaStream_t st) {
     return true;
 }
 
-template void vcycle<double>(hierarchy<double> &, cudaStream_t, int, int, bool, bool);
-template void vcycle<float>(hierarchy<float> &, cudaStream_t, int, int, bool, bool);
+template void vcycle<double>(hierarchy<double> &, cudaStream_t, int, int, bool, bool, bool);
+template void vcycle<float>(hierarchy<float> &, cudaStream_t, int, int, bool, bool, bool);
 template void top_sweep<double>(hierarchy<double> &, cudaStream_t);
 template void top_sweep<float>(hierarchy<float> &, cudaStream_t);
 template void top_residual_sqnorm<double>(hierarchy<double> &, const norm_sink &, cudaStream_t);

@@ -177,10 +177,12 @@ struct norm_sink {
 // zero_start: the top-level z is taken as zero (the first cycle of a pass);
 // the V-cycle then clears it itself or never reads it.  residual_known: the
 // last launch that touched h's top z, b and r was top_residual_sqnorm, whose r
-// a cycle in correction form (FP64) starts from.
+// a cycle in correction form (FP64) starts from.  plain: no correction form,
+// for a cycle that is itself the result: the pairs' 2^-48 is relative to the
+// correction, which only a loop that goes on from the residual makes small.
 template <typename T>
 void vcycle(hierarchy<T> &h, cudaStream_t st, int bottom_sweeps, int bottom_fp64, bool zero_start = false,
-            bool residual_known = false);
+            bool residual_known = false, bool plain = false);
 template <typename T> void top_sweep(hierarchy<T> &h, cudaStream_t st);
 // FP64 V-cycles in correction form (mg_small.cu): pair_residual leaves
 // r = b - A z of the top level as float pairs in its r array (and, with a

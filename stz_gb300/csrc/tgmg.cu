@@ -781,6 +781,8 @@ template <int B> struct tg {
     // the FP64 residual, corrections added in FP64): FP32 levels sharing the
     // class maps of lv, their tables and the FP32 coarsest inverse.
     bool mixed = false, have32 = false;
+    // every level in FP64 (single iterations, whose result no residual is tested on)
+    bool plain = false;
     glevel<B, float> lf[kMaxLevels];
     size_t stf_cap[kMaxLevels] = {0};
     float *inv_f = nullptr;
@@ -790,7 +792,7 @@ template <int B> struct tg {
     hview<B, float> v32() const { return hview<B, float>{lf, inv ? inv_f : nullptr, inv_n, tail_start_f}; }
     // graph of one iteration of the last (type, omega, cycles) used
     cudaGraphExec_t gexec = nullptr;
-    int gkey[5] = {-1, 0, 0, 0, 0};
+    int gkey[6] = {-1, 0, 0, 0, 0, 0};
     double gomega = 0;
     long gnodes = 0;
     double last_ms = 0;
@@ -898,7 +900,7 @@ template <int B, typename T> void vc(tg<B> *g, const hview<B, T> &h, int i, int 
         return;
     }
     if constexpr (B == 2 && sizeof(T) == 8) {
-        if (g->small.active() && i == g->small.first() && cd == 1 && cu == 1 && !sym && hb == kBottomSweeps) {
+        if (!g->plain && g->small.active() && i == g->small.first() && cd == 1 && cu == 1 && !sym && hb == kBottomSweeps) {
             g->small.launch(reinterpret_cast<const double2 *>(h.lv[i].b), reinterpret_cast<double2 *>(h.lv[i].z), g->st);
             g->kernels++;
             return;
@@ -1015,7 +1017,7 @@ template <int B> void drop_graph(tg<B> *g) {
 
 template <int B> int run_iterations(tg<B> *g, int type, int count, double omega, int cd, int cu, int hb) {
     if (count <= 0) return STZG_OK;
-    const int key[5] = {type, cd, cu, hb, uses_mixed(g, type) ? 2 : 1};
+    const int key[6] = {type, cd, cu, hb, uses_mixed(g, type) ? 2 : 1, g->plain};
     if (!g->gexec || std::memcmp(key, g->gkey, sizeof(key)) != 0 || g->gomega != omega) {
         drop_graph(g);
         const long k0 = g->kernels;
@@ -1553,7 +1555,10 @@ int tg_solve_fixed(tg<B> *g, int type, int per_loop, int max_loops, double omega
 template <int B> int tg_iterate(tg<B> *g, int type, int count, double omega, int cd, int cu, int hb) {
     timed<B> t(g);
     if (uses_mixed(g, type) && count > 0) resid_split(g);
-    STZG_CHECK(run_iterations(g, type, count, omega, cd, cu, hb));
+    g->plain = true;
+    const int st = run_iterations(g, type, count, omega, cd, cu, hb);
+    g->plain = false;
+    STZG_CHECK(st);
     t.done();
     STZG_CUDA(cudaGetLastError());
     return STZG_OK;
