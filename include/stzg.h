@@ -66,8 +66,10 @@ typedef struct {
                           (0: 4194304); reaching it returns STZG_ESUBSTEP */
     int advection;     /* STZG_ADV_AUTO (0) or STZG_ADV_SPLIT: the advection (and the explicit
                           step) takes its increments from 64-bit fixed-point copies of the
-                          FP64 fields, with exact differences and ENO choices and one FP64
-                          rounding per updated value; mixed-precision handles also run the
+                          FP64 fields, with exact differences and ENO choices, within the
+                          rounding of the values each update is computed from (parts
+                          of the grid whose values spread too far for that run in
+                          FP64); mixed-precision handles also run the
                           projection source and the stress correction in float-float
                           arithmetic (pairs of floats, ~2^-44 relative) on the FP64 state.
                           STZG_ADV_FP64 keeps all of them in FP64, bit-exact with the

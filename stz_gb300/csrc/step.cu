@@ -426,11 +426,17 @@ __device__ __forceinline__ double add_ff(double a, ff inc) { return a + ff_to_d(
 // comparison of their magnitudes and the ENO value (at most 2^62) are then
 // exact, so near ties need no margin.  The products with the velocity times
 // dt/(2 dx), scaled likewise, are the high words of 64 x 64 bit products (cut
-// at about 2^-57 of the largest increment), and each field takes its increment
-// in one FP64 addition.  An update therefore carries the one rounding the FP64
-// form's last operation has.
-// Tiles with an infinity or a NaN in a field or the velocity are listed and
-// take k_advect's arithmetic in k_advect_rest, as do the cells that the yield
+// within four units of 2^-57 of the largest increment), and each field takes its
+// increment in one FP64 addition.
+// Those cuts are relative to the tile's largest values.  An update stays within
+// 32 roundings of the values it is computed from, the error bound of the FP64
+// form, where one value of its stencil reaches 2^50 units of the increment
+// (fx_weak; with a velocity dt/(2 dx) of 0.1, 2^-7 of the tile's largest); a
+// cell where none does, which takes fields over many orders of magnitude within
+// a tile, lists its 32 x 8 half.  Mixed handles, whose solves and source leave
+// 2^-44, ask for 2^47 units.
+// The listed halves take k_advect's arithmetic in k_advect_rest, as do tiles with
+// an infinity or a NaN in a field or the velocity, and the cells that the yield
 // test (on the leading 24 bits, with a margin) cannot certify as elastic.
 // A block takes 32 x 16 cells, two rows of eight threads after one another: the
 // staged halo is 1.4 times the cells (1.7 at 32 x 8, where converting it was a
@@ -439,6 +445,19 @@ __device__ __forceinline__ double add_ff(double a, ff inc) { return a + ff_to_d(
 // instructions a cell, the integers' conversions among them).
 constexpr int FXY = 2 * ATY, FROWS = FXY + 4;
 constexpr unsigned kFxBytes = F_COUNT * FROWS * ACOLS * sizeof(double);
+// Of a field's increments in a tile: minus their unit, and the quick test's
+// threshold with its double (zero for a field that cannot fail it).
+struct alignas(16) fx_scale {
+    double unit;
+    int thr;
+    unsigned span;
+    __device__ __forceinline__ void set(int K, int t) {
+        unit = -power_of_two(K);
+        thr = t;
+        span = 2u * (unsigned)t;
+    }
+    __device__ __forceinline__ bool below(long long v) const { return (unsigned)((int)(v >> 32) + thr) < span; }
+};
 struct fx_smem {
     union {
         double d[F_COUNT][FROWS][ACOLS];  // TMA destination (128-byte aligned)
@@ -446,6 +465,8 @@ struct fx_smem {
     } t;
     long long nu[FXY + 1][ATX + 1], nv[FXY + 1][ATX + 1];  // node velocities, walls substituted
     unsigned top[F_COUNT + 1];  // largest high word's magnitude per field; then of the velocity
+    unsigned redo;              // halves to list
+    fx_scale scale[F_COUNT];
     int xs[ACOLS], col[ACOLS];  // period shift and storage column of tile column c-2
     uint64_t bar;
 };
@@ -454,6 +475,7 @@ struct fx_smem {
 struct advect_fx_consts {
     long long hmx, hmy;
     int he;
+    int floor = 0;  // explicit step: what its viscous and diffusive sums ask of fx_threshold
     double xf, yf;  // 1/(2 dt dx), 1/(2 dt dy) of projection_step
 };
 
@@ -491,6 +513,37 @@ __device__ __forceinline__ long long fx_products(const fx_factor &u, long long a
     return (long long)u.hi * a1 + (long long)v.hi * b1 + (mid >> 31);
 }
 
+// Whether no integer of the cross of two columns and two rows around c reaches
+// 2^32 thr.
+__device__ __forceinline__ bool below(long long v, int thr) {
+    return (unsigned)((int)(v >> 32) + thr) < 2u * (unsigned)thr;
+}
+__device__ __forceinline__ bool stencil_below(const long long *c, int thr) {
+    bool b = below(c[0], thr);
+    for (int k = 1; k <= 2; k++)
+        b = b && below(c[k], thr) && below(c[-k], thr) && below(c[k * ACOLS], thr) && below(c[-k * ACOLS], thr);
+    return b;
+}
+// 2^(K - 32) for the test above, K = 33 at least; 2^30, which nothing reaches, for
+// an increment that large.
+__device__ __forceinline__ int fx_threshold(int K) { return 1 << min(max(K - 32, 1), 30); }
+
+// Whether a cell (and node) that failed the quick test may be off by more than
+// its own values' rounding: a field, unless it or the velocity is zero in the
+// whole tile, or the velocity at the cell's corners, whose differences are the
+// spin, is everywhere small.
+__device__ __noinline__ bool fx_weak(const fx_smem &Sm, int row, int tx, bool node, int thr) {
+    if (Sm.top[F_COUNT] == 0) return false;
+    const int at = (row + 2) * ACOLS + tx + 2;
+    for (int f = 0; f < F_COUNT; f++)
+        if (Sm.top[f] != 0 && (node || (f != F_X && f != F_Y)) && stencil_below(&Sm.t.v[f][0][0] + at, thr)) return true;
+    constexpr int slow = 1 << (50 - 32);
+    bool b = true;
+    for (int k = 0; k < 4; k++)
+        b = b && below(Sm.nu[row + (k >> 1)][tx + (k & 1)], slow) && below(Sm.nv[row + (k >> 1)][tx + (k & 1)], slow);
+    return b;
+}
+
 // Yield test on the leading 24 bits: 3q^2 + s^2 + tau^2 within 5e-7; a cell
 // clearly below the cut-offs of k_advect (1e-24, or an athermal law below
 // yield) is elastic there too, any other one takes the FP64 test and law.
@@ -523,6 +576,7 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         Sm.xs[tid] = u < 0 ? -1 : (u >= m ? 1 : 0);
     }
     if (tid < F_COUNT + 1) Sm.top[tid] = 0;
+    if (tid == 0) Sm.redo = 0;
     __syncthreads();
     if (tid == 0) {
         mbar_expect_tx(&Sm.bar, kFxBytes);
@@ -584,6 +638,9 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         E[f] = max((int)(Sm.top[f] >> 20), 128);
         finite = finite && E[f] < 0x7ff;
     }
+    const int Ku = Eu + h.he - 2037;  // an increment is its integer times -2^(E + Ku)
+#pragma unroll
+    for (int f = 0; f < F_COUNT; f++) finite = finite && E[f] + Ku < 1000;
     if (!finite) {  // the same for the whole block
         // two of k_advect's tiles
         if (tid < 2 && j0 + tid * ATY < n)
@@ -593,6 +650,11 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
     // the map's values are unwrapped across the seam: room for the period
     E[F_X] = max(E[F_X], (int)((unsigned)__double2hiint(c.lx) >> 20)) + 1;
     const long long lx = to_fixed(c.lx, E[F_X]);
+    const int thr = fx_threshold((PRE ? 50 : 47) + Ku + 1081);
+    if (tid == 0) {
+#pragma unroll
+        for (int f = 0; f < F_COUNT; f++) Sm.scale[f].set(E[f] + Ku, Sm.top[f] && Sm.top[F_COUNT] ? thr : 0);
+    }
     for (int p = tid; p < FROWS * ACOLS; p += ATX * ATY) {
 #pragma unroll
         for (int f = 0; f < F_COUNT; f++) {
@@ -613,15 +675,15 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         }
     }
     __syncthreads();
-    if (i >= m) return;
-    const int Ku = Eu + h.he - 2037;  // an increment is its integer times -2^(E + Ku)
+    unsigned flows = 0, unsure = 0;  // of this thread's two cells, those not surely elastic; those to look at again
 #pragma unroll 1
-    for (int row = ty; row < FXY; row += ATY) {
+    for (int row = ty; row < FXY && i < m && j0 + row < n; row += ATY) {
         const int j = j0 + row;
-        if (j >= n) return;
         const size_t ci = (size_t)(j + 1) * m + i;
+        bool weak = false;
         auto upwind = [&](int f, const fx_factor &uh, int dx, const fx_factor &vh, int dy, bool inner) {
             const long long *q = &Sm.t.v[f][row + 2][tx + 2];
+            weak = weak || Sm.scale[f].below(q[0]);
             return fx_products(uh, eno_fx(q, dx, true), vh, eno_fx(q, dy, inner));
         };
         const long long u00 = Sm.nu[row][tx], v00 = Sm.nv[row][tx];
@@ -632,12 +694,13 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
             const bool inner = v00 > 0 ? j > 1 : j < n - 1;
 #pragma unroll
             for (int f = F_X; f <= F_Y; f++)
-                B[f][ci] = fma((double)upwind(f, uh, dx, vh, dy, inner), -power_of_two(E[f] + Ku), A[f][ci]);
+                B[f][ci] = fma((double)upwind(f, uh, dx, vh, dy, inner), Sm.scale[f].unit, A[f][ci]);
         }
         // staggered velocity and spin (shear_sim.cc:330-333)
         const long long u10 = Sm.nu[row][tx + 1], u01 = Sm.nu[row + 1][tx], u11 = Sm.nu[row + 1][tx + 1];
         const long long v10 = Sm.nv[row][tx + 1], v01 = Sm.nv[row + 1][tx], v11 = Sm.nv[row + 1][tx + 1];
         const long long u4 = (u00 + u10) + (u01 + u11), v4 = (v00 + v10) + (v01 + v11);
+        weak = weak || (below(u4, 1 << (52 - 32)) && below(v4, 1 << (52 - 32)));
         const double two_omega = (double)(__mul64hi((v10 - v00) + (v11 - v01), h.hmx) -
                                           __mul64hi((u01 - u00) + (u11 - u10), h.hmy)) *
                                  power_of_two(64 + Eu - 1081 + h.he);
@@ -649,16 +712,27 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         for (int f = 0; f < 5; f++) a[f] = A[f][ci];
 #pragma unroll
         for (int f = 0; f < 5; f++) {
-            const double inc = (double)upwind(f, uh, dx, vh, dy, inner), sc = -power_of_two(E[f] + Ku);
+            const double inc = (double)upwind(f, uh, dx, vh, dy, inner), sc = Sm.scale[f].unit;
             if (f == F_S) v[f] = a[f] + fma(inc, sc, two_omega * a[F_TAU]);
             else if (f == F_TAU) v[f] = a[f] + fma(inc, sc, -two_omega * a[F_S]);
             else v[f] = fma(inc, sc, a[f]);
             B[f][ci] = v[f];
         }
-        if (!surely_elastic(c, a[F_Q], a[F_S], a[F_TAU])) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
+        if (!surely_elastic(c, a[F_Q], a[F_S], a[F_TAU])) flows |= row < ATY ? 1u : 2u;
         F.ddev[ci] = 0;
         if (PRE) write_pre(F, ci, h.xf, h.yf, v[F_P], v[F_Q], v[F_S], v[F_TAU]);
+        if (weak) unsure |= row < ATY ? 1u : 2u;
     }
+#pragma unroll 1
+    for (int k = 0; k < 2; k++)
+        if ((unsure >> k & 1) && fx_weak(Sm, ty + k * ATY, tx, j0 + ty + k * ATY > 0, thr)) atomicOr(&Sm.redo, 1u << k);
+    __syncthreads();
+    const unsigned redo = Sm.redo;
+    if (tid < 2 && (redo >> tid & 1)) F.tlist[atomicAdd(F.pcount + 1, 1u)] = (2 * blockIdx.y + tid) * gridDim.x + blockIdx.x;
+    flows &= ~redo;
+    for (int k = 0; k < 2; k++)
+        if (flows >> k & 1)
+            F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)((size_t)(j0 + ty + k * ATY + 1) * m + i);
 }
 
 // What k_advect_fx left: the listed cells' plastic part (k_advect's FP64 yield
@@ -834,7 +908,8 @@ __global__ void __launch_bounds__(ATX * ATY) k_direct(step_consts c, direct_cons
 // velocity gradient and the viscous term.  k_direct is bound by its ~160 FP64
 // operations per cell (0.70 ms a step at 1024 x 768 with flow everywhere; 0.11
 // this kernel, 0.14 the plastic law in k_direct_rest).  Tiles with a value that is not finite and cells near
-// yield are listed for k_direct_rest.
+// yield are listed for k_direct_rest, and, as in k_advect_fx, the 32 x 8 halves with
+// a cell whose own values lie too far below the tile's largest (fxd_weak).
 struct fxd_smem {
     union {
         double d[DF_COUNT][FROWS][ACOLS];  // TMA destination of the first seven (128-byte aligned)
@@ -844,8 +919,46 @@ struct fxd_smem {
     int xs[ACOLS], col[ACOLS];
     // -hx, -hy times the scale of the stresses' sums; hx, hy, hxxv, hyyv times that of the velocities
     double xfs, yfs, hx[2], hy[2], vx[2], vy[2];
+    fx_scale scale[DF_COUNT];
+    int rates, force;        // quick thresholds of the velocity at the corners and of the stresses
+    double chi;              // the unit of chi's integers
+    unsigned redo;           // halves to list
+    int by[DF_COUNT];        // shift to the stresses', or the velocities', common scale
     uint64_t bar;
 };
+
+// An integer at the scale of exponent E, cut to a coarser one.
+__device__ __forceinline__ long long fx_cut(long long v, int by) { return v >> min(by, 63); }
+
+// Whether a cell that failed the quick test, or its lower-left node (node), may be
+// off by more than its own values' rounding (as fx_weak): a field that is
+// everywhere small on its stencil, the velocity at the corners (the rates), or
+// the four cells' stresses (the force on the node), unless zero in the whole tile.
+// The force's and the rates' sums are cut at no more than sixteen units of 2^-59
+// of the tile's largest value, and their bounds take in 16 and 8 such terms.
+__device__ __noinline__ bool fxd_weak(const fxd_smem &Sm, int row, int tx, bool node, int thr, bool diffuses) {
+    const int at = (row + 2) * ACOLS + tx + 2;
+    constexpr int slow = 1 << (50 - 32);
+    const bool moves = Sm.top[DF_U] || Sm.top[DF_V];
+    for (int f = 0; f < DF_COUNT; f++) {
+        if (Sm.top[f] == 0 || !(moves || (f == F_CHI && diffuses))) continue;
+        if ((node || f <= F_CHI) && stencil_below(&Sm.t.v[f][0][0] + at, thr)) return true;
+    }
+    bool still = moves, slack = node;
+    bool stressed = false;
+    for (int f = 0; f < DF_COUNT; f++) {
+        const bool vel = f >= DF_U;
+        if (!vel && f != F_P && f != F_Q && f != F_S && f != F_TAU) continue;
+        stressed = stressed || (!vel && Sm.top[f]);
+        for (int k = 0; k < 4; k++) {
+            const int o = vel ? (k & 1) + (k >> 1) * ACOLS : -(k & 1) - (k >> 1) * ACOLS;
+            const bool b = below(fx_cut((&Sm.t.v[f][0][0])[at + o], Sm.by[f]), slow);
+            if (vel) still = still && b;
+            else slack = slack && b;
+        }
+    }
+    return still || (slack && stressed);
+}
 
 __global__ void __launch_bounds__(ATX * ATY, 4)
     k_direct_fx(step_consts c, direct_consts d, advect_fx_consts h, const __grid_constant__ field_boxes maps,
@@ -867,6 +980,7 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         Sm.xs[tid] = u < 0 ? -1 : (u >= m ? 1 : 0);
     }
     if (tid < DF_COUNT) Sm.top[tid] = 0;
+    if (tid == 0) Sm.redo = 0;
     __syncthreads();
     if (tid == 0) {
         mbar_expect_tx(&Sm.bar, kFxBytes);
@@ -931,6 +1045,9 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         E[f] = max((int)(Sm.top[f] >> 20), 128);
         finite = finite && E[f] < 0x7ff;
     }
+    const int Ku = max(E[DF_U], E[DF_V]) + h.he - 2037;
+#pragma unroll
+    for (int f = 0; f < DF_COUNT; f++) finite = finite && E[f] + Ku < 1000;
     if (!finite) {  // the same for the whole block: two of k_direct's tiles
         if (tid < 2 && j0 + tid * ATY < n)
             F.tlist[atomicAdd(F.pcount + 1, 1u)] = (2 * blockIdx.y + tid) * gridDim.x + blockIdx.x;
@@ -940,8 +1057,18 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
     const long long lx = to_fixed(c.lx, E[F_X]);
     // the stresses at one scale, and both velocities at one (cut to it)
     const int Es = max(max(E[F_P], E[F_Q]), max(E[F_S], E[F_TAU])), Eu = max(E[DF_U], E[DF_V]);
-    auto cut = [](long long v, int by) { return v >> min(by, 63); };
+    auto cut = [](long long v, int by) { return fx_cut(v, by); };
+    const int thr = fx_threshold(max(50 + Ku + 1081, h.floor));
+    const bool moves = Sm.top[DF_U] || Sm.top[DF_V];
     if (tid == 0) {
+#pragma unroll
+        for (int f = 0; f < DF_COUNT; f++) {
+            Sm.scale[f].set(E[f] + Ku, Sm.top[f] && (moves || (f == F_CHI && d.hccd != 0)) ? thr : 0);
+            Sm.by[f] = (f >= DF_U ? Eu : Es) - E[f];
+        }
+        Sm.chi = power_of_two(E[F_CHI] - 1081);
+        Sm.rates = moves ? 1 << (52 - 32) : 0;
+        Sm.force = Sm.top[F_P] || Sm.top[F_Q] || Sm.top[F_S] || Sm.top[F_TAU] ? 1 << (52 - 32) : 0;
         const double ss = power_of_two(Es - 1081);
         Sm.xfs = -d.hx * ss;
         Sm.yfs = -d.hy * ss;
@@ -965,23 +1092,22 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         }
     }
     __syncthreads();
-    if (i >= m) return;
-    const int Ku = Eu + h.he - 2037;
+    unsigned flows = 0, unsure = 0;
 #pragma unroll 1
-    for (int row = ty; row < FXY; row += ATY) {
+    for (int row = ty; row < FXY && i < m && j0 + row < n; row += ATY) {
         const int j = j0 + row;
-        if (j >= n) return;
+        bool weak = false;
         const size_t ci = (size_t)(j + 1) * m + i;
         const int at = (row + 2) * ACOLS + tx + 2;
         auto fld = [&](int f) { return &Sm.t.v[f][0][0] + at; };
         auto upwind = [&](int f, const fx_factor &uh, int dx, const fx_factor &vh, int dy, bool inner) {
-            return -(double)fx_products(uh, eno_fx(fld(f), dx, true), vh, eno_fx(fld(f), dy, inner)) *
-                   power_of_two(E[f] + Ku);
+            weak = weak || Sm.scale[f].below(fld(f)[0]);
+            return (double)fx_products(uh, eno_fx(fld(f), dx, true), vh, eno_fx(fld(f), dy, inner)) * Sm.scale[f].unit;
         };
         const long long *U = fld(DF_U), *V = fld(DF_V);
         if (j > 0) {
             const long long u0 = U[0], v0 = V[0];
-            const fx_factor uh(4 * cut(u0, Eu - E[DF_U]), h.hmx), vh(4 * cut(v0, Eu - E[DF_V]), h.hmy);
+            const fx_factor uh(4 * cut(u0, Sm.by[DF_U]), h.hmx), vh(4 * cut(v0, Sm.by[DF_V]), h.hmy);
             const int dx = u0 > 0 ? 1 : -1, dy = v0 > 0 ? ACOLS : -ACOLS;
             const bool inner = v0 > 0 ? j > 1 : j < n - 1;
             // net force from the cells (i-1,j-1), (i,j-1), (i-1,j), (i,j)
@@ -989,12 +1115,14 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int o = (k & 1) - 1 + ((k >> 1) - 1) * ACOLS;
-                const long long pq = cut(fld(F_P)[o], Es - E[F_P]) + cut(fld(F_Q)[o], Es - E[F_Q]);
-                const long long sv = cut(fld(F_S)[o], Es - E[F_S]);
+                const long long pq = cut(fld(F_P)[o], Sm.by[F_P]) + cut(fld(F_Q)[o], Sm.by[F_Q]);
+                const long long sv = cut(fld(F_S)[o], Sm.by[F_S]);
                 a[k] = pq - sv;
                 b[k] = pq + sv;
-                t[k] = cut(fld(F_TAU)[o], Es - E[F_TAU]);
+                t[k] = cut(fld(F_TAU)[o], Sm.by[F_TAU]);
             }
+            const int force = Sm.force;
+            weak = weak || (below(a[3], force) && below(b[3], force) && below(t[3], force));
             const double xfs = Sm.xfs, yfs = Sm.yfs;
             const double fx = fma(xfs, (double)((a[1] - a[0]) + (a[3] - a[2])),
                                   yfs * (double)((t[0] - t[2]) + (t[1] - t[3])));
@@ -1015,12 +1143,13 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         const long long u00 = U[0], u10 = U[1], u01 = U[ACOLS], u11 = U[ACOLS + 1];
         const long long v00 = V[0], v10 = V[1], v01 = V[ACOLS], v11 = V[ACOLS + 1];
         const long long u4 = (u00 + u10) + (u01 + u11), v4 = (v00 + v10) + (v01 + v11);
+        weak = weak || (below(cut(u4, Sm.by[DF_U]), Sm.rates) && below(cut(v4, Sm.by[DF_V]), Sm.rates));
         const double ux = Sm.hx[0] * (double)((u10 - u00) + (u11 - u01));
         const double uy = Sm.hy[0] * (double)((u01 - u00) + (u11 - u10));
         const double vx = Sm.hx[1] * (double)((v10 - v00) + (v11 - v01));
         const double vy = Sm.hy[1] * (double)((v01 - v00) + (v11 - v10));
         const double two_omega = vx - uy, div = ux + vy;
-        const fx_factor uh(cut(u4, Eu - E[DF_U]), h.hmx), vh(cut(v4, Eu - E[DF_V]), h.hmy);
+        const fx_factor uh(cut(u4, Sm.by[DF_U]), h.hmx), vh(cut(v4, Sm.by[DF_V]), h.hmy);
         const int dx = u4 > 0 ? 1 : -1, dy = v4 > 0 ? ACOLS : -ACOLS;
         const bool inner = v4 > 0 ? j > 0 : j < n - 1;
         auto inc = [&](int f) { return upwind(f, uh, dx, vh, dy, inner); };
@@ -1032,14 +1161,26 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         double cchi = A[F_CHI][ci] + inc(F_CHI);
         if (d.hccd != 0) {
             const long long *H = fld(F_CHI);
-            cchi += power_of_two(E[F_CHI] - 1081) *
+            cchi += Sm.chi *
                     fma(d.hxxcd, (double)((H[1] - H[0]) + (H[-1] - H[0])),
                         d.hyycd * (double)((H[ACOLS] - H[0]) + (H[-ACOLS] - H[0])));
         }
         B[F_CHI][ci] = cchi;
-        if (!surely_elastic(c, q, s, t)) F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)ci;
+        if (!surely_elastic(c, q, s, t)) flows |= row < ATY ? 1u : 2u;
         F.ddev[ci] = 0;
+        if (weak) unsure |= row < ATY ? 1u : 2u;
     }
+#pragma unroll 1
+    for (int k = 0; k < 2; k++)
+        if ((unsure >> k & 1) && fxd_weak(Sm, ty + k * ATY, tx, j0 + ty + k * ATY > 0, thr, d.hccd != 0))
+            atomicOr(&Sm.redo, 1u << k);
+    __syncthreads();
+    const unsigned redo = Sm.redo;
+    if (tid < 2 && (redo >> tid & 1)) F.tlist[atomicAdd(F.pcount + 1, 1u)] = (2 * blockIdx.y + tid) * gridDim.x + blockIdx.x;
+    flows &= ~redo;
+    for (int k = 0; k < 2; k++)
+        if (flows >> k & 1)
+            F.plist[atomicAdd(F.pcount, 1u)] = (unsigned)((size_t)(j0 + ty + k * ATY + 1) * m + i);
 }
 
 // What k_direct_fx left: the listed cells' plastic part and the listed tiles.
@@ -1430,7 +1571,7 @@ void advection(const step_consts &c, const field_maps &maps, fields_dev &F, int 
     a.xf = 0.5 / dt * c.xsp;
     a.yf = 0.5 / dt * c.ysp;
     const dim3 grid(ceil_div(c.m, ATX), ceil_div(c.n, ATY));
-    if (c.fixed_point) {
+    if (c.fixed_point && std::isfinite(a.hx + a.hy)) {
         advect_fx_consts h = fx_consts(a.hx, a.hy);
         h.xf = a.xf;
         h.yf = a.yf;
@@ -1469,8 +1610,12 @@ void direct_step(const step_consts &c, const field_maps &maps, double viscosity,
     d.hccd = 2 * (d.hxxcd + d.hyycd);
     dim3 blk(ATX, ATY);
     const dim3 grid = g2(c.m, c.n, blk);
-    if (c.fixed_point) {
-        const advect_fx_consts h = fx_consts(hx, hy);
+    if (c.fixed_point && std::isfinite(hx + hy)) {
+        advect_fx_consts h = fx_consts(hx, hy);
+        // second differences times these factors, cut at four units of 2^-59
+        const double second = std::max((d.hxxv + d.hyyv) * d.mu_inv, d.hxxcd + d.hyycd);
+        if (second > 0) std::frexp(second, &h.floor);
+        h.floor += second > 0 ? 50 : 0;
         cudaMemsetAsync(F.pcount, 0, 2 * sizeof(unsigned), st);
         k_direct_fx<<<dim3(grid.x, ceil_div(c.n, FXY)), blk, sizeof(fxd_smem) + 128, st>>>(c, d, h, maps.tall, F, cur,
                                                                                           bv);

@@ -44,7 +44,7 @@ struct fields_dev {
     // Y2 = xf tau + yf B, A = p+q-s, B = p+q+s (xf, yf of projection_step).
     double *pre[4];
     // Fixed-point advection: cells that its yield test cannot certify as elastic,
-    // tiles with a value that is not finite, and their counts (two words).
+    // 32 x 8 tiles that it leaves to FP64, and their counts (two words).
     unsigned *plist;
     unsigned *tlist;
     unsigned *pcount;
