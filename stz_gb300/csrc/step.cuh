@@ -97,8 +97,8 @@ __device__ __forceinline__ bool mag_gt(double a, double b) {
 // second differences d1 = p0 - 2p1 + p2 and d2 = p1 - 2p2 + p3, |d1| > |d2|
 // selects 3p1 - 4p2 + p3 = d2 + 2(p1 - p2), otherwise p0 - p2 = d1 + 2(p1 - p2).
 // Written through first differences: six FP64 operations and an integer
-// compare.  The adjoint takes its branch decisions from eno2_pick, so both
-// see the same choice.
+// compare.  The adjoint takes its branch decisions from eno2_pick and runs its
+// forward steps with this arithmetic, so both see the same choice.
 __device__ __forceinline__ bool eno2_pick(double p0, double p1, double p2, double p3) {
     const double e = p1 - p2;
     return mag_gt((p0 - p1) - e, e - (p2 - p3));
