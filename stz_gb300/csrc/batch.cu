@@ -118,6 +118,24 @@ void drop_batch_graph(stzg_batch *b) {
     b->g_nsteps = -1;
 }
 
+// The cycles captured while this lives share the chip with `together` - 1 others.
+struct shared_chip {
+    stzg_sim *s;
+    explicit shared_chip(stzg_sim *q, size_t together) : s(q) {
+        set(s->h64, together > 1, together > 20 ? 4 : (together > 12 ? 8 : 16));
+        set(s->h32, together > 1, together > 20 ? 4 : (together > 12 ? 8 : 16));
+    }
+    ~shared_chip() {
+        set(s->h64, false, 16);
+        set(s->h32, false, 16);
+    }
+    template <typename T> static void set(hierarchy<T> &h, bool crowded, int blocks) {
+        h.crowded = crowded;
+        h.small_blocks = blocks;
+        h.long_marches = blocks < 16;
+    }
+};
+
 // Appends instance k's step loop to the root graph.
 int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, long *kernels) {
     stzg_sim *s = b->sims[k];
@@ -140,9 +158,8 @@ int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, 
     // levels (16 / 8 / 4 / 2 blocks, 12 instances: 9.1 / 9.5 / 10.3 / 11.4 ms;
     // 24: 15.4 / 13.8 / 13.6 / 14.9; 32: 12.7 / 11.1 / 10.3 / 11.1) and the top
     // level's long marches, whose halo is smaller (32: 10.3 ms, short 10.8).
-    const size_t together = b->sims.size();
-    s->h64.crowded = s->h32.crowded = together > 1;
-    s->h64.small_blocks = s->h32.small_blocks = together > 20 ? 4 : (together > 12 ? 8 : 16);
+    // The batch's graph alone takes this: a handle stepped by itself has the chip.
+    const shared_chip share(s, b->sims.size());
     double *clk = b->dclock + (size_t)k * CLK_COUNT;
     int *ctr = b->dctr + (size_t)k * CTR_COUNT;
     // the captured step kernels read time, wall data and buffer index from the clock

@@ -2526,7 +2526,7 @@ template <typename T> void launch_lev_up(level_view<T> &F, level_view<T> &C, cud
 // hide them: V-cycle at 256^2 / 512^2 / 1024^2 with 8 rows 45 / 62 / 84 us, so
 // 36 / 54 / 73 us (2048^2 keeps 8).
 template <typename T> static int top_rows(const hierarchy<T> &h, int strips, int cn) {
-    return h.small_blocks < 16 ? kTopRows : std::min(march_rows(strips, cn), kTopRows);
+    return h.long_marches ? kTopRows : std::min(march_rows(strips, cn), kTopRows);
 }
 
 // The streaming top-level kernels (single precision only): the swept z goes

@@ -113,6 +113,8 @@ template <typename T> class hierarchy {
     // other cycles run at the same time: no early launches, whose waiting
     // blocks take the others' slots
     bool crowded = false;
+    // the top level's longest marches, whose halo is smaller
+    bool long_marches = false;
     // single precision: the coarse levels at most 512 wide and the tail in
     // one cooperative persistent kernel (set by the owner once
     // coarse_persist_supported() holds; bar: two zeroed device words for its
