@@ -15,6 +15,7 @@
 // costs 10 to 20 issue slots on the FP32 pipe where an FP64 one blocks its
 // quarter of the SM for 64 clocks.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 
@@ -260,7 +261,7 @@ template <> struct scalar_of<double> { typedef ff type; };
 // Largest cluster the device takes for the small-level kernels (probed once
 // per device; at least 1).
 int max_blocks() {
-    static int known[64];
+    static std::atomic<int> known[64];  // several host threads may probe at once, to the same result
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
     if (!known[dev]) {
@@ -390,7 +391,7 @@ void launch_tile(void (*kern)(K...), const tile_level &L, bool bands, size_t sme
 }
 
 bool prepare_tiles() {
-    static int known[64];
+    static std::atomic<int> known[64];  // several host threads may probe at once, to the same result
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     if (!known[dev]) {

@@ -3,6 +3,7 @@
 #include "mg_small.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
 }
 
 int max_blocks() {
-    static int known[64];
+    static std::atomic<int> known[64];  // several host threads may probe at once, to the same result
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     if (!known[dev]) {
