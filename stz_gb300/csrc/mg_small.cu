@@ -447,6 +447,7 @@ int build_dense(hierarchy<double> &h, const std::vector<double> &inverse, std::v
             P.dense = next;
             if (!layout_small(P, l, l + 1, 1, kSmallMax)) return STZG_OK;  // the older kernels serve it
             k_dense_columns<<<(unsigned)N, kSmallThreads, P.bytes>>>(P, M);
+            note_launch();
             STZG_CUDA(cudaGetLastError());
         }
         next = reinterpret_cast<const float4 *>(M);

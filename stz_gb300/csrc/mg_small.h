@@ -16,16 +16,17 @@ namespace stzg {
 struct small_desc {
     int m, n;
     bool rows;             // the stencil depends on the row only
-    std::vector<int> ids;  // stencil of every row (rows) or point
+    const std::vector<int> *ids;  // stencil of every row (rows) or point
+    bool ids_kept;                // the same as at the last setup
     std::vector<double> table;  // 40 doubles per stencil: nine blocks and the inverse centre
 };
 
 class small_cycle {
   public:
     // Lays out the levels first..ml of desc (bottom: the coarsest level's matrix,
-    // 2mn x 2mn row-major) on stream st; the host data must live until st is
-    // synchronised.  *moved is set where a launch captured before does not fit
-    // any more.  active() tells whether the levels can be taken.
+    // 2mn x 2mn row-major) on stream st; ids must live until st is synchronised.
+    // *moved is set where a launch captured before does not fit any more, also
+    // when an error is returned.  active() tells whether the levels can be taken.
     int setup(const std::vector<small_desc> &desc, int yp, const std::vector<double> &bottom, cudaStream_t st,
               bool *moved);
     bool active() const { return t_ > 0; }

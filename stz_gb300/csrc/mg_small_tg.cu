@@ -130,10 +130,10 @@ int small_cycle::need(buffer &b, size_t bytes, bool *moved) {
     if (b.cap >= bytes) return STZG_OK;
     if (b.p) cudaFree(b.p);
     b = buffer();
+    *moved = true;
     const cudaError_t e = cudaMalloc(&b.p, bytes);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(small levels)");
     b.cap = bytes;
-    *moved = true;
     return STZG_OK;
 }
 
@@ -179,16 +179,18 @@ int small_cycle::setup(const std::vector<small_desc> &desc, int yp, const std::v
                 pairs_[l][20 * c + 2 * e + 1] = make_float4(o[0], o[1], o[2], o[3]);
             }
         STZG_CHECK(need(tab_[l], pairs_[l].size() * sizeof(float4), moved));
-        STZG_CHECK(need(cls_[l], D.ids.size() * sizeof(int), moved));
+        const bool sent = D.ids_kept && cls_[l].cap;
+        STZG_CHECK(need(cls_[l], D.ids->size() * sizeof(int), moved));
         STZG_CUDA(cudaMemcpyAsync(tab_[l].p, pairs_[l].data(), pairs_[l].size() * sizeof(float4),
                                   cudaMemcpyHostToDevice, st));
-        STZG_CUDA(cudaMemcpyAsync(cls_[l].p, D.ids.data(), D.ids.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+        if (!sent)
+            STZG_CUDA(cudaMemcpyAsync(cls_[l].p, D.ids->data(), D.ids->size() * sizeof(int), cudaMemcpyHostToDevice, st));
         small_level<ff> &S = P.lv[l];
         S.m = D.m;
         S.n = D.n;
         S.homog = D.rows;
         S.nst = nst;
-        S.ncls = (int)D.ids.size();
+        S.ncls = (int)D.ids->size();
         S.cls = (const int *)cls_[l].p;
         S.st = (const float4 *)tab_[l].p;
     }
@@ -211,6 +213,7 @@ int small_cycle::setup(const std::vector<small_desc> &desc, int yp, const std::v
         if (!layout_small(Q, l, l + 1, 1, kSmallMax)) return done(nullptr);
         if (yp) k_block_columns<true><<<(unsigned)N, kSmallThreads, Q.bytes, st>>>(Q, (float2 *)dense_[l].p);
         else k_block_columns<false><<<(unsigned)N, kSmallThreads, Q.bytes, st>>>(Q, (float2 *)dense_[l].p);
+        note_launch();
         STZG_CUDA(cudaGetLastError());
     }
     P.dense = (const float4 *)dense_[d].p;

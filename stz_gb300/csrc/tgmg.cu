@@ -774,7 +774,11 @@ template <int B> struct tg {
     int tail_start = 1 << 30;  // first level handled by k_tg_tail (none if > nl-1)
     double *partials = nullptr, *dsum = nullptr, *hsum = nullptr;
     std::vector<double> inv_host;  // the coarsest inverse, for its FP32 copy
-    small_cycle small;             // 2x2 blocks, x periodic: the small levels in one launch
+    // 2x2 blocks, x periodic: the small levels in one launch, laid out by the first
+    // iteration that takes them on a new operator (small_kept: laid out since the
+    // class map of the level changed)
+    small_cycle small;
+    bool small_ready = false, small_kept[kMaxLevels] = {};
     std::vector<std::vector<gst<B, float>>> host32;  // FP32 tables as uploaded
     std::vector<float> inv_host32;
     // Mixed precision (V-cycle solves as refinement passes: FP32 V-cycles on
@@ -1015,8 +1019,80 @@ template <int B> void drop_graph(tg<B> *g) {
     g->gkey[0] = -1;
 }
 
+// The coarsest level as a matrix: its inverse, or the linear map of the
+// bottom's sweeps from zero (the first kBottomSweeps down, as many up).
+std::vector<double> bottom_matrix(const host_level<2> &L, int xp, int yp, const std::vector<double> &inverse) {
+    if (!inverse.empty()) return inverse;
+    const int pts = L.m * L.n, N = 2 * pts;
+    std::vector<double> M;
+    if (N > 256) return M;
+    M.assign((size_t)N * N, 0.0);
+    const int cxn = (xp && (L.m & 1)) ? 3 : 2, cyn = (yp && (L.n & 1)) ? 3 : 2;
+#pragma omp parallel for schedule(static)
+    for (int col = 0; col < N; col++) {
+        std::vector<double> z(N, 0.0);
+        for (int s = 0; s < 2 * kBottomSweeps; s++)
+            for (int cy = 0; cy < cyn; cy++)
+                for (int cx = 0; cx < cxn; cx++)
+                    for (int j = 0; j < L.n; j++) {
+                        if ((cyn == 3 && j == L.n - 1 ? 2 : (j & 1)) != cy) continue;
+                        for (int i = 0; i < L.m; i++) {
+                            if ((cxn == 3 && i == L.m - 1 ? 2 : (i & 1)) != cx) continue;
+                            const int p = j * L.m + i;
+                            const gst<2> &st = L.table[L.cls[p]];
+                            double rx = 2 * p == col ? 1 : 0, ry = 2 * p + 1 == col ? 1 : 0;
+                            for (int k = 0; k < 9; k++) {
+                                const int y = nbr(j, k / 3 - 1, L.n, yp), x = nbr(i, k % 3 - 1, L.m, xp);
+                                if (k == 4 || x < 0 || y < 0) continue;
+                                const double *e = st.e[k].c, *v = &z[2 * (y * L.m + x)];
+                                rx -= e[0] * v[0] + e[1] * v[1];
+                                ry -= e[2] * v[0] + e[3] * v[1];
+                            }
+                            const double *e = st.e[9].c;
+                            z[2 * p] = e[0] * rx + e[1] * ry;
+                            z[2 * p + 1] = e[2] * rx + e[3] * ry;
+                        }
+                    }
+        for (int r = 0; r < N; r++) M[(size_t)r * N + col] = z[r];
+    }
+    return M;
+}
+
+// Lays out the small levels for iterations that take them (vc): FP64 V-cycles with
+// one sweep each way and the default bottom on 2x2 blocks periodic in x.  Other
+// iterations, mixed-precision ones among them, do not pay for them.
+int ready_small(tg<1> *, int, int, int, int) { return STZG_OK; }
+int ready_small(tg<2> *g, int type, int cd, int cu, int hb) {
+    const bool taken = (type == STZG_TGMG_VCYCLE || type == STZG_TGMG_FMG) && !uses_mixed(g, type) && !g->plain &&
+                       cd == 1 && cu == 1 && hb == kBottomSweeps;
+    if (!taken || !g->xp || g->small_ready) return STZG_OK;
+    std::vector<small_desc> desc(g->nl);
+    for (int l = 0; l < g->nl; l++) {
+        const host_level<2> &H = g->host[l];
+        small_desc &D = desc[l];
+        D.m = H.m;
+        D.n = H.n;
+        if (l == 0) continue;
+        D.rows = H.rows;
+        D.ids = H.rows ? &H.row_ids : &H.cls;
+        D.ids_kept = g->small_kept[l];
+        D.table.resize(40 * H.table.size());
+        for (size_t c = 0; c < H.table.size(); c++)
+            for (int e = 0; e < 10; e++)
+                for (int q = 0; q < 4; q++) D.table[40 * c + 4 * e + q] = H.table[c].e[e].c[q];
+    }
+    bool moved = false;
+    const int st = g->small.setup(desc, g->yp, bottom_matrix(g->host.back(), g->xp, g->yp, g->inv_host), g->st, &moved);
+    if (moved) drop_graph(g);
+    STZG_CHECK(st);
+    for (bool &k : g->small_kept) k = g->small.active();
+    g->small_ready = true;
+    return STZG_OK;
+}
+
 template <int B> int run_iterations(tg<B> *g, int type, int count, double omega, int cd, int cu, int hb) {
     if (count <= 0) return STZG_OK;
+    STZG_CHECK(ready_small(g, type, cd, cu, hb));
     const int key[6] = {type, cd, cu, hb, uses_mixed(g, type) ? 2 : 1, g->plain};
     if (!g->gexec || std::memcmp(key, g->gkey, sizeof(key)) != 0 || g->gomega != omega) {
         drop_graph(g);
@@ -1164,66 +1240,6 @@ template <int B> int upload_f32(tg<B> *g, bool *moved) {
     return STZG_OK;
 }
 
-// The coarsest level as a matrix: its inverse, or the linear map of the
-// bottom's sweeps from zero (the first kBottomSweeps down, as many up).
-std::vector<double> bottom_matrix(const host_level<2> &L, int xp, int yp, const std::vector<double> &inverse) {
-    if (!inverse.empty()) return inverse;
-    const int pts = L.m * L.n, N = 2 * pts;
-    std::vector<double> M;
-    if (N > 256) return M;
-    M.assign((size_t)N * N, 0.0);
-    const int cxn = (xp && (L.m & 1)) ? 3 : 2, cyn = (yp && (L.n & 1)) ? 3 : 2;
-#pragma omp parallel for schedule(static)
-    for (int col = 0; col < N; col++) {
-        std::vector<double> z(N, 0.0);
-        for (int s = 0; s < 2 * kBottomSweeps; s++)
-            for (int cy = 0; cy < cyn; cy++)
-                for (int cx = 0; cx < cxn; cx++)
-                    for (int j = 0; j < L.n; j++) {
-                        if ((cyn == 3 && j == L.n - 1 ? 2 : (j & 1)) != cy) continue;
-                        for (int i = 0; i < L.m; i++) {
-                            if ((cxn == 3 && i == L.m - 1 ? 2 : (i & 1)) != cx) continue;
-                            const int p = j * L.m + i;
-                            const gst<2> &st = L.table[L.cls[p]];
-                            double rx = 2 * p == col ? 1 : 0, ry = 2 * p + 1 == col ? 1 : 0;
-                            for (int k = 0; k < 9; k++) {
-                                const int y = nbr(j, k / 3 - 1, L.n, yp), x = nbr(i, k % 3 - 1, L.m, xp);
-                                if (k == 4 || x < 0 || y < 0) continue;
-                                const double *e = st.e[k].c, *v = &z[2 * (y * L.m + x)];
-                                rx -= e[0] * v[0] + e[1] * v[1];
-                                ry -= e[2] * v[0] + e[3] * v[1];
-                            }
-                            const double *e = st.e[9].c;
-                            z[2 * p] = e[0] * rx + e[1] * ry;
-                            z[2 * p + 1] = e[2] * rx + e[3] * ry;
-                        }
-                    }
-        for (int r = 0; r < N; r++) M[(size_t)r * N + col] = z[r];
-    }
-    return M;
-}
-
-// The small levels of a 2x2-block hierarchy with x periodic.
-int setup_small(tg<1> *, std::vector<small_desc> &, bool *) { return STZG_OK; }
-int setup_small(tg<2> *g, std::vector<small_desc> &desc, bool *moved) {
-    if (!g->xp) return STZG_OK;
-    desc.resize(g->nl);
-    for (int l = 0; l < g->nl; l++) {
-        const host_level<2> &H = g->host[l];
-        small_desc &D = desc[l];
-        D.m = H.m;
-        D.n = H.n;
-        if (l == 0) continue;
-        D.rows = H.rows;
-        D.ids = H.rows ? H.row_ids : H.cls;
-        D.table.resize(40 * H.table.size());
-        for (size_t c = 0; c < H.table.size(); c++)
-            for (int e = 0; e < 10; e++)
-                for (int q = 0; q < 4; q++) D.table[40 * c + 4 * e + q] = H.table[c].e[e].c[q];
-    }
-    return g->small.setup(desc, g->yp, bottom_matrix(g->host.back(), g->xp, g->yp, g->inv_host), g->st, moved);
-}
-
 // Galerkin hierarchy below the top and its upload.  A level's class map goes
 // up only when it changed (the top's when the caller says so), so a new
 // operator on the same stencil pattern (the sheared-coordinates step: the
@@ -1280,8 +1296,8 @@ template <int B> int build_hierarchy(tg<B> *g, bool top_cls_kept = false) {
         }
     }
     if (g->have32) STZG_CHECK(upload_f32(g, &moved));
-    std::vector<small_desc> desc;  // lives until the stream is synchronised below
-    STZG_CHECK(setup_small(g, desc, &moved));
+    g->small_ready = false;
+    for (int l = 0; l < g->nl; l++) g->small_kept[l] = g->small_kept[l] && g->host[l].cls_kept;
     if (moved || g->inv != inv_was) drop_graph(g);
     STZG_CUDA(cudaStreamSynchronize(g->st));  // the host vectors are uploaded before they go
     return STZG_OK;
