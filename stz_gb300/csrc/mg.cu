@@ -2202,9 +2202,8 @@ __global__ void __launch_bounds__(1024) k_tail_pairs(tail_levels tl, hierarchy_v
     tail_inv_prefetch(tl, tail_raw, w * 32 + lane, 32 * nw);
     pdl_trigger();
     pdl_wait();
-    tail_pairs_body(
-        [&](const float2 *b, float2 *z, int nd) { dense_rows(tl.dense, b, z, nd, threadIdx.y, blockDim.y, threadIdx.x); },
-        tl, H, tail_raw, S, offs, lane, w, nw);
+    // launched without a matrix: the small-level kernel takes the levels that have one
+    tail_pairs_body([](const float2 *, float2 *, int) {}, tl, H, tail_raw, S, offs, lane, w, nw);
 }
 
 // ---------------------------------------------------------------------------
