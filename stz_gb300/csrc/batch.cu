@@ -154,7 +154,7 @@ int add_instance(stzg_batch *b, cudaGraph_t root, int k, double dt, int nsteps, 
     // The instances share the chip.  None of their kernels starts early, whose
     // waiting blocks would hold slots the others need (24 mixed instances of
     // 64^2 to 512^2, graph time: 18.9 ms with early launches, 13.6 without; 6
-    // of them: 8.6, 7.8).  Many of them take smaller clusters for their small
+    // of them: 8.6, 7.8).  Many of them, whatever their sizes, take smaller clusters for their small
     // levels (16 / 8 / 4 / 2 blocks, 12 instances: 9.1 / 9.5 / 10.3 / 11.4 ms;
     // 24: 15.4 / 13.8 / 13.6 / 14.9; 32: 12.7 / 11.1 / 10.3 / 11.1) and the top
     // level's long marches, whose halo is smaller (32: 10.3 ms, short 10.8).

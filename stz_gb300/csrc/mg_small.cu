@@ -307,22 +307,27 @@ bool plan_small(const hierarchy<T> &h, int t, int blocks, bool zero_start, small
     return layout_small(P, t, h.dense_from, blocks, kSmallMax);
 }
 
-// Levels of at most this many nodes go to the small-level kernel.  Its blocks
-// are one cluster, 16 of the chip's 152 SMs, so wider levels are faster as one
-// launch each over the whole chip.  Measured whole V-cycles, first level at
-// 17,000 / 66,000 nodes, FP32 at 512^2: 76 / 82 us; 17,000 / 27,000, float
-// pairs at 1024^2: 280 / 272 us (before the matrix of the coarsest levels).
-constexpr long kSmallPoints32 = 17000, kSmallPoints64 = 27000;
+// Levels of at most this many nodes go to the small-level kernel, where its
+// shared memory holds them.  Its blocks are one cluster, 16 of the chip's 152
+// SMs, so wider levels are faster as one launch each over the whole chip.  Whole
+// V-cycles with the limit at 9,000 / 17,000 / 35,000 nodes, us:
+//   float pairs, 158x157 59.7 / 59.7 / 71.8, 256x256 64.1 / 60.3 / 60.2,
+//     256x400 71.5 / 71.5 / 76.6, 96x256 48.2 / 48.3 / 46.4, 96x330 54.6 / 54.6
+//     / 76.3; 512^2 and 1024^2 change by 1 percent or not at all (their next
+//     level does not fit);
+//   FP32, 158x157 40.3 / 40.2 / 45.2, 256x256 41.8 / 35.9 / 36.0, 1024^2 74.5 /
+//     71.9 / 71.8 (77.8 without a limit); narrow grids would take more (64x400
+//     51.2 / 51.2 / 28.5, 96x256 31.2 / 31.2 / 27.3).
+constexpr long kSmallPoints = 17000;
 
 // First level of the small-level kernel and its cluster size; false where no
 // level fits.
 template <typename T>
 bool choose_small(const hierarchy<T> &h, bool zero_start, small_plan<typename scalar_of<T>::type> &P) {
-    const long limit = sizeof(T) == 4 ? kSmallPoints32 : kSmallPoints64;
     const int cap = std::min(max_blocks(), std::max(1, h.small_blocks));
     if (!h.dense) return false;
     for (int t = 0; t < h.dense_from; t++) {
-        if ((long)h.lv[t].m * h.lv[t].n > limit) continue;
+        if ((long)h.lv[t].m * h.lv[t].n > kSmallPoints) continue;
         for (int c = cap; c >= 1; c >>= 1)
             if (plan_small(h, t, c, zero_start, P)) return true;
     }

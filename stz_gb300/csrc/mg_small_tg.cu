@@ -64,8 +64,9 @@ struct io_env : block_env {
 constexpr unsigned kBlockMax = kSmallMax - 256;  // the rest for io_env's words
 
 // FP64 V-cycle of a 512 x 256 grid of 2x2 blocks, y periodic: 520 us with one
-// FP64 launch per colour and a single-block FP64 tail of 215 us; the four steps
-// of that grid that the cycle dominates went from 25.0 to 12.3 ms with this kernel.
+// FP64 launch per colour on every level and a single-block FP64 tail of 215 us;
+// 161 us with this kernel from level 2 (128 x 64) on, levels 0 and 1 still one
+// launch per colour.  Four steps of that grid went from 25.0 to 12.8 ms.
 template <bool FAST, bool YP>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_small_blocks(const __grid_constant__ small_plan<ff> P) {
     extern __shared__ __align__(16) unsigned char small_raw[];
@@ -112,8 +113,12 @@ int max_blocks() {
     return known[dev] - 1;
 }
 
-// Levels of at most this many nodes: the alternative is eleven FP64 launches
-// of about 7 us per level.
+// Levels of at most this many nodes, where the blocks' shared memory holds them (a
+// short grid has rows for few blocks: 256 x 128 nodes under 512 x 256, y
+// periodic, do not fit, 128 x 251 under 256 x 500 do); the alternative is eleven
+// FP64 launches of about 7 us per level.  V-cycles with the limit at 9,000 /
+// 17,000 / 33,000: 256x500 160 / 161 / 134 us, 128x900 155 / 154 / 130, 256x256 y
+// periodic 142 / 107 / 109; more than 33,000 changed nothing.
 constexpr long kBlockPoints = 33000;
 
 }  // namespace
