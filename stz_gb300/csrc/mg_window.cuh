@@ -783,10 +783,13 @@ template <typename S> struct small_plan {
 };
 
 // First row of block c on level l: level d's cut scaled up, the line's end
-// for c == blocks.
+// for c == blocks.  A bounded line of even n has a coarse row beyond its last
+// one, so the scaled cut of the last block can lie beyond the line's end (8 rows
+// of level d cut into 8 over 50 rows: 7 << 3); its band is empty then, and what it
+// owns of the coarser levels it computes from its halo rows.
 template <typename S> MGW_BOTH int band_row(const small_plan<S> &P, int l, int c) {
-    if (c >= P.blocks) return P.lv[l].n;
-    return ((c * P.lv[P.d].n) >> P.shift) << (P.d - l);
+    const int n = P.lv[l].n, row = ((c * P.lv[P.d].n) >> P.shift) << (P.d - l);
+    return c >= P.blocks || row > n ? n : row;
 }
 template <typename S> MGW_BOTH int band_below(const small_plan<S> &P, int l) {
     return P.top && l == P.t ? kTopBelow : kLevBelow;
