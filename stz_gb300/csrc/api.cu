@@ -1176,6 +1176,7 @@ int stzg_time_kernel(stzg_sim *s, double dt, int kernel, int reps, double *ms) {
         }
         return STZG_OK;
     };
+    if (kernel == 3) pair_begin(s->h64, s->st);
     STZG_CHECK(one());  // warm-up
     STZG_CUDA(cudaEventRecord(s->ev0, s->st));
     for (int r = 0; r < reps; r++) STZG_CHECK(one());

@@ -289,6 +289,8 @@ __device__ __forceinline__ bool advect_tile(const step_consts &c, const advect_c
     // j0-1..) by TMA while the block sets up the column tables.
     if (tid == 0 && use == 0) mbar_init(&Sm.bar, 1);
     tile_columns(T, i0, m, c.lx);
+    // the last tile's stores to the copies' destination, before the next copies
+    if (use) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (tid == 0) {
         mbar_expect_tx(&Sm.bar, kTileBytes);
@@ -1143,13 +1145,14 @@ __global__ void __launch_bounds__(ATX * ATY, 4)
         const long long u00 = U[0], u10 = U[1], u01 = U[ACOLS], u11 = U[ACOLS + 1];
         const long long v00 = V[0], v10 = V[1], v01 = V[ACOLS], v11 = V[ACOLS + 1];
         const long long u4 = (u00 + u10) + (u01 + u11), v4 = (v00 + v10) + (v01 + v11);
-        weak = weak || (below(cut(u4, Sm.by[DF_U]), Sm.rates) && below(cut(v4, Sm.by[DF_V]), Sm.rates));
+        const long long us = cut(u4, Sm.by[DF_U]), vs = cut(v4, Sm.by[DF_V]);
+        weak = weak || (below(us, Sm.rates) && below(vs, Sm.rates));
         const double ux = Sm.hx[0] * (double)((u10 - u00) + (u11 - u01));
         const double uy = Sm.hy[0] * (double)((u01 - u00) + (u11 - u10));
         const double vx = Sm.hx[1] * (double)((v10 - v00) + (v11 - v01));
         const double vy = Sm.hy[1] * (double)((v01 - v00) + (v11 - v10));
         const double two_omega = vx - uy, div = ux + vy;
-        const fx_factor uh(cut(u4, Sm.by[DF_U]), h.hmx), vh(cut(v4, Sm.by[DF_V]), h.hmy);
+        const fx_factor uh(us, h.hmx), vh(vs, h.hmy);
         const int dx = u4 > 0 ? 1 : -1, dy = v4 > 0 ? ACOLS : -ACOLS;
         const bool inner = v4 > 0 ? j > 0 : j < n - 1;
         auto inc = [&](int f) { return upwind(f, uh, dx, vh, dy, inner); };
